@@ -159,17 +159,19 @@ int p2b_cfr_solve(const void* subgames, const void* nodes, int32_t num_subgames,
 int64_t p2b_cfr_scratch_floats(int32_t max_internal, int32_t num_blocks);
 int64_t p2b_cfr_solve_scratch_floats(int32_t max_internal, int32_t max_children, int32_t num_blocks,
                                      int32_t num_subgames, int64_t rows);
+int64_t p2b_cfr_step_scratch_floats(int32_t max_internal, int32_t num_subgames, int64_t rows);
 int p2b_cfr_default_blocks(void);
-/* Which kernel runs the iteration passes of a p2b_cfr_solve whose leaves are all terminal (process-wide
- * setting, no counterpart in the upstream project).  0, the default: the lean kernel, except for batches so
- * small that the general kernel is quicker (at most one subgame per SM; or fewer than eight per SM while
- * max_internal x max_children + 1 exceeds 160, i.e. some subgame may be too large for the lean kernel).
- * 1: the lean kernel whenever it applies.  Results are the same bits either way.  Returns the previous
- * setting; a negative argument only queries. */
+/* Which kernels run the iteration passes of a p2b_cfr_solve whose leaves are all terminal (process-wide
+ * setting, no counterpart in the upstream project).  0, the default: the lean kernel, a block per subgame, from
+ * 1.5 subgames per SM on (8 per SM when max_internal x max_children + 1 exceeds 160, i.e. some subgame may be too
+ * large for it); below that, and for solves it does not cover, the split kernels, which spread a subgame over the
+ * chip (they need the scratch area of p2b_cfr_solve_scratch_floats as sized under the same setting; else the general
+ * kernel runs).  1: the lean kernel whenever it applies.  Results are the same bits either way.  Returns the
+ * previous setting; a negative argument only queries. */
 int p2b_cfr_path_policy(int32_t policy);
 /* Measurement aid (no counterpart in the upstream project): with timing enabled on the current
- * device, a p2b_cfr_solve that runs its iteration passes in the lean kernel brackets that one
- * launch with CUDA events on the caller's stream; p2b_cfr_iteration_ms waits for it and writes
+ * device, a p2b_cfr_solve of more subgames than SMs (eight times as many where some may exceed the lean
+ * kernel's limit, or whenever the lean kernel runs) brackets its iteration passes with CUDA events on the caller's stream; p2b_cfr_iteration_ms waits for it and writes
  * its duration in milliseconds to the HOST float *ms. */
 int p2b_cfr_iteration_timing(int32_t enable);
 int p2b_cfr_iteration_ms(float* ms);
@@ -195,8 +197,10 @@ int p2b_cfr_iteration_ms(float* ms);
  * step(pass, 2); }, or step(-1, 1); for every pass { leaf_values = model(leaf_beliefs);
  * pass == iterations ? step(pass, 2) : step(pass..pass+1, 16); }.  Arrays as in p2b_cfr_solve, plus state
  * carried between calls:
- *  scratch      p2b_cfr_scratch_floats(max_internal, 1) * num_subgames floats (one set of
- *               work rows per subgame instead of per block)
+ *  scratch      at least p2b_cfr_scratch_floats(max_internal, 1) * num_subgames floats (one set of
+ *               work rows per subgame instead of per block).  With p2b_cfr_step_scratch_floats(max_internal,
+ *               num_subgames, rows) floats the iteration passes run in the split kernels, which spread a
+ *               subgame over the chip; same results, bit for bit.  All calls of a solve pass the same area
  *  carry_sums   [rows,2] floats ([2,rows,2] with flags bit 2 or 3), carry_roots [num_subgames,4,1344] floats (opaque)
  *  leaf_begin   [num_subgames] int32: first leaf slot of each subgame; a node of kind 3 uses
  *               slot leaf_begin[subgame] + its internal_idx field; leaf_slots = number of slots

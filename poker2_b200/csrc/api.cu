@@ -92,6 +92,10 @@ int64_t p2b_cfr_scratch_floats(int32_t max_internal, int32_t num_blocks) {
     return cfr_scratch_floats(max_internal) * num_blocks;
 }
 
+int64_t p2b_cfr_step_scratch_floats(int32_t max_internal, int32_t num_subgames, int64_t rows) {
+    return cfr_step_scratch_floats(max_internal, num_subgames, rows);
+}
+
 int64_t p2b_cfr_solve_scratch_floats(int32_t max_internal, int32_t max_children, int32_t num_blocks,
                                      int32_t num_subgames, int64_t rows) {
     if (num_blocks <= 0) num_blocks = cfr_default_blocks();
@@ -149,6 +153,7 @@ int p2b_cfr_solve(const void* subgames, const void* nodes, int32_t num_subgames,
     p.br_values = br_values;
     p.scratch = scratch;
     p.scratch_stride = cfr_scratch_floats(max_internal);
+    p.scratch_floats = scratch_floats;
     p.max_internal = max_internal;
     p.scalars = static_cast<const IterScalars*>(scalars);
     p.iterations = iterations;
@@ -237,6 +242,7 @@ int p2b_cfr_step(const void* subgames, const void* nodes, int32_t num_subgames, 
     p.br_values = br_values;
     p.scratch = scratch;
     p.scratch_stride = cfr_scratch_floats(max_internal);
+    p.scratch_floats = scratch_floats;
     p.max_internal = max_internal;
     p.scalars = static_cast<const IterScalars*>(scalars);
     p.iterations = iterations;

@@ -30,6 +30,7 @@
 
 #include "cfr.cuh"
 #include "cfr_dev.cuh"
+#include "cfr_split.cuh"
 #include "exactdiv.cuh"
 #include "showdown.cuh"
 
@@ -1531,13 +1532,17 @@ int sm_count();
 
 int cfr_default_blocks() { return sm_count(); }
 
+static int check_records(const CfrParams& p, cudaStream_t stream) {
+    cfr_validate_kernel<<<p.num_subgames, kCfrMaxNodes, 0, stream>>>(p);
+    return check_cuda(cudaGetLastError(), "cfr_validate_kernel");
+}
+
 static int dispatch_cfr(const CfrParams& p, int num_blocks, int max_children, cudaStream_t stream) {
     if (max_children > kCfrMaxChildren)
         return set_error(P2B_ERR_ARG, "at most %d actions per node are supported, got %d", kCfrMaxChildren, max_children);
     // every launch is checked, also the later steps of a stepped solve: the launcher has cleared the
     // status word and the queue, and the kernel must not walk records the check refuses
-    cfr_validate_kernel<<<p.num_subgames, kCfrMaxNodes, 0, stream>>>(p);
-    const int rc = check_cuda(cudaGetLastError(), "cfr_validate_kernel");
+    const int rc = check_records(p, stream);
     if (rc) return rc;
     // one kernel serves every child count up to its width: node bodies are specialised per count inside it
     if (max_children <= kMaxC) return launch_kernel<2, kMaxC>(p, num_blocks, stream);
@@ -1567,12 +1572,12 @@ IterTiming* iter_timing_of_current_device() {
 }
 }  // namespace
 
-// Which kernel runs the iteration passes of a plain one-call solve.  0 (default): the lean kernel, unless the
-// batch is so small that the general kernel is quicker -- at most one subgame per SM (a lone 448-thread block
-// leaves an SM idler than the general kernel's 672 threads: 22.3 against 30.2 ms for 148 subgames x 64
-// iterations), or fewer than eight per SM when some subgame may exceed the lean kernel's node limit (the lean
-// launch and the launch for the large subgames would then both run half empty, one after the other: 36 against
-// 64 ms for 192 ragged subgames of up to 237 nodes x 24 iterations).  1: the lean kernel whenever it applies.
+// Which kernels run the iteration passes of a one-call solve whose leaves are all terminal.  0 (default): the lean
+// kernel, whose blocks keep a subgame each and so want two subgames an SM; the split kernels (cfr_split.cu), which
+// spread every subgame over the chip, for batches below 1.5 an SM, and below 8 an SM when some subgame may exceed
+// the lean kernel's node limit.  Measured, ms for 16 iterations with start and final pass, split / lean: trees of 54
+// nodes, 64 subgames 4.5 / 6.2, 192 8.6 / 9.4, 256 10.4 / 9.8, 592 21.8 / 19.4; up to 261 nodes, 64 subgames 10.7 / 40,
+// 296 25 / 49, 1184 89 / 92, 2048 152 / 151.  1: the lean kernel whenever it applies.
 static std::atomic<int> g_path_policy{0};
 
 int cfr_path_policy(int policy) {
@@ -1608,12 +1613,69 @@ static int clear_counters(int32_t* work_counter, cudaStream_t stream) {
     return check_cuda(cudaMemsetAsync(work_counter, 0, 4 * sizeof(int32_t), stream), "cudaMemsetAsync(work counter)");
 }
 
-long long cfr_solve_scratch_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows) {
+// Some subgame of the batch may be too large for the lean kernel.
+static bool maybe_large(int max_internal, int max_children) { return (long long)max_internal * max_children + 1 > kIterMaxNodes; }
+
+static bool lean_preferred(int num_subgames, int max_internal, int max_children) {
+    if (g_path_policy.load() != 0) return true;
+    return num_subgames >= (maybe_large(max_internal, max_children) ? 8 * sm_count() : 3 * sm_count() / 2);
+}
+
+// Work space of a one-call solve before the hand-over rows: one set of work rows per block, or the space of the split
+// passes, which the start and final pass use in turn.
+static long long solve_work_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows) {
     long long per_block = cfr_scratch_floats(max_internal);
     const long long iter_block = cfr_iter_scratch_floats(max_internal, max_children);
     if (iter_block > per_block) per_block = iter_block;
+    const long long blocks = per_block * num_blocks, split = split_scratch_floats(num_subgames, rows);
+    const bool lean = max_children <= kIterMaxChildren && lean_preferred(num_subgames, max_internal, max_children);
+    return !lean && split > blocks ? split : blocks;
+}
+
+long long cfr_solve_scratch_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows) {
     const long long carry_sums = rows * 4;  // current-policy sums and, for cfr_avg, average-policy sums
-    return per_block * num_blocks + (long long)num_subgames * 4 * P2B_HPAD + carry_sums;
+    return solve_work_floats(max_internal, max_children, num_blocks, num_subgames, rows) + (long long)num_subgames * 4 * P2B_HPAD +
+           carry_sums;
+}
+
+long long cfr_step_scratch_floats(int max_internal, int num_subgames, long long rows) {
+    const long long one_each = cfr_scratch_floats(max_internal) * num_subgames, split = split_scratch_floats(num_subgames, rows);
+    return one_each > split ? one_each : split;
+}
+
+// The record check and a launch of the general kernel for the passes and phases given.
+static int general_passes(CfrParams p, int num_blocks, int max_children, int begin, int end, int phases, cudaStream_t stream) {
+    p.pass_begin = begin;
+    p.pass_end = end;
+    p.phases = phases;
+    int rc = clear_counters(p.work_counter, stream);
+    return rc ? rc : dispatch_cfr(p, num_blocks, max_children, stream);
+}
+
+// The same for iteration passes on the split kernels.
+static int split_passes(const CfrParams& p, int max_children, int begin, int end, bool down, bool up, cudaStream_t stream) {
+    int rc = clear_counters(p.work_counter, stream);
+    if (!rc) rc = check_records(p, stream);
+    return rc ? rc : launch_split_passes(p, max_children, begin, end, down, up, stream);
+}
+
+// A call of a stepped solve: start and final pass in the general kernel, iteration passes in the split kernels.
+static int launch_stepped(const CfrParams& p, int num_blocks, int max_children, cudaStream_t stream) {
+    const int T = p.iterations;
+    int rc = P2B_OK;
+    if (p.phases == 16) {
+        const int t = p.pass_begin;
+        rc = t < 0 ? general_passes(p, num_blocks, max_children, t, t, 2, stream) : P2B_OK;
+        if (!rc && t + 1 < T) return split_passes(p, max_children, t < 0 ? 0 : t, t + 1, t < 0, false, stream);
+        if (!rc && t >= 0) rc = split_passes(p, max_children, t, t, false, true, stream);
+        return rc ? rc : general_passes(p, num_blocks, max_children, T, T, 1, stream);
+    }
+    const bool down = (p.phases & 1) != 0, up = (p.phases & 2) != 0;
+    const int first = p.pass_begin < 0 ? 0 : p.pass_begin, last = p.pass_end < T ? p.pass_end : T - 1;
+    if (p.pass_begin < 0) rc = general_passes(p, num_blocks, max_children, -1, -1, p.phases, stream);
+    if (!rc && first <= last) rc = split_passes(p, max_children, first, last, down, up, stream);
+    if (!rc && p.pass_end == T) rc = general_passes(p, num_blocks, max_children, T, T, p.phases, stream);
+    return rc;
 }
 
 int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, cudaStream_t stream, bool fast_scratch) {
@@ -1629,13 +1691,35 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
     // leaves all terminal, all passes in this call: the iteration kernel applies (a start policy only concerns
     // the start pass, a warm start of type `model` is a kernel of its own between that pass and the iterations)
     const bool plain = !p.stepped && !p.leaf_beliefs && !p.leaf_values && !p.cfr_avg && !p.linear;
+    if (p.stepped && p.phases != 4 && p.phases != 8 && split_applies(p, max_children, p.scratch_floats))
+        return launch_stepped(p, num_blocks, max_children, stream);
     long long per_block = cfr_scratch_floats(p.max_internal);
     const long long iter_block = cfr_iter_scratch_floats(p.max_internal, max_children);
     if (iter_block > per_block) per_block = iter_block;
-    const bool maybe_large = (long long)p.max_internal * max_children + 1 > kIterMaxNodes;
-    const bool few = g_path_policy.load() == 0 &&
-                     (p.num_subgames <= sm_count() || (maybe_large && p.num_subgames < 8 * sm_count()));
-    if (!(plain && fast_scratch && max_children <= kIterMaxChildren && !few)) {
+    const bool large = maybe_large(p.max_internal, max_children);
+    const bool lean = plain && fast_scratch && max_children <= kIterMaxChildren &&
+                      lean_preferred(p.num_subgames, p.max_internal, max_children);
+    if (!p.stepped && fast_scratch && !lean && split_applies(p, max_children, p.scratch_floats)) {
+        IterTiming* timing = iter_timing_of_current_device();
+        const bool timed = timing && timing->enabled && p.num_subgames > (large ? 8 : 1) * sm_count();
+        CfrParams q = p;
+        q.scratch_stride = per_block;
+        q.carry_roots = p.scratch + solve_work_floats(p.max_internal, max_children, num_blocks, p.num_subgames, p.rows);
+        q.carry_sums = q.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;
+        q.stepped = 1;
+        q.scratch_per_block = 1;
+        rc = general_passes(q, num_blocks, max_children, -1, -1, 3, stream);
+        if (!rc && p.warm_weight > 0.0f)
+            rc = launch_cfr_warm_seed(p.nodes, p.rows, p.start_policy, p.warm_weight, p.regrets, p.weight_sums, stream);
+        if (timed) cudaEventRecord(timing->start, stream);
+        if (!rc) rc = split_passes(q, max_children, 0, p.iterations - 1, true, true, stream);
+        if (timed) {
+            cudaEventRecord(timing->stop, stream);
+            timing->recorded = true;
+        }
+        return rc ? rc : general_passes(q, num_blocks, max_children, p.iterations, p.iterations, 3, stream);
+    }
+    if (!lean) {
         if (p.warm_weight > 0.0f) {
             // the general kernel in two launches around the seeding: start pass, then every other pass
             if (p.stepped) return set_error(P2B_ERR_ARG, "a stepped solve seeds its warm start itself");
@@ -1644,7 +1728,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
                                               "(hand-over rows between the launches)");
             CfrParams q = p;
             q.scratch_stride = per_block;
-            q.carry_roots = p.scratch + per_block * num_blocks;
+            q.carry_roots = p.scratch + solve_work_floats(p.max_internal, max_children, num_blocks, p.num_subgames, p.rows);
             q.carry_sums = q.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;
             q.stepped = 1;
             q.scratch_per_block = 1;
@@ -1671,7 +1755,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
     // pass with the best responses (cfr_solve_kernel).  Root rows and their sums travel between the
     // launches in the tail of the scratch area; work rows do not, so each launch keeps one set per block.
     p.scratch_stride = per_block;
-    p.carry_roots = p.scratch + per_block * num_blocks;
+    p.carry_roots = p.scratch + solve_work_floats(p.max_internal, max_children, num_blocks, p.num_subgames, p.rows);
     p.carry_sums = p.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;
     p.stepped = 1;
     p.scratch_per_block = 1;
@@ -1683,8 +1767,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
         rc = clear_counters(q.work_counter, stream);
         if (rc) return rc;
         if (part == 1) {
-            cfr_validate_kernel<<<q.num_subgames, kCfrMaxNodes, 0, stream>>>(q);
-            rc = check_cuda(cudaGetLastError(), "cfr_validate_kernel");
+            rc = check_records(q, stream);
             if (rc) return rc;
             IterTiming* timing = iter_timing_of_current_device();
             const bool timed = timing && timing->enabled;
@@ -1697,7 +1780,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
             // Subgames with more nodes than the iteration kernel holds in shared memory were skipped by it:
             // the general kernel runs their iteration passes.  The batch can only contain such a subgame
             // if the bound below exceeds the limit.
-            if (!rc && maybe_large) {
+            if (!rc && large) {
                 rc = clear_counters(q.work_counter, stream);
                 if (rc) return rc;
                 q.large_only = 1;

@@ -104,6 +104,7 @@ struct CfrParams {
     float* br_values;            // [B][2] best-response value of each player at the root (out, may be null)
     float* scratch;              // per-block work rows
     long long scratch_stride;    // floats per block
+    long long scratch_floats;    // size of the whole scratch area
     int32_t max_internal;        // largest n_internal over the batch
     const IterScalars* scalars;  // [iterations]
     int32_t iterations;
@@ -162,6 +163,7 @@ __host__ __device__ inline long long cfr_scratch_floats(int max_internal) {
 int launch_cfr_solve(const CfrParams& p, int num_blocks, int max_children, cudaStream_t stream, bool fast_scratch = false);
 long long cfr_iter_scratch_floats(int max_internal, int max_children);
 long long cfr_solve_scratch_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows);
+long long cfr_step_scratch_floats(int max_internal, int num_subgames, long long rows);
 int launch_cfr_iter(const CfrParams& p, int num_blocks, cudaStream_t stream);
 int cfr_path_policy(int policy);  // returns the previous one; < 0 only queries
 int cfr_iteration_timing(int enable);

@@ -453,7 +453,7 @@ class SteppedSolver(SubgameSolver):
     def __init__(self, layout: DeviceTreeLayout, boards: torch.Tensor, device: torch.device, **kw):
         super().__init__(layout, boards, device, **kw)
         f32 = dict(device=device, dtype=torch.float32)
-        n_scratch = int(_lib.lib().p2b_cfr_scratch_floats(layout.max_internal, 1)) * self.B
+        n_scratch = int(_lib.lib().p2b_cfr_step_scratch_floats(layout.max_internal, self.B, layout.rows))
         self.scratch = torch.empty(n_scratch, **f32)
         self.carry_sums = torch.zeros(2, layout.rows, 2, **f32)  # current-policy sums, average-policy sums
         self.carry_roots = torch.zeros(self.B, 4, HPAD, **f32)
@@ -536,11 +536,10 @@ class SteppedSolver(SubgameSolver):
         launching their kernels and the leaf model's one by one; same kernels, same results.  Ignored
         where the host works between the passes (cfr_avg, running_values, policy_delta).  The leaf model must
         be capturable: device work only, the same shapes every pass, no host synchronisation.
-        joint_sweeps: with model leaves, launch the bottom-up sweep of a pass together with the top-down sweep
-        of the next one (`phases` 16 of `p2b_cfr_step`) wherever the host has nothing to do between them, so
-        that a pass is one solver launch instead of two; same results.  Off by default: measured on 192
-        flop subgames of 273 nodes it changes nothing (2.50 against 2.47 ms per pass), the time of a pass is
-        the blocks' walk over the subgames, not the launches."""
+        joint_sweeps: count the bottom-up sweep of a pass and the top-down sweep of the next one as one in
+        `launches`.  With model leaves the two go into one call (`phases` 16 of `p2b_cfr_step`) in any case, wherever
+        the host has nothing to do between them: that saves deriving the current policy anew (0.09 of 1.4 ms a pass on
+        192 flop subgames of 77 nodes); same results."""
         assert root_beliefs.shape == (self.B, 2, HPAD) and root_beliefs.dtype == torch.float32
         assert root_beliefs.is_contiguous() and root_beliefs.device == self.device
         ws = int(warm_start_iterations)
@@ -590,8 +589,7 @@ class SteppedSolver(SubgameSolver):
             for t, q in pstats.delta_checkpoints(ws, all_scalars.shape[0]).items():
                 delta_at[t - ws + (0 if ws > 0 else -1)] = q
         # the bottom-up sweep of a pass waits for the top-down sweep of the next one where they can share a launch
-        fuse = (joint_sweeps and n_leaves > 0 and graphed is None
-                and not (cfr_avg or running_values or policy_delta is not None))
+        fuse = n_leaves > 0 and graphed is None and not (cfr_avg or running_values or policy_delta is not None)
         pending_up = None
         for pas in range(-1, iterations + 1):
             if pas == 0 and warm_br:
@@ -632,6 +630,8 @@ class SteppedSolver(SubgameSolver):
             if pending_up is not None:
                 self._step(root_beliefs, sc, iterations, flags_pass, pending_up, pas, 16)
                 pending_up = None
+                if not joint_sweeps:
+                    self.launches += 1  # two sweeps
             else:
                 self._step(root_beliefs, sc, iterations, flags_pass, pas, pas, 1)
             vals = leaf_fn(self.leaf_beliefs[:n_leaves])

@@ -1,0 +1,67 @@
+"""The split kernels (a pass as one kernel over all nodes and one over all hands) against the general kernel, which walks
+the tree: equal bits in every output, over the batch sizes at which the column kernel changes its shape, the widest
+nodes and the solve options that change what a pass does."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def auto_policy(cuda_device):
+    from poker2_b200 import solver
+
+    before = solver.set_path_policy("auto")
+    yield
+    solver.set_path_policy(before)
+
+
+def _both(cuda_device, B, *, bins=(0.5, 1.0), cap=2, iterations=5, cfr_type="discounted", deep=False, **kw):
+    """The same solve with the full scratch area and with the minimal one, which keeps every pass in the general kernel."""
+    import bench
+    from poker2_b200 import solver, tree as ptree
+
+    boards, ranges, pot, stack = bench.make_inputs(B, 11 + B)
+    if deep:
+        pot, stack = torch.full((B,), 60), torch.full((B,), 500)
+    trees = ptree.build_trees(ptree.root_states(pot.numpy(), stack.numpy()), list(bins), 8, max_raises=cap)
+    layout = solver.device_layout(trees, boards.numpy())
+    rb = solver.pad_rows(ranges.to(cuda_device)).contiguous()
+    scal = solver.iteration_scalars(iterations, cfr_type=cfr_type, dcfr_delay=1)
+    out = []
+    for lean in (True, False):
+        sv = solver.SubgameSolver(layout, boards, cuda_device, exploitability=True, keep_policy=True, sampling=True,
+                                  lean_iterations=lean)
+        sv.set_sampling_schedule(torch.arange(B) % iterations + 1)
+        r = sv.solve(rb, scal, check=True, **kw)
+        out.append([x.clone() for x in (r.policy_avg, r.regrets, r.weight_sums, r.policy, r.policy_sample, r.root_values[..., :1326],
+                                        r.values_avg[..., :1326], r.exploitability, r.br_values)] + [r.beliefs_last.clone()])
+    return layout, out
+
+
+@pytest.mark.parametrize("B", [1, 7, 8, 60])  # one hand a thread up to 7, two from 8 on
+def test_batch_sizes(cuda_device, B):
+    for a, b in zip(*_both(cuda_device, B)[1]):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("opts", [
+    dict(bins=(0.5, 0.75, 1.0, 1.5, 2.0), cap=1),  # up to 8 actions at a node
+    dict(cap=None, deep=True),  # more nodes than the lean kernel holds
+    dict(cfr_type="linear", cfr_plus=True),
+    dict(cfr_avg=True, enforce_zero_sum=True),
+    dict(cfr_type="discounted_plus", iterations=1),
+])
+def test_options(cuda_device, opts):
+    layout, out = _both(cuda_device, 5, **opts)
+    if opts.get("deep"):
+        assert np.asarray(layout.subgames["n_nodes"]).max() > 160
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("B", [160, 600])  # two warps and one warp a slice; beyond the lean kernel's 8 actions limit
+def test_wide_batches(cuda_device, B):
+    for a, b in zip(*_both(cuda_device, B, bins=(0.5, 0.75, 1.0, 1.5, 2.0), cap=1, iterations=2)[1]):
+        assert torch.equal(a, b)
