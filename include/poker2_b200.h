@@ -392,6 +392,14 @@ int p2b_chance_expand_features(const float* pre_beliefs, int64_t player_stride, 
                                int64_t feature_stride, int64_t* root_lookup, void* stream);
 int p2b_indexed_mean_bf16(const void* src_bf16, int64_t src_stride, const int64_t* sample_offsets,
                           int64_t num_roots, float* out, int64_t out_player_stride, void* stream);
+/* A bf16 value network called once per leaf (set_leaf_values, src/p2/search/cfr_evaluator.py:1025-1047):
+ * p2b_leaf_features_bf16 rounds both players' beliefs of every leaf (rows player_stride floats apart) into the first
+ * 2 x 1326 columns of its input row; p2b_leaf_values_bf16 widens the first 2 x 1326 columns of its output rows into
+ * the leaf's two value rows.  Strides in elements, all even. */
+int p2b_leaf_features_bf16(const float* beliefs, int64_t player_stride, int64_t leaves, void* features_bf16,
+                           int64_t feature_stride, void* stream);
+int p2b_leaf_values_bf16(const void* values_bf16, int64_t value_stride, int64_t leaves, float* out, int64_t player_stride,
+                         void* stream);
 /* Flop chance node (src/p2/search/chance_node_helper.py:218-357).  p2b_expand_on_boards:
  * post_beliefs [num_roots*num_boards, 2, 1326] = the beliefs of every root re-blocked and
  * re-normalised on every given board (boards [num_boards, board_len] int64, -1 = empty slot;

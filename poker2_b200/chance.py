@@ -35,7 +35,7 @@ def expand_next_card(pre_beliefs: torch.Tensor, boards: torch.Tensor):
     post = torch.empty(S, 2, NUM_HANDS, device=boards.device, dtype=torch.float32)
     lookup = torch.empty(S, dtype=torch.int64, device=boards.device)
     samples = torch.empty(S, L, dtype=torch.int64, device=boards.device)
-    with torch.cuda.device(boards.device):
+    with _lib.on(boards.device):
         _lib.call("p2b_chance_expand", _lib.ptr(pre_beliefs), _lib.ptr(boards), L, _lib.ptr(offsets), B, S,
                   _lib.ptr(post), _lib.ptr(lookup), _lib.ptr(samples), _lib.stream_ptr(boards.device))
     return post, lookup, samples
@@ -51,7 +51,7 @@ def indexed_add_rows(out: torch.Tensor, index: torch.Tensor, src: torch.Tensor, 
     assert out.dtype == torch.float32 == src.dtype and index.dtype == torch.int64
     assert src.shape[0] == index.shape[0] and src.shape[1:] == out.shape[1:]
     width = out[0].numel() if out.shape[0] else 0
-    with torch.cuda.device(out.device):
+    with _lib.on(out.device):
         _lib.call("p2b_indexed_add_rows", _lib.ptr(out), _lib.ptr(index), _lib.ptr(src), src.shape[0], out.shape[0],
                   width, int(mean), int(accumulate), _lib.stream_ptr(out.device))
     return out
@@ -89,7 +89,7 @@ def expand_features_bf16(pre_beliefs: torch.Tensor, boards: torch.Tensor, offset
     if out is None:
         out = torch.empty(num_samples, feature_stride, device=pre_beliefs.device, dtype=torch.bfloat16)
     assert out.dtype == torch.bfloat16 and out.is_contiguous() and tuple(out.shape) == (num_samples, feature_stride)
-    with torch.cuda.device(pre_beliefs.device):
+    with _lib.on(pre_beliefs.device):
         _lib.call("p2b_chance_expand_features", _lib.ptr(pre_beliefs), pre_beliefs.stride(1), _lib.ptr(boards),
                   boards.shape[1], _lib.ptr(offsets), B, num_samples, _lib.ptr(context), _lib.ptr(out), feature_stride,
                   None, _lib.stream_ptr(pre_beliefs.device))
@@ -102,7 +102,7 @@ def indexed_mean_bf16(src: torch.Tensor, offsets: torch.Tensor, out: torch.Tenso
     _lib.require_cuda(src, "indexed_mean_bf16")
     assert src.dtype == torch.bfloat16 and src.stride(1) == 1 and out.dtype == torch.float32
     assert out.stride(2) == 1 and out.stride(0) == 2 * out.stride(1)
-    with torch.cuda.device(src.device):
+    with _lib.on(src.device):
         _lib.call("p2b_indexed_mean_bf16", _lib.ptr(src), src.stride(0), _lib.ptr(offsets), out.shape[0], _lib.ptr(out),
                   out.stride(1), _lib.stream_ptr(src.device))
     return out

@@ -132,7 +132,7 @@ def build_device_layout(roots: ptree.RoundState, boards, bet_bins, max_depth: in
     level_counts = torch.empty(B, D + 1, **i32)
     stream = _lib.stream_ptr(device)
     p = _lib.ptr
-    with torch.cuda.device(device):
+    with _lib.on(device):
         _lib.call("p2b_tree_count", p(packed), B, bins, n_bins, D, cap, p(counts), p(level_counts), stream)
         # prefix sums over the subgames (plumbing): rows, model-leaf slots, level-major bases
         # (scans run along the contiguous dimension of transposed copies: torch's scan along the
@@ -163,7 +163,7 @@ def build_device_layout(roots: ptree.RoundState, boards, bet_bins, max_depth: in
     to_lm = torch.empty(rows, device=device, dtype=torch.int64)
     model_rows = torch.empty(n_model, device=device, dtype=torch.int64)
     state = torch.empty(rows, 8, **i32) if node_state else None
-    with torch.cuda.device(device):
+    with _lib.on(device):
         _lib.call("p2b_tree_records", p(packed), p(boards_dev), int(boards_dev.shape[1]), B, bins, n_bins, D, cap,
                   p(node_begin), p(leaf_begin), p(level_base), p(subgames), p(nodes), p(to_lm),
                   p(model_rows) if n_model else None, p(state), stream)

@@ -178,7 +178,7 @@ class SubgameEvaluator:
                                          warm_start_iterations=ws)
         if ws > 0 and start_policy is None:  # uniform over the children of every parent
             cc = torch.from_numpy(self.trees.child_count[self.trees.parent_index.clip(min=0)]).clamp(min=1)
-            start_policy = (1.0 / cc.to(torch.float32))[:, None].expand(-1, NUM_HANDS).contiguous()
+            start_policy = (1.0 / cc.to(torch.float32)).to(self.device)[:, None].expand(-1, NUM_HANDS)
         first = None
         if ws > 0:
             first = psolver.warm_start_mix_scalars(scal, cfr_type=self.cfr_type, gamma=self.gamma,

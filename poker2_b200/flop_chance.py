@@ -70,7 +70,7 @@ def expand_on_boards(pre_beliefs: torch.Tensor, boards: torch.Tensor) -> torch.T
     boards = boards.to(device=pre_beliefs.device, dtype=torch.int64).contiguous()
     B, F = pre_beliefs.shape[0], boards.shape[0]
     post = torch.empty(B * F, 2, NUM_HANDS, device=pre_beliefs.device, dtype=torch.float32)
-    with torch.cuda.device(pre_beliefs.device):
+    with _lib.on(pre_beliefs.device):
         _lib.call("p2b_expand_on_boards", _lib.ptr(pre_beliefs), pre_beliefs.stride(1), _lib.ptr(boards), boards.shape[1],
                   B, F, _lib.ptr(post), _lib.stream_ptr(pre_beliefs.device))
     return post
@@ -82,7 +82,7 @@ def mean_over_hand_perms(values: torch.Tensor, perms: torch.Tensor) -> torch.Ten
     assert values.dtype == torch.float32 and values.is_contiguous() and values.shape[-1] == NUM_HANDS
     perms = perms.to(device=values.device, dtype=torch.int32).contiguous()
     out = torch.empty_like(values)
-    with torch.cuda.device(values.device):
+    with _lib.on(values.device):
         _lib.call("p2b_mean_over_hand_perms", _lib.ptr(values), _lib.ptr(perms), perms.shape[0],
                   values.numel() // NUM_HANDS, _lib.ptr(out), _lib.stream_ptr(values.device))
     return out

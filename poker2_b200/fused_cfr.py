@@ -26,7 +26,7 @@ def _require() -> None:
 
 
 def _call(name: str, dev: torch.device, *args) -> None:
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         _lib.call(name, *args, _lib.stream_ptr(dev))
 
 
@@ -468,7 +468,7 @@ class GraphedCFRIteration:
         prev_skip = ev._skip_t_scalars_update
         ev._skip_t_scalars_update = True
         try:
-            with torch.cuda.device(ev.device):
+            with _lib.on(ev.device):
                 side = torch.cuda.Stream()
                 side.wait_stream(torch.cuda.current_stream())
                 with torch.cuda.stream(side):

@@ -15,7 +15,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from . import chance
+from . import _lib, chance
 
 NUM_HANDS = 1326
 
@@ -96,21 +96,25 @@ class ChanceLeafEvaluator:
             off = chance.sample_offsets_of(self.boards[a:b])
             self._chunks.append((a, b, off, int(off[-1].item())))
 
-    def _call_fused(self, leaf_beliefs: torch.Tensor) -> torch.Tensor:
-        L, W = leaf_beliefs.shape[0], leaf_beliefs.shape[2]
-        out = torch.zeros(L, 2, W, device=leaf_beliefs.device, dtype=torch.float32)
+    def evaluate_into(self, leaf_beliefs: torch.Tensor, out: torch.Tensor) -> None:
+        """Values of all leaves into out[..., :1326] (fp32 [L,2,W])."""
+        if not self.fused:
+            out[..., :NUM_HANDS].copy_(self(leaf_beliefs))
+            return
         for a, b, off, n_samples in self._chunks:
             x = chance.expand_features_bf16(leaf_beliefs[a:b], self.boards[a:b], off, n_samples, self.context[a:b],
                                             self.model.IN_PADDED)
-            y = self.model.net(x)
+            with torch.no_grad():
+                y = self.model.net(x)
             chance.indexed_mean_bf16(y, off, out[a:b])
         self.calls += 1
-        return out
 
     def __call__(self, leaf_beliefs: torch.Tensor) -> torch.Tensor:
-        if self.fused:
-            return self._call_fused(leaf_beliefs)
         L = leaf_beliefs.shape[0]
+        if self.fused:
+            out = torch.zeros(L, 2, leaf_beliefs.shape[2], device=leaf_beliefs.device, dtype=torch.float32)
+            self.evaluate_into(leaf_beliefs, out)
+            return out
         out = torch.empty(L, 2, NUM_HANDS, device=leaf_beliefs.device, dtype=torch.float32)
         for a in range(0, L, self.chunk):
             b = min(a + self.chunk, L)
@@ -131,5 +135,39 @@ class DirectLeafEvaluator:
         self.boards = boards.to(device=device, dtype=torch.int64).contiguous()
         self.context = context.to(device=device, dtype=torch.float32).contiguous()
 
+        # a bf16 `ValueMLP` reads rows that the feature kernel writes: the columns that no pass changes (board
+        # one-hot, context, padding) are filled in once
+        self._rows = None
+        if type(model) is ValueMLP and model.dtype == torch.bfloat16 and self.boards.shape[0] > 0:
+            L, first = self.boards.shape[0], 2 * NUM_HANDS
+            x = torch.zeros(L, ValueMLP.IN_PADDED, device=device, dtype=torch.bfloat16)
+            card = torch.arange(52, device=device)
+            x[:, first: first + 52] = (self.boards[:, :, None] == card).any(dim=1)
+            x[:, first + 52: ValueMLP.IN_FEATURES] = self.context
+            self._rows = x
+
+    def evaluate_into(self, leaf_beliefs: torch.Tensor, out: torch.Tensor) -> None:
+        """Values of all leaves into out[..., :1326] (fp32 [L,2,W])."""
+        if self._rows is None or not _paired_rows(leaf_beliefs) or not _paired_rows(out):
+            out[..., :NUM_HANDS].copy_(self.model(leaf_beliefs[..., :NUM_HANDS].contiguous(), self.boards, self.context))
+            return
+        p, L = _lib.ptr, leaf_beliefs.shape[0]
+        with _lib.on(out.device), torch.no_grad():
+            stream = _lib.stream_ptr(out.device)
+            _lib.call("p2b_leaf_features_bf16", p(leaf_beliefs), leaf_beliefs.stride(1), L, p(self._rows),
+                      self._rows.stride(0), stream)
+            y = self.model.net(self._rows)
+            _lib.call("p2b_leaf_values_bf16", p(y), y.stride(0), L, p(out), out.stride(1), stream)
+
     def __call__(self, leaf_beliefs: torch.Tensor) -> torch.Tensor:
-        return self.model(leaf_beliefs[..., :NUM_HANDS].contiguous(), self.boards, self.context)
+        if self._rows is None:
+            return self.model(leaf_beliefs[..., :NUM_HANDS].contiguous(), self.boards, self.context)
+        out = torch.empty(leaf_beliefs.shape[0], 2, NUM_HANDS, device=leaf_beliefs.device, dtype=torch.float32)
+        self.evaluate_into(leaf_beliefs, out)
+        return out
+
+
+def _paired_rows(t: torch.Tensor) -> bool:
+    """[L,2,W] fp32, rows of whole pairs of hands one after the other."""
+    return (t.is_cuda and t.dtype == torch.float32 and t.stride(2) == 1 and t.stride(0) == 2 * t.stride(1)
+            and t.stride(1) % 2 == 0 and t.data_ptr() % 8 == 0)

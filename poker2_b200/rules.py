@@ -35,7 +35,7 @@ def compare_7_single_batch(ab_batch: torch.Tensor) -> torch.Tensor:
     _lib.require_cuda(ab_batch, "CUDA hand evaluator")
     planes = ab_batch.contiguous().to(torch.int8)
     out = torch.empty((planes.shape[0],), device=planes.device, dtype=torch.int32)
-    with torch.cuda.device(planes.device):
+    with _lib.on(planes.device):
         _lib.call("p2b_compare7_planes", _lib.ptr(planes), planes.shape[0], _lib.ptr(out),
                   _lib.stream_ptr(planes.device))
     return out
@@ -64,7 +64,7 @@ def compare_7_cards_single_batch(cards_batch: torch.Tensor) -> torch.Tensor:
     _lib.require_cuda(cards_batch, "CUDA hand evaluator")
     cards = _as_i16(cards_batch)
     out = torch.empty((cards.shape[0],), device=cards.device, dtype=torch.int32)
-    with torch.cuda.device(cards.device):
+    with _lib.on(cards.device):
         _lib.call("p2b_compare7_cards", _lib.ptr(cards), cards.shape[0], _lib.ptr(out),
                   _lib.stream_ptr(cards.device))
     return out
@@ -79,7 +79,7 @@ def rank_7_cards_single_batch(cards_batch: torch.Tensor) -> torch.Tensor:
     _lib.require_cuda(cards_batch, "CUDA hand evaluator")
     cards = _as_i16(cards_batch)
     out = torch.empty((cards.shape[0],), device=cards.device, dtype=torch.int32)
-    with torch.cuda.device(cards.device):
+    with _lib.on(cards.device):
         _lib.call("p2b_rank7_cards", _lib.ptr(cards), cards.shape[0], _lib.ptr(out),
                   _lib.stream_ptr(cards.device))
     return out
@@ -96,7 +96,7 @@ def rank_hands(board: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     m = b16.shape[0]
     scores = torch.empty((m, NUM_HANDS), device=board.device, dtype=torch.int32)
     order = torch.empty((m, NUM_HANDS), device=board.device, dtype=torch.int64)
-    with torch.cuda.device(board.device):
+    with _lib.on(board.device):
         _lib.call("p2b_rank_hands", _lib.ptr(b16), m, _lib.ptr(scores), _lib.ptr(order), None,
                   _lib.stream_ptr(board.device))
     return scores, order

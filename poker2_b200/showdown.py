@@ -24,7 +24,7 @@ class BoardTables:
         self.num_boards = boards.shape[0]
         b16 = boards.contiguous().to(torch.int16)
         self.blob = torch.empty((self.num_boards, _lib.TABLE_BYTES), device=self.device, dtype=torch.uint8)
-        with torch.cuda.device(self.device):
+        with _lib.on(self.device):
             _lib.call("p2b_rank_hands", _lib.ptr(b16), self.num_boards, None, None, _lib.ptr(self.blob),
                       _lib.stream_ptr(self.device))
 
@@ -56,7 +56,7 @@ def showdown_values(
     if out is None:
         out = torch.empty_like(beliefs)
     assert out.is_contiguous() and out.shape == beliefs.shape and out.dtype == torch.float32
-    with torch.cuda.device(beliefs.device):
+    with _lib.on(beliefs.device):
         _lib.call("p2b_showdown_values", _lib.ptr(tables.blob), _lib.ptr(table_of_row), _lib.ptr(beliefs),
                   2 * NUM_HANDS, _lib.ptr(potential), _lib.ptr(scale), _lib.ptr(out), 2 * NUM_HANDS, rows,
                   _lib.stream_ptr(beliefs.device))

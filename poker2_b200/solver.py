@@ -316,7 +316,7 @@ class SubgameSolver:
         rows = layout.rows
         B = int(layout.subgames_dev.shape[0]) if built_on_device else layout.subgames.shape[0]
         self.B = B
-        with torch.cuda.device(device):
+        with _lib.on(device):
             blocks = num_blocks if num_blocks > 0 else int(_lib.lib().p2b_cfr_default_blocks())
         self.num_blocks = min(blocks, B)
         f32 = dict(device=device, dtype=torch.float32)
@@ -339,13 +339,7 @@ class SubgameSolver:
         self.beliefs_avg = torch.zeros(rows, 2, HPAD, **f32) if keep_node_values else None
         self.exploitability = torch.zeros(B, **f32) if (exploitability and keep_node_values) else None
         self.br_values = torch.zeros(B, 2, **f32) if (exploitability and keep_node_values) else None
-        # the larger area lets a solve without optional outputs run its iteration passes in the lean kernel
-        if lean_iterations:
-            n_scratch = int(_lib.lib().p2b_cfr_solve_scratch_floats(layout.max_internal, layout.max_children,
-                                                                    self.num_blocks, B, rows))
-        else:
-            n_scratch = int(_lib.lib().p2b_cfr_scratch_floats(layout.max_internal, self.num_blocks))
-        self.scratch = torch.empty(n_scratch, **f32)
+        self.scratch = torch.empty(self._scratch_floats(lean_iterations), **f32)
         self.work_counter = torch.zeros(4, device=device, dtype=torch.int32)
         # the thread blocks take subgames from a queue: largest trees first, so that the blocks that finish
         # last hold small ones (a stable sort: equal sizes keep their input order)
@@ -359,6 +353,14 @@ class SubgameSolver:
         self.beliefs_last = torch.zeros(rows, 2, HPAD, **f32) if sampling else None
         self.sample_pass = torch.full((B,), -2, device=device, dtype=torch.int32) if sampling else None
         self.launches = 0
+
+    def _scratch_floats(self, lean_iterations: bool) -> int:
+        """The larger area lets a solve run its iteration passes in the lean or in the split kernels."""
+        layout, lib = self.layout, _lib.lib()
+        if lean_iterations:
+            return int(lib.p2b_cfr_solve_scratch_floats(layout.max_internal, layout.max_children, self.num_blocks, self.B,
+                                                        layout.rows))
+        return int(lib.p2b_cfr_scratch_floats(layout.max_internal, self.num_blocks))
 
     def set_sampling_schedule(self, t_sample: torch.Tensor, warm_start_iterations: int = 0) -> None:
         """t_sample [B]: iteration at whose start each subgame's current policy is kept
@@ -417,7 +419,7 @@ class SubgameSolver:
         sc = torch.from_numpy(scalars.view(np.uint8).reshape(max(iterations, 0), 32).copy()).to(self.device)
         self._scalars = sc
         p = _lib.ptr
-        with torch.cuda.device(self.device):
+        with _lib.on(self.device):
             _lib.call(
                 "p2b_cfr_solve", p(self.subgames), p(self.nodes), self.B, self.layout.rows, self.layout.max_children,
                 self.layout.max_internal, p(self.tables.blob) if self.tables is not None else None, p(root_beliefs),
@@ -453,8 +455,6 @@ class SteppedSolver(SubgameSolver):
     def __init__(self, layout: DeviceTreeLayout, boards: torch.Tensor, device: torch.device, **kw):
         super().__init__(layout, boards, device, **kw)
         f32 = dict(device=device, dtype=torch.float32)
-        n_scratch = int(_lib.lib().p2b_cfr_step_scratch_floats(layout.max_internal, self.B, layout.rows))
-        self.scratch = torch.empty(n_scratch, **f32)
         self.carry_sums = torch.zeros(2, layout.rows, 2, **f32)  # current-policy sums, average-policy sums
         self.carry_roots = torch.zeros(self.B, 4, HPAD, **f32)
         slots = max(layout.num_model_leaves, 1)
@@ -462,38 +462,61 @@ class SteppedSolver(SubgameSolver):
         self.leaf_beliefs = torch.zeros(slots, 2, HPAD, **f32)
         self.leaf_values = torch.zeros(slots, 2, HPAD, **f32)
 
-    start_policy_rows = None  # [rows,1344] policy of the start pass (None: uniform)
-    _last_model_values = None
-    _graphed = None  # (key, GraphedPass) of the last solve with graph=True
+    def _scratch_floats(self, lean_iterations: bool) -> int:
+        return int(_lib.lib().p2b_cfr_step_scratch_floats(self.layout.max_internal, self.B, self.layout.rows))
 
-    def _de_average(self, vals, t, scalars, enforce_zero_sum, n_leaves):
+    start_policy_rows = None  # [rows,1344] policy of the start pass (None: uniform)
+    _last_model_values = None  # the model's values of the evaluation before (cfr_avg), padded rows
+    _spare_model_values = None  # the buffer that takes the next ones
+    _graphed = None  # (key, GraphedPass) of the last solve with graph=True
+    _mix_table = None  # the scalar table of the whole solve on the device, for the mixes between the passes
+
+    def _mix_zero_sum(self, a, b, beliefs, ignore, t: int, coef_a: str, coef_b: str, scale: str, out, subtract: bool,
+                      enforce_zero_sum: bool) -> None:
+        """out = (a * coef_a (+|-) b * coef_b) / scale over rows of [2,1344], minus the zero-sum shift by the beliefs if
+        asked (fp32 sums in the order of the CPU row reduction).  The coefficients are fields of iteration t's row of
+        the scalar table on the device."""
+        row = self._mix_table.data_ptr() + t * SCALAR_DTYPE.itemsize
+        at = lambda name: row + SCALAR_DTYPE.fields[name][1]  # noqa: E731
+        p = _lib.ptr
+        with _lib.on(self.device):
+            _lib.call("p2b_step_mix_zero_sum", p(a), p(b), p(beliefs), p(ignore), at(coef_a), at(coef_b), at(scale), p(out),
+                      a.shape[0], HPAD, 2 | int(subtract), 2 if enforce_zero_sum else 0, _lib.stream_ptr(self.device))
+
+    def _de_average(self, leaf_fn, t, enforce_zero_sum, n: int) -> None:
         """The CFR-AVG branch of `_set_model_values_impl` (cfr_evaluator.py:997-1018): from t = 2 on the
         model's values are read as the average over the iterations, so this iteration's are
         ((old + new) * values - old * last) / new, shifted to zero sum by the leaf beliefs if asked."""
-        raw = vals[..., :NUM_HANDS].to(torch.float32)
-        last, self._last_model_values = self._last_model_values, raw.clone()
+        raw = self._spare_model_values
+        if raw is None:
+            raw = torch.zeros_like(self.leaf_values)
+        self._value_leaves(leaf_fn, n, raw)
+        last, self._last_model_values, self._spare_model_values = self._last_model_values, raw, self._last_model_values
         if t <= 1 or last is None:
-            return vals
-        row = scalars[t]
-        old, total = float(row["mix_old"]), float(row["mix_total"])
-        new = torch.tensor(float(row["mix_new"]), device=raw.device, dtype=torch.float32)
-        unmixed = (total * raw - old * last) / new  # a tensor divisor: an IEEE division, like the CPU's
-        if enforce_zero_sum:
-            from . import fused_cfr as F
+            self.leaf_values[:n].copy_(raw[:n])
+        else:
+            self._mix_zero_sum(raw[:n], last[:n], self.leaf_beliefs[:n], None, t, "mix_total", "mix_old", "mix_new",
+                               self.leaf_values[:n], True, enforce_zero_sum)
 
-            one, zero = (torch.tensor(v, device=raw.device, dtype=torch.float32) for v in (1.0, 0.0))
-            out = torch.empty_like(unmixed)
-            # unmixed * 1 - 0 * 0 is unmixed itself; the kernel adds the shift, its sums in the CPU's order
-            F.mix_zero_sum(unmixed.contiguous(), torch.zeros_like(unmixed),
-                           self.leaf_beliefs[:n_leaves, :, :NUM_HANDS].contiguous(), one, zero, out, mode=2)
-            unmixed = out
-        return unmixed
+    def _value_leaves(self, leaf_fn, n: int, out: torch.Tensor | None = None) -> None:
+        """The caller's values of the first n leaf slots into `out` (default: the rows the bottom-up sweep reads); an
+        evaluator that can write in place does."""
+        out = self.leaf_values if out is None else out
+        into = getattr(leaf_fn, "evaluate_into", None)
+        if into is not None:
+            into(self.leaf_beliefs[:n], out[:n])
+            return
+        vals = leaf_fn(self.leaf_beliefs[:n])
+        if vals.shape[-1] == NUM_HANDS:
+            out[:n, :, :NUM_HANDS].copy_(vals)
+        else:
+            out[:n].copy_(vals)
 
     def _step(self, root_beliefs, sc, iterations, flags, pass_begin, pass_end, phases, sample_pass=None) -> None:
         p = _lib.ptr
         if sample_pass is None:
             sample_pass = self.sample_pass
-        with torch.cuda.device(self.device):
+        with _lib.on(self.device):
             _lib.call(
                 "p2b_cfr_step", p(self.subgames), p(self.nodes), self.B, self.layout.rows, self.layout.max_children,
                 self.layout.max_internal, p(self.tables.blob) if self.tables is not None else None, p(root_beliefs),
@@ -569,7 +592,9 @@ class SteppedSolver(SubgameSolver):
         if n_leaves and leaf_fn is None:
             raise ValueError("the trees have model-valued leaves: a leaf_fn is required")
         self._last_model_values = None
-        self._running = None
+        self._running = self._spare_running = None
+        if cfr_avg or running_values:
+            self._mix_table = torch.from_numpy(all_scalars.view(np.uint8).reshape(-1, SCALAR_DTYPE.itemsize).copy()).to(self.device)
         self.policy_deltas = {}
         graphed = None
         if graph and not (cfr_avg or running_values or policy_delta is not None) and iterations >= 4:
@@ -600,7 +625,7 @@ class SteppedSolver(SubgameSolver):
                 if self.weight_sums is not None:
                     self.weight_sums.fill_(weight)
             elif pas == 0 and ws > 0:
-                with torch.cuda.device(self.device):
+                with _lib.on(self.device):
                     _lib.call("p2b_cfr_warm_seed", _lib.ptr(self.nodes), self.layout.rows, _lib.ptr(self.start_policy_rows),
                               float(ws) * float(warm_start_multiplier), _lib.ptr(self.regrets), _lib.ptr(self.weight_sums),
                               _lib.stream_ptr(self.device))
@@ -623,7 +648,7 @@ class SteppedSolver(SubgameSolver):
             if n_leaves == 0:
                 self._step(root_beliefs, sc, iterations, flags_pass, pas, pas, 3)
                 if running_values:
-                    self._mix_running_values(pas, ws, all_scalars, enforce_zero_sum)
+                    self._mix_running_values(pas, ws, enforce_zero_sum)
                 if before is not None:
                     self.policy_deltas[delta_at[pas]] = policy_delta(before, policy_delta.policy_of(self.regrets))
                 continue
@@ -634,16 +659,13 @@ class SteppedSolver(SubgameSolver):
                     self.launches += 1  # two sweeps
             else:
                 self._step(root_beliefs, sc, iterations, flags_pass, pas, pas, 1)
-            vals = leaf_fn(self.leaf_beliefs[:n_leaves])
             if cfr_avg:
                 # iteration the pass belongs to, as `set_leaf_values(t)` sees it: the start pass, the pass
                 # that follows a warm start and the final pass pass t = 0 (:1511, :1288)
                 t = 0 if (pas < 0 or pas == iterations) else (pas if ws == 0 else (0 if pas == 0 else ws + pas - 1))
-                vals = self._de_average(vals, t, all_scalars, enforce_zero_sum, n_leaves)
-            if vals.shape[-1] == NUM_HANDS:
-                self.leaf_values[:n_leaves, :, :NUM_HANDS].copy_(vals)
+                self._de_average(leaf_fn, t, enforce_zero_sum, n_leaves)
             else:
-                self.leaf_values[:n_leaves].copy_(vals)
+                self._value_leaves(leaf_fn, n_leaves)
             if self.beliefs_last is not None and pas == iterations - 1:
                 # beliefs of the last iteration at the model leaves (the states sampling continues from)
                 self.beliefs_last[layout_tensor(self.layout, "model_rows", self.device)] = self.leaf_beliefs[:n_leaves]
@@ -652,7 +674,7 @@ class SteppedSolver(SubgameSolver):
                 continue
             self._step(root_beliefs, sc, iterations, flags_pass, pas, pas, 2)
             if running_values:
-                self._mix_running_values(pas, ws, all_scalars, enforce_zero_sum)
+                self._mix_running_values(pas, ws, enforce_zero_sum)
             if before is not None:
                 self.policy_deltas[delta_at[pas]] = policy_delta(before, policy_delta.policy_of(self.regrets))
         return self._result()
@@ -661,31 +683,25 @@ class SteppedSolver(SubgameSolver):
     _running = None  # [rows,2,1344] the running average
     _terminal = None  # [rows] uint8: 1 at the leaves that end the hand (exempt from the zero-sum shift)
 
-    def _mix_running_values(self, pas, ws, scalars, enforce_zero_sum) -> None:
+    def _mix_running_values(self, pas, ws, enforce_zero_sum) -> None:
         """After the bottom-up sweep of pass `pas` (whose node values are in self.values_avg, the average
         beliefs in self.beliefs_avg): the start pass, or the pass that follows a warm start, sets the
         average to the values (cfr_evaluator.py:1513); an iteration pass mixes them in with the weights
         of its iteration and shifts the result to zero sum (:1260-1274)."""
-        from . import fused_cfr as F
-
         first = 0 if ws > 0 else -1
         if pas < first:
             return
         if pas == first:
             self._running = self.values_avg.clone()
+            self._spare_running = torch.empty_like(self._running)
             return
         t = pas if ws == 0 else ws + pas - 1
-        row = scalars[t]
-        dev = self.device
-        old, new, total = (torch.tensor(float(row[k]), device=dev, dtype=torch.float32)
-                           for k in ("mix_old", "mix_new", "mix_total"))
         if self._terminal is None:
             kind = self.nodes.view(torch.uint8).reshape(-1, 16)[:, 5] & 3  # the kind_act byte of every record
             self._terminal = ((kind == 1) | (kind == 2)).to(torch.uint8).contiguous()
-        out = torch.empty_like(self._running)
-        F.mix_zero_sum_rows(self._running, self.values_avg, self.beliefs_avg, self._terminal, old, new, total, out,
-                            divide=True, mode=2 if enforce_zero_sum else 0)
-        self._running = out
+        self._mix_zero_sum(self._running, self.values_avg, self.beliefs_avg, self._terminal, t, "mix_old", "mix_new", "mix_total",
+                           self._spare_running, False, enforce_zero_sum)
+        self._running, self._spare_running = self._spare_running, self._running
 
     def _finish_running_values(self, root_beliefs, sc, iterations, flags, leaf_fn, n_leaves) -> None:
         """No final evaluation of the average policy in this mode: the final pass still runs, because the
@@ -700,11 +716,7 @@ class SteppedSolver(SubgameSolver):
             self._step(root_beliefs, sc, iterations, flags_final, iterations, iterations, 3)
         else:
             self._step(root_beliefs, sc, iterations, flags_final, iterations, iterations, 1)
-            vals = leaf_fn(self.leaf_beliefs[:n_leaves])
-            if vals.shape[-1] == NUM_HANDS:
-                self.leaf_values[:n_leaves, :, :NUM_HANDS].copy_(vals)
-            else:
-                self.leaf_values[:n_leaves].copy_(vals)
+            self._value_leaves(leaf_fn, n_leaves)
             self._step(root_beliefs, sc, iterations, flags_final, iterations, iterations, 2)
         self.exploitability = expl
         self.values_avg = running
@@ -755,11 +767,7 @@ class GraphedPass:
             sv._step(*args, 3, sample_pass=self.sample_window)
             return
         sv._step(*args, 1, sample_pass=self.sample_window)
-        vals = self.leaf_fn(sv.leaf_beliefs[:n_leaves])
-        if vals.shape[-1] == NUM_HANDS:
-            sv.leaf_values[:n_leaves, :, :NUM_HANDS].copy_(vals)
-        else:
-            sv.leaf_values[:n_leaves].copy_(vals)
+        sv._value_leaves(self.leaf_fn, n_leaves)
         sv._step(*args, 2, sample_pass=self.sample_window)
 
     def capture(self, t_capture: int) -> None:
@@ -802,7 +810,7 @@ def solve_noalloc(sv: SubgameSolver, root_beliefs: torch.Tensor, scalars_dev: to
     Calls share that work area, so do not overlap two of them on one GPU."""
     assert root_beliefs.shape == (sv.B, 2, HPAD) and root_beliefs.is_contiguous()
     p = _lib.ptr
-    with torch.cuda.device(sv.device):
+    with _lib.on(sv.device):
         _lib.call(
             "p2b_cfr_solve_noalloc", p(sv.subgames), p(sv.nodes), sv.B, sv.layout.rows, sv.layout.max_children,
             sv.layout.max_internal, p(sv.tables.blob) if sv.tables is not None else None, p(root_beliefs),
@@ -822,7 +830,7 @@ def noalloc_status(device) -> int:
 
     device = torch.device(device)
     out = ctypes.c_int32(-1)
-    with torch.cuda.device(device):
+    with _lib.on(device):
         _lib.call("p2b_cfr_noalloc_status", ctypes.byref(out), _lib.stream_ptr(device))
     return int(out.value)
 

@@ -65,3 +65,23 @@ def test_options(cuda_device, opts):
 def test_wide_batches(cuda_device, B):
     for a, b in zip(*_both(cuda_device, B, bins=(0.5, 0.75, 1.0, 1.5, 2.0), cap=1, iterations=2)[1]):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("L,W", [(1, 1344), (3, 1326), (257, 1344)])
+def test_network_per_leaf_in_place(cuda_device, L, W):
+    """The rows the feature kernel feeds a bf16 ValueMLP and the values written back, against the model called on the
+    same beliefs: the same bits, padding untouched."""
+    from poker2_b200 import leaf_eval
+
+    g = torch.Generator(device=cuda_device).manual_seed(L)
+    beliefs = torch.rand(L, 2, W, device=cuda_device, generator=g)
+    boards = torch.rand(L, 52, device=cuda_device, generator=g).argsort(dim=1)[:, :5]
+    boards[:, 3:] = -1
+    ctx = torch.rand(L, 3, device=cuda_device, generator=g)
+    model = leaf_eval.ValueMLP(64, 2, dtype=torch.bfloat16, seed=1).to(cuda_device)
+    ev = leaf_eval.DirectLeafEvaluator(model, boards, ctx, cuda_device)
+    want = model(beliefs[..., :1326].contiguous(), boards, ctx)
+    out = torch.full((L, 2, W), 7.0, device=cuda_device)
+    ev.evaluate_into(beliefs, out)
+    assert torch.equal(out[..., :1326], want) and torch.equal(ev(beliefs), want)
+    assert (out[..., 1326:] == 7.0).all()
