@@ -163,8 +163,8 @@ int64_t p2b_cfr_step_scratch_floats(int32_t max_internal, int32_t num_subgames, 
 int p2b_cfr_default_blocks(void);
 /* Which kernels run the iteration passes of a p2b_cfr_solve whose leaves are all terminal (process-wide
  * setting, no counterpart in the upstream project).  0, the default: the lean kernel, a block per subgame, from
- * 1.5 subgames per SM on (8 per SM when max_internal x max_children + 1 exceeds 160, i.e. some subgame may be too
- * large for it); below that, and for solves it does not cover, the split kernels, which spread a subgame over the
+ * two subgames per SM on unless max_internal x max_children + 1 exceeds 160, i.e. some subgame may be too
+ * large for it; else, and for solves it does not cover, the split kernels, which spread a subgame over the
  * chip (they need the scratch area of p2b_cfr_solve_scratch_floats as sized under the same setting; else the general
  * kernel runs).  1: the lean kernel whenever it applies.  Results are the same bits either way.  Returns the
  * previous setting; a negative argument only queries. */

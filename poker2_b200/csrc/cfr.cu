@@ -1573,11 +1573,10 @@ IterTiming* iter_timing_of_current_device() {
 }  // namespace
 
 // Which kernels run the iteration passes of a one-call solve whose leaves are all terminal.  0 (default): the lean
-// kernel, whose blocks keep a subgame each and so want two subgames an SM; the split kernels (cfr_split.cu), which
-// spread every subgame over the chip, for batches below 1.5 an SM, and below 8 an SM when some subgame may exceed
-// the lean kernel's node limit.  Measured, ms for 16 iterations with start and final pass, split / lean: trees of 54
-// nodes, 64 subgames 4.5 / 6.2, 192 8.6 / 9.4, 256 10.4 / 9.8, 592 21.8 / 19.4; up to 261 nodes, 64 subgames 10.7 / 40,
-// 296 25 / 49, 1184 89 / 92, 2048 152 / 151.  1: the lean kernel whenever it applies.
+// kernel, whose blocks keep a subgame each, for batches of at least two subgames an SM of which none may exceed its node
+// limit; else the split kernels (cfr_split.cu), which spread every subgame over the chip.  Measured, ms a pass, split /
+// lean: trees of 54 nodes, 64 subgames 0.18 / 0.33, 192 0.34 / 0.46, 296 0.48 / 0.48, 1184 1.89 / 1.77, 4096 6.41 / 6.08;
+// up to 261 nodes, 64 subgames 0.30 / 2.2, 592 2.0 / 2.8, 2048 6.6 / 7.6.  1: the lean kernel whenever it applies.
 static std::atomic<int> g_path_policy{0};
 
 int cfr_path_policy(int policy) {
@@ -1618,7 +1617,7 @@ static bool maybe_large(int max_internal, int max_children) { return (long long)
 
 static bool lean_preferred(int num_subgames, int max_internal, int max_children) {
     if (g_path_policy.load() != 0) return true;
-    return num_subgames >= (maybe_large(max_internal, max_children) ? 8 * sm_count() : 3 * sm_count() / 2);
+    return num_subgames >= 2 * sm_count() && !maybe_large(max_internal, max_children);
 }
 
 // Work space of a one-call solve before the hand-over rows: one set of work rows per block, or the space of the split

@@ -9,20 +9,21 @@
 //     at a node is the product of the current policies along the path, so all nodes can be worked on at once.
 //   * What couples the nodes (value backup, regrets, next policy, average policy) is elementwise in the hand.
 //
-// So a pass is split_rows_kernel, one block per internal node of the whole batch, followed by
-// split_columns_kernel, where a block owns a slice of hands of one subgame and goes up the tree level by level,
-// one warp a node.  A solve whose leaves are valued by the caller's model has the model between the two.
-// The reach rows of the other kernels do not exist here: both kernels multiply along the path (3 to 5 rows that
-// are in L2), and the old average policy of the ancestors, which the average-policy mix weights by, is still in
-// place when a node is visited bottom-up.
+// So a pass is split_rows_kernel, one block per internal node of the whole batch, followed by split_up_kernel,
+// where the warps of a block own a slice of the hands of one subgame and go up the tree level by level, a warp a node.  A solve whose leaves are valued by the caller's model has the model between the two.
+// There is no top-down sweep: the row kernel multiplies along the path (3 to 5 rows that are in L2), and does the
+// same with the average policy of the pass before, by which the average-policy mix weights.
 //
 // Arithmetic and results are those of cfr.cu, bit for bit: same operations in the same order, also in the fp64 sums.
 //
-// Measured on a B200, a pass in the general kernel / here: one subgame of 57 nodes 0.32 / 0.036 ms, 37 of 96 nodes
-// 1.15 / 0.21 ms, 192 flop subgames of 77 nodes (largest 271) 1.4 / 0.48 ms.  The row kernel takes 6.3 us an SM and
-// node with two blocks resident; shared-memory wavefronts bound it (0.68 of their peak over the whole kernel, gathers of
-// the per-card sums and of the showdown tables), with half of the issue slots used.  The column kernel is bound by the
-// latency of its row accesses at small batches and runs at 0.6 of the memory bandwidth at large ones.
+// Measured on a B200, a pass in the general kernel / here: one subgame of 57 nodes 0.32 / 0.033 ms, 37 of 96 nodes
+// 1.15 / 0.16 ms, 192 flop subgames of 77 nodes (largest 271) 1.4 / 0.39 ms.  The row kernel takes 6.3 us an SM and
+// node with two blocks resident; shared-memory wavefronts (0.65 of their peak, mostly the gathers of the per-card sums and
+// of the showdown tables) and the barriers between its phases bound it, with half of the issue slots used.  The up kernel
+// is bound by memory at large batches (2.55 ms on 4096 subgames of 54 nodes, 0.9 of the copy bandwidth over the 15 GB it
+// moves) and by the latency of a warp's walk at small ones.
+#include <atomic>
+
 #include "cfr_split.cuh"
 
 #include "cfr_dev.cuh"
@@ -63,7 +64,9 @@ enum RecRow {
     kRecSeen = 1,    // the policy as each hand of the player who does not choose sees it
     kRecWeight = 2,  // regret weights of the acting player's hands (internal nodes)
     kRecValue = 3,   // values of player 0, then of player 1 (internal nodes and showdown leaves)
-    kRecRows = 5
+    kRecReach = 5,   // the acting player's reach under the current policy and under the old average policy (internal
+    kRecOldReach = 6,  // nodes, passes that mix)
+    kRecRows = 7
 };
 constexpr int kRec = kRecRows * P2B_HPAD;  // floats from a node's record to the next
 
@@ -263,6 +266,13 @@ __device__ __forceinline__ FV<VPT> path_product(const float* base, int stride, c
     return r;
 }
 
+// The root's row of the pass becomes what the node beliefs of the next pass derive from.
+__device__ __forceinline__ void advance_root(const CfrParams& p, int s, int h) {
+    float* cr = p.carry_roots + (long long)s * 4 * P2B_HPAD + h;
+    stc<2>(cr, ldc<2>(cr + 2 * P2B_HPAD));
+    stc<2>(cr + P2B_HPAD, ldc<2>(cr + 3 * P2B_HPAD));
+}
+
 // Average-policy mix and renormalisation of K siblings (cfr_evaluator.py:1195-1258): A <- mix of A and P, weighted by
 // the acting player's reach under the old average policy (rba) and under the current one (ra).
 template <int VPT, int K>
@@ -329,187 +339,344 @@ __device__ __forceinline__ void mix_average(const IterScalars& sc, const FV<VPT>
             if (sum.v[i] > 1e-5f) A[c].v[i] = q[c].v[i];
 }
 
-enum ColumnMode {
-    kColInit = 0,  // current policy from the regrets, the root's rows moved on to the coming pass
-    kColMix = 1,   // average-policy mix alone: solves whose beliefs are taken under the updated average policy
-    kColUp = 2     // values, average-policy mix (unless kColMix has done it), regrets, the next policy
-};
+// The two elementwise passes over the nodes that need no values: the first current policy from the regrets (and the root's
+// rows moved on to the coming pass), and the average-policy mix alone, for solves whose beliefs are taken under the updated
+// average policy.  A warp takes a node for 64 hands, from the deepest level up: the old average policy of a node's ancestors
+// is still in place when it is visited.
+enum PrepMode { kPrepPolicy = 0, kPrepMix = 1 };
 
-// One node for the hands of a warp: VPT consecutive ones a thread.  The stages are ordered so that about three rows a
-// child are live at a time: values and backup, average-policy mix, regrets, next policy.
-template <int VPT, int K, int MODE>
-__device__ __forceinline__ void column_node(const CfrParams& p, const SplitWork& w, const SplitItem& it,
-                                            const NodeRecPacked* nodes, const FV<VPT>& mask, int h, int pass, int leaf0,
-                                            bool sample, bool mixed) {
-    const int a = it.to_act, j = it.node, fc = it.first_child;
-    const long long kids = (long long)(it.node_begin + fc) * P2B_HPAD + h;
-    float* rec = w.rec + (long long)(it.node_begin + fc) * kRec + h;  // of the first child
-    float* R_row = p.regrets + kids;
-    FV<VPT> P[K];
-    if (MODE == kColInit) {
+template <int K, int MODE>
+__device__ __forceinline__ void prep_node(const CfrParams& p, const SplitWork& w, const SplitItem& it, const FV<2>& mask, int h,
+                                          const IterScalars& sc) {
+    const long long kids = (long long)(it.node_begin + it.first_child) * P2B_HPAD + h;
+    float* rec = w.rec + (long long)(it.node_begin + it.first_child) * kRec + h;  // of the first child
+    FV<2> P[K];
+    if (MODE == kPrepPolicy) {
 #pragma unroll
-        for (int c = 0; c < K; ++c) P[c] = ldc<VPT>(R_row + c * P2B_HPAD);
-        regret_matching<VPT, K>(P);
+        for (int c = 0; c < K; ++c) P[c] = ldc<2>(p.regrets + kids + c * P2B_HPAD);
+        regret_matching<2, K>(P);
 #pragma unroll
-        for (int c = 0; c < K; ++c) stc<VPT>(rec + c * kRec, P[c]);
+        for (int c = 0; c < K; ++c) stc<2>(rec + c * kRec, P[c]);
         return;
     }
-    const bool update = MODE == kColUp && pass + 1 < p.iterations;
-    const IterScalars sc = p.scalars[pass];
-    const bool mix_here = MODE == kColMix || !mixed, mix = mix_here && (sc.do_mix & 1) != 0;
     float* A_row = p.policy_avg + kids;
 #pragma unroll
-    for (int c = 0; c < K; ++c) P[c] = ldc<VPT>(rec + c * kRec);
-    FV<VPT> A[K], ra, rba;
-    if (mix) {
+    for (int c = 0; c < K; ++c) P[c] = ldc<2>(rec + c * kRec);
+    if (sc.do_mix & 1) {
+        FV<2> A[K];
 #pragma unroll
-        for (int c = 0; c < K; ++c) A[c] = ldc<VPT>(A_row + c * P2B_HPAD);
-        ra = path_product<VPT>(w.rec + (long long)it.node_begin * kRec + h, kRec, it.path, it.n_path[0], mask);
-        rba = path_product<VPT>(p.policy_avg + (long long)it.node_begin * P2B_HPAD + h, P2B_HPAD, it.path, it.n_path[0], mask);
-    }
-    FV<VPT> Va[K], acc_a, wgt;
-    const bool tracked = update && p.weight_sums != nullptr;
-    float* W_row = p.weight_sums + kids;
-    if (MODE == kColUp) {
-        // value backup (:1095-1115)
-        FV<VPT> acc_o;
+        for (int c = 0; c < K; ++c) A[c] = ldc<2>(A_row + c * P2B_HPAD);
+        const FV<2> ra = path_product<2>(w.rec + (long long)it.node_begin * kRec + h, kRec, it.path, it.n_path[0], mask);
+        const FV<2> rba = path_product<2>(p.policy_avg + (long long)it.node_begin * P2B_HPAD + h, P2B_HPAD, it.path,
+                                          it.n_path[0], mask);
+        mix_average<2, K>(sc, ra, rba, P, A);
 #pragma unroll
-        for (int i = 0; i < VPT; ++i) acc_a.v[i] = acc_o.v[i] = 0.0f;
-        const int va_off = (kRecValue + a) * P2B_HPAD, vo_off = (kRecValue + 1 - a) * P2B_HPAD;
-        float* me = w.rec + (long long)(it.node_begin + j) * kRec + h;
-        if (update) wgt = ldc<VPT>(me + kRecWeight * P2B_HPAD);
-        FV<VPT> Q[K], Vo[K];
+        for (int c = 0; c < K; ++c) stc<2>(A_row + c * P2B_HPAD, A[c]);
+    } else {
 #pragma unroll
-        for (int c = 0; c < K; ++c) {
-            Q[c] = ldc<VPT>(rec + c * kRec + kRecSeen * P2B_HPAD);
-            const int kind = it.kind[c];
-            const float *va = rec + c * kRec + va_off, *vo = rec + c * kRec + vo_off;
-            if (kind == kModelLeaf && p.leaf_values) {
-                const float* v = p.leaf_values + (long long)(leaf0 + nodes[fc + c].internal_idx) * 2 * P2B_HPAD + h;
-                va = v + a * P2B_HPAD;
-                vo = v + (1 - a) * P2B_HPAD;
-            }
-            if (kind == kFoldLeaf || (kind == kModelLeaf && !p.leaf_values)) {
-                const float v0 = kind == kFoldLeaf ? nodes[fc + c].v0 : 0.0f, f = a == 0 ? v0 : -v0;
-#pragma unroll
-                for (int i = 0; i < VPT; ++i) {
-                    Va[c].v[i] = f;
-                    Vo[c].v[i] = -f;
-                }
-            } else {
-                Va[c] = ldc<VPT>(va);
-                Vo[c] = ldc<VPT>(vo);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < K; ++c)
-#pragma unroll
-            for (int i = 0; i < VPT; ++i) {
-                acc_a.v[i] = __fadd_rn(acc_a.v[i], __fmul_rn(Va[c].v[i], P[c].v[i]));
-                acc_o.v[i] = __fadd_rn(acc_o.v[i], __fmul_rn(Vo[c].v[i], Q[c].v[i]));
-            }
-        if (j != 0) {
-            stc<VPT>(me + va_off, acc_a);
-            stc<VPT>(me + vo_off, acc_o);
-        }
-        if (p.iter_values && p.values_avg) {  // the values of this iteration at the node and at the leaves below it
-            float* out = p.values_avg + (long long)it.node_begin * 2 * P2B_HPAD + h;
-            stc<VPT>(out + (2 * j + a) * P2B_HPAD, acc_a);
-            stc<VPT>(out + (2 * j + 1 - a) * P2B_HPAD, acc_o);
-#pragma unroll
-            for (int c = 0; c < K; ++c)
-                if (it.kind[c] != kInternal) {
-                    stc<VPT>(out + (2 * (fc + c) + a) * P2B_HPAD, Va[c]);
-                    stc<VPT>(out + (2 * (fc + c) + 1 - a) * P2B_HPAD, Vo[c]);
-                }
-        }
-        if (p.policy && pass == p.iterations - 1) {
-#pragma unroll
-            for (int c = 0; c < K; ++c) stc<VPT>(p.policy + kids + c * P2B_HPAD, P[c]);
-        }
-        if (sample) {
-#pragma unroll
-            for (int c = 0; c < K; ++c) stc<VPT>(p.policy_sample + kids + c * P2B_HPAD, P[c]);
-        }
-    }
-    if (mix_here) {
-        if (mix) {
-            mix_average<VPT, K>(sc, ra, rba, P, A);
-#pragma unroll
-            for (int c = 0; c < K; ++c) stc<VPT>(A_row + c * P2B_HPAD, A[c]);
-        } else {
-#pragma unroll
-            for (int c = 0; c < K; ++c) stc<VPT>(A_row + c * P2B_HPAD, P[c]);
-        }
-    }
-    if (update) {
-        // instantaneous regrets of this pass folded into the discounted update of the next (:1117-1165, :1346-1368)
-        const IterScalars sn = p.scalars[pass + 1];
-        const Divisor d_pos = make_divisor(sn.den_pos), d_neg = make_divisor(sn.den_neg);
-        const bool no_regret = ((sn.do_mix >> 1) & 3) == a + 1;  // linear CFR: this player's actions get none
-        FV<VPT> R[K], W[K];
-#pragma unroll
-        for (int c = 0; c < K; ++c) R[c] = ldc<VPT>(R_row + c * P2B_HPAD);
-        if (tracked) {
-#pragma unroll
-            for (int c = 0; c < K; ++c) W[c] = ldc<VPT>(W_row + c * P2B_HPAD);
-        }
-#pragma unroll
-        for (int c = 0; c < K; ++c) {
-            DivGuard g = guard_begin(d_pos.ok && d_neg.ok);
-            FV<VPT> rn, rq, wn, wq, dy;
-#pragma unroll
-            for (int i = 0; i < VPT; ++i) {
-                const bool pos = R[c].v[i] > 0.0f;
-                const float num = pos ? sn.num_pos : sn.num_neg, dr = pos ? d_pos.r : d_neg.r;
-                dy.v[i] = pos ? d_pos.y : d_neg.y;
-                rn.v[i] = __fmul_rn(R[c].v[i], num);
-                rq.v[i] = div_g<false>(rn.v[i], dy.v[i], dr, g);
-                if (tracked) {
-                    wn.v[i] = __fmul_rn(W[c].v[i], num);
-                    wq.v[i] = div_g<true>(wn.v[i], dy.v[i], dr, g);
-                }
-            }
-            if (__builtin_expect(guard_bad(g), 0)) {
-#pragma unroll
-                for (int i = 0; i < VPT; ++i) {
-                    rq.v[i] = __fdiv_rn(rn.v[i], dy.v[i]);
-                    if (tracked) wq.v[i] = __fdiv_rn(wn.v[i], dy.v[i]);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < VPT; ++i) {
-                const float reg = no_regret ? 0.0f : __fmul_rn(wgt.v[i], __fsub_rn(Va[c].v[i], acc_a.v[i]));
-                float rr = __fadd_rn(rq.v[i], reg);
-                if (p.cfr_plus) rr = fmaxf(rr, 0.0f);
-                R[c].v[i] = rr;
-                if (tracked) W[c].v[i] = __fadd_rn(wq.v[i], 1.0f);
-            }
-            stc<VPT>(R_row + c * P2B_HPAD, R[c]);
-            if (tracked) stc<VPT>(W_row + c * P2B_HPAD, W[c]);
-        }
-        regret_matching<VPT, K>(R);
-#pragma unroll
-        for (int c = 0; c < K; ++c) stc<VPT>(rec + c * kRec, R[c]);
+        for (int c = 0; c < K; ++c) stc<2>(A_row + c * P2B_HPAD, P[c]);
     }
 }
 
-// A block holds `slices` slices of 32 VPT hands of one subgame with `lanes` warps each, which take the nodes of a level
-// in turn; a level is complete when they meet at the slice's barrier.
-template <int VPT, int MAXK, int MODE>
-__global__ void __launch_bounds__(256, 3) split_columns_kernel(const CfrParams p, const SplitWork w, int pass, bool advance,
-                                                               bool mixed, int lanes, int slices) {
-    constexpr int kSlices = P2B_HPAD / (32 * VPT);
+constexpr int kPrepWarps = 4;
+template <int MAXK, int MODE>
+__global__ void __launch_bounds__(32 * kPrepWarps) split_prep_kernel(const CfrParams p, const SplitWork w, int pass) {
+    constexpr int kSlices = P2B_HPAD / 64;
+    if (p.work_counter[1] != 0) return;
+    const int q = blockIdx.x / kSlices, warp = threadIdx.x >> 5;
+    const int h = (blockIdx.x - q * kSlices) * 64 + (threadIdx.x & 31) * 2;
+    const int s = p.queue_order ? p.queue_order[q] : q;
+    const SubgameRec sg = p.subgames[s];
+    const SplitLevels* lv = w.levels + q;
+    const SplitItem* items = w.items + lv->item_begin;
+    FV<2> mask;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const bool real = h + i < P2B_NUM_HANDS;
+        const int hc = real ? h + i : P2B_NUM_HANDS - 1;
+        const bool blocked = (((sg.board_mask >> p.combos->c1[hc]) | (sg.board_mask >> p.combos->c2[hc])) & 1ull) != 0;
+        mask.v[i] = real && !blocked ? 1.0f : 0.0f;
+    }
+    const IterScalars sc = p.scalars[pass];
+    for (int d = lv->n_levels - 1; d >= 0; --d) {
+        for (int x = lv->begin[d] + warp; x < lv->begin[d + 1]; x += kPrepWarps) {
+            const SplitItem& it = items[x];
+            with_children<MAXK>(it.n_children, [&](auto kc) { prep_node<decltype(kc)::value, MODE>(p, w, it, mask, h, sc); });
+        }
+        if (MODE == kPrepMix) __syncthreads();
+    }
+    if (MODE == kPrepPolicy && warp == 0) advance_root(p, s, h);
+}
+
+// ---- columns --------------------------------------------------------------------------------------
+// The bottom-up half of a pass: value backup (cfr_evaluator.py:1095-1115), average-policy mix and renormalisation
+// (:1195-1258), instantaneous regrets (:1117-1165) folded into the discounted update of the next pass (:1346-1368) and
+// the policy that follows from it (:1168-1185), all elementwise in the hand.
+//
+// A warp owns a slice of 64 hands and takes one node at a time.  A node's rows (7 a child, 256 bytes each for the slice) are
+// copied into the warp's part of shared memory while the warp works on the node before, so that neither the child loops have
+// to be unrolled to have loads in flight nor a register is spent on a row that waits: with the loads in registers and a body
+// per child count the kernel ran at 20 warps an SM, half of their stalls on loads and a fifth on instruction fetches.
+constexpr int kUpThreads = 256;  // at most
+enum UpSlot { kUpPolicy = 0, kUpSeen = 1, kUpRegret = 2, kUpSum = 3, kUpAverage = 4, kUpValueA = 5, kUpValueO = 6, kUpSlots = 7 };
+constexpr int kUpNodeRows = 3;  // behind the children's rows: regret weights, reach, old average reach
+constexpr int kUpRow = 64;      // floats
+__host__ __device__ constexpr int up_rows(int children) { return kUpSlots * children + kUpNodeRows; }
+
+__device__ __forceinline__ void async_pair(float* shared, const float* global) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(shared)), "l"(global) : "memory");
+}
+
+// The kernels of consecutive passes follow one another without a gap: each lets the next one be scheduled as soon as its own
+// blocks run (launch_next), and the next one reads what no pass changes (work lists, records, board tables) before it
+// waits for this one's results (previous_done).
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void previous_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+struct UpPass {  // what a pass does, uniform over the grid
+    bool update, tracked, mix, mixed, keep_values, keep_policy, sample;
+    IterScalars sc, sn;
+    Divisor d_pos, d_neg;
+};
+
+// Starts the copies of a node's rows, except the values of its internal children, which may not be there yet.
+__device__ __forceinline__ void up_stage(const CfrParams& p, const SplitWork& w, const UpPass& u, const SplitItem& it,
+                                         const NodeRecPacked* nodes, int h, int leaf0, float* at) {
+    const int k = it.n_children, a = it.to_act;
+    const long long row = it.node_begin + it.first_child;
+    const float* rec = w.rec + row * kRec + h;
+    const long long kids = row * P2B_HPAD + h;
+    const float *R = p.regrets + kids, *W = p.weight_sums + kids, *A = p.policy_avg + kids;
+    float* d = at;
+#pragma unroll 1
+    for (int c = 0; c < k; ++c) {
+        async_pair(d + kUpPolicy * kUpRow, rec + kRecPolicy * P2B_HPAD);
+        async_pair(d + kUpSeen * kUpRow, rec + kRecSeen * P2B_HPAD);
+        if (u.update) async_pair(d + kUpRegret * kUpRow, R);
+        if (u.tracked) async_pair(d + kUpSum * kUpRow, W);
+        if (u.mix) async_pair(d + kUpAverage * kUpRow, A);
+        const int kind = it.kind[c];
+        if (kind == kShowdownLeaf || (kind == kModelLeaf && p.leaf_values)) {
+            const float* v = kind == kShowdownLeaf
+                                 ? rec + kRecValue * P2B_HPAD
+                                 : p.leaf_values + (long long)(leaf0 + nodes[it.first_child + c].internal_idx) * 2 * P2B_HPAD + h;
+            async_pair(d + kUpValueA * kUpRow, v + a * P2B_HPAD);
+            async_pair(d + kUpValueO * kUpRow, v + (1 - a) * P2B_HPAD);
+        } else if (kind != kInternal) {
+            const float v0 = kind == kFoldLeaf ? nodes[it.first_child + c].v0 : 0.0f, f = a == 0 ? v0 : -v0;
+            *reinterpret_cast<float2*>(d + kUpValueA * kUpRow) = make_float2(f, f);
+            *reinterpret_cast<float2*>(d + kUpValueO * kUpRow) = make_float2(-f, -f);
+        }
+        d += kUpSlots * kUpRow;
+        rec += kRec;
+        R += P2B_HPAD;
+        W += P2B_HPAD;
+        A += P2B_HPAD;
+    }
+    const float* me = w.rec + (long long)(it.node_begin + it.node) * kRec + h;
+    if (u.update) async_pair(d, me + kRecWeight * P2B_HPAD);
+    if (u.mix) {
+        async_pair(d + kUpRow, me + kRecReach * P2B_HPAD);
+        async_pair(d + 2 * kUpRow, me + kRecOldReach * P2B_HPAD);
+    }
+}
+
+__device__ __forceinline__ void up_stage_values(const SplitWork& w, const SplitItem& it, int h, float* at) {
+    const float* v = w.rec + (long long)(it.node_begin + it.first_child) * kRec + kRecValue * P2B_HPAD + h;
+#pragma unroll 1
+    for (int c = 0; c < it.n_children; ++c) {
+        if (it.kind[c] == kInternal) {
+            async_pair(at + (kUpSlots * c + kUpValueA) * kUpRow, v + c * kRec + it.to_act * P2B_HPAD);
+            async_pair(at + (kUpSlots * c + kUpValueO) * kUpRow, v + c * kRec + (1 - it.to_act) * P2B_HPAD);
+        }
+    }
+}
+
+__device__ __forceinline__ void up_node(const CfrParams& p, const SplitWork& w, const UpPass& u, const SplitItem& it, int h,
+                                        float* at) {
+    const int k = it.n_children, a = it.to_act, j = it.node, fc = it.first_child;
+    const long long kids = (long long)(it.node_begin + fc) * P2B_HPAD + h;
+    const float* node_rows = at + k * kUpSlots * kUpRow;
+    auto slot = [&](int c, int which) { return at + (kUpSlots * c + which) * kUpRow; };
+    FV<2> acc_a, acc_o;
+    acc_a.v[0] = acc_a.v[1] = acc_o.v[0] = acc_o.v[1] = 0.0f;
+#pragma unroll 2
+    for (int c = 0; c < k; ++c) {
+        const FV<2> P = ldc<2>(slot(c, kUpPolicy)), Q = ldc<2>(slot(c, kUpSeen));
+        const FV<2> Va = ldc<2>(slot(c, kUpValueA)), Vo = ldc<2>(slot(c, kUpValueO));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            acc_a.v[i] = __fadd_rn(acc_a.v[i], __fmul_rn(Va.v[i], P.v[i]));
+            acc_o.v[i] = __fadd_rn(acc_o.v[i], __fmul_rn(Vo.v[i], Q.v[i]));
+        }
+    }
+    if (j != 0) {
+        float* v = w.rec + (long long)(it.node_begin + j) * kRec + kRecValue * P2B_HPAD + h;
+        stc<2>(v + a * P2B_HPAD, acc_a);
+        stc<2>(v + (1 - a) * P2B_HPAD, acc_o);
+    }
+    if (u.keep_values) {  // the values of this iteration at the node and at the leaves below it
+        float* out = p.values_avg + (long long)it.node_begin * 2 * P2B_HPAD + h;
+        stc<2>(out + (2 * j + a) * P2B_HPAD, acc_a);
+        stc<2>(out + (2 * j + 1 - a) * P2B_HPAD, acc_o);
+#pragma unroll 1
+        for (int c = 0; c < k; ++c)
+            if (it.kind[c] != kInternal) {
+                stc<2>(out + (2 * (fc + c) + a) * P2B_HPAD, ldc<2>(slot(c, kUpValueA)));
+                stc<2>(out + (2 * (fc + c) + 1 - a) * P2B_HPAD, ldc<2>(slot(c, kUpValueO)));
+            }
+    }
+    if (u.keep_policy || u.sample) {
+#pragma unroll 1
+        for (int c = 0; c < k; ++c) {
+            const FV<2> P = ldc<2>(slot(c, kUpPolicy));
+            if (u.keep_policy) stc<2>(p.policy + kids + c * P2B_HPAD, P);
+            if (u.sample) stc<2>(p.policy_sample + kids + c * P2B_HPAD, P);
+        }
+    }
+    float* A_row = p.policy_avg + kids;
+    if (u.mix) {
+        const FV<2> ra = ldc<2>(node_rows + kUpRow), rba = ldc<2>(node_rows + 2 * kUpRow);
+        FV<2> ro, rn, sum;
+        Divisor d[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            ro.v[i] = __fmul_rn(rba.v[i], u.sc.mix_old);
+            rn.v[i] = __fmul_rn(ra.v[i], u.sc.mix_new);
+            const float den = __fadd_rn(ro.v[i], rn.v[i]);
+            const bool weighted = den > 1e-5f;  // else: (numerically) no reach, the plain iteration weights (:1231-1239)
+            ro.v[i] = weighted ? ro.v[i] : u.sc.mix_old;
+            rn.v[i] = weighted ? rn.v[i] : u.sc.mix_new;
+            d[i] = make_divisor(weighted ? den : u.sc.mix_total);
+            sum.v[i] = 0.0f;
+        }
+#pragma unroll 2
+        for (int c = 0; c < k; ++c) {
+            const FV<2> P = ldc<2>(slot(c, kUpPolicy)), A = ldc<2>(slot(c, kUpAverage));
+            DivGuard g = guard_begin(d[0].ok && d[1].ok);
+            FV<2> num, q;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                num.v[i] = __fadd_rn(__fmul_rn(ro.v[i], A.v[i]), __fmul_rn(rn.v[i], P.v[i]));
+                q.v[i] = div_g<true>(num.v[i], d[i].y, d[i].r, g);
+            }
+            if (__builtin_expect(guard_bad(g), 0)) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) q.v[i] = __fdiv_rn(num.v[i], d[i].y);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) sum.v[i] = __fadd_rn(sum.v[i], q.v[i]);
+            stc<2>(slot(c, kUpAverage), q);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) d[i] = make_divisor(sum.v[i]);
+#pragma unroll 2
+        for (int c = 0; c < k; ++c) {
+            FV<2> x = ldc<2>(slot(c, kUpAverage)), q;
+            DivGuard g = guard_begin(d[0].ok && d[1].ok);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) q.v[i] = div_g<true>(x.v[i], d[i].y, d[i].r, g);
+            if (__builtin_expect(guard_bad(g), 0)) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) q.v[i] = __fdiv_rn(x.v[i], sum.v[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (sum.v[i] > 1e-5f) x.v[i] = q.v[i];
+            stc<2>(A_row + c * P2B_HPAD, x);
+        }
+    } else if (!u.mixed) {
+#pragma unroll 1
+        for (int c = 0; c < k; ++c) stc<2>(A_row + c * P2B_HPAD, ldc<2>(slot(c, kUpPolicy)));
+    }
+    if (!u.update) return;
+    const FV<2> wgt = ldc<2>(node_rows);
+    const bool no_regret = ((u.sn.do_mix >> 1) & 3) == a + 1;  // linear CFR: this player's actions get none
+    FV<2> sum;
+    sum.v[0] = sum.v[1] = 0.0f;
+#pragma unroll 2
+    for (int c = 0; c < k; ++c) {
+        FV<2> R = ldc<2>(slot(c, kUpRegret)), W;
+        const FV<2> Va = ldc<2>(slot(c, kUpValueA));
+        W = R;
+        if (u.tracked) W = ldc<2>(slot(c, kUpSum));
+        DivGuard g = guard_begin(u.d_pos.ok && u.d_neg.ok);
+        FV<2> rn, rq, wn, wq, dy;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const bool pos = R.v[i] > 0.0f;
+            const float num = pos ? u.sn.num_pos : u.sn.num_neg, dr = pos ? u.d_pos.r : u.d_neg.r;
+            dy.v[i] = pos ? u.d_pos.y : u.d_neg.y;
+            rn.v[i] = __fmul_rn(R.v[i], num);
+            rq.v[i] = div_g<false>(rn.v[i], dy.v[i], dr, g);
+            if (u.tracked) {
+                wn.v[i] = __fmul_rn(W.v[i], num);
+                wq.v[i] = div_g<true>(wn.v[i], dy.v[i], dr, g);
+            }
+        }
+        if (__builtin_expect(guard_bad(g), 0)) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                rq.v[i] = __fdiv_rn(rn.v[i], dy.v[i]);
+                if (u.tracked) wq.v[i] = __fdiv_rn(wn.v[i], dy.v[i]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float reg = no_regret ? 0.0f : __fmul_rn(wgt.v[i], __fsub_rn(Va.v[i], acc_a.v[i]));
+            float rr = __fadd_rn(rq.v[i], reg);
+            if (p.cfr_plus) rr = fmaxf(rr, 0.0f);
+            R.v[i] = rr;
+            if (u.tracked) W.v[i] = __fadd_rn(wq.v[i], 1.0f);
+        }
+        stc<2>(p.regrets + kids + c * P2B_HPAD, R);
+        if (u.tracked) stc<2>(p.weight_sums + kids + c * P2B_HPAD, W);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            R.v[i] = fmaxf(R.v[i], 0.0f);
+            sum.v[i] = __fadd_rn(sum.v[i], R.v[i]);
+        }
+        stc<2>(slot(c, kUpRegret), R);
+    }
+    const float invk = __fdiv_rn(1.0f, (float)k);
+    Divisor d[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) d[i] = make_divisor(fmaxf(sum.v[i], 1e-8f));
+    float* P_row = w.rec + (long long)(it.node_begin + fc) * kRec + h;
+#pragma unroll 2
+    for (int c = 0; c < k; ++c) {
+        const FV<2> x = ldc<2>(slot(c, kUpRegret));
+        DivGuard g = guard_begin(d[0].ok && d[1].ok);
+        FV<2> q;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) q.v[i] = div_g<true>(x.v[i], d[i].y, d[i].r, g);
+        if (__builtin_expect(guard_bad(g), 0)) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) q.v[i] = __fdiv_rn(x.v[i], d[i].y);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) q.v[i] = sum.v[i] > 1e-8f ? q.v[i] : invk;
+        stc<2>(P_row + c * kRec, q);
+    }
+}
+
+// A block holds `slices` slices of one subgame with `lanes` warps each, which take the nodes of a level in turn; a level is
+// complete when the warps of a slice meet at its barrier.  `ring`: rows of a warp's staging area; two nodes that follow one
+// another lie at its two ends if they fit together, else the second is copied once the first is done.
+__global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p, const SplitWork w, int pass, bool advance,
+                                                              bool mixed, int lanes, int slices, int ring) {
+    constexpr int kSlices = P2B_HPAD / kUpRow;
     extern __shared__ __align__(16) unsigned char smem[];
     if (p.work_counter[1] != 0) return;
     const int per_subgame = kSlices / slices;
     const int q = blockIdx.x / per_subgame;
     const int s = p.queue_order ? p.queue_order[q] : q;
-    const int tid = threadIdx.x, warp = tid >> 5, mine = warp / lanes, lane_warp = warp - mine * lanes;
-    const int h = ((blockIdx.x - q * per_subgame) * slices + mine) * 32 * VPT + (tid & 31) * VPT;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mine = warp / lanes, lane_warp = warp - mine * lanes;
+    const int h = ((blockIdx.x - q * per_subgame) * slices + mine) * kUpRow + lane * 2;
     const SubgameRec sg = p.subgames[s];
-    SplitItem* items = reinterpret_cast<SplitItem*>(smem);
-    NodeRecPacked* nodes = reinterpret_cast<NodeRecPacked*>(smem + sg.n_internal * sizeof(SplitItem));
+    float* stage = reinterpret_cast<float*>(smem) + (long long)warp * ring * kUpRow + lane * 2;
+    SplitItem* items = reinterpret_cast<SplitItem*>(smem + (size_t)lanes * slices * ring * kUpRow * 4);
+    NodeRecPacked* nodes = reinterpret_cast<NodeRecPacked*>(items + sg.n_internal);
     const SplitLevels* lv = w.levels + q;
     {
         const uint4* ns = reinterpret_cast<const uint4*>(p.nodes + sg.node_begin);
@@ -517,35 +684,56 @@ __global__ void __launch_bounds__(256, 3) split_columns_kernel(const CfrParams p
         const uint4* is = reinterpret_cast<const uint4*>(w.items + lv->item_begin);
         for (int i = tid; i < sg.n_internal * 4; i += blockDim.x) reinterpret_cast<uint4*>(items)[i] = is[i];
     }
-    FV<VPT> mask;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-        const bool real = h + i < P2B_NUM_HANDS;
-        const int hc = real ? h + i : P2B_NUM_HANDS - 1;
-        const bool blocked = (((sg.board_mask >> p.combos->c1[hc]) | (sg.board_mask >> p.combos->c2[hc])) & 1ull) != 0;
-        mask.v[i] = real && !blocked ? 1.0f : 0.0f;
-    }
+    UpPass u;
+    u.sc = p.scalars[pass];
+    u.update = pass + 1 < p.iterations;
+    u.sn = p.scalars[u.update ? pass + 1 : pass];
+    u.tracked = u.update && p.weight_sums != nullptr;
+    u.mixed = mixed;
+    u.mix = !mixed && (u.sc.do_mix & 1) != 0;
+    u.keep_values = p.iter_values && p.values_avg != nullptr;
+    u.keep_policy = p.policy != nullptr && pass == p.iterations - 1;
+    u.sample = p.policy_sample != nullptr && p.sample_pass[s] == pass;
+    u.d_pos = make_divisor(u.sn.den_pos);
+    u.d_neg = make_divisor(u.sn.den_neg);
     const int leaf0 = p.leaf_begin ? p.leaf_begin[s] : 0;
-    const bool sample = p.policy_sample && p.sample_pass[s] == pass;
     __syncthreads();
+    launch_next();
+    previous_done();
+
     // one warp a slice: straight up the tree, no barrier
     const bool alone = lanes == 1;
-    for (int d = alone ? 0 : lv->n_levels - 1; d >= 0; --d) {
-        const int begin = alone ? 0 : lv->begin[d], end = alone ? sg.n_internal : lv->begin[d + 1];
-        for (int x = end - 1 - lane_warp; x >= begin; x -= lanes) {
-            const SplitItem& it = items[x];
-            with_children<MAXK>(it.n_children, [&](auto kc) {
-                column_node<VPT, decltype(kc)::value, MODE>(p, w, it, nodes, mask, h, pass, leaf0, sample, mixed);
-            });
-        }
-        if (!alone) asm volatile("bar.sync %0, %1;" ::"r"(mine + 1), "r"(32 * lanes) : "memory");
+    const int n_levels = alone ? 1 : lv->n_levels;
+    auto begin_of = [&](int d) { return alone ? 0 : (int)lv->begin[d]; };
+    auto first_of = [&](int d) { return (alone ? sg.n_internal : (int)lv->begin[d + 1]) - 1 - lane_warp; };
+    int d = n_levels - 1, level = d;
+    int x = first_of(d);
+    while (d > 0 && x < begin_of(d)) x = first_of(--d);
+    bool any = x >= begin_of(d), top = false;
+    if (any) up_stage(p, w, u, items[x], nodes, h, leaf0, stage);
+    while (any) {
+        for (; level > d; --level) asm volatile("bar.sync %0, %1;" ::"r"(mine + 1), "r"(32 * lanes) : "memory");
+        const SplitItem& it = items[x];
+        const int rows = up_rows(it.n_children);
+        float* at = stage + (top ? (ring - rows) * kUpRow : 0);
+        up_stage_values(w, it, h, at);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        int nx = x - lanes, nd = d;
+        while (nd > 0 && nx < begin_of(nd)) nx = first_of(--nd);
+        const bool more = nx >= begin_of(nd);
+        const int next_rows = more ? up_rows(items[nx].n_children) : 0;
+        float* next_at = stage + (top ? 0 : (ring - next_rows) * kUpRow);
+        const bool ahead = rows + next_rows <= ring;
+        if (more && ahead) up_stage(p, w, u, items[nx], nodes, h, leaf0, next_at);
+        up_node(p, w, u, it, h, at);
+        if (more && !ahead) up_stage(p, w, u, items[nx], nodes, h, leaf0, next_at);
+        x = nx;
+        d = nd;
+        any = more;
+        top = !top;
     }
-    // the root's row of the pass becomes what the node beliefs of the next pass derive from
-    if (advance && lane_warp == 0) {
-        float* cr = p.carry_roots + (long long)s * 4 * P2B_HPAD + h;
-        stc<VPT>(cr, ldc<VPT>(cr + 2 * P2B_HPAD));
-        stc<VPT>(cr + P2B_HPAD, ldc<VPT>(cr + 3 * P2B_HPAD));
-    }
+    for (; level > 0; --level) asm volatile("bar.sync %0, %1;" ::"r"(mine + 1), "r"(32 * lanes) : "memory");
+    if (advance && lane_warp == 0) advance_root(p, s, h);
 }
 
 // ---- rows ---------------------------------------------------------------------------------------
@@ -665,7 +853,7 @@ __device__ __forceinline__ void card_sums(const float* rows, int n_cs, double* c
             if (live && q == 0) cs[r * 52 + c] = ((t0 + t1) + t2) + t3;
         }
     }
-    // total mass of a row, a warp each (the 18 padding entries are zero)
+    // total mass of a row, a warp each from the last one down (the 18 padding entries are zero)
     for (int r = kRowThreads / 32 - 1 - warp; r < n_cs; r += kRowThreads / 32) {
         const float* __restrict__ x = rows + r * P2B_HPAD;
         double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -682,19 +870,18 @@ __device__ __forceinline__ void card_sums(const float* rows, int n_cs, double* c
     }
 }
 
-// Tables of the showdown formula for the row x of slot 0 (the other player's beliefs) and of slot 1 (the leaf row);
-// `slots` = 3 builds both, 2 only slot 1's.
-__device__ __forceinline__ void showdown_tables(const BoardTabView& tv, const float* x0, const float* x1, int slots,
-                                                float* pref_out, float* pc_out, float* tot_out, double* scan) {
+// Tables of the showdown formula for two ranges (x: the other player's beliefs x0, y: the leaf row x1), their entries side by
+// side, so that one gather of a hand's position serves both.  Of each range, four warps scan a quarter of the strength
+// order each (a quarter's offset is the sum of the earlier ones, which they hand one another) and 208 threads take a
+// quarter of a card's list each.
+__device__ __forceinline__ void showdown_tables(const BoardTabView& tv, const float* x0, const float* x1, float2* pref2, float2* pc2,
+                                                float2* tot2, double* scan) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint16_t* __restrict__ sorted = tv.sorted;
-    if (warp < 8 && ((slots >> (warp & 1)) & 1)) {
-        // quarter scan: prefix of 352 sorted positions; the offset is the sum of the earlier quarters, which the four
-        // warps of a slot hand one another
-        const int slot = warp & 1, qi = 3 - (warp >> 1);
+    if (warp < 8) {
+        const uint16_t* __restrict__ sorted = tv.sorted;
+        const int slot = warp & 1, qi = 3 - (warp >> 1), k0 = qi * kScanQuarter + 11 * lane;
         const float* __restrict__ x = slot ? x1 : x0;
-        float* __restrict__ pref = pref_out + slot * P2B_HPAD;
-        const int k0 = qi * kScanQuarter + 11 * lane;
+        float* __restrict__ pref = reinterpret_cast<float*>(pref2) + slot;
         float v[11];
 #pragma unroll
         for (int i = 0; i < 11; ++i) v[i] = (k0 + i < P2B_NUM_HANDS) ? x[sorted[k0 + i]] : 0.0f;
@@ -722,14 +909,13 @@ __device__ __forceinline__ void showdown_tables(const BoardTabView& tv, const fl
 #pragma unroll
         for (int i = 0; i < 11; ++i) {
             run += (double)v[i];
-            if (k0 + i < P2B_NUM_HANDS) pref[k0 + i + 1] = (float)run;
+            if (k0 + i < P2B_NUM_HANDS) pref[2 * (k0 + i + 1)] = (float)run;
         }
     }
-    // per-card prefix sums: a quarter list a thread, slot 1 from the last 208 threads of the block down
+    // the lists: the second range from the last 208 threads of the block down
     const int back = kRowThreads - 1 - tid;
     if (back < 416) {
         const int slot = back < 208 ? 1 : 0, u = 207 - (back - (slot ? 0 : 208)), c = u >> 2, q = u & 3;
-        const bool live = ((slots >> slot) & 1) != 0;
         const float* __restrict__ x = slot ? x1 : x0;
         const uint16_t* __restrict__ at = tv.cardlist + 13 * q * 52 + c;
         float v[13];
@@ -746,67 +932,74 @@ __device__ __forceinline__ void showdown_tables(const BoardTabView& tv, const fl
         const int g = lane & ~3;
         const double t0 = __shfl_sync(0xffffffffu, mine, g), t1 = __shfl_sync(0xffffffffu, mine, g + 1);
         const double t2 = __shfl_sync(0xffffffffu, mine, g + 2);
-        if (live) {
-            double acc = q == 0 ? 0.0 : (q == 1 ? t0 : (q == 2 ? t0 + t1 : (t0 + t1) + t2));
-            float* __restrict__ row = pc_out + slot * 52 * 52 + c * 52;
-            if (q == 0) row[0] = 0.0f;
-            float* __restrict__ out = row + 13 * q + 1;
+        double acc = q == 0 ? 0.0 : (q == 1 ? t0 : (q == 2 ? t0 + t1 : (t0 + t1) + t2));
+        float* __restrict__ row = reinterpret_cast<float*>(pc2) + 2 * c * 52 + slot;
+        if (q == 0) row[0] = 0.0f;
+        float* __restrict__ out = row + 2 * (13 * q + 1);
 #pragma unroll
-            for (int i = 0; i < 12; ++i) {
-                acc += (double)v[i];
-                out[i] = (float)acc;
-            }
-            if (q < 3) out[12] = (float)(acc + (double)v[12]);
-            else tot_out[slot * 64 + c] = (float)acc;  // == row[51]
+        for (int i = 0; i < 12; ++i) {
+            acc += (double)v[i];
+            out[2 * i] = (float)acc;
         }
+        if (q < 3) out[24] = (float)(acc + (double)v[12]);
+        else reinterpret_cast<float*>(tot2)[2 * c + slot] = (float)acc;  // == row[51]
     }
 }
 
-// Showdown EV (before the pot scaling) of this thread's hands: ev0 (if BOTH) against the range x0 with the tables of
-// slot 0, ev1 against x1 with those of slot 1.  The formula of showdown_hand_ev; a hand's positions in the tables are
-// unpacked once for both.
-template <bool BOTH>
-__device__ __forceinline__ void showdown_rows(const BoardTabView& tv, const float* x0, const float* x1, const float* pref,
-                                              const float* pc, const float* tot, const Hands& hi, Row3& ev0, Row3& ev1) {
+// Showdown EV (before the pot scaling) of this thread's hands against the two ranges: the formula of showdown_hand_ev, a
+// hand's positions in the tables unpacked once for both.
+__device__ __forceinline__ void showdown_rows(const BoardTabView& tv, const float* x0, const float* x1, const float2* pref,
+                                              const float2* pc, const float2* tot, const Hands& hi, Row3& ev0, Row3& ev1) {
     const int tid = threadIdx.x;
     DivGuard g = guard_begin(true);
+    auto one = [&](float PL, float PR, float C1, float D1, float C2, float D2, float T1, float T2, float xh, bool allowed) {
+        const float win = __fsub_rn(__fsub_rn(PL, C1), C2);
+        const float tie = __fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(PR, PL), __fsub_rn(D1, C1)), __fsub_rn(D2, C2)), xh);
+        const float den = fmaxf(__fadd_rn(__fsub_rn(__fsub_rn(1.0f, T1), T2), xh), 1e-8f);
+        const Divisor d = make_divisor(den);
+        g.dok = g.dok && d.ok;
+        const float wp = div_g<false>(win, d.y, d.r, g), tp = div_g<false>(tie, d.y, d.r, g);
+        const float ev = __fsub_rn(wp, __fsub_rn(__fsub_rn(1.0f, wp), tp));
+        return (allowed && den > 1e-8f) ? ev : 0.0f;
+    };
 #pragma unroll
     for (int i = 0; i < kHandsPerThread; ++i) {
         const int h = tid + i * kRowThreads, hc = hi.real[i] ? h : 0;
         const uint2 rec = *reinterpret_cast<const uint2*>(tv.rec + hc);
-        const int l = rec.x & 0xffffu, r = rec.x >> 16;
-        const int a0 = hi.c1[i] * 52 + (rec.y & 0xff), a1 = hi.c1[i] * 52 + ((rec.y >> 8) & 0xff);
-        const int b0 = hi.c2[i] * 52 + ((rec.y >> 16) & 0xff), b1 = hi.c2[i] * 52 + (rec.y >> 24);
-#pragma unroll
-        for (int slot = BOTH ? 0 : 1; slot < 2; ++slot) {
-            const float* P = pref + slot * P2B_HPAD;
-            const float* C = pc + slot * 52 * 52;
-            const float* T = tot + slot * 64;
-            const float xh = (slot ? x1 : x0)[h];
-            const float PL = P[l], C1 = C[a0], C2 = C[b0];
-            const float win = __fsub_rn(__fsub_rn(PL, C1), C2);
-            const float tie = __fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(P[r], PL), __fsub_rn(C[a1], C1)), __fsub_rn(C[b1], C2)), xh);
-            const float den = fmaxf(__fadd_rn(__fsub_rn(__fsub_rn(1.0f, T[hi.c1[i]]), T[hi.c2[i]]), xh), 1e-8f);
-            const Divisor d = make_divisor(den);
-            g.dok = g.dok && d.ok;
-            const float wp = div_g<false>(win, d.y, d.r, g), tp = div_g<false>(tie, d.y, d.r, g);
-            const float ev = __fsub_rn(wp, __fsub_rn(__fsub_rn(1.0f, wp), tp));
-            (slot ? ev1 : ev0).v[i] = (hi.allowed[i] && den > 1e-8f) ? ev : 0.0f;
-        }
+        const float2 PL = pref[rec.x & 0xffffu], PR = pref[rec.x >> 16];
+        const float2* r1 = pc + hi.c1[i] * 52;
+        const float2* r2 = pc + hi.c2[i] * 52;
+        const float2 C1 = r1[rec.y & 0xff], D1 = r1[(rec.y >> 8) & 0xff], C2 = r2[(rec.y >> 16) & 0xff], D2 = r2[rec.y >> 24];
+        const float2 T1 = tot[hi.c1[i]], T2 = tot[hi.c2[i]];
+        ev0.v[i] = one(PL.x, PR.x, C1.x, D1.x, C2.x, D2.x, T1.x, T2.x, x0[h], hi.allowed[i]);
+        ev1.v[i] = one(PL.y, PR.y, C1.y, D1.y, C2.y, D2.y, T1.y, T2.y, x1[h], hi.allowed[i]);
     }
-    if (__builtin_expect(guard_bad(g), 0)) {
+    if (__builtin_expect(guard_bad(g), 0)) {  // the same with IEEE divisions
 #pragma unroll 1
-        for (int slot = BOTH ? 0 : 1; slot < 2; ++slot)
-#pragma unroll
-            for (int i = 0; i < kHandsPerThread; ++i) {
-                const int h = tid + i * kRowThreads;
-                if (!hi.real[i]) continue;
-                const float ev = showdown_hand_ev(tv.rec[h], hi.c1[i], hi.c2[i], (slot ? x1 : x0)[h], hi.allowed[i],
-                                                  pref + slot * P2B_HPAD, pc + slot * 52 * 52, tot[slot * 64 + hi.c1[i]],
-                                                  tot[slot * 64 + hi.c2[i]]);
-                if (slot) ev1.v[i] = ev;
-                else ev0.v[i] = ev;
+        for (int i = 0; i < kHandsPerThread; ++i) {
+            const int h = tid + i * kRowThreads;
+            const HandRec rec = tv.rec[h < P2B_NUM_HANDS ? h : 0];
+            const int c1 = i == 0 ? hi.c1[0] : i == 1 ? hi.c1[1] : hi.c1[2], c2 = i == 0 ? hi.c2[0] : i == 1 ? hi.c2[1] : hi.c2[2];
+            const bool allowed = i == 0 ? hi.allowed[0] : i == 1 ? hi.allowed[1] : hi.allowed[2];
+#pragma unroll 1
+            for (int slot = 0; slot < 2; ++slot) {
+                auto at = [&](const float2& t) { return slot ? t.y : t.x; };
+                const float PL = at(pref[rec.lpos]), PR = at(pref[rec.rpos]);
+                const float C1 = at(pc[c1 * 52 + rec.nb0]), D1 = at(pc[c1 * 52 + rec.ne0]);
+                const float C2 = at(pc[c2 * 52 + rec.nb1]), D2 = at(pc[c2 * 52 + rec.ne1]);
+                const float xh = (slot ? x1 : x0)[h];
+                const float win = __fsub_rn(__fsub_rn(PL, C1), C2);
+                const float tie = __fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(PR, PL), __fsub_rn(D1, C1)), __fsub_rn(D2, C2)), xh);
+                const float den = fmaxf(__fadd_rn(__fsub_rn(__fsub_rn(1.0f, at(tot[c1])), at(tot[c2])), xh), 1e-8f);
+                const float wp = __fdiv_rn(win, den), tp = __fdiv_rn(tie, den);
+                const float e = __fsub_rn(wp, __fsub_rn(__fsub_rn(1.0f, wp), tp));
+                const float ev = (allowed && den > 1e-8f) ? e : 0.0f;
+                Row3& out = slot ? ev1 : ev0;
+                if (i == 0) out.v[0] = ev;
+                else if (i == 1) out.v[1] = ev;
+                else out.v[2] = ev;
             }
+        }
     }
 }
 
@@ -817,9 +1010,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float* rows = reinterpret_cast<float*>(smem + L.rows);
     float* leaf = rows + L.leaf_row * P2B_HPAD;
-    float* pref = reinterpret_cast<float*>(smem + L.pref);
-    float* pc = reinterpret_cast<float*>(smem + L.pc);
-    float* tot = reinterpret_cast<float*>(smem + L.tot);
+    float2* pref = reinterpret_cast<float2*>(smem + L.pref);
+    float2* pc = reinterpret_cast<float2*>(smem + L.pc);
+    float2* tot = reinterpret_cast<float2*>(smem + L.tot);
     double* scan = reinterpret_cast<double*>(smem + L.scan);
     double* cs = reinterpret_cast<double*>(smem + L.cs);
     double* S = reinterpret_cast<double*>(smem + L.S);
@@ -852,6 +1045,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
             idx[i] = word;
         }
     }
+    const bool mix = (p.scalars[pass].do_mix & 1) != 0;
+    launch_next();
+    bool waited = false;
     // a block takes consecutive items: mostly nodes of one subgame, whose board tables stay in shared memory
     const int total = w.total[0], each = (total + gridDim.x - 1) / gridDim.x;
     const int first = blockIdx.x * each, last = min(first + each, total);
@@ -874,6 +1070,10 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
             hi.allowed[i] = hi.real[i] && (((sg.board_mask >> hi.c1[i]) | (sg.board_mask >> hi.c2[i])) & 1ull) == 0;
             mask.v[i] = hi.allowed[i] ? 1.0f : 0.0f;
         }
+        if (!waited) {
+            previous_done();
+            waited = true;
+        }
         const long long nb = (long long)sg.node_begin * P2B_HPAD;
         float* rec = w.rec + (long long)sg.node_begin * kRec;
         float* cr = p.carry_roots + (long long)it.subgame * 4 * P2B_HPAD;
@@ -892,6 +1092,11 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
             const Row3 r_a = path3(rec, kRec, it.path, it.n_path[0], mask, tid);
             const Row3 r_o = path3(rec, kRec, it.path + it.n_path[0], it.n_path[1], mask, tid);
             const Row3 u_a = mul3(prior_a, r_a), u_o = mul3(prior_o, r_o);
+            if (!AVG && mix) {  // what the average-policy mix weights by
+                st3(rec + j * kRec + kRecReach * P2B_HPAD, tid, r_a);
+                st3(rec + j * kRec + kRecOldReach * P2B_HPAD, tid,
+                    path3(p.policy_avg + nb, P2B_HPAD, it.path, it.n_path[0], mask, tid));
+            }
             Row3 bbar_a, bbar_o;  // beliefs under the average policy
             if (AVG) {
                 const Row3 rw_a = path3(p.policy_avg + nb, P2B_HPAD, it.path, it.n_path[0], mask, tid);
@@ -980,7 +1185,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
         __syncthreads();
         card_sums(rows, 2 + k, cs, S, idx);
         const BoardTabView tv = view_tables(smem + L.tab);
-        if (showdown) showdown_tables(tv, rows + P2B_HPAD, leaf, 3, pref, pc, tot, scan);
+        if (showdown) showdown_tables(tv, rows + P2B_HPAD, leaf, pref, pc, tot, scan);
         __syncthreads();
 
         const Row3 b_a = ld3(rows, tid), x_o = ld3(rows + P2B_HPAD, tid);
@@ -1017,7 +1222,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
         if (!showdown) continue;
         // the acting player's hands against the other player's beliefs, and the reverse at each showdown leaf
         Row3 eva, evo;
-        showdown_rows<true>(tv, rows + P2B_HPAD, leaf, pref, pc, tot, hi, eva, evo);
+        showdown_rows(tv, rows + P2B_HPAD, leaf, pref, pc, tot, hi, eva, evo);
         const Divisor dscale = make_divisor(sg.scale);
 #pragma unroll 1
         for (int c = it.first_sd; c < k; ++c) {
@@ -1030,9 +1235,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
                 __syncthreads();
                 st3(leaf, tid, normalised(u, avg_sums[2 + c], sg.allowed_prob, hi));
                 __syncthreads();
-                showdown_tables(tv, rows + P2B_HPAD, leaf, 2, pref, pc, tot, scan);
+                showdown_tables(tv, rows + P2B_HPAD, leaf, pref, pc, tot, scan);
                 __syncthreads();
-                showdown_rows<false>(tv, rows + P2B_HPAD, leaf, pref, pc, tot, hi, eva, evo);
+                showdown_rows(tv, rows + P2B_HPAD, leaf, pref, pc, tot, hi, eva, evo);
             }
             const NodeRec ch = load_node(p.nodes + sg.node_begin + fc + c);
             const float pot_a = a == 0 ? ch.v0 : ch.v1, pot_o = a == 0 ? ch.v1 : ch.v0;
@@ -1059,54 +1264,90 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
     }
 }
 
+// Raises a kernel's shared-memory limit on the current device, once for each size it has not had there (the call takes as
+// long as a launch).
+struct SharedLimit {
+    std::atomic<int> bytes[64] = {};
+};
+int allow_shared(SharedLimit& had, const void* kernel, int bytes) {
+    int dev = 0;
+    int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    if (rc) return rc;
+    const bool known = dev >= 0 && dev < 64;
+    if (known && had.bytes[dev].load() >= bytes) return P2B_OK;
+    rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "shared-memory attribute");
+    if (!rc && known) {
+        int seen = had.bytes[dev].load();
+        while (seen < bytes && !had.bytes[dev].compare_exchange_weak(seen, bytes)) {
+        }
+    }
+    return rc;
+}
+
+// `follows`: the launch before it on the stream was one of these kernels (see launch_next).
+template <typename... Params, typename... Args>
+int launch_pass_kernel(void (*kernel)(Params...), const char* name, unsigned grid, unsigned threads, int bytes, bool follows,
+                       cudaStream_t stream, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = (size_t)bytes;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = follows ? 1 : 0;
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...), name);
+}
+
 template <int MAXK, bool SD, bool AVG>
-int launch_rows(const CfrParams& p, const SplitWork& w, int pass, cudaStream_t stream) {
+int launch_rows(const CfrParams& p, const SplitWork& w, int pass, bool follows, cudaStream_t stream) {
     constexpr int kBytes = row_layout(MAXK, SD).bytes;
     static_assert(kBytes <= 227 * 1024, "one block must fit an SM");
-    int rc = check_cuda(cudaFuncSetAttribute(split_rows_kernel<MAXK, SD, AVG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes),
-                        "split_rows_kernel shared-memory attribute");
+    static SharedLimit had;
+    int rc = allow_shared(had, reinterpret_cast<const void*>(split_rows_kernel<MAXK, SD, AVG>), kBytes);
     if (rc) return rc;
     const long long most = (long long)p.num_subgames * p.max_internal, fit = 2ll * sm_count();
-    split_rows_kernel<MAXK, SD, AVG><<<(unsigned)(most < fit ? most : fit), kRowThreads, kBytes, stream>>>(p, w, pass);
-    return check_cuda(cudaGetLastError(), "split_rows_kernel");
+    return launch_pass_kernel(split_rows_kernel<MAXK, SD, AVG>, "split_rows_kernel", (unsigned)(most < fit ? most : fit), kRowThreads,
+                              kBytes, follows, stream, p, w, pass);
 }
 
 template <int MAXK>
-int launch_rows(const CfrParams& p, const SplitWork& w, int pass, bool avg, cudaStream_t stream) {
+int launch_rows(const CfrParams& p, const SplitWork& w, int pass, bool avg, bool follows, cudaStream_t stream) {
     if (p.tables)
-        return avg ? launch_rows<MAXK, true, true>(p, w, pass, stream) : launch_rows<MAXK, true, false>(p, w, pass, stream);
-    return avg ? launch_rows<MAXK, false, true>(p, w, pass, stream) : launch_rows<MAXK, false, false>(p, w, pass, stream);
+        return avg ? launch_rows<MAXK, true, true>(p, w, pass, follows, stream)
+                   : launch_rows<MAXK, true, false>(p, w, pass, follows, stream);
+    return avg ? launch_rows<MAXK, false, true>(p, w, pass, follows, stream)
+               : launch_rows<MAXK, false, false>(p, w, pass, follows, stream);
 }
 
-template <int VPT, int MAXK>
-int launch_columns(const CfrParams& p, const SplitWork& w, ColumnMode mode, int pass, bool advance, bool mixed, int max_children,
-                   cudaStream_t stream) {
+template <int MODE>
+int launch_prep(const CfrParams& p, const SplitWork& w, int pass, int max_children, cudaStream_t stream) {
+    const unsigned grid = (unsigned)p.num_subgames * (P2B_HPAD / 64);
+    if (max_children <= kIterMaxChildren) split_prep_kernel<6, MODE><<<grid, 32 * kPrepWarps, 0, stream>>>(p, w, pass);
+    else split_prep_kernel<8, MODE><<<grid, 32 * kPrepWarps, 0, stream>>>(p, w, pass);
+    return check_cuda(cudaGetLastError(), "split_prep_kernel");
+}
+
+int launch_up(const CfrParams& p, const SplitWork& w, int pass, bool advance, bool mixed, int max_children, bool follows,
+              cudaStream_t stream) {
+    // Warps a slice: one warp's walk up a tree is the time of a small batch, so nodes of a level are spread over up to eight;
+    // more warps than it takes to keep the memory busy only wait at the levels with few nodes.  Measured (us a pass; 8 / 4 /
+    // 2 / 1 warps a slice): 1 subgame 17 / 21 / 29 / 49, 37 of 96 nodes 76 / 79 / 114 / 198, 192 of 77 nodes 318 / 257 /
+    // 231 / 264, 4096 of 54 nodes - / - / 2550 / 2730.
+    const int lanes = p.num_subgames >= sm_count() ? 2 : 8, slices = lanes == 2 ? 3 : 1;
+    int ring = 40;  // two nodes of two or three actions, the usual ones, fit together; 18 warps an SM
+    if (ring < up_rows(max_children)) ring = up_rows(max_children);
     long long nodes = (long long)p.max_internal * max_children + 1;
     if (nodes > kCfrMaxNodes) nodes = kCfrMaxNodes;
-    const int bytes = p.max_internal * (int)sizeof(SplitItem) + (int)nodes * (int)sizeof(NodeRecPacked);
-    // Warps a slice: as many as it takes to fill the chip with about 16 warps an SM; more of them than that only wait at
-    // the levels with few nodes.  Measured (us a pass, 8 / 2 / 1 warps a slice): 37 subgames of 96 nodes 120 / 197 / 350,
-    // 192 of 77 nodes 428 / 335 / 506, 4096 of 54 nodes 6680 / 4070 / 3750.
-    const int B = p.num_subgames, sms = sm_count();
-    int lanes = 8, slices = 1;
-    if (B >= 4 * sms) lanes = 1, slices = VPT == 2 ? 7 : 6;
-    else if (B >= sms) lanes = 2, slices = 3;
-    const unsigned grid = (unsigned)B * (P2B_HPAD / (32 * VPT) / slices), threads = 32 * lanes * slices;
-    if (mode == kColInit) split_columns_kernel<VPT, MAXK, kColInit><<<grid, threads, bytes, stream>>>(p, w, pass, advance, mixed, lanes, slices);
-    else if (mode == kColMix) split_columns_kernel<VPT, MAXK, kColMix><<<grid, threads, bytes, stream>>>(p, w, pass, advance, mixed, lanes, slices);
-    else split_columns_kernel<VPT, MAXK, kColUp><<<grid, threads, bytes, stream>>>(p, w, pass, advance, mixed, lanes, slices);
-    return check_cuda(cudaGetLastError(), "split_columns_kernel");
-}
-
-int columns(const CfrParams& p, const SplitWork& w, ColumnMode mode, int pass, bool advance, bool mixed, int max_children,
-            cudaStream_t stream) {
-    // one hand a thread while two would leave SMs without a block: a warp's walk is 25 % shorter then
-    const bool one = p.num_subgames * (P2B_HPAD / 64) < sm_count();
-    if (max_children <= kIterMaxChildren)
-        return one ? launch_columns<1, 6>(p, w, mode, pass, advance, mixed, max_children, stream)
-                   : launch_columns<2, 6>(p, w, mode, pass, advance, mixed, max_children, stream);
-    return one ? launch_columns<1, 8>(p, w, mode, pass, advance, mixed, max_children, stream)
-               : launch_columns<2, 8>(p, w, mode, pass, advance, mixed, max_children, stream);
+    const int bytes = lanes * slices * ring * kUpRow * 4 + p.max_internal * (int)sizeof(SplitItem) + (int)nodes * (int)sizeof(NodeRecPacked);
+    static SharedLimit had;
+    int rc = allow_shared(had, reinterpret_cast<const void*>(split_up_kernel), bytes);
+    if (rc) return rc;
+    const unsigned grid = (unsigned)p.num_subgames * (P2B_HPAD / kUpRow / slices);
+    return launch_pass_kernel(split_up_kernel, "split_up_kernel", grid, 32 * lanes * slices, bytes, follows, stream, p, w, pass, advance,
+                              mixed, lanes, slices, ring);
 }
 
 }  // namespace
@@ -1124,19 +1365,27 @@ int launch_split_passes(const CfrParams& p, int max_children, int pass_begin, in
     const SplitWork w = carve(p.scratch, p.num_subgames, p.rows);
     const bool avg = p.cfr_avg != 0 || p.iter_values != 0;
     int rc = P2B_OK;
+    bool follows = false;
     if (down) {
         split_items_kernel<<<p.num_subgames, kCfrMaxNodes, 0, stream>>>(p, w);
         rc = check_cuda(cudaGetLastError(), "split_items_kernel");
-        if (!rc) rc = columns(p, w, kColInit, pass_begin, true, avg, max_children, stream);
+        if (!rc) rc = launch_prep<kPrepPolicy>(p, w, pass_begin, max_children, stream);
     }
     for (int pass = pass_begin; pass <= pass_end && !rc; ++pass) {
         if (pass > pass_begin || down) {
-            if (avg) rc = columns(p, w, kColMix, pass, false, avg, max_children, stream);
+            if (avg) {
+                rc = launch_prep<kPrepMix>(p, w, pass, max_children, stream);
+                follows = false;
+            }
             if (!rc)
-                rc = max_children <= kIterMaxChildren ? launch_rows<6>(p, w, pass, avg, stream)
-                                                      : launch_rows<8>(p, w, pass, avg, stream);
+                rc = max_children <= kIterMaxChildren ? launch_rows<6>(p, w, pass, avg, follows, stream)
+                                                      : launch_rows<8>(p, w, pass, avg, follows, stream);
+            follows = true;
         }
-        if (!rc && (pass < pass_end || up)) rc = columns(p, w, kColUp, pass, pass < pass_end, avg, max_children, stream);
+        if (!rc && (pass < pass_end || up)) {
+            rc = launch_up(p, w, pass, pass < pass_end, avg, max_children, follows, stream);
+            follows = true;
+        }
     }
     return rc;
 }

@@ -40,7 +40,7 @@ def _both(cuda_device, B, *, bins=(0.5, 1.0), cap=2, iterations=5, cfr_type="dis
     return layout, out
 
 
-@pytest.mark.parametrize("B", [1, 7, 8, 60])  # one hand a thread up to 7, two from 8 on
+@pytest.mark.parametrize("B", [1, 7, 8, 60])  # eight warps a slice of hands
 def test_batch_sizes(cuda_device, B):
     for a, b in zip(*_both(cuda_device, B)[1]):
         assert torch.equal(a, b)
@@ -61,7 +61,7 @@ def test_options(cuda_device, opts):
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("B", [160, 600])  # two warps and one warp a slice; beyond the lean kernel's 8 actions limit
+@pytest.mark.parametrize("B", [160, 600])  # two warps a slice; beyond the lean kernel's 8 actions limit
 def test_wide_batches(cuda_device, B):
     for a, b in zip(*_both(cuda_device, B, bins=(0.5, 0.75, 1.0, 1.5, 2.0), cap=1, iterations=2)[1]):
         assert torch.equal(a, b)
