@@ -1651,29 +1651,32 @@ static int general_passes(CfrParams p, int num_blocks, int max_children, int beg
     return rc ? rc : dispatch_cfr(p, num_blocks, max_children, stream);
 }
 
-// The same for iteration passes on the split kernels.
-static int split_passes(const CfrParams& p, int max_children, int begin, int end, bool down, bool up, cudaStream_t stream) {
-    int rc = clear_counters(p.work_counter, stream);
-    if (!rc) rc = check_records(p, stream);
-    return rc ? rc : launch_split_passes(p, max_children, begin, end, down, up, stream);
-}
-
-// A call of a stepped solve: start and final pass in the general kernel, iteration passes in the split kernels.
+// A call of a stepped solve on the split kernels.  Only a start pass whose node values are kept stays in the general kernel:
+// the best-response pass of a `model_br` warm start goes on from that kernel's work rows.
 static int launch_stepped(const CfrParams& p, int num_blocks, int max_children, cudaStream_t stream) {
     const int T = p.iterations;
     int rc = P2B_OK;
+    if (p.pass_begin < 0 && p.iter_values) {
+        rc = general_passes(p, num_blocks, max_children, -1, -1, p.phases == 16 ? 2 : p.phases, stream);
+        if (rc || p.pass_end < 0) return rc;
+    }
+    rc = clear_counters(p.work_counter, stream);
+    if (!rc) rc = check_records(p, stream);
+    if (rc) return rc;
+    const bool start = p.pass_begin < 0 && !p.iter_values;
+    if (p.phases == 4) return launch_split_final(p, max_children, false, false, true, stream);
     if (p.phases == 16) {
         const int t = p.pass_begin;
-        rc = t < 0 ? general_passes(p, num_blocks, max_children, t, t, 2, stream) : P2B_OK;
-        if (!rc && t + 1 < T) return split_passes(p, max_children, t < 0 ? 0 : t, t + 1, t < 0, false, stream);
-        if (!rc && t >= 0) rc = split_passes(p, max_children, t, t, false, true, stream);
-        return rc ? rc : general_passes(p, num_blocks, max_children, T, T, 1, stream);
+        if (start) rc = launch_split_start(p, max_children, false, true, t + 1 < T, stream);
+        if (!rc && t + 1 < T) return launch_split_passes(p, max_children, t < 0 ? 0 : t, t + 1, t < 0, false, start, stream);
+        if (!rc && t >= 0) rc = launch_split_passes(p, max_children, t, t, false, true, false, stream);
+        return rc ? rc : launch_split_final(p, max_children, true, false, false, stream);
     }
     const bool down = (p.phases & 1) != 0, up = (p.phases & 2) != 0;
     const int first = p.pass_begin < 0 ? 0 : p.pass_begin, last = p.pass_end < T ? p.pass_end : T - 1;
-    if (p.pass_begin < 0) rc = general_passes(p, num_blocks, max_children, -1, -1, p.phases, stream);
-    if (!rc && first <= last) rc = split_passes(p, max_children, first, last, down, up, stream);
-    if (!rc && p.pass_end == T) rc = general_passes(p, num_blocks, max_children, T, T, p.phases, stream);
+    if (start) rc = launch_split_start(p, max_children, down, up, first <= last, stream);
+    if (!rc && first <= last) rc = launch_split_passes(p, max_children, first, last, down, up, start, stream);
+    if (!rc && p.pass_end == T) rc = launch_split_final(p, max_children, down, up, up, stream);
     return rc;
 }
 
@@ -1690,7 +1693,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
     // leaves all terminal, all passes in this call: the iteration kernel applies (a start policy only concerns
     // the start pass, a warm start of type `model` is a kernel of its own between that pass and the iterations)
     const bool plain = !p.stepped && !p.leaf_beliefs && !p.leaf_values && !p.cfr_avg && !p.linear;
-    if (p.stepped && p.phases != 4 && p.phases != 8 && split_applies(p, max_children, p.scratch_floats))
+    if (p.stepped && p.phases != 8 && split_applies(p, max_children, p.scratch_floats))
         return launch_stepped(p, num_blocks, max_children, stream);
     long long per_block = cfr_scratch_floats(p.max_internal);
     const long long iter_block = cfr_iter_scratch_floats(p.max_internal, max_children);
@@ -1702,21 +1705,21 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
         IterTiming* timing = iter_timing_of_current_device();
         const bool timed = timing && timing->enabled && p.num_subgames > (large ? 8 : 1) * sm_count();
         CfrParams q = p;
-        q.scratch_stride = per_block;
         q.carry_roots = p.scratch + solve_work_floats(p.max_internal, max_children, num_blocks, p.num_subgames, p.rows);
         q.carry_sums = q.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;
-        q.stepped = 1;
-        q.scratch_per_block = 1;
-        rc = general_passes(q, num_blocks, max_children, -1, -1, 3, stream);
-        if (!rc && p.warm_weight > 0.0f)
+        const bool warm = p.warm_weight > 0.0f;  // works on the regrets of the start pass before the iterations read them
+        rc = clear_counters(q.work_counter, stream);
+        if (!rc) rc = check_records(q, stream);
+        if (!rc) rc = launch_split_start(q, max_children, true, true, !warm, stream);
+        if (!rc && warm)
             rc = launch_cfr_warm_seed(p.nodes, p.rows, p.start_policy, p.warm_weight, p.regrets, p.weight_sums, stream);
         if (timed) cudaEventRecord(timing->start, stream);
-        if (!rc) rc = split_passes(q, max_children, 0, p.iterations - 1, true, true, stream);
+        if (!rc) rc = launch_split_passes(q, max_children, 0, p.iterations - 1, true, true, !warm, stream);
         if (timed) {
             cudaEventRecord(timing->stop, stream);
             timing->recorded = true;
         }
-        return rc ? rc : general_passes(q, num_blocks, max_children, p.iterations, p.iterations, 3, stream);
+        return rc ? rc : launch_split_final(q, max_children, true, true, true, stream);
     }
     if (!lean) {
         if (p.warm_weight > 0.0f) {

@@ -66,6 +66,8 @@ enum RecRow {
     kRecValue = 3,   // values of player 0, then of player 1 (internal nodes and showdown leaves)
     kRecReach = 5,   // the acting player's reach under the current policy and under the old average policy (internal
     kRecOldReach = 6,  // nodes, passes that mix)
+    kRecActing = 2,  // final pass: beliefs of the acting player
+    kRecBelief = 5,  // final pass: beliefs of player 0, then of player 1; later the best-response values of the second sweep
     kRecRows = 7
 };
 constexpr int kRec = kRecRows * P2B_HPAD;  // floats from a node's record to the next
@@ -433,7 +435,14 @@ __device__ __forceinline__ void async_pair(float* shared, const float* global) {
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void previous_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+enum UpJob {
+    kUpIter = 0,   // second half of an iteration pass
+    kUpStart = 1,  // of the start pass: no regrets and sums yet
+    kUpFinal = 2,  // of the final pass: values only, the root's too
+    kUpBase = 3    // plain expectation under the average policy from the clamped leaf values (:732-735), for the exploitability
+};
 struct UpPass {  // what a pass does, uniform over the grid
+    int job;
     bool update, tracked, mix, mixed, keep_values, keep_policy, sample;
     IterScalars sc, sn;
     Divisor d_pos, d_neg;
@@ -452,11 +461,20 @@ __device__ __forceinline__ void up_stage(const CfrParams& p, const SplitWork& w,
     for (int c = 0; c < k; ++c) {
         async_pair(d + kUpPolicy * kUpRow, rec + kRecPolicy * P2B_HPAD);
         async_pair(d + kUpSeen * kUpRow, rec + kRecSeen * P2B_HPAD);
-        if (u.update) async_pair(d + kUpRegret * kUpRow, R);
-        if (u.tracked) async_pair(d + kUpSum * kUpRow, W);
+        if (u.job == kUpStart) {
+            *reinterpret_cast<float2*>(d + kUpRegret * kUpRow) = make_float2(0.0f, 0.0f);
+            *reinterpret_cast<float2*>(d + kUpSum * kUpRow) = make_float2(0.0f, 0.0f);
+        } else {
+            if (u.update) async_pair(d + kUpRegret * kUpRow, R);
+            if (u.tracked) async_pair(d + kUpSum * kUpRow, W);
+        }
         if (u.mix) async_pair(d + kUpAverage * kUpRow, A);
         const int kind = it.kind[c];
-        if (kind == kShowdownLeaf || (kind == kModelLeaf && p.leaf_values)) {
+        if (u.job == kUpBase && kind != kInternal) {
+            const float* v = p.values_avg + 2 * (row + c) * P2B_HPAD + h;
+            async_pair(d + kUpValueA * kUpRow, v + a * P2B_HPAD);
+            async_pair(d + kUpValueO * kUpRow, v + (1 - a) * P2B_HPAD);
+        } else if (kind == kShowdownLeaf || (kind == kModelLeaf && p.leaf_values)) {
             const float* v = kind == kShowdownLeaf
                                  ? rec + kRecValue * P2B_HPAD
                                  : p.leaf_values + (long long)(leaf0 + nodes[it.first_child + c].internal_idx) * 2 * P2B_HPAD + h;
@@ -503,18 +521,27 @@ __device__ __forceinline__ void up_node(const CfrParams& p, const SplitWork& w, 
 #pragma unroll 2
     for (int c = 0; c < k; ++c) {
         const FV<2> P = ldc<2>(slot(c, kUpPolicy)), Q = ldc<2>(slot(c, kUpSeen));
-        const FV<2> Va = ldc<2>(slot(c, kUpValueA)), Vo = ldc<2>(slot(c, kUpValueO));
+        FV<2> Va = ldc<2>(slot(c, kUpValueA)), Vo = ldc<2>(slot(c, kUpValueO));
+        if (u.job == kUpBase && it.kind[c] != kInternal) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                Va.v[i] = fminf(fmaxf(Va.v[i], -1.0f), 1.0f);
+                Vo.v[i] = fminf(fmaxf(Vo.v[i], -1.0f), 1.0f);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             acc_a.v[i] = __fadd_rn(acc_a.v[i], __fmul_rn(Va.v[i], P.v[i]));
             acc_o.v[i] = __fadd_rn(acc_o.v[i], __fmul_rn(Vo.v[i], Q.v[i]));
         }
     }
-    if (j != 0) {
-        float* v = w.rec + (long long)(it.node_begin + j) * kRec + kRecValue * P2B_HPAD + h;
+    if (j != 0 || u.job >= kUpFinal) {
+        float* v = j == 0 && u.job == kUpBase ? p.carry_roots + (long long)it.subgame * 4 * P2B_HPAD + h
+                                              : w.rec + (long long)(it.node_begin + j) * kRec + kRecValue * P2B_HPAD + h;
         stc<2>(v + a * P2B_HPAD, acc_a);
         stc<2>(v + (1 - a) * P2B_HPAD, acc_o);
     }
+    if (u.job >= kUpFinal) return;
     if (u.keep_values) {  // the values of this iteration at the node and at the leaves below it
         float* out = p.values_avg + (long long)it.node_begin * 2 * P2B_HPAD + h;
         stc<2>(out + (2 * j + a) * P2B_HPAD, acc_a);
@@ -663,7 +690,7 @@ __device__ __forceinline__ void up_node(const CfrParams& p, const SplitWork& w, 
 // A block holds `slices` slices of one subgame with `lanes` warps each, which take the nodes of a level in turn; a level is
 // complete when the warps of a slice meet at its barrier.  `ring`: rows of a warp's staging area; two nodes that follow one
 // another lie at its two ends if they fit together, else the second is copied once the first is done.
-__global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p, const SplitWork w, int pass, bool advance,
+__global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p, const SplitWork w, int job, int pass, bool advance,
                                                               bool mixed, int lanes, int slices, int ring) {
     constexpr int kSlices = P2B_HPAD / kUpRow;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -685,15 +712,16 @@ __global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p,
         for (int i = tid; i < sg.n_internal * 4; i += blockDim.x) reinterpret_cast<uint4*>(items)[i] = is[i];
     }
     UpPass u;
-    u.sc = p.scalars[pass];
-    u.update = pass + 1 < p.iterations;
-    u.sn = p.scalars[u.update ? pass + 1 : pass];
+    u.job = job;
+    u.sc = p.scalars[job == kUpIter ? pass : 0];
+    u.update = job <= kUpStart && pass + 1 < p.iterations;
+    u.sn = p.scalars[u.update ? pass + 1 : 0];
     u.tracked = u.update && p.weight_sums != nullptr;
     u.mixed = mixed;
-    u.mix = !mixed && (u.sc.do_mix & 1) != 0;
+    u.mix = job == kUpIter && !mixed && (u.sc.do_mix & 1) != 0;
     u.keep_values = p.iter_values && p.values_avg != nullptr;
-    u.keep_policy = p.policy != nullptr && pass == p.iterations - 1;
-    u.sample = p.policy_sample != nullptr && p.sample_pass[s] == pass;
+    u.keep_policy = job == kUpIter && p.policy != nullptr && pass == p.iterations - 1;
+    u.sample = job == kUpIter && p.policy_sample != nullptr && p.sample_pass[s] == pass;
     u.d_pos = make_divisor(u.sn.den_pos);
     u.d_neg = make_divisor(u.sn.den_neg);
     const int leaf0 = p.leaf_begin ? p.leaf_begin[s] : 0;
@@ -827,6 +855,20 @@ __device__ __forceinline__ Row3 normalised(Row3 x, float sum, float allowed_prob
 // Per-card sums and totals of the rows 0 .. n_cs-1 (cs, S).  Thread t < 416 adds quarter (t / 4 mod 52, t mod 4) of
 // the 51 hands that hold a card, for the even or (t >= 208) the odd rows: the indices of its 13 hands belong to the
 // thread for the whole kernel and are held in registers as byte offsets, two to a word.
+__device__ __forceinline__ void card_indices(int tid, uint32_t (&idx)[7]) {
+    const int u = tid >= 208 ? tid - 208 : tid, c = (u >> 2) % 52, q = u & 3;
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        uint32_t word = 0;
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int e = q + 4 * (2 * i + b);
+            if (2 * i + b < 13 && e < 51)
+                word |= (uint32_t)(4 * (e < c ? combo_index(e, c) : combo_row_offset(c) - c + e)) << (16 * b);
+        }
+        idx[i] = word;
+    }
+}
 __device__ __forceinline__ void card_sums(const float* rows, int n_cs, double* cs, double* S, const uint32_t (&idx)[7]) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int half = tid >= 208 ? 1 : 0, u = tid - 208 * half, c = u >> 2, q = u & 3;
@@ -1003,8 +1045,101 @@ __device__ __forceinline__ void showdown_rows(const BoardTabView& tv, const floa
     }
 }
 
-template <int MAXK, bool SD, bool AVG>
+// The start pass at one node.  Upstream pushes the beliefs down one level at a time and re-normalises EVERY row after each
+// level (cfr_evaluator.py:855-875): a node at level L is normalised init_depth - L + 1 times, its children derive from its
+// once-normalised row, and the root's row, which its children take as given, is normalised once a level itself.
+template <int K>
+__device__ __forceinline__ void start_rows(const CfrParams& p, const SubgameRec& sg, const SplitItem& it, float* rows, float* sums,
+                                           float* leaf, float* rec, float* cr, int leaf0, const Hands& hi, int tid) {
+    const int a = it.to_act, o = 1 - a, j = it.node, fc = it.first_child, lane = tid & 31, warp = tid >> 5;
+    const int depth = it.n_path[0] + it.n_path[1];
+    const long long nb = (long long)sg.node_begin * P2B_HPAD;
+    auto normalise = [&](Row3& u, Row3& v, int times) {
+#pragma unroll 1
+        for (int t = 0; t < times; ++t) {
+            __syncthreads();
+            st3(rows, tid, u);
+            st3(rows + P2B_HPAD, tid, v);
+            __syncthreads();
+            if (warp < 2) {
+                const float sum = row_sum_reference_order(rows + warp * P2B_HPAD);
+                if (lane == 0) sums[warp] = sum;
+            }
+            __syncthreads();
+            u = normalised(u, sums[0], sg.allowed_prob, hi);
+            v = normalised(v, sums[1], sg.allowed_prob, hi);
+        }
+    };
+    auto policy = [&](int node) {  // the start policy: the caller's, or uniform over the siblings
+        if (p.start_policy) return ld3(p.start_policy + nb + (long long)node * P2B_HPAD, tid);
+        const int siblings = load_node(p.nodes + sg.node_begin + load_node(p.nodes + sg.node_begin + node).parent).n_children;
+        Row3 r;
+        r.v[0] = r.v[1] = r.v[2] = __fdiv_rn(1.0f, (float)siblings);
+        return r;
+    };
+    const float* given = p.root_beliefs + (long long)it.subgame * 2 * P2B_HPAD;
+    Row3 r_a = ld3(given + a * P2B_HPAD, tid), r_o = ld3(given + o * P2B_HPAD, tid);
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) {
+        r_a.v[i] = hi.allowed[i] ? r_a.v[i] : 0.0f;
+        r_o.v[i] = hi.allowed[i] ? r_o.v[i] : 0.0f;
+    }
+    if (j == 0) {
+        st3(cr + a * P2B_HPAD, tid, r_a);
+        st3(cr + o * P2B_HPAD, tid, r_o);
+    }
+#pragma unroll 1
+    for (int ia = 0, io = it.n_path[0]; ia + io < it.n_path[0] + depth;) {  // down the path, both players' nodes in order
+        const bool acting = io >= depth || (ia < it.n_path[0] && it.path[ia] < it.path[io]);
+        const Row3 P = policy(acting ? it.path[ia] : it.path[io]);
+        if (acting) {
+            r_a = mul3(r_a, P);
+            ++ia;
+        } else {
+            r_o = mul3(r_o, P);
+            ++io;
+        }
+        normalise(r_a, r_o, 1);
+    }
+    Row3 b_a = r_a, b_o = r_o;
+    normalise(b_a, b_o, j == 0 ? max(p.init_depth, 1) : p.init_depth - depth);
+    if (j == 0) {
+        st3(cr + (2 + a) * P2B_HPAD, tid, b_a);
+        st3(cr + (2 + o) * P2B_HPAD, tid, b_o);
+    }
+#pragma unroll 1
+    for (int c = 0; c < K; ++c) {
+        const Row3 P = policy(fc + c);
+        st3(p.policy_avg + nb + (fc + c) * P2B_HPAD, tid, P);
+        st3(rec + (fc + c) * kRec, tid, P);
+        if (it.kind[c] == kShowdownLeaf || (it.kind[c] == kModelLeaf && p.leaf_beliefs)) {
+            Row3 x_a = mul3(r_a, P), x_o = r_o;
+            normalise(x_a, x_o, p.init_depth - depth);
+            if (it.kind[c] == kModelLeaf) {
+                float* out = p.leaf_beliefs + 2ll * (leaf0 + load_node(p.nodes + sg.node_begin + fc + c).internal_idx) * P2B_HPAD;
+                st3(out + a * P2B_HPAD, tid, x_a);
+                st3(out + o * P2B_HPAD, tid, x_o);
+            } else {
+                st3(c == it.first_sd ? leaf : rec + (fc + c) * kRec + kRecValue * P2B_HPAD, tid, x_a);
+            }
+        }
+        st3(rows + (2 + c) * P2B_HPAD, tid, mul3(b_a, P));
+    }
+    __syncthreads();
+    st3(rows, tid, b_a);
+    st3(rows + P2B_HPAD, tid, b_o);
+}
+
+enum RowKind {
+    kRowIter = 0,   // iteration pass, beliefs under the current policy
+    kRowAvg = 1,    // iteration pass that also needs the beliefs under the average policy (cfr_avg, kept values)
+    kRowStart = 2,  // start pass: the start policy, beliefs re-normalised once per level (:830-886)
+    kRowFinal = 3   // final pass: the average policy (`update_average_values_final`, :1276-1292)
+};
+
+template <int MAXK, bool SD, int KIND>
 __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrParams p, const SplitWork w, int pass) {
+    constexpr bool AVG = KIND == kRowAvg;
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr RowLayout L = row_layout(MAXK, SD);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1030,22 +1165,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
         hi.c1[i] = p.combos->c1[hc];
         hi.c2[i] = p.combos->c2[hc];
     }
-    uint32_t idx[7];  // see card_sums
-    {
-        const int u = tid >= 208 ? tid - 208 : tid, c = (u >> 2) % 52, q = u & 3;
-#pragma unroll
-        for (int i = 0; i < 7; ++i) {
-            uint32_t word = 0;
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const int e = q + 4 * (2 * i + b);
-                if (2 * i + b < 13 && e < 51)
-                    word |= (uint32_t)(4 * (e < c ? combo_index(e, c) : combo_row_offset(c) - c + e)) << (16 * b);
-            }
-            idx[i] = word;
-        }
-    }
-    const bool mix = (p.scalars[pass].do_mix & 1) != 0;
+    uint32_t idx[7];
+    card_indices(tid, idx);
+    const bool mix = KIND == kRowIter && (p.scalars[pass].do_mix & 1) != 0;
     launch_next();
     bool waited = false;
     // a block takes consecutive items: mostly nodes of one subgame, whose board tables stay in shared memory
@@ -1085,14 +1207,23 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
 
         with_children<MAXK>(k, [&](auto kc) {
             constexpr int K = decltype(kc)::value;
+            if constexpr (KIND == kRowStart) {
+                start_rows<K>(p, sg, it, rows, sums, leaf, rec, cr, leaf0, hi, tid);
+                return;
+            }
             Row3 P[K];
+            const float* policy = KIND == kRowFinal ? p.policy_avg + nb : rec;
+            constexpr int kPolicyStride = KIND == kRowFinal ? P2B_HPAD : kRec;
 #pragma unroll
-            for (int c = 0; c < K; ++c) P[c] = ld3(rec + (fc + c) * kRec, tid);
+            for (int c = 0; c < K; ++c) {
+                P[c] = ld3(policy + (fc + c) * kPolicyStride, tid);
+                if (KIND == kRowFinal) st3(rec + (fc + c) * kRec, tid, P[c]);
+            }
             const Row3 prior_a = ld3(cr + a * P2B_HPAD, tid), prior_o = ld3(cr + o * P2B_HPAD, tid);
-            const Row3 r_a = path3(rec, kRec, it.path, it.n_path[0], mask, tid);
-            const Row3 r_o = path3(rec, kRec, it.path + it.n_path[0], it.n_path[1], mask, tid);
+            const Row3 r_a = path3(policy, kPolicyStride, it.path, it.n_path[0], mask, tid);
+            const Row3 r_o = path3(policy, kPolicyStride, it.path + it.n_path[0], it.n_path[1], mask, tid);
             const Row3 u_a = mul3(prior_a, r_a), u_o = mul3(prior_o, r_o);
-            if (!AVG && mix) {  // what the average-policy mix weights by
+            if (KIND == kRowIter && mix) {  // what the average-policy mix weights by
                 st3(rec + j * kRec + kRecReach * P2B_HPAD, tid, r_a);
                 st3(rec + j * kRec + kRecOldReach * P2B_HPAD, tid,
                     path3(p.policy_avg + nb, P2B_HPAD, it.path, it.n_path[0], mask, tid));
@@ -1153,7 +1284,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
             const Row3 b_a = normalised(u_a, sums[0], sg.allowed_prob, hi);
             const Row3 b_o = normalised(u_o, sums[1], sg.allowed_prob, hi);
             const Row3 x_o = avgb ? bbar_o : b_o;
-            if (j == 0) {  // the root's own row, and its sums, for the pass after this one
+            if (KIND != kRowFinal && j == 0) {  // the root's own row, and its sums, for the pass after this one
                 st3(cr + (2 + a) * P2B_HPAD, tid, b_a);
                 st3(cr + (2 + o) * P2B_HPAD, tid, b_o);
                 if (tid == 0) {
@@ -1161,7 +1292,17 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
                     p.carry_sums[2ll * sg.node_begin + o] = sums[1];
                 }
             }
-            if (p.beliefs_last && pass == p.iterations - 1) {
+            if (KIND == kRowFinal) {  // for the value outputs and the best responses
+                st3(rec + j * kRec + kRecActing * P2B_HPAD, tid, b_a);
+                st3(rec + j * kRec + (kRecBelief + a) * P2B_HPAD, tid, b_a);
+                st3(rec + j * kRec + (kRecBelief + o) * P2B_HPAD, tid, b_o);
+                if (p.beliefs_avg) {
+                    float* out = p.beliefs_avg + 2 * nb;
+                    st3(out + (2 * j + a) * P2B_HPAD, tid, b_a);
+                    st3(out + (2 * j + o) * P2B_HPAD, tid, b_o);
+                }
+            }
+            if (KIND != kRowFinal && p.beliefs_last && pass == p.iterations - 1) {
                 float* out = p.beliefs_last + 2 * nb;
                 st3(out + (2 * j + a) * P2B_HPAD, tid, b_a);
                 st3(out + (2 * j + o) * P2B_HPAD, tid, b_o);
@@ -1169,8 +1310,14 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
 #pragma unroll
             for (int c = 0; c < K; ++c) {
                 float* row = rows + (2 + c) * P2B_HPAD;
-                if (SD && c == it.first_sd) {
-                    st3(leaf, tid, normalised(ld3(row, tid), avg_sums[2 + c], sg.allowed_prob, hi));
+                if (SD && it.kind[c] == kShowdownLeaf) {
+                    const Row3 x = normalised(ld3(row, tid), avg_sums[2 + c], sg.allowed_prob, hi);
+                    st3(c == it.first_sd ? leaf : rec + (fc + c) * kRec + kRecValue * P2B_HPAD, tid, x);
+                    if (KIND == kRowFinal && p.beliefs_avg) {
+                        float* out = p.beliefs_avg + 2 * nb + 2 * (fc + c) * P2B_HPAD;
+                        st3(out + a * P2B_HPAD, tid, x);
+                        st3(out + o * P2B_HPAD, tid, b_o);
+                    }
                 } else if (it.kind[c] == kModelLeaf && p.leaf_beliefs) {
                     const int slot = leaf0 + load_node(p.nodes + sg.node_begin + fc + c).internal_idx;
                     float* out = p.leaf_beliefs + 2ll * slot * P2B_HPAD;
@@ -1199,7 +1346,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
                 d[i] = make_divisor(unblocked(cs, S[0], hi.c1[i], hi.c2[i], b_a.v[i]));
                 ok = ok && d[i].ok;
             }
-            st3(rec + j * kRec + kRecWeight * P2B_HPAD, tid, wgt);
+            if (KIND != kRowFinal) st3(rec + j * kRec + kRecWeight * P2B_HPAD, tid, wgt);
 #pragma unroll 1
             for (int c = 0; c < k; ++c) {
                 const Row3 m = ld3(rows + (2 + c) * P2B_HPAD, tid);
@@ -1228,12 +1375,11 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
         for (int c = it.first_sd; c < k; ++c) {
             if (it.kind[c] != kShowdownLeaf) continue;
             if (c != it.first_sd) {
-                // a further showdown child (a call and an all-in of the same size; rare): its tables in place of the first one's
-                const Row3 r = path3(avgb ? p.policy_avg + nb : rec, avgb ? P2B_HPAD : kRec, it.path, it.n_path[0], mask, tid);
-                const Row3 P = avgb ? ld3(p.policy_avg + nb + (fc + c) * P2B_HPAD, tid) : ld3(rec + (fc + c) * kRec, tid);
-                const Row3 u = mul3(ld3(cr + a * P2B_HPAD, tid), mul3(r, P));
+                // a further showdown child (a call and an all-in of the same size; rare): its tables in place of the first
+                // one's, from its beliefs, which wait in its value row
+                const Row3 x = ld3(rec + (fc + c) * kRec + kRecValue * P2B_HPAD, tid);
                 __syncthreads();
-                st3(leaf, tid, normalised(u, avg_sums[2 + c], sg.allowed_prob, hi));
+                st3(leaf, tid, x);
                 __syncthreads();
                 showdown_tables(tv, rows + P2B_HPAD, leaf, pref, pc, tot, scan);
                 __syncthreads();
@@ -1262,6 +1408,214 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
             st3(v + o * P2B_HPAD, tid, vo);
         }
     }
+}
+
+// ---- values and best responses after the final pass -----------------------------------------------
+// The outputs of the final pass at a node and at the leaves below it, with the zero-sum shift where asked (:957-980: at every
+// node that does not end the hand, the mean over the players of sum_h values * beliefs).
+__global__ void __launch_bounds__(kRowThreads) split_values_kernel(const CfrParams p, const SplitWork w) {
+    __shared__ __align__(16) float prod[2][P2B_HPAD];
+    __shared__ float sums[2];
+    if (p.work_counter[1] != 0) return;
+    const int tid = threadIdx.x;
+    for (int x = blockIdx.x; x < w.total[0]; x += gridDim.x) {
+        const SplitItem& it = w.items[x];
+        const int leaf0 = p.leaf_begin ? p.leaf_begin[it.subgame] : 0;
+        auto shift_of = [&](const Row3& v0, const Row3& b0, const Row3& v1, const Row3& b1) {
+            __syncthreads();
+            st3(prod[0], tid, mul3(v0, b0));
+            st3(prod[1], tid, mul3(v1, b1));
+            __syncthreads();
+            if (tid < 64) {
+                const float sum = row_sum_reference_order(prod[tid >> 5]);
+                if ((tid & 31) == 0) sums[tid >> 5] = sum;
+            }
+            __syncthreads();
+            return __fmul_rn(__fadd_rn(sums[0], sums[1]), 0.5f);
+        };
+        auto minus = [&](Row3 v, float s) {
+#pragma unroll
+            for (int i = 0; i < kHandsPerThread; ++i) v.v[i] = __fsub_rn(v.v[i], s);
+            return v;
+        };
+        if (!p.values_avg && it.node != 0) continue;
+        {
+            const float* me = w.rec + (long long)(it.node_begin + it.node) * kRec;
+            Row3 v0 = ld3(me + kRecValue * P2B_HPAD, tid), v1 = ld3(me + (kRecValue + 1) * P2B_HPAD, tid);
+            if (p.enforce_zero_sum) {
+                const float s = shift_of(v0, ld3(me + kRecBelief * P2B_HPAD, tid), v1, ld3(me + (kRecBelief + 1) * P2B_HPAD, tid));
+                v0 = minus(v0, s);
+                v1 = minus(v1, s);
+            }
+            if (p.values_avg) {
+                float* out = p.values_avg + 2ll * (it.node_begin + it.node) * P2B_HPAD;
+                st3(out, tid, v0);
+                st3(out + P2B_HPAD, tid, v1);
+            }
+            if (it.node == 0) {
+                float* out = p.root_values + 2ll * it.subgame * P2B_HPAD;
+                st3(out, tid, v0);
+                st3(out + P2B_HPAD, tid, v1);
+            }
+        }
+        if (!p.values_avg) continue;
+        for (int c = 0; c < it.n_children; ++c) {
+            const int kind = it.kind[c];
+            if (kind == kInternal) continue;
+            const long long row = it.node_begin + it.first_child + c;
+            const NodeRec nd = load_node(p.nodes + row);
+            Row3 v0, v1;
+            if (kind == kShowdownLeaf) {
+                v0 = ld3(w.rec + row * kRec + kRecValue * P2B_HPAD, tid);
+                v1 = ld3(w.rec + row * kRec + (kRecValue + 1) * P2B_HPAD, tid);
+            } else {
+                const bool model = kind == kModelLeaf && p.leaf_values;
+                const float f = kind == kFoldLeaf ? nd.v0 : 0.0f;
+                const long long slot = 2ll * (leaf0 + nd.internal_idx) * P2B_HPAD;
+#pragma unroll
+                for (int i = 0; i < kHandsPerThread; ++i) {
+                    v0.v[i] = f;
+                    v1.v[i] = -f;
+                }
+                if (model) {
+                    v0 = ld3(p.leaf_values + slot, tid);
+                    v1 = ld3(p.leaf_values + slot + P2B_HPAD, tid);
+                }
+                if (p.enforce_zero_sum && kind == kModelLeaf && p.leaf_beliefs) {
+                    const float s = shift_of(v0, ld3(p.leaf_beliefs + slot, tid), v1, ld3(p.leaf_beliefs + slot + P2B_HPAD, tid));
+                    v0 = minus(v0, s);
+                    v1 = minus(v1, s);
+                }
+            }
+            float* out = p.values_avg + 2 * row * P2B_HPAD;
+            st3(out, tid, v0);
+            st3(out + P2B_HPAD, tid, v1);
+        }
+    }
+}
+
+// One level of the best-response sweeps (`_best_response_values`, :603-716) of both players: block (subgame, deviator, lane)
+// takes every lanes-th node of level d.  Where the deviator acts, its best action per hand decides which beliefs the other
+// player meets, whose per-card sums make the node's weights; elsewhere the weights are the final pass's own.  Values of
+// sweep 0 lie in the value rows of the final pass, those of sweep 1 in its belief rows, both spent by then.
+template <int MAXK>
+__global__ void __launch_bounds__(kRowThreads, 2) split_best_response_kernel(const CfrParams p, const SplitWork w, int d, int lanes) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* rows = reinterpret_cast<float*>(smem);  // beliefs of the acting player, then a row a child
+    double* cs = reinterpret_cast<double*>(smem + (1 + MAXK) * P2B_HPAD * 4);
+    double* S = cs + (1 + MAXK) * 52;
+    if (p.work_counter[1] != 0) return;
+    const int tid = threadIdx.x;
+    const int q = blockIdx.x / (2 * lanes), rest = blockIdx.x - q * 2 * lanes, deviator = rest / lanes;
+    const SplitLevels* lv = w.levels + q;
+    if (d >= lv->n_levels) return;
+    uint32_t idx[7];
+    card_indices(tid, idx);
+    const int mine = deviator == 0 ? kRecValue : kRecBelief;
+    for (int x = lv->begin[d] + rest - deviator * lanes; x < lv->begin[d + 1]; x += lanes) {
+        const SplitItem& it = w.items[lv->item_begin + x];
+        const int a = it.to_act, o = 1 - a, k = it.n_children;
+        const bool deviates = deviator == a;
+        float* me = w.rec + (long long)(it.node_begin + it.node) * kRec;
+        const float* kids = w.rec + (long long)(it.node_begin + it.first_child) * kRec;
+        auto value = [&](int c, int pl) {
+            if (it.kind[c] == kInternal) return ld3(kids + c * kRec + (mine + pl) * P2B_HPAD, tid);
+            Row3 v = ld3(p.values_avg + (2ll * (it.node_begin + it.first_child + c) + pl) * P2B_HPAD, tid);
+#pragma unroll
+            for (int i = 0; i < kHandsPerThread; ++i) v.v[i] = fminf(fmaxf(v.v[i], -1.0f), 1.0f);
+            return v;
+        };
+        Row3 acc_a, acc_o, b_a;
+        int best[kHandsPerThread];
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) {
+            acc_a.v[i] = acc_o.v[i] = b_a.v[i] = 0.0f;
+            best[i] = 0;
+        }
+        if (deviates) {
+            // best action per hand: the first maximum (argmax, :653-660)
+            acc_a = value(0, a);
+#pragma unroll 1
+            for (int c = 1; c < k; ++c) {
+                const Row3 v = value(c, a);
+#pragma unroll
+                for (int i = 0; i < kHandsPerThread; ++i)
+                    if (v.v[i] > acc_a.v[i]) {
+                        acc_a.v[i] = v.v[i];
+                        best[i] = c;
+                    }
+            }
+            b_a = ld3(me + kRecActing * P2B_HPAD, tid);
+            __syncthreads();  // the tables of the node before have been read
+            st3(rows, tid, b_a);
+#pragma unroll 1
+            for (int c = 0; c < k; ++c) {
+                Row3 m;
+#pragma unroll
+                for (int i = 0; i < kHandsPerThread; ++i) m.v[i] = best[i] == c ? b_a.v[i] : 0.0f;
+                st3(rows + (1 + c) * P2B_HPAD, tid, m);
+            }
+            __syncthreads();
+            card_sums(rows, 1 + k, cs, S, idx);
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (int c = 0; c < k; ++c) {
+            const Row3 Vo = value(c, o);
+            Row3 weight;
+            if (deviates) {
+#pragma unroll
+                for (int i = 0; i < kHandsPerThread; ++i) {
+                    const int h = tid + i * kRowThreads, hc = h < P2B_NUM_HANDS ? h : P2B_NUM_HANDS - 1;
+                    const int c1 = p.combos->c1[hc], c2 = p.combos->c2[hc];
+                    const float blk = unblocked(cs + (1 + c) * 52, S[1 + c], c1, c2, best[i] == c ? b_a.v[i] : 0.0f);
+                    const float den = unblocked(cs, S[0], c1, c2, b_a.v[i]);
+                    weight.v[i] = den > 1e-5f ? __fdiv_rn(blk, den) : 0.0f;
+                }
+            } else {
+                weight = ld3(kids + c * kRec + kRecSeen * P2B_HPAD, tid);
+                const Row3 P = ld3(kids + c * kRec + kRecPolicy * P2B_HPAD, tid), Va = value(c, a);
+#pragma unroll
+                for (int i = 0; i < kHandsPerThread; ++i) acc_a.v[i] = __fadd_rn(acc_a.v[i], __fmul_rn(Va.v[i], P.v[i]));
+            }
+#pragma unroll
+            for (int i = 0; i < kHandsPerThread; ++i) acc_o.v[i] = __fadd_rn(acc_o.v[i], __fmul_rn(weight.v[i], Vo.v[i]));
+        }
+        st3(me + (mine + a) * P2B_HPAD, tid, acc_a);
+        st3(me + (mine + o) * P2B_HPAD, tid, acc_o);
+    }
+}
+
+// Local exploitability (:718-764) from the root values of the two sweeps and of the plain expectation, which the up kernel has
+// left in the rows of the hand-over area where the root's prior was.
+__global__ void __launch_bounds__(kRowThreads) split_exploitability_kernel(const CfrParams p, const SplitWork w) {
+    __shared__ __align__(16) float prod[4][P2B_HPAD];
+    __shared__ float sums[4];
+    if (p.work_counter[1] != 0) return;
+    const int s = blockIdx.x, tid = threadIdx.x;
+    const float* cr = p.carry_roots + (long long)s * 4 * P2B_HPAD;
+    const float* root = w.rec + (long long)p.subgames[s].node_begin * kRec;
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        const Row3 rb = ld3(cr + (2 + d) * P2B_HPAD, tid), base = ld3(cr + d * P2B_HPAD, tid);
+        const Row3 best = ld3(root + ((d == 0 ? kRecValue : kRecBelief) + d) * P2B_HPAD, tid);
+        Row3 gain, value;
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) {
+            gain.v[i] = __fmul_rn(__fsub_rn(best.v[i], base.v[i]), rb.v[i]);
+            value.v[i] = __fmul_rn(best.v[i], rb.v[i]);
+        }
+        st3(prod[d], tid, gain);
+        st3(prod[2 + d], tid, value);
+    }
+    __syncthreads();
+    if (tid < 128) {
+        const float sum = row_sum_reference_order(prod[tid >> 5]);
+        if ((tid & 31) == 0) sums[tid >> 5] = sum;
+    }
+    __syncthreads();
+    if (tid == 0) p.exploitability[s] = __fadd_rn(sums[0], sums[1]);
+    if (tid < 2 && p.br_values) p.br_values[(long long)s * 2 + tid] = sums[2 + tid];
 }
 
 // Raises a kernel's shared-memory limit on the current device, once for each size it has not had there (the call takes as
@@ -1301,25 +1655,27 @@ int launch_pass_kernel(void (*kernel)(Params...), const char* name, unsigned gri
     return check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...), name);
 }
 
-template <int MAXK, bool SD, bool AVG>
+template <int MAXK, bool SD, int KIND>
 int launch_rows(const CfrParams& p, const SplitWork& w, int pass, bool follows, cudaStream_t stream) {
     constexpr int kBytes = row_layout(MAXK, SD).bytes;
     static_assert(kBytes <= 227 * 1024, "one block must fit an SM");
     static SharedLimit had;
-    int rc = allow_shared(had, reinterpret_cast<const void*>(split_rows_kernel<MAXK, SD, AVG>), kBytes);
+    int rc = allow_shared(had, reinterpret_cast<const void*>(split_rows_kernel<MAXK, SD, KIND>), kBytes);
     if (rc) return rc;
     const long long most = (long long)p.num_subgames * p.max_internal, fit = 2ll * sm_count();
-    return launch_pass_kernel(split_rows_kernel<MAXK, SD, AVG>, "split_rows_kernel", (unsigned)(most < fit ? most : fit), kRowThreads,
+    return launch_pass_kernel(split_rows_kernel<MAXK, SD, KIND>, "split_rows_kernel", (unsigned)(most < fit ? most : fit), kRowThreads,
                               kBytes, follows, stream, p, w, pass);
 }
 
-template <int MAXK>
-int launch_rows(const CfrParams& p, const SplitWork& w, int pass, bool avg, bool follows, cudaStream_t stream) {
-    if (p.tables)
-        return avg ? launch_rows<MAXK, true, true>(p, w, pass, follows, stream)
-                   : launch_rows<MAXK, true, false>(p, w, pass, follows, stream);
-    return avg ? launch_rows<MAXK, false, true>(p, w, pass, follows, stream)
-               : launch_rows<MAXK, false, false>(p, w, pass, follows, stream);
+template <int MAXK, int KIND>
+int launch_rows(const CfrParams& p, const SplitWork& w, int pass, bool follows, cudaStream_t stream) {
+    return p.tables ? launch_rows<MAXK, true, KIND>(p, w, pass, follows, stream)
+                    : launch_rows<MAXK, false, KIND>(p, w, pass, follows, stream);
+}
+template <int KIND>
+int launch_rows(const CfrParams& p, const SplitWork& w, int pass, int max_children, bool follows, cudaStream_t stream) {
+    return max_children <= kIterMaxChildren ? launch_rows<6, KIND>(p, w, pass, follows, stream)
+                                            : launch_rows<8, KIND>(p, w, pass, follows, stream);
 }
 
 template <int MODE>
@@ -1330,7 +1686,7 @@ int launch_prep(const CfrParams& p, const SplitWork& w, int pass, int max_childr
     return check_cuda(cudaGetLastError(), "split_prep_kernel");
 }
 
-int launch_up(const CfrParams& p, const SplitWork& w, int pass, bool advance, bool mixed, int max_children, bool follows,
+int launch_up(const CfrParams& p, const SplitWork& w, UpJob job, int pass, bool advance, bool mixed, int max_children, bool follows,
               cudaStream_t stream) {
     // Warps a slice: one warp's walk up a tree is the time of a small batch, so nodes of a level are spread over up to eight;
     // more warps than it takes to keep the memory busy only wait at the levels with few nodes.  Measured (us a pass; 8 / 4 /
@@ -1346,8 +1702,8 @@ int launch_up(const CfrParams& p, const SplitWork& w, int pass, bool advance, bo
     int rc = allow_shared(had, reinterpret_cast<const void*>(split_up_kernel), bytes);
     if (rc) return rc;
     const unsigned grid = (unsigned)p.num_subgames * (P2B_HPAD / kUpRow / slices);
-    return launch_pass_kernel(split_up_kernel, "split_up_kernel", grid, 32 * lanes * slices, bytes, follows, stream, p, w, pass, advance,
-                              mixed, lanes, slices, ring);
+    return launch_pass_kernel(split_up_kernel, "split_up_kernel", grid, 32 * lanes * slices, bytes, follows, stream, p, w, job, pass,
+                              advance, mixed, lanes, slices, ring);
 }
 
 }  // namespace
@@ -1361,12 +1717,13 @@ bool split_applies(const CfrParams& p, int max_children, long long scratch_float
            scratch_floats >= split_scratch_floats(p.num_subgames, p.rows);
 }
 
-int launch_split_passes(const CfrParams& p, int max_children, int pass_begin, int pass_end, bool down, bool up, cudaStream_t stream) {
+int launch_split_passes(const CfrParams& p, int max_children, int pass_begin, int pass_end, bool down, bool up, bool continued,
+                        cudaStream_t stream) {
     const SplitWork w = carve(p.scratch, p.num_subgames, p.rows);
     const bool avg = p.cfr_avg != 0 || p.iter_values != 0;
     int rc = P2B_OK;
     bool follows = false;
-    if (down) {
+    if (down && !continued) {
         split_items_kernel<<<p.num_subgames, kCfrMaxNodes, 0, stream>>>(p, w);
         rc = check_cuda(cudaGetLastError(), "split_items_kernel");
         if (!rc) rc = launch_prep<kPrepPolicy>(p, w, pass_begin, max_children, stream);
@@ -1378,16 +1735,60 @@ int launch_split_passes(const CfrParams& p, int max_children, int pass_begin, in
                 follows = false;
             }
             if (!rc)
-                rc = max_children <= kIterMaxChildren ? launch_rows<6>(p, w, pass, avg, follows, stream)
-                                                      : launch_rows<8>(p, w, pass, avg, follows, stream);
+                rc = avg ? launch_rows<kRowAvg>(p, w, pass, max_children, follows, stream)
+                         : launch_rows<kRowIter>(p, w, pass, max_children, follows, stream);
             follows = true;
         }
         if (!rc && (pass < pass_end || up)) {
-            rc = launch_up(p, w, pass, pass < pass_end, avg, max_children, follows, stream);
+            rc = launch_up(p, w, kUpIter, pass, pass < pass_end, avg, max_children, follows, stream);
             follows = true;
         }
     }
     return rc;
+}
+
+int launch_split_start(const CfrParams& p, int max_children, bool down, bool up, bool advance, cudaStream_t stream) {
+    const SplitWork w = carve(p.scratch, p.num_subgames, p.rows);
+    int rc = P2B_OK;
+    if (down) {
+        split_items_kernel<<<p.num_subgames, kCfrMaxNodes, 0, stream>>>(p, w);
+        rc = check_cuda(cudaGetLastError(), "split_items_kernel");
+        if (!rc) rc = launch_rows<kRowStart>(p, w, 0, max_children, false, stream);
+    }
+    if (!rc && up) rc = launch_up(p, w, kUpStart, -1, advance, true, max_children, down, stream);
+    return rc;
+}
+
+int launch_split_final(const CfrParams& p, int max_children, bool down, bool up, bool best_responses, cudaStream_t stream) {
+    const SplitWork w = carve(p.scratch, p.num_subgames, p.rows);
+    const int B = p.num_subgames, sms = sm_count();
+    int rc = P2B_OK;
+    if (down) rc = launch_rows<kRowFinal>(p, w, p.iterations, max_children, false, stream);
+    if (!rc && up) {
+        rc = launch_up(p, w, kUpFinal, p.iterations, false, true, max_children, down, stream);
+        if (rc) return rc;
+        const long long most = (long long)B * p.max_internal, fit = 4ll * sms;
+        split_values_kernel<<<(unsigned)(most < fit ? most : fit), kRowThreads, 0, stream>>>(p, w);
+        rc = check_cuda(cudaGetLastError(), "split_values_kernel");
+    }
+    if (rc || !best_responses || !p.exploitability || !p.values_avg) return rc;
+    rc = launch_up(p, w, kUpBase, p.iterations, false, true, max_children, false, stream);
+    if (rc) return rc;
+    // as many blocks a subgame and sweep as it takes to fill the chip, up to a level's worth of nodes
+    int lanes = sms / B;
+    lanes = lanes < 1 ? 1 : lanes > 16 ? 16 : lanes;
+    const bool wide = max_children > kIterMaxChildren;
+    const auto kernel = wide ? split_best_response_kernel<kCfrMaxChildren> : split_best_response_kernel<kIterMaxChildren>;
+    const int bytes = (1 + (wide ? kCfrMaxChildren : kIterMaxChildren)) * (P2B_HPAD * 4 + 52 * 8 + 8);
+    static SharedLimit had[2];
+    rc = allow_shared(had[wide], reinterpret_cast<const void*>(kernel), bytes);
+    for (int d = p.init_depth; d >= 0 && !rc; --d) {
+        kernel<<<(unsigned)(B * 2 * lanes), kRowThreads, bytes, stream>>>(p, w, d, lanes);
+        rc = check_cuda(cudaGetLastError(), "split_best_response_kernel");
+    }
+    if (rc) return rc;
+    split_exploitability_kernel<<<(unsigned)B, kRowThreads, 0, stream>>>(p, w);
+    return check_cuda(cudaGetLastError(), "split_exploitability_kernel");
 }
 
 }  // namespace p2b
