@@ -988,59 +988,22 @@ __device__ __forceinline__ void showdown_tables(const BoardTabView& tv, const fl
     }
 }
 
-// Showdown EV (before the pot scaling) of this thread's hands against the two ranges: the formula of showdown_hand_ev, a
-// hand's positions in the tables unpacked once for both.
+// Showdown EV (before the pot scaling) of this thread's hands against the two ranges.
 __device__ __forceinline__ void showdown_rows(const BoardTabView& tv, const float* x0, const float* x1, const float2* pref,
                                               const float2* pc, const float2* tot, const Hands& hi, Row3& ev0, Row3& ev1) {
-    const int tid = threadIdx.x;
     DivGuard g = guard_begin(true);
-    auto one = [&](float PL, float PR, float C1, float D1, float C2, float D2, float T1, float T2, float xh, bool allowed) {
-        const float win = __fsub_rn(__fsub_rn(PL, C1), C2);
-        const float tie = __fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(PR, PL), __fsub_rn(D1, C1)), __fsub_rn(D2, C2)), xh);
-        const float den = fmaxf(__fadd_rn(__fsub_rn(__fsub_rn(1.0f, T1), T2), xh), 1e-8f);
-        const Divisor d = make_divisor(den);
-        g.dok = g.dok && d.ok;
-        const float wp = div_g<false>(win, d.y, d.r, g), tp = div_g<false>(tie, d.y, d.r, g);
-        const float ev = __fsub_rn(wp, __fsub_rn(__fsub_rn(1.0f, wp), tp));
-        return (allowed && den > 1e-8f) ? ev : 0.0f;
-    };
 #pragma unroll
     for (int i = 0; i < kHandsPerThread; ++i) {
-        const int h = tid + i * kRowThreads, hc = hi.real[i] ? h : 0;
-        const uint2 rec = *reinterpret_cast<const uint2*>(tv.rec + hc);
-        const float2 PL = pref[rec.x & 0xffffu], PR = pref[rec.x >> 16];
-        const float2* r1 = pc + hi.c1[i] * 52;
-        const float2* r2 = pc + hi.c2[i] * 52;
-        const float2 C1 = r1[rec.y & 0xff], D1 = r1[(rec.y >> 8) & 0xff], C2 = r2[(rec.y >> 16) & 0xff], D2 = r2[rec.y >> 24];
-        const float2 T1 = tot[hi.c1[i]], T2 = tot[hi.c2[i]];
-        ev0.v[i] = one(PL.x, PR.x, C1.x, D1.x, C2.x, D2.x, T1.x, T2.x, x0[h], hi.allowed[i]);
-        ev1.v[i] = one(PL.y, PR.y, C1.y, D1.y, C2.y, D2.y, T1.y, T2.y, x1[h], hi.allowed[i]);
+        const int h = threadIdx.x + i * kRowThreads;
+        showdown_hand_pair<false>(*reinterpret_cast<const uint2*>(tv.rec + (hi.real[i] ? h : 0)), hi.c1[i], hi.c2[i], x0[h], x1[h],
+                                  hi.allowed[i], pref, pc, tot, g, ev0.v[i], ev1.v[i]);
     }
-    if (__builtin_expect(guard_bad(g), 0)) {  // the same with IEEE divisions
-#pragma unroll 1
+    if (__builtin_expect(guard_bad(g), 0)) {
+#pragma unroll
         for (int i = 0; i < kHandsPerThread; ++i) {
-            const int h = tid + i * kRowThreads;
-            const HandRec rec = tv.rec[h < P2B_NUM_HANDS ? h : 0];
-            const int c1 = i == 0 ? hi.c1[0] : i == 1 ? hi.c1[1] : hi.c1[2], c2 = i == 0 ? hi.c2[0] : i == 1 ? hi.c2[1] : hi.c2[2];
-            const bool allowed = i == 0 ? hi.allowed[0] : i == 1 ? hi.allowed[1] : hi.allowed[2];
-#pragma unroll 1
-            for (int slot = 0; slot < 2; ++slot) {
-                auto at = [&](const float2& t) { return slot ? t.y : t.x; };
-                const float PL = at(pref[rec.lpos]), PR = at(pref[rec.rpos]);
-                const float C1 = at(pc[c1 * 52 + rec.nb0]), D1 = at(pc[c1 * 52 + rec.ne0]);
-                const float C2 = at(pc[c2 * 52 + rec.nb1]), D2 = at(pc[c2 * 52 + rec.ne1]);
-                const float xh = (slot ? x1 : x0)[h];
-                const float win = __fsub_rn(__fsub_rn(PL, C1), C2);
-                const float tie = __fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(PR, PL), __fsub_rn(D1, C1)), __fsub_rn(D2, C2)), xh);
-                const float den = fmaxf(__fadd_rn(__fsub_rn(__fsub_rn(1.0f, at(tot[c1])), at(tot[c2])), xh), 1e-8f);
-                const float wp = __fdiv_rn(win, den), tp = __fdiv_rn(tie, den);
-                const float e = __fsub_rn(wp, __fsub_rn(__fsub_rn(1.0f, wp), tp));
-                const float ev = (allowed && den > 1e-8f) ? e : 0.0f;
-                Row3& out = slot ? ev1 : ev0;
-                if (i == 0) out.v[0] = ev;
-                else if (i == 1) out.v[1] = ev;
-                else out.v[2] = ev;
-            }
+            const int h = threadIdx.x + i * kRowThreads;
+            showdown_hand_pair<true>(*reinterpret_cast<const uint2*>(tv.rec + (hi.real[i] ? h : 0)), hi.c1[i], hi.c2[i], x0[h], x1[h],
+                                     hi.allowed[i], pref, pc, tot, g, ev0.v[i], ev1.v[i]);
         }
     }
 }
@@ -1171,8 +1134,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
     launch_next();
     bool waited = false;
     // a block takes consecutive items: mostly nodes of one subgame, whose board tables stay in shared memory
-    const int total = w.total[0], each = (total + gridDim.x - 1) / gridDim.x;
-    const int first = blockIdx.x * each, last = min(first + each, total);
+    const long long total = w.total[0];
+    const int first = (int)(blockIdx.x * total / gridDim.x), last = (int)((blockIdx.x + 1) * total / gridDim.x);
     int table = -1;
     for (int x = first; x < last; ++x) {
         __syncthreads();  // every thread is done with the shared memory of the item before

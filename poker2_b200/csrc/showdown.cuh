@@ -84,4 +84,37 @@ __device__ __forceinline__ float showdown_hand_ev(const HandRec r, int c1, int c
     return showdown_hand_ev(r, c1, c2, xh, allowed, P, PC, PC[c1 * 52 + 51], PC[c2 * 52 + 51]);
 }
 
+// The same for two ranges whose tables lie side by side (x: the first range's entry, y: the second's), so that one gather
+// of a hand's position serves both.  The quotients go through the short sequence; the caller collects its guard over a
+// group of hands and redoes the group with IEEE = true if it asks for it.
+template <bool IEEE>
+__device__ __forceinline__ void showdown_hand_pair(uint2 rec, int c1, int c2, float x0, float x1, bool allowed,
+                                                   const float2* __restrict__ P, const float2* __restrict__ PC,
+                                                   const float2* __restrict__ tot, DivGuard& g, float& ev0, float& ev1) {
+    const float2 PL = P[rec.x & 0xffffu], PR = P[rec.x >> 16];  // the fields of HandRec
+    const float2* r1 = PC + c1 * 52;
+    const float2* r2 = PC + c2 * 52;
+    const float2 a0 = r1[rec.y & 0xffu], a1 = r1[(rec.y >> 8) & 0xffu], b0 = r2[(rec.y >> 16) & 0xffu], b1 = r2[rec.y >> 24];
+    const float2 t1 = tot[c1], t2 = tot[c2];
+    auto one = [&](float pl, float pr, float c, float d, float e, float f, float u, float v, float x) {
+        const float win = __fsub_rn(__fsub_rn(pl, c), e);
+        const float tie = __fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(pr, pl), __fsub_rn(d, c)), __fsub_rn(f, e)), x);
+        const float den = fmaxf(__fadd_rn(__fsub_rn(__fsub_rn(1.0f, u), v), x), 1e-8f);
+        float wp, tp;
+        if (IEEE) {
+            wp = __fdiv_rn(win, den);
+            tp = __fdiv_rn(tie, den);
+        } else {
+            const Divisor y = make_divisor(den);
+            g.dok = g.dok && y.ok;
+            wp = div_g<false>(win, y.y, y.r, g);
+            tp = div_g<false>(tie, y.y, y.r, g);
+        }
+        const float ev = __fsub_rn(wp, __fsub_rn(__fsub_rn(1.0f, wp), tp));
+        return (allowed && den > 1e-8f) ? ev : 0.0f;
+    };
+    ev0 = one(PL.x, PR.x, a0.x, a1.x, b0.x, b1.x, t1.x, t2.x, x0);
+    ev1 = one(PL.y, PR.y, a0.y, a1.y, b0.y, b1.y, t1.y, t2.y, x1);
+}
+
 }  // namespace p2b
