@@ -32,10 +32,13 @@ int p2b_version(void);
 /* rank_7_cards_single_batch_triton (rules_triton.py:96-117): cards [n,7] int16 ids
  * 0..51 -> out [n] int32 packed score type<<20|k1<<16|..|k5. */
 int p2b_rank7_cards(const int16_t* cards, int64_t n, int32_t* out, void* stream);
+/* the same on int64 ids (of which the low 16 bits count), without a converted copy */
+int p2b_rank7_cards_i64(const int64_t* cards, int64_t n, int32_t* out, void* stream);
 
 /* compare_7_cards_single_batch_triton (rules_triton.py:78-93): cards [n,2,7] int16 ->
  * out [n] int32 in {1,-1,0}. */
 int p2b_compare7_cards(const int16_t* cards, int64_t n, int32_t* out, void* stream);
+int p2b_compare7_cards_i64(const int64_t* cards, int64_t n, int32_t* out, void* stream);
 
 /* compare_7_single_batch_triton (rules_triton.py:36-51): planes [n,2,4,13] int8 one-hot
  * -> out [n] int32 in {1,-1,0}. */
@@ -57,6 +60,10 @@ int p2b_showdown_values(const unsigned char* tables, const int32_t* table_of_row
                         const float* beliefs, int64_t belief_row_stride,
                         const int64_t* potential, const float* scale, float* values,
                         int64_t value_row_stride, int64_t rows, void* stream);
+/* the same on rows row_index[i] of beliefs and values (i < rows; potential, scale and table_of_row stay by i) */
+int p2b_showdown_values_at(const unsigned char* tables, const int32_t* table_of_row, const int64_t* row_index,
+                           const float* beliefs, int64_t belief_row_stride, const int64_t* potential, const float* scale,
+                           float* values, int64_t value_row_stride, int64_t rows, void* stream);
 
 /* showdown_ev_triton (src/p2/search/fused_cfr_triton.py:2271-2320): the EV of every strength-sorted
  * position straight from sorted-order inputs, `rows` rows of `hands` (<= 1344) entries each:
@@ -366,6 +373,30 @@ int p2b_step_reach_weights(float* reach, const float* policy, const uint8_t* all
 int p2b_step_deep_beliefs(float* out, const float* root_beliefs, const float* reach, const float* allowed_prob,
                           const int64_t* root_index, int64_t num_roots, int64_t total, int32_t H, float eps,
                           void* stream);
+
+/* ---- whole steps of one iteration (step_evaluator.StepCFREvaluator) -------------------------
+ * Arrays in the upstream layout with rows of 1326: [M,H] or [M,2,H] fp32, level-major topology (children of a node
+ * consecutive; child_offsets / child_count / to_act of the first num_parents nodes), index arrays int64.
+ *  p2b_steps_regrets  instantaneous regrets (cfr_evaluator.py:1117-1165), the discounted update of cumulative and
+ *                     weight_sums (:1346-1368) and regret matching into policy (:1168-1185); scalars4 = {t^a, t^b,
+ *                     t^a+1, t^b+1}; uniform = the policy where no regret is positive
+ *  p2b_steps_reach    reach [M,2,H] under `policy` (:332-361) and, unless beliefs is NULL, beliefs [M,2,H] = prior
+ *                     [roots,2,H] x reach, normalised (:363-380).  path [M,depth] int32: 2 * node + acting player of
+ *                     every node from below the root down to the row's own, -1 behind the last.  prior and beliefs
+ *                     must not overlap
+ *  p2b_steps_average  average-policy mix and renormalisation (:1195-1258)
+ *  p2b_steps_seen     policy of every child as each hand of the player who does not choose sees it (:1076-1093) */
+int p2b_steps_regrets(const float* values, const float* beliefs, const int64_t* to_act, const int64_t* child_offsets,
+                      const int64_t* child_count, const float* uniform, const float* scalars4, float* cumulative,
+                      float* weight_sums, float* policy, int64_t num_roots, int64_t num_parents, int apply_dcfr, int cfr_plus,
+                      void* stream);
+int p2b_steps_reach(const float* policy, const uint8_t* allowed, const float* allowed_prob, const int32_t* path, int32_t depth,
+                    const int64_t* root_index, const float* prior, float* reach, float* beliefs, int64_t nodes, void* stream);
+int p2b_steps_average(const float* reach, const float* reach_avg, const float* policy, const int64_t* to_act,
+                      const int64_t* child_offsets, const int64_t* child_count, const float* old_w, const float* new_w,
+                      const float* total_w, float* policy_avg, int64_t num_parents, void* stream);
+int p2b_steps_seen(const float* beliefs, const float* policy, const int64_t* to_act, const int64_t* child_offsets,
+                   const int64_t* child_count, float* seen, int64_t num_parents, void* stream);
 
 /* ---- chance nodes (src/p2/search/chance_node_helper.py:359-479, single_card_chance_values) --
  * p2b_chance_expand: for each root b, one sample per card not on its board (ascending card

@@ -27,9 +27,12 @@ _f32 = ctypes.c_float
 _SIGNATURES = {
     "p2b_rank7_cards": [_vp, _i64, _vp, _vp],
     "p2b_compare7_cards": [_vp, _i64, _vp, _vp],
+    "p2b_rank7_cards_i64": [_vp, _i64, _vp, _vp],
+    "p2b_compare7_cards_i64": [_vp, _i64, _vp, _vp],
     "p2b_compare7_planes": [_vp, _i64, _vp, _vp],
     "p2b_rank_hands": [_vp, _i64, _vp, _vp, _vp, _vp],
     "p2b_showdown_values": [_vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _vp],
+    "p2b_showdown_values_at": [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _vp],
     "p2b_showdown_ev_sorted": [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _vp, _vp],
     "p2b_cfr_solve": [_vp, _vp, _i32, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64,
                       _vp, _i32, _i32, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _f32, _vp],
@@ -58,6 +61,10 @@ _SIGNATURES = {
     "p2b_step_weighted_parent_sum": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _vp],
     "p2b_step_reach_weights": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _vp],
     "p2b_step_deep_beliefs": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _f32, _vp],
+    "p2b_steps_regrets": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i32, _vp],
+    "p2b_steps_reach": [_vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _i64, _vp],
+    "p2b_steps_average": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp],
+    "p2b_steps_seen": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp],
     "p2b_chance_expand": [_vp, _vp, _i32, _vp, _i64, _i64, _vp, _vp, _vp, _vp],
     "p2b_indexed_add_rows": [_vp, _vp, _vp, _i64, _i64, _i64, _i32, _i32, _vp],
     "p2b_chance_expand_features": [_vp, _i64, _vp, _i32, _vp, _i64, _i64, _vp, _vp, _i64, _vp, _vp],

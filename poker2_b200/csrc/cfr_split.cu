@@ -770,8 +770,6 @@ __global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p,
 //
 // 448 threads with three hands each, a third of a row apart: consecutive threads touch consecutive hands in global
 // and shared memory, and two blocks fit an SM (72 registers a thread).
-constexpr int kRowThreads = 448, kHandsPerThread = 3;
-static_assert(kRowThreads * kHandsPerThread == P2B_HPAD, "rows are covered exactly");
 constexpr int kScanQuarter = 352;  // 32 lanes x 11 sorted positions
 
 struct RowLayout {  // byte offsets into dynamic shared memory
@@ -850,66 +848,6 @@ __device__ __forceinline__ Row3 normalised(Row3 x, float sum, float allowed_prob
 #pragma unroll
     for (int i = 0; i < kHandsPerThread; ++i) q.v[i] = sum > 1e-5f ? q.v[i] : (hi.allowed[i] ? allowed_prob : 0.0f);
     return q;
-}
-
-// Per-card sums and totals of the rows 0 .. n_cs-1 (cs, S).  Thread t < 416 adds quarter (t / 4 mod 52, t mod 4) of
-// the 51 hands that hold a card, for the even or (t >= 208) the odd rows: the indices of its 13 hands belong to the
-// thread for the whole kernel and are held in registers as byte offsets, two to a word.
-__device__ __forceinline__ void card_indices(int tid, uint32_t (&idx)[7]) {
-    const int u = tid >= 208 ? tid - 208 : tid, c = (u >> 2) % 52, q = u & 3;
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        uint32_t word = 0;
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const int e = q + 4 * (2 * i + b);
-            if (2 * i + b < 13 && e < 51)
-                word |= (uint32_t)(4 * (e < c ? combo_index(e, c) : combo_row_offset(c) - c + e)) << (16 * b);
-        }
-        idx[i] = word;
-    }
-}
-__device__ __forceinline__ void card_sums(const float* rows, int n_cs, double* cs, double* S, const uint32_t (&idx)[7]) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int half = tid >= 208 ? 1 : 0, u = tid - 208 * half, c = u >> 2, q = u & 3;
-    if (tid < 416) {
-        for (int r0 = 0; r0 < n_cs; r0 += 2) {
-            const int r = r0 + half;
-            const bool live = r < n_cs;
-            const char* __restrict__ x = reinterpret_cast<const char*>(rows + (live ? r : 0) * P2B_HPAD);
-            float v[13];
-#pragma unroll
-            for (int i = 0; i < 12; ++i)
-                v[i] = *reinterpret_cast<const float*>(x + (i & 1 ? idx[i >> 1] >> 16 : idx[i >> 1] & 0xffffu));
-            v[12] = q < 3 ? *reinterpret_cast<const float*>(x + idx[6]) : 0.0f;
-            double t_even = 0.0, t_odd = 0.0;
-#pragma unroll
-            for (int i = 0; i < 13; ++i) {
-                if (i & 1) t_odd += (double)v[i];
-                else t_even += (double)v[i];
-            }
-            const double mine = t_even + t_odd;
-            const int g = lane & ~3;
-            const double t0 = __shfl_sync(0xffffffffu, mine, g), t1 = __shfl_sync(0xffffffffu, mine, g + 1);
-            const double t2 = __shfl_sync(0xffffffffu, mine, g + 2), t3 = __shfl_sync(0xffffffffu, mine, g + 3);
-            if (live && q == 0) cs[r * 52 + c] = ((t0 + t1) + t2) + t3;
-        }
-    }
-    // total mass of a row, a warp each from the last one down (the 18 padding entries are zero)
-    for (int r = kRowThreads / 32 - 1 - warp; r < n_cs; r += kRowThreads / 32) {
-        const float* __restrict__ x = rows + r * P2B_HPAD;
-        double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-        for (int b = 0; b < 7; ++b) {
-            float v[6];
-#pragma unroll
-            for (int i = 0; i < 6; ++i) v[i] = x[lane + 32 * (6 * b + i)];
-#pragma unroll
-            for (int i = 0; i < 6; ++i) acc[i] += (double)v[i];
-        }
-        const double tot = warp_sum(((acc[0] + acc[1]) + (acc[2] + acc[3])) + (acc[4] + acc[5]));
-        if (lane == 0) S[r] = tot;
-    }
 }
 
 // Tables of the showdown formula for two ranges (x: the other player's beliefs x0, y: the leaf row x1), their entries side by

@@ -1,7 +1,9 @@
 // Hand-ranking kernels: packed score of [N,7] card ids, pairwise comparison of card-id
-// and one-hot-plane hands.  HBM-bound by design: 14 B in + 4 B out per hand; a thread owns
-// four consecutive hands (56 B, seven 8-byte loads) and prefetches its next four while it
-// scores the current ones.
+// and one-hot-plane hands.  A thread owns four consecutive hands (int16: 56 B, seven 8-byte loads;
+// int64: 224 B, fourteen 16-byte loads) and fetches its next four while it scores the current ones.
+// int64 ids are read as they are: their converted copy cost a pass over memory and a launch (300,000 hands 19 us, now 10).
+#include <atomic>
+
 #include "common.cuh"
 #include "rank7.cuh"
 
@@ -9,31 +11,13 @@ namespace p2b {
 
 constexpr int kRankThreads = 256;
 constexpr int kHandsPerThread = 4;
-constexpr int kTileHands = kRankThreads * kHandsPerThread;  // 1024 hands = 14336 B per tile
 
-// cards: [n,7] int16; out: [n] int32.  VEC = base pointer is 8-byte aligned.
-// A block keeps the 32 KB rank table, the type table and a card -> suit-lane-bit table in
-// shared memory; a hand of distinct cards is scored by the table walk of rank7.cuh
-// (score_distinct_lut), a hand with repeated ids by the general bit-mask scorer.
-template <bool VEC>
-__global__ void __launch_bounds__(kRankThreads) rank7_cards_kernel(const int16_t* __restrict__ cards,
-                                                                   int32_t* __restrict__ out, int64_t n,
-                                                                   const RankLut* __restrict__ lut) {
-    __shared__ __align__(16) uint32_t T[kRankLutEntries];
-    __shared__ uint32_t TT[32];
-    {
-        const uint4* src = reinterpret_cast<const uint4*>(lut->mask_entry);
-        for (int i = threadIdx.x; i < kRankLutEntries / 4; i += kRankThreads) reinterpret_cast<uint4*>(T)[i] = __ldg(src + i);
-        if (threadIdx.x < 32) TT[threadIdx.x] = threadIdx.x < kTypeLutEntries ? lut->type_entry[threadIdx.x] : 0u;
-    }
-    __syncthreads();
-    // A thread takes four consecutive hands: 56 bytes = seven 8-byte words (VEC: 8-byte aligned),
-    // read straight from global memory; the words of its next tile are fetched while the current
-    // four hands are scored, so no barrier separates loading from scoring.
-    const int64_t num_tiles = (n + kTileHands - 1) / kTileHands;
-    auto load_words = [&](int64_t t, uint32_t (&w)[14]) {
-        const int64_t h0 = t * kTileHands + kHandsPerThread * threadIdx.x;
-        if (t < num_tiles && VEC && h0 + kHandsPerThread <= n) {
+// The 28 card ids of hands h0 .. h0+3 as 14 words of two 16-bit ids (ids beyond hand n: 0).  T = int16_t or int64_t, of
+// which the low 16 bits count; VEC: the base pointer is aligned for the wide loads.
+template <typename T, bool VEC>
+__device__ __forceinline__ void load_words(const T* __restrict__ cards, int64_t h0, int64_t n, uint32_t (&w)[14]) {
+    if (VEC && h0 + kHandsPerThread <= n) {
+        if constexpr (sizeof(T) == 2) {
             const uint2* mine = reinterpret_cast<const uint2*>(cards + h0 * 7);
 #pragma unroll
             for (int i = 0; i < 7; ++i) {
@@ -42,76 +26,113 @@ __global__ void __launch_bounds__(kRankThreads) rank7_cards_kernel(const int16_t
                 w[2 * i + 1] = v.y;
             }
         } else {
+            const uint4* mine = reinterpret_cast<const uint4*>(cards + h0 * 7);
 #pragma unroll
             for (int i = 0; i < 14; ++i) {
-                const int64_t e = h0 * 7 + 2 * i;
-                const uint32_t a0 = (t < num_tiles && e < n * 7) ? (uint16_t)cards[e] : 0u;
-                const uint32_t a1 = (t < num_tiles && e + 1 < n * 7) ? (uint16_t)cards[e + 1] : 0u;
-                w[i] = a0 | (a1 << 16);
+                const uint4 v = __ldcs(mine + i);
+                w[i] = __byte_perm(v.x, v.z, 0x5410);
             }
         }
-    };
-    uint32_t w[14], wn[14];
-    load_words(blockIdx.x, w);
-    for (int64_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-        const int64_t hand0 = t * kTileHands;
-        const int64_t remaining = n - hand0;
-        const int hands = remaining < kTileHands ? (int)remaining : kTileHands;
-        load_words(t + gridDim.x, wn);
-        // card id -> bit position in the four 16-bit suit lanes (id + 3 * suit), for both 16-bit
-        // halves of a word at once: (id * 79) >> 10 is id / 13 for ids below 52 and the product
-        // of the low half cannot carry into the high half
-        uint32_t bp[14];
+    } else {
 #pragma unroll
-        for (int k = 0; k < 14; ++k) bp[k] = w[k] + 3u * (((w[k] * 79u) >> 10) & 0x003F003Fu);
-        int32_t score[kHandsPerThread];
+        for (int i = 0; i < 14; ++i) {
+            const int64_t e = h0 * 7 + 2 * i;
+            const uint32_t a0 = e < n * 7 ? (uint16_t)cards[e] : 0u;
+            const uint32_t a1 = e + 1 < n * 7 ? (uint16_t)cards[e + 1] : 0u;
+            w[i] = a0 | (a1 << 16);
+        }
+    }
+}
+
+// Scores of the four hands in w; rank(m0, m1, m2, m3) scores a hand of distinct cards from its suit masks.
+template <typename Rank>
+__device__ __forceinline__ void score_four(const uint32_t (&w)[14], int32_t (&score)[kHandsPerThread], Rank&& rank) {
+    // card id -> bit position in the four 16-bit suit lanes (id + 3 * suit), for both 16-bit
+    // halves of a word at once: (id * 79) >> 10 is id / 13 for ids below 52 and the product
+    // of the low half cannot carry into the high half
+    uint32_t bp[14];
 #pragma unroll
-        for (int j = 0; j < kHandsPerThread; ++j) {
-            uint32_t lo = 0, hi = 0;
+    for (int k = 0; k < 14; ++k) bp[k] = w[k] + 3u * (((w[k] * 79u) >> 10) & 0x003F003Fu);
+#pragma unroll
+    for (int j = 0; j < kHandsPerThread; ++j) {
+        uint32_t lo = 0, hi = 0;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            const int e = 7 * j + i;  // 16-bit element of the thread's 28
+            const uint32_t bit = (e & 1) ? (bp[e >> 1] >> 16) : (bp[e >> 1] & 0xffffu);
+            uint32_t blo, bhi;  // 1 << bit as two words: shl.b32 gives 0 for shift counts above 31
+            asm("shl.b32 %0, 1, %1;" : "=r"(blo) : "r"(bit));
+            asm("shl.b32 %0, 1, %1;" : "=r"(bhi) : "r"(bit - 32u));
+            lo |= blo;
+            hi |= bhi;
+        }
+        const uint32_t m0 = lo & 0x1fffu, m1 = (lo >> 16) & 0x1fffu, m2 = hi & 0x1fffu, m3 = (hi >> 16) & 0x1fffu;
+        if (__popc(lo) + __popc(hi) == 7) {
+            score[j] = rank(m0, m1, m2, m3);
+        } else {  // repeated (or out-of-range) ids: the general scorer on the ids themselves
+            int c[7];
 #pragma unroll
             for (int i = 0; i < 7; ++i) {
-                const int e = 7 * j + i;  // 16-bit element of the thread's 28
-                const uint32_t bit = (e & 1) ? (bp[e >> 1] >> 16) : (bp[e >> 1] & 0xffffu);
-                uint32_t blo, bhi;  // 1 << bit as two words: shl.b32 gives 0 for shift counts above 31
-                asm("shl.b32 %0, 1, %1;" : "=r"(blo) : "r"(bit));
-                asm("shl.b32 %0, 1, %1;" : "=r"(bhi) : "r"(bit - 32u));
-                lo |= blo;
-                hi |= bhi;
+                const int e = 7 * j + i;
+                c[i] = (int)(int16_t)((e & 1) ? (w[e >> 1] >> 16) : (w[e >> 1] & 0xffffu));
             }
-            if (__popc(lo) + __popc(hi) == 7) {
-                score[j] = score_distinct_lut(lo & 0x1fffu, (lo >> 16) & 0x1fffu, hi & 0x1fffu, (hi >> 16) & 0x1fffu, T, TT);
-            } else {  // repeated (or out-of-range) ids: the general scorer on the ids themselves
-                int c[7];
-#pragma unroll
-                for (int i = 0; i < 7; ++i) {
-                    const int e = 7 * j + i;
-                    c[i] = (int)(int16_t)((e & 1) ? (w[e >> 1] >> 16) : (w[e >> 1] & 0xffffu));
-                }
-                score[j] = score_cards<7>(c);
-            }
+            score[j] = score_cards<7>(c);
         }
-        const int h0 = kHandsPerThread * threadIdx.x;
-        if (h0 + kHandsPerThread <= hands && ((reinterpret_cast<uintptr_t>(out + hand0) & 15) == 0)) {
-            __stcs(reinterpret_cast<int4*>(out + hand0 + h0), make_int4(score[0], score[1], score[2], score[3]));
-        } else {
+    }
+}
+
+__device__ __forceinline__ void store_four(int32_t* __restrict__ out, int64_t h0, int64_t n, const int32_t (&score)[kHandsPerThread]) {
+    if (h0 + kHandsPerThread <= n && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
+        __stcs(reinterpret_cast<int4*>(out + h0), make_int4(score[0], score[1], score[2], score[3]));
+    } else {
 #pragma unroll
-            for (int j = 0; j < kHandsPerThread; ++j)
-                if (h0 + j < hands) out[hand0 + h0 + j] = score[j];
-        }
+        for (int j = 0; j < kHandsPerThread; ++j)
+            if (h0 + j < n) out[h0 + j] = score[j];
+    }
+}
+
+// cards: [n,7]; out: [n] int32.  A block's threads take consecutive groups of four hands, one grid's worth at a time.
+template <typename T, bool VEC, typename Rank>
+__device__ __forceinline__ void rank_all(const T* __restrict__ cards, int32_t* __restrict__ out, int64_t n, Rank&& rank) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x * kHandsPerThread;
+    int64_t h0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kHandsPerThread;
+    uint32_t w[14], wn[14];
+    load_words<T, VEC>(cards, h0, n, w);
+    for (; h0 < n; h0 += step) {
+        load_words<T, VEC>(cards, h0 + step, n, wn);
+        int32_t score[kHandsPerThread];
+        score_four(w, score, rank);
+        store_four(out, h0, n, score);
 #pragma unroll
         for (int i = 0; i < 14; ++i) w[i] = wn[i];
     }
 }
 
-// cards: [n,2,7] int16 -> {1,-1,0}
-__global__ void __launch_bounds__(256) compare7_cards_kernel(const int16_t* __restrict__ cards,
-                                                            int32_t* __restrict__ out, int64_t n) {
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(kRankThreads) rank7_cards_kernel(const T* __restrict__ cards, int32_t* __restrict__ out,
+                                                                   int64_t n, const RankLut* __restrict__ lut) {
+    __shared__ __align__(16) uint32_t table[kRankLutEntries];
+    __shared__ uint32_t types[32];
+    {
+        const uint4* src = reinterpret_cast<const uint4*>(lut->mask_entry);
+        for (int i = threadIdx.x; i < kRankLutEntries / 4; i += kRankThreads) reinterpret_cast<uint4*>(table)[i] = __ldg(src + i);
+        if (threadIdx.x < 32) types[threadIdx.x] = threadIdx.x < kTypeLutEntries ? lut->type_entry[threadIdx.x] : 0u;
+    }
+    __syncthreads();
+    rank_all<T, VEC>(cards, out, n, [&](uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+        return score_distinct_lut(m0, m1, m2, m3, table, types);
+    });
+}
+
+// cards: [n,2,7] -> {1,-1,0}
+template <typename T>
+__global__ void __launch_bounds__(256) compare7_cards_kernel(const T* __restrict__ cards, int32_t* __restrict__ out, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int a[7], b[7];
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
-            a[k] = cards[i * 14 + k];
-            b[k] = cards[i * 14 + 7 + k];
+            a[k] = (int16_t)cards[i * 14 + k];
+            b[k] = (int16_t)cards[i * 14 + 7 + k];
         }
         const int32_t sa = score_cards<7>(a), sb = score_cards<7>(b);
         out[i] = (sa > sb) - (sa < sb);
@@ -149,32 +170,42 @@ static int grid_for(int64_t work_items, int per_block, int max_blocks) {
 
 int sm_count();
 
-int launch_rank7_cards(const int16_t* cards, int64_t n, int32_t* out, cudaStream_t stream) {
-    if (n == 0) return P2B_OK;
-    int rc = ensure_tables();
-    if (rc) return rc;
-    const bool vec = (reinterpret_cast<uintptr_t>(cards) & 7) == 0;
+template <typename T, bool VEC>
+static int launch_rank(const T* cards, int64_t n, int32_t* out, cudaStream_t stream) {
     // one wave of resident blocks: the tile loop is strided by the grid, so a partial second wave
     // would leave most SMs idle at the end
-    static int resident[2] = {0, 0};
-    if (resident[vec] == 0) {
+    static std::atomic<int> resident{0};
+    if (resident.load() == 0) {
         int per_sm = 0;
-        cudaError_t e = vec ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rank7_cards_kernel<true>, kRankThreads, 0)
-                            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rank7_cards_kernel<false>, kRankThreads, 0);
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rank7_cards_kernel<T, VEC>, kRankThreads, 0);
         if (e != cudaSuccess) return check_cuda(e, "rank7 occupancy query");
-        resident[vec] = per_sm > 0 ? per_sm : 1;
+        resident.store(per_sm > 0 ? per_sm : 1);
     }
-    const int grid = grid_for(n, kTileHands, sm_count() * resident[vec]);
-    if (vec) rank7_cards_kernel<true><<<grid, kRankThreads, 0, stream>>>(cards, out, n, device_rank_lut());
-    else rank7_cards_kernel<false><<<grid, kRankThreads, 0, stream>>>(cards, out, n, device_rank_lut());
+    const int grid = grid_for(n, kRankThreads * kHandsPerThread, sm_count() * resident.load());
+    rank7_cards_kernel<T, VEC><<<grid, kRankThreads, 0, stream>>>(cards, out, n, device_rank_lut());
     return check_cuda(cudaGetLastError(), "rank7_cards_kernel");
 }
 
-int launch_compare7_cards(const int16_t* cards, int64_t n, int32_t* out, cudaStream_t stream) {
+template <typename T>
+static int rank_cards(const T* cards, int64_t n, int32_t* out, cudaStream_t stream) {
     if (n == 0) return P2B_OK;
-    compare7_cards_kernel<<<grid_for(n, 256, sm_count() * 8), 256, 0, stream>>>(cards, out, n);
+    const int rc = ensure_tables();
+    if (rc) return rc;
+    const bool vec = (reinterpret_cast<uintptr_t>(cards) & (sizeof(T) == 2 ? 7 : 15)) == 0;
+    return vec ? launch_rank<T, true>(cards, n, out, stream) : launch_rank<T, false>(cards, n, out, stream);
+}
+
+template <typename T>
+static int compare_cards(const T* cards, int64_t n, int32_t* out, cudaStream_t stream) {
+    if (n == 0) return P2B_OK;
+    compare7_cards_kernel<T><<<grid_for(n, 256, sm_count() * 8), 256, 0, stream>>>(cards, out, n);
     return check_cuda(cudaGetLastError(), "compare7_cards_kernel");
 }
+
+int launch_rank7_cards(const int16_t* cards, int64_t n, int32_t* out, cudaStream_t s) { return rank_cards(cards, n, out, s); }
+int launch_rank7_cards(const int64_t* cards, int64_t n, int32_t* out, cudaStream_t s) { return rank_cards(cards, n, out, s); }
+int launch_compare7_cards(const int16_t* cards, int64_t n, int32_t* out, cudaStream_t s) { return compare_cards(cards, n, out, s); }
+int launch_compare7_cards(const int64_t* cards, int64_t n, int32_t* out, cudaStream_t s) { return compare_cards(cards, n, out, s); }
 
 int launch_compare7_planes(const int8_t* planes, int64_t n, int32_t* out, cudaStream_t stream) {
     if (n == 0) return P2B_OK;

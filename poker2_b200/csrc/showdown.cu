@@ -348,9 +348,11 @@ constexpr int kEvTot = kEvCombo + 2 * 1328;             // float [2][64] mass of
 constexpr int kEvalSmem = kEvTot + 2 * 64 * 4;
 static_assert(kEvQ % 8 == 0, "alignment");
 
+// AT: beliefs and values by row_index[row] instead of row.
+template <bool AT>
 __global__ void __launch_bounds__(kEvalThreads, 2) showdown_eval_kernel(
-    const unsigned char* __restrict__ tabs, const int32_t* __restrict__ tab_of_row, const ComboTable* __restrict__ combos,
-    const float* __restrict__ beliefs, int64_t belief_row_stride, const long long* __restrict__ potential,
+    const unsigned char* __restrict__ tabs, const int32_t* __restrict__ tab_of_row, const int64_t* __restrict__ row_index,
+    const ComboTable* __restrict__ combos, const float* __restrict__ beliefs, int64_t belief_row_stride, const long long* __restrict__ potential,
     const float* __restrict__ scale, float* __restrict__ values, int64_t value_row_stride, int64_t rows) {
     extern __shared__ __align__(16) unsigned char smem[];
     float* P = reinterpret_cast<float*>(smem + kEvP);   // P[p*HPAD + k] = prefix of player p's range, strength order
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(kEvalThreads, 2) showdown_eval_kernel(
                 const unsigned d = (unsigned)__cvta_generic_to_shared(dst + 16 * i);
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + 16 * i) : "memory");
             }
-            const float* brow = beliefs + row * belief_row_stride;
+            const float* brow = beliefs + (AT ? row_index[row] : row) * belief_row_stride;
             float* xd = reinterpret_cast<float*>(dst + kEvX);
             if (vec_in) {
                 for (int i = tid; i < 2 * P2B_NUM_HANDS / 4; i += kEvalThreads) {
@@ -484,7 +486,7 @@ __global__ void __launch_bounds__(kEvalThreads, 2) showdown_eval_kernel(
 
         // ---- C. per-hand formula ----
         const unsigned long long bmask = *tv.board_mask;
-        float* vrow = values + row * value_row_stride;
+        float* vrow = values + (AT ? row_index[row] : row) * value_row_stride;
         const float pot0 = (float)potential[row * 2], pot1 = (float)potential[row * 2 + 1];
         const Divisor dscale = make_divisor(scale[row]);
         // a thread takes a hand for both players: cards, board check and the hand's record are shared
@@ -517,20 +519,21 @@ int launch_board_setup(const int16_t* boards, int64_t m, unsigned char* tabs, in
     return check_cuda(cudaGetLastError(), "board_setup_kernel");
 }
 
-int launch_showdown_eval(const unsigned char* tabs, const int32_t* tab_of_row, const float* beliefs,
+int launch_showdown_eval(const unsigned char* tabs, const int32_t* tab_of_row, const int64_t* row_index, const float* beliefs,
                          int64_t belief_row_stride, const long long* potential, const float* scale, float* values,
                          int64_t value_row_stride, int64_t rows, cudaStream_t stream) {
     if (rows == 0) return P2B_OK;
     int rc = ensure_tables();
     if (rc) return rc;
-    rc = check_cuda(cudaFuncSetAttribute(showdown_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEvalSmem),
+    const auto kernel = row_index ? showdown_eval_kernel<true> : showdown_eval_kernel<false>;
+    rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEvalSmem),
                     "showdown_eval_kernel smem attribute");
     if (rc) return rc;
     int64_t grid = rows;
     const int64_t cap = (int64_t)sm_count() * 2;
     if (grid > cap) grid = cap;
-    showdown_eval_kernel<<<(unsigned)grid, kEvalThreads, kEvalSmem, stream>>>(
-        tabs, tab_of_row, device_combo_table(), beliefs, belief_row_stride, potential, scale, values, value_row_stride,
+    kernel<<<(unsigned)grid, kEvalThreads, kEvalSmem, stream>>>(
+        tabs, tab_of_row, row_index, device_combo_table(), beliefs, belief_row_stride, potential, scale, values, value_row_stride,
         rows);
     return check_cuda(cudaGetLastError(), "showdown_eval_kernel");
 }

@@ -505,6 +505,290 @@ __global__ void deep_beliefs_kernel(float* __restrict__ out, const float* __rest
     }
 }
 
+// ---- whole steps of `step_evaluator.StepCFREvaluator` ------------------------------------------
+// The kernels above mirror the upstream wrappers one for one, which leaves an iteration at 64 launches and several passes
+// over every tensor (0.80 ms for 64 roots, 0.66 of it kernel time; 0.31 ms and 14 launches now, bound by the rows' way through
+// memory at 2 to 4 TB/s and, in two of the kernels, the per-card sums).  These do a step of the iteration each, a block of 448
+// threads per parent or node with the rows it couples in registers and shared memory; same operations in the same order.
+// Rows are 1326 wide; the topology is level-major with the children of a node consecutive.
+struct StepRow {
+    float v[kHandsPerThread];
+};
+__device__ __forceinline__ StepRow ld_row(const float* __restrict__ row) {
+    StepRow r;
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) {
+        const int h = threadIdx.x + i * kRowThreads;
+        r.v[i] = h < P2B_NUM_HANDS ? row[h] : 0.0f;
+    }
+    return r;
+}
+__device__ __forceinline__ void st_row(float* __restrict__ row, const StepRow& r) {
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) {
+        const int h = threadIdx.x + i * kRowThreads;
+        if (h < P2B_NUM_HANDS) row[h] = r.v[i];
+    }
+}
+__device__ __forceinline__ void stage_row(float* shared, const StepRow& r) {  // padded with zeros
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) shared[threadIdx.x + i * kRowThreads] = r.v[i];
+}
+struct StepCards {
+    int c1[kHandsPerThread], c2[kHandsPerThread];
+};
+__device__ __forceinline__ StepCards load_cards(const ComboTable* __restrict__ combos) {
+    StepCards c;
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) {
+        const int h = threadIdx.x + i * kRowThreads, hc = h < P2B_NUM_HANDS ? h : P2B_NUM_HANDS - 1;
+        c.c1[i] = combos->c1[hc];
+        c.c2[i] = combos->c2[hc];
+    }
+    return c;
+}
+
+// Instantaneous regrets (cfr_evaluator.py:1117-1165), the discounted update (:1346-1368) and regret matching (:1168-1185)
+// of the children of one parent; a root's own row takes part in the update with no regret.
+__global__ void __launch_bounds__(kRowThreads, 2) step_regrets_kernel(
+    const float* __restrict__ values, const float* __restrict__ beliefs, const long long* __restrict__ to_act,
+    const long long* __restrict__ child_offsets, const long long* __restrict__ child_count, const ComboTable* __restrict__ combos,
+    const float* __restrict__ uniform, const float* __restrict__ scal, float* __restrict__ cumul, float* __restrict__ weights,
+    float* __restrict__ policy, long long num_roots, int apply_dcfr, int cfr_plus) {
+    constexpr int H = P2B_NUM_HANDS;
+    __shared__ __align__(16) float xs[P2B_HPAD];
+    __shared__ double cs[52], S[1];
+    const long long par = blockIdx.x;
+    const int k = (int)child_count[par];
+    DcfrScalars sc;
+    sc.an = scal[0];
+    sc.bn = scal[1];
+    sc.da = make_divisor(scal[2]);
+    sc.db = make_divisor(scal[3]);
+    if (par < num_roots) {
+        StepRow c = ld_row(cumul + par * H), w = ld_row(weights + par * H);
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) dcfr_update_one(c.v[i], w.v[i], 0.0f, sc, apply_dcfr, cfr_plus);
+        st_row(cumul + par * H, c);
+        st_row(weights + par * H, w);
+    }
+    if (k == 0) return;
+    const int a = (int)to_act[par];
+    const long long first = child_offsets[par];
+    uint32_t idx[7];
+    card_indices(threadIdx.x, idx);
+    const StepCards cards = load_cards(combos);
+    const StepRow b = ld_row(beliefs + (par * 2 + 1 - a) * H), v = ld_row(values + (par * 2 + a) * H);
+    stage_row(xs, b);
+    __syncthreads();
+    card_sums(xs, 1, cs, S, idx);
+    __syncthreads();
+    StepRow wgt, sum;
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) {
+        wgt.v[i] = unblocked(cs, S[0], cards.c1[i], cards.c2[i], b.v[i]);
+        sum.v[i] = 0.0f;
+    }
+#pragma unroll 2
+    for (int c = 0; c < k; ++c) {
+        const long long row = first + c;
+        StepRow r = ld_row(cumul + row * H), w = ld_row(weights + row * H);
+        const StepRow vc = ld_row(values + (row * 2 + a) * H);
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) {
+            dcfr_update_one(r.v[i], w.v[i], __fmul_rn(wgt.v[i], __fsub_rn(vc.v[i], v.v[i])), sc, apply_dcfr, cfr_plus);
+            sum.v[i] = __fadd_rn(sum.v[i], fmaxf(r.v[i], 0.0f));
+        }
+        st_row(cumul + row * H, r);
+        st_row(weights + row * H, w);
+    }
+    Divisor d[kHandsPerThread];
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) d[i] = make_divisor(fmaxf(sum.v[i], 1e-8f));
+#pragma unroll 2
+    for (int c = 0; c < k; ++c) {
+        const StepRow r = ld_row(cumul + (first + c) * H);  // as this thread has just stored them
+        StepRow u = ld_row(uniform + (first + c) * H);
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) u.v[i] = sum.v[i] > 1e-8f ? div_exact(fmaxf(r.v[i], 0.0f), d[i]) : u.v[i];
+        st_row(policy + (first + c) * H, u);
+    }
+}
+
+// Reach of both players at one node (cfr_evaluator.py:332-361) and, unless `beliefs` is null, the beliefs that follow from
+// the root's (:363-380): the product of the policies along the path, which is `path[node][depth]` from the root down,
+// each entry 2 * node + the player who chose it, -1 behind the last.
+__global__ void __launch_bounds__(kRowThreads) step_reach_kernel(
+    const float* __restrict__ policy, const unsigned char* __restrict__ allowed, const float* __restrict__ allowed_prob,
+    const int32_t* __restrict__ path, int depth, const long long* __restrict__ root_index, const float* __restrict__ prior,
+    float* __restrict__ reach, float* __restrict__ beliefs) {
+    constexpr int H = P2B_NUM_HANDS;
+    __shared__ __align__(16) float xs[2][P2B_HPAD];
+    __shared__ float sums[2];
+    const long long node = blockIdx.x;
+    StepRow r[2];
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) {
+        const int h = threadIdx.x + i * kRowThreads;
+        r[0].v[i] = r[1].v[i] = (h < H && allowed[node * H + h]) ? 1.0f : 0.0f;
+    }
+    for (int e = 0; e < depth; ++e) {
+        const int code = path[node * depth + e];
+        if (code < 0) break;
+        const StepRow P = ld_row(policy + (long long)(code >> 1) * H);
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) {
+            if (code & 1) r[1].v[i] = __fmul_rn(r[1].v[i], P.v[i]);
+            else r[0].v[i] = __fmul_rn(r[0].v[i], P.v[i]);
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p) st_row(reach + (node * 2 + p) * H, r[p]);
+    if (!beliefs) return;
+    const long long root = root_index[node];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const StepRow b = ld_row(prior + (root * 2 + p) * H);
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) r[p].v[i] = __fmul_rn(b.v[i], r[p].v[i]);
+        stage_row(xs[p], r[p]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        const float s = row_sum_reference_order(xs[threadIdx.x >> 5]);
+        if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = s;
+    }
+    __syncthreads();
+    const StepRow fallback = ld_row(allowed_prob + node * H);
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const Divisor d = make_divisor(sums[p]);
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) r[p].v[i] = sums[p] > 1e-5f ? div_exact(r[p].v[i], d) : fallback.v[i];
+        st_row(beliefs + (node * 2 + p) * H, r[p]);
+    }
+}
+
+// Average-policy mix and renormalisation of the children of one parent (cfr_evaluator.py:1195-1258).
+__global__ void __launch_bounds__(kRowThreads, 2) step_average_kernel(
+    const float* __restrict__ reach, const float* __restrict__ reach_avg, const float* __restrict__ policy,
+    const long long* __restrict__ to_act, const long long* __restrict__ child_offsets, const long long* __restrict__ child_count,
+    const float* __restrict__ old_p, const float* __restrict__ new_p, const float* __restrict__ tot_p, float* __restrict__ avg) {
+    constexpr int H = P2B_NUM_HANDS;
+    const long long par = blockIdx.x;
+    const int k = (int)child_count[par];
+    if (k == 0) return;
+    const long long first = child_offsets[par], side = (par * 2 + to_act[par]) * H;
+    const float o = *old_p, w = *new_p, tot = *tot_p;
+    StepRow ra = ld_row(reach_avg + side), rn = ld_row(reach + side), sum;
+    Divisor d[kHandsPerThread];
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) {
+        const float x = __fmul_rn(ra.v[i], o), y = __fmul_rn(rn.v[i], w), den = __fadd_rn(x, y);
+        const bool weighted = den > 1e-5f;
+        ra.v[i] = weighted ? x : o;
+        rn.v[i] = weighted ? y : w;
+        d[i] = make_divisor(weighted ? den : tot);
+        sum.v[i] = 0.0f;
+    }
+#pragma unroll 2
+    for (int c = 0; c < k; ++c) {
+        StepRow A = ld_row(avg + (first + c) * H);
+        const StepRow P = ld_row(policy + (first + c) * H);
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) {
+            A.v[i] = div_exact(__fadd_rn(__fmul_rn(ra.v[i], A.v[i]), __fmul_rn(rn.v[i], P.v[i])), d[i]);
+            sum.v[i] = __fadd_rn(sum.v[i], A.v[i]);
+        }
+        st_row(avg + (first + c) * H, A);
+    }
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) d[i] = make_divisor(fmaxf(sum.v[i], 1e-5f));
+#pragma unroll 2
+    for (int c = 0; c < k; ++c) {
+        StepRow A = ld_row(avg + (first + c) * H);  // as this thread has just stored them
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i)
+            if (sum.v[i] > 1e-5f) A.v[i] = div_exact(A.v[i], d[i]);
+        st_row(avg + (first + c) * H, A);
+    }
+}
+
+constexpr int kSeenRows = 8;
+// Policy of the children of one parent as each hand of the other player sees it (cfr_evaluator.py:1076-1093).
+__global__ void __launch_bounds__(kRowThreads, 2) step_seen_kernel(
+    const float* __restrict__ beliefs, const float* __restrict__ policy, const long long* __restrict__ to_act,
+    const long long* __restrict__ child_offsets, const long long* __restrict__ child_count, const ComboTable* __restrict__ combos,
+    float* __restrict__ seen) {
+    constexpr int H = P2B_NUM_HANDS;
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* rows = reinterpret_cast<float*>(smem);
+    double* cs = reinterpret_cast<double*>(smem + (1 + kSeenRows) * P2B_HPAD * 4);
+    double* S = cs + (1 + kSeenRows) * 52;
+    const long long par = blockIdx.x;
+    const int k = (int)child_count[par];
+    if (k == 0) return;
+    const long long first = child_offsets[par];
+    uint32_t idx[7];
+    card_indices(threadIdx.x, idx);
+    const StepCards cards = load_cards(combos);
+    const StepRow b = ld_row(beliefs + (par * 2 + to_act[par]) * H);
+    stage_row(rows, b);
+    for (int c0 = 0; c0 < k; c0 += kSeenRows) {  // as many children at a time as there are rows for
+        const int n = min(kSeenRows, k - c0);
+#pragma unroll 2
+        for (int c = 0; c < n; ++c) {
+            StepRow P = ld_row(policy + (first + c0 + c) * H);
+#pragma unroll
+            for (int i = 0; i < kHandsPerThread; ++i) P.v[i] = __fmul_rn(b.v[i], P.v[i]);
+            stage_row(rows + (1 + c) * P2B_HPAD, P);
+        }
+        __syncthreads();
+        card_sums(rows, 1 + n, cs, S, idx);
+        __syncthreads();
+        Divisor d[kHandsPerThread];
+#pragma unroll
+        for (int i = 0; i < kHandsPerThread; ++i) d[i] = make_divisor(unblocked(cs, S[0], cards.c1[i], cards.c2[i], b.v[i]));
+#pragma unroll 1
+        for (int c = 0; c < n; ++c) {
+            StepRow q;
+#pragma unroll
+            for (int i = 0; i < kHandsPerThread; ++i) {
+                const float m = rows[(1 + c) * P2B_HPAD + threadIdx.x + i * kRowThreads];
+                const float x = unblocked(cs + (1 + c) * 52, S[1 + c], cards.c1[i], cards.c2[i], m);
+                q.v[i] = d[i].y > 1e-5f ? div_exact(x, d[i]) : 0.0f;
+            }
+            st_row(seen + (first + c0 + c) * H, q);
+        }
+        __syncthreads();
+    }
+}
+
+// weighted_parent_sum_kernel for rows of 1326: a block per parent, six sums a thread.
+__global__ void __launch_bounds__(kRowThreads) weighted_parent_rows_kernel(
+    float* __restrict__ values, const long long* __restrict__ prev_actor, const float* __restrict__ pol_hero,
+    const float* __restrict__ pol_opp, const long long* __restrict__ child_offsets, const long long* __restrict__ child_count,
+    long long parent_base) {
+    constexpr int H = P2B_NUM_HANDS;
+    const long long first = child_offsets[blockIdx.x], k = child_count[blockIdx.x], par = parent_base + blockIdx.x;
+    if (k == 0) return;
+    StepRow acc[2];
+#pragma unroll
+    for (int i = 0; i < kHandsPerThread; ++i) acc[0].v[i] = acc[1].v[i] = 0.0f;
+#pragma unroll 2
+    for (long long c = first; c < first + k; ++c) {
+        const int a = (int)prev_actor[c];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const StepRow pol = ld_row((a == p ? pol_hero : pol_opp) + c * H), v = ld_row(values + (c * 2 + p) * H);
+#pragma unroll
+            for (int i = 0; i < kHandsPerThread; ++i) acc[p].v[i] = __fadd_rn(acc[p].v[i], __fmul_rn(v.v[i], pol.v[i]));
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p) st_row(values + (par * 2 + p) * H, acc[p]);
+}
+
 }  // namespace
 
 int sm_count();
@@ -645,6 +929,12 @@ int p2b_step_weighted_parent_sum(float* values, const int64_t* prev_actor, const
                                  const float* policy_opp, const int64_t* child_offsets, const int64_t* child_count,
                                  int64_t parent_base, int64_t num_parents, int32_t H, void* stream) {
     if (num_parents <= 0) return P2B_OK;
+    if (H == P2B_NUM_HANDS) {
+        weighted_parent_rows_kernel<<<(unsigned)num_parents, kRowThreads, 0, (cudaStream_t)stream>>>(
+            values, (const long long*)prev_actor, policy_hero, policy_opp, (const long long*)child_offsets,
+            (const long long*)child_count, parent_base);
+        STEP_CHECK("weighted_parent_rows_kernel");
+    }
     weighted_parent_sum_kernel<<<GRID_ELEMS(num_parents * 2 * H), kThreads, 0, (cudaStream_t)stream>>>(
         values, (const long long*)prev_actor, policy_hero, policy_opp, (const long long*)child_offsets,
         (const long long*)child_count, parent_base, num_parents, H);
@@ -666,6 +956,52 @@ int p2b_step_deep_beliefs(float* out, const float* root_beliefs, const float* re
     deep_beliefs_kernel<<<GRID_ROWS((total - num_roots) * 2), kThreads, 0, (cudaStream_t)stream>>>(
         out, root_beliefs, reach, allowed_prob, (const long long*)root_index, num_roots, total, H, eps);
     STEP_CHECK("deep_beliefs_kernel");
+}
+
+int p2b_steps_regrets(const float* values, const float* beliefs, const int64_t* to_act, const int64_t* child_offsets,
+                      const int64_t* child_count, const float* uniform, const float* scalars4, float* cumulative,
+                      float* weight_sums, float* policy, int64_t num_roots, int64_t num_parents, int apply_dcfr, int cfr_plus,
+                      void* stream) {
+    if (num_parents <= 0) return P2B_OK;
+    const int rc = ensure_tables();
+    if (rc) return rc;
+    step_regrets_kernel<<<(unsigned)num_parents, kRowThreads, 0, (cudaStream_t)stream>>>(
+        values, beliefs, (const long long*)to_act, (const long long*)child_offsets, (const long long*)child_count,
+        device_combo_table(), uniform, scalars4, cumulative, weight_sums, policy, num_roots, apply_dcfr, cfr_plus);
+    STEP_CHECK("step_regrets_kernel");
+}
+
+int p2b_steps_reach(const float* policy, const uint8_t* allowed, const float* allowed_prob, const int32_t* path, int32_t depth,
+                    const int64_t* root_index, const float* prior, float* reach, float* beliefs, int64_t nodes, void* stream) {
+    if (nodes <= 0) return P2B_OK;
+    step_reach_kernel<<<(unsigned)nodes, kRowThreads, 0, (cudaStream_t)stream>>>(
+        policy, allowed, allowed_prob, path, depth, (const long long*)root_index, prior, reach, beliefs);
+    STEP_CHECK("step_reach_kernel");
+}
+
+int p2b_steps_average(const float* reach, const float* reach_avg, const float* policy, const int64_t* to_act,
+                      const int64_t* child_offsets, const int64_t* child_count, const float* old_w, const float* new_w,
+                      const float* total_w, float* policy_avg, int64_t num_parents, void* stream) {
+    if (num_parents <= 0) return P2B_OK;
+    step_average_kernel<<<(unsigned)num_parents, kRowThreads, 0, (cudaStream_t)stream>>>(
+        reach, reach_avg, policy, (const long long*)to_act, (const long long*)child_offsets, (const long long*)child_count,
+        old_w, new_w, total_w, policy_avg);
+    STEP_CHECK("step_average_kernel");
+}
+
+int p2b_steps_seen(const float* beliefs, const float* policy, const int64_t* to_act, const int64_t* child_offsets,
+                   const int64_t* child_count, float* seen, int64_t num_parents, void* stream) {
+    if (num_parents <= 0) return P2B_OK;
+    int rc = ensure_tables();
+    if (rc) return rc;
+    constexpr int kBytes = (1 + kSeenRows) * (P2B_HPAD * 4 + 53 * 8);
+    rc = check_cuda(cudaFuncSetAttribute(step_seen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes),
+                    "step_seen_kernel shared-memory attribute");
+    if (rc) return rc;
+    step_seen_kernel<<<(unsigned)num_parents, kRowThreads, kBytes, (cudaStream_t)stream>>>(
+        beliefs, policy, (const long long*)to_act, (const long long*)child_offsets, (const long long*)child_count,
+        device_combo_table(), seen);
+    STEP_CHECK("step_seen_kernel");
 }
 
 }  // extern "C"

@@ -370,27 +370,21 @@ class TScalars:
     them on the host with `update` before launching (or replaying) the step kernels."""
 
     def __init__(self, device: torch.device, dtype: torch.dtype = torch.float32) -> None:
-        z = lambda: torch.zeros((), dtype=dtype, device=device)  # noqa: E731
         self.device, self.dtype = device, dtype
-        self.t_alpha_num, self.t_beta_num, self.t_alpha_den, self.t_beta_den = z(), z(), z(), z()
-        self.mix_old, self.mix_new, self.mix_total, self.mix_inv_total = z(), z(), z(), z()
-        self.mix_onon, self.mix_oon = z(), z()
+        # one array, so that an iteration's scalars arrive in one copy
+        self._all = torch.zeros(10, dtype=dtype, device=device)
+        (self.t_alpha_num, self.t_beta_num, self.t_alpha_den, self.t_beta_den, self.mix_old, self.mix_new, self.mix_total,
+         self.mix_inv_total, self.mix_onon, self.mix_oon) = self._all.unbind()
         self.t_tensor = torch.zeros((), dtype=torch.long, device=device)
 
     def update(self, t: int, dcfr_alpha: float, dcfr_beta: float, mix_old: float, mix_new: float) -> None:
         an, bn = float(t ** dcfr_alpha), float(t ** dcfr_beta)
-        self.t_alpha_num.fill_(an)
-        self.t_beta_num.fill_(bn)
-        self.t_alpha_den.fill_(an + 1.0)
-        self.t_beta_den.fill_(bn + 1.0)
-        total = float(mix_old) + float(mix_new)
-        self.mix_old.fill_(float(mix_old))
-        self.mix_new.fill_(float(mix_new))
-        self.mix_total.fill_(total)
-        self.mix_inv_total.fill_(1.0 / total if total != 0.0 else 1.0)
-        if float(mix_new) != 0.0:
-            self.mix_onon.fill_(total / float(mix_new))
-            self.mix_oon.fill_(float(mix_old) / float(mix_new))
+        old, new = float(mix_old), float(mix_new)
+        total = old + new
+        values = [an, bn, an + 1.0, bn + 1.0, old, new, total, 1.0 / total if total != 0.0 else 1.0]
+        if new != 0.0:
+            values += [total / new, old / new]
+        self._all[: len(values)].copy_(torch.tensor(values, dtype=self.dtype))
         self.t_tensor.fill_(int(t))
 
 

@@ -62,6 +62,17 @@ class ValueMLP(torch.nn.Module):
         return y.to(torch.float32).view(S, 2, NUM_HANDS)
 
 
+    @torch.no_grad()
+    def layers(self, x: torch.Tensor) -> torch.Tensor:
+        """`self.net` on input rows x, activations in place (half the memory traffic and footprint of a GELU, same bits)."""
+        for layer in self.net:
+            if type(layer) is torch.nn.GELU and layer.approximate == "none":
+                x = torch.ops.aten.gelu_(x)
+            else:
+                x = layer(x)
+        return x
+
+
 def leaf_context(trees, node_index) -> torch.Tensor:
     """[L,3] fp32 context of the tree nodes `node_index` (upstream numbering): pot and both
     stacks as fractions of the two starting stacks together."""
@@ -104,8 +115,7 @@ class ChanceLeafEvaluator:
         for a, b, off, n_samples in self._chunks:
             x = chance.expand_features_bf16(leaf_beliefs[a:b], self.boards[a:b], off, n_samples, self.context[a:b],
                                             self.model.IN_PADDED)
-            with torch.no_grad():
-                y = self.model.net(x)
+            y = self.model.layers(x)
             chance.indexed_mean_bf16(y, off, out[a:b])
         self.calls += 1
 
@@ -156,7 +166,7 @@ class DirectLeafEvaluator:
             stream = _lib.stream_ptr(out.device)
             _lib.call("p2b_leaf_features_bf16", p(leaf_beliefs), leaf_beliefs.stride(1), L, p(self._rows),
                       self._rows.stride(0), stream)
-            y = self.model.net(self._rows)
+            y = self.model.layers(self._rows)
             _lib.call("p2b_leaf_values_bf16", p(y), y.stride(0), L, p(out), out.stride(1), stream)
 
     def __call__(self, leaf_beliefs: torch.Tensor) -> torch.Tensor:

@@ -50,6 +50,13 @@ def compare_7_batches(a_batch: torch.Tensor, b_batch: torch.Tensor) -> torch.Ten
     return compare_7_single_batch(torch.stack([a_batch, b_batch], dim=1).bool())
 
 
+def _card_ids(t: torch.Tensor):
+    """(contiguous card ids, suffix of the entry point that reads them): int16 and int64 as they are."""
+    if t.dtype == torch.int64:
+        return t.contiguous(), "_i64"
+    return _as_i16(t), ""
+
+
 def _as_i16(t: torch.Tensor) -> torch.Tensor:
     if t.dtype == torch.int16 and t.is_contiguous():
         return t
@@ -62,10 +69,10 @@ def compare_7_cards_single_batch(cards_batch: torch.Tensor) -> torch.Tensor:
     if cards_batch.dim() != 3 or tuple(cards_batch.shape[1:]) != (2, 7):
         raise ValueError(f"Expected [N, 2, 7] input, got {tuple(cards_batch.shape)}")
     _lib.require_cuda(cards_batch, "CUDA hand evaluator")
-    cards = _as_i16(cards_batch)
+    cards, kind = _card_ids(cards_batch)
     out = torch.empty((cards.shape[0],), device=cards.device, dtype=torch.int32)
     with _lib.on(cards.device):
-        _lib.call("p2b_compare7_cards", _lib.ptr(cards), cards.shape[0], _lib.ptr(out),
+        _lib.call("p2b_compare7_cards" + kind, _lib.ptr(cards), cards.shape[0], _lib.ptr(out),
                   _lib.stream_ptr(cards.device))
     return out
 
@@ -77,10 +84,10 @@ def rank_7_cards_single_batch(cards_batch: torch.Tensor) -> torch.Tensor:
     if cards_batch.dim() != 2 or cards_batch.shape[1] != 7:
         raise ValueError(f"Expected [N, 7] input, got {tuple(cards_batch.shape)}")
     _lib.require_cuda(cards_batch, "CUDA hand evaluator")
-    cards = _as_i16(cards_batch)
+    cards, kind = _card_ids(cards_batch)
     out = torch.empty((cards.shape[0],), device=cards.device, dtype=torch.int32)
     with _lib.on(cards.device):
-        _lib.call("p2b_rank7_cards", _lib.ptr(cards), cards.shape[0], _lib.ptr(out),
+        _lib.call("p2b_rank7_cards" + kind, _lib.ptr(cards), cards.shape[0], _lib.ptr(out),
                   _lib.stream_ptr(cards.device))
     return out
 

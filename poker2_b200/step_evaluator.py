@@ -8,7 +8,8 @@ tests and tools call directly: `initialize_policy_and_beliefs`, `set_leaf_values
 `poker2_b200.fused_cfr` and `poker2_b200.showdown` the way the upstream fused evaluator composes its
 Triton kernels (p2/search/fused_sparse_cfr_evaluator.py:144-527), so the state can be inspected
 between any two steps.  It is the slow, transparent form: a whole solve belongs in
-`solver.SubgameSolver` (three launches), which ends in the same state.
+`solver.SubgameSolver` (three launches), which ends in the same state.  `cfr_iteration` and the steps it is made of run in
+kernels that do a whole step each (`p2b_steps_*`); the start and `update_policy` by itself go through the one-for-one ones.
 
 Covered: uniform start, `cfr_type` standard / discounted / discounted_plus with optional CFR+ clamp,
 leaves valued by showdown, fold constants and an optional `leaf_fn`; value targets from the final
@@ -20,6 +21,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from . import _lib
 from . import fused_cfr as F
 from . import showdown
 
@@ -88,28 +90,35 @@ class StepCFREvaluator:
         self.latest_values[fold, 0] = fv[fold][:, None]
         self.latest_values[fold, 1] = -fv[fold][:, None]
         self.values_avg = self.latest_values.clone()
+        # the path to every node from below its root: 2 * node + the player who chose it, -1 behind the last
+        parent, actor = np.asarray(t.parent_index), np.asarray(t.prev_actor)
+        path = np.full((M, max(self.tree_depth, 1)), -1, dtype=np.int32)
+        for d in range(self.tree_depth):
+            b, c = self.depth_offsets[d + 1], self.depth_offsets[d + 2]
+            path[b:c] = path[parent[b:c]]
+            path[b:c, d] = 2 * np.arange(b, c) + actor[b:c]
+        self._path = torch.from_numpy(path).to(dev)
+        # the slices of the topology that every iteration hands to a kernel
+        self._levels = [(a, self.child_offsets[a:b].contiguous(), self.child_count[a:b].contiguous())
+                        for a, b in zip(self.depth_offsets[:-2], self.depth_offsets[1:-1])]
+        self._allowed_bytes = self.allowed_hands.view(torch.uint8)
+        self._seen = z(M, NUM_HANDS)
         # iteration scalars on the device, so that one captured iteration can be replayed for another t
         # (fused_sparse_cfr_evaluator.py:100-107, 535-550)
         self._t_scalars = F.TScalars(dev)
         self._skip_t_scalars_update = False
 
     # ---- reach and beliefs (cfr_evaluator.py:248-273, 332-380) ------------------------------
-    def _calculate_reach_weights(self, target: torch.Tensor, policy: torch.Tensor) -> None:
-        offs = self.depth_offsets
-        target.zero_()
-        target[: self.root_nodes] = self.allowed_hands[: self.root_nodes, None, :].to(torch.float32)
-        for d in range(self.tree_depth):
-            F.fused_reach_weights_depth_(target, policy, self.allowed_hands, self.parent_index, self.prev_actor,
-                                         offs[d + 1], offs[d + 2])
+    def _call(self, name: str, *args) -> None:
+        with _lib.on(self.device):
+            _lib.call(name, *[a.data_ptr() if torch.is_tensor(a) else a for a in args], _lib.stream_ptr(self.device))
 
-    def _propagate_all_beliefs(self, target: torch.Tensor, reach: torch.Tensor) -> None:
-        """Every row = its root's row x reach, blocked and normalised; the root rows themselves are
-        normalised once more per call, like every other row upstream."""
-        N = self.root_nodes
-        F.fused_deep_beliefs_(target, target, reach, self.allowed_hands_prob, self.root_of, num_roots=N)
-        roots = target[:N]
-        roots.mul_(reach[:N])
-        F.fused_block_and_normalize_beliefs_(roots, self.allowed_hands[:N], self.allowed_hands_prob[:N])
+    def _calculate_reach_weights(self, target: torch.Tensor, policy: torch.Tensor, beliefs: torch.Tensor | None = None) -> None:
+        """Reach under `policy`; with `beliefs` also those: every row = its root's row x reach, blocked and normalised (the
+        root rows themselves are normalised once more per call, like every other row upstream)."""
+        prior = None if beliefs is None else beliefs[: self.root_nodes].clone()
+        self._call("p2b_steps_reach", policy, self._allowed_bytes, self.allowed_hands_prob, self._path, self._path.shape[1],
+                   self.root_of, prior, target, beliefs, self.total_nodes)
 
     # ---- start of evaluate_cfr (cfr_evaluator.py:832-886, 1503-1513) ------------------------
     def initialize_policy_and_beliefs(self) -> None:
@@ -132,34 +141,26 @@ class StepCFREvaluator:
 
     # ---- leaves and backup (cfr_evaluator.py:1025-1115) -------------------------------------
     def set_leaf_values(self, t: int = 0, beliefs: torch.Tensor | None = None) -> None:
-        beliefs = self.beliefs if beliefs is None else beliefs
+        beliefs = self.beliefs if beliefs is None else beliefs.contiguous()
         if self.model_indices.numel():
             vals = self.leaf_fn(beliefs[self.model_indices], self.model_indices)
             self.latest_values[self.model_indices] = vals[..., :NUM_HANDS].to(torch.float32)
         if self.showdown_indices.numel():
-            vals = showdown.showdown_values(self._tables, beliefs[self.showdown_indices].contiguous(), self._sd_potential,
-                                            self._sd_scale, table_of_row=self._sd_table)
-            self.latest_values[self.showdown_indices] = vals
+            stride = 2 * NUM_HANDS
+            self._call("p2b_showdown_values_at", self._tables.blob, self._sd_table, self.showdown_indices, beliefs, stride,
+                       self._sd_potential, self._sd_scale, self.latest_values, stride, self.showdown_indices.numel())
 
     def compute_expected_values(self, policy=None, beliefs=None, leaf_values=None, values=None) -> None:
-        policy = self.policy_probs if policy is None else policy
-        beliefs = self.beliefs if beliefs is None else beliefs
+        policy = self.policy_probs if policy is None else policy.contiguous()
+        beliefs = self.beliefs if beliefs is None else beliefs.contiguous()
         leaf_values = self.latest_values if leaf_values is None else leaf_values
         values = leaf_values if values is None else values
-        if leaf_values is values:
-            values.masked_fill_((~self.leaf_mask)[:, None, None], 0.0)
-        else:
+        if leaf_values is not values:  # (in place, the inner rows are overwritten below)
             torch.where(self.leaf_mask[:, None, None], leaf_values, torch.zeros((), device=self.device), out=values)
-        N, top, offs = self.root_nodes, self.top, self.depth_offsets
-        idx = self.to_act[:top, None, None].expand(-1, -1, NUM_HANDS)
-        actor_beliefs = beliefs[:top].gather(1, idx).squeeze(1).contiguous()
-        marginal = (actor_beliefs.index_select(0, self.parent_index[N:]) * policy[N:]).contiguous()
-        opp = torch.zeros_like(policy)
-        opp[N:] = F.unblocked_mass_ratio_indirect_triton(marginal, actor_beliefs, self.parent_index[N:].contiguous())
-        for d in range(self.tree_depth - 1, -1, -1):
-            a, b = offs[d], offs[d + 1]
-            F.fused_weighted_parent_sum(values, self.prev_actor, policy, opp, self.child_offsets[a:b].contiguous(),
-                                        self.child_count[a:b].contiguous(), parent_base=a, max_children=self.num_actions)
+        self._call("p2b_steps_seen", beliefs, policy, self.to_act, self.child_offsets, self.child_count, self._seen, self.top)
+        for a, offsets, counts in reversed(self._levels):
+            self._call("p2b_step_weighted_parent_sum", values, self.prev_actor, policy, self._seen, offsets, counts, a,
+                       offsets.numel(), NUM_HANDS)
 
     # ---- one iteration (cfr_evaluator.py:1117-1258, 1331-1381) ------------------------------
     def compute_instantaneous_regrets(self, values: torch.Tensor | None = None) -> torch.Tensor:
@@ -184,15 +185,9 @@ class StepCFREvaluator:
         if (self.cfr_type in ("discounted", "discounted_plus") and t <= self.dcfr_delay) or t == 0:
             self.policy_probs_avg.copy_(self.policy_probs)
             return
-        N, top = self.root_nodes, self.top
-        avg, ts = self.policy_probs_avg, self._t_scalars
-        F.fused_average_policy_mix_with_tensors_(avg, self.policy_probs, self.self_reach, self.self_reach_avg, self.to_act,
-                                                 self.parent_index, ts.mix_old, ts.mix_new, ts.mix_total, bottom=N)
-        psum = F.fused_parent_sum(avg, self.child_offsets[:top].contiguous(), self.child_count[:top].contiguous(),
-                                  max_children=self.num_actions)
-        child = avg[N:].contiguous()
-        F.fused_divide_by_parent_sum_(child, child, psum, self.parent_index[N:].contiguous(), avg[N:], eps=1e-5)
-        avg[:N] = 0.0
+        ts = self._t_scalars
+        self._call("p2b_steps_average", self.self_reach, self.self_reach_avg, self.policy_probs, self.to_act, self.child_offsets,
+                   self.child_count, ts.mix_old, ts.mix_new, ts.mix_total, self.policy_probs_avg, self.top)
 
     def update_policy(self, t: int) -> None:
         N, top = self.root_nodes, self.top
@@ -201,11 +196,13 @@ class StepCFREvaluator:
                                         max_children=self.num_actions)
         F.fused_divide_by_parent_sum_(pos[N:].contiguous(), self.uniform_policy[N:].contiguous(), parent_sum,
                                       self.parent_index[N:].contiguous(), self.policy_probs[N:])
-        self._calculate_reach_weights(self.self_reach, self.policy_probs)
-        self._propagate_all_beliefs(self.beliefs, self.self_reach)
+        self._follow_policy(t)
+
+    def _follow_policy(self, t: int) -> None:
+        """Reach, beliefs and average policy of the current policy."""
+        self._calculate_reach_weights(self.self_reach, self.policy_probs, self.beliefs)
         self.update_average_policy(t)
-        self._calculate_reach_weights(self.self_reach_avg, self.policy_probs_avg)
-        self._propagate_all_beliefs(self.beliefs_avg, self.self_reach_avg)
+        self._calculate_reach_weights(self.self_reach_avg, self.policy_probs_avg, self.beliefs_avg)
 
     def prepare_replay(self, t: int) -> None:
         """Fills the device scalars of iteration t (discount factors, mixing weights); `cfr_iteration` does it
@@ -219,12 +216,12 @@ class StepCFREvaluator:
     def cfr_iteration(self, t: int) -> None:
         if not self._skip_t_scalars_update:
             self.prepare_replay(t)
-        regrets = self.compute_instantaneous_regrets(self.latest_values)
-        ts = self._t_scalars
-        F.fused_dcfr_update_with_tensors_(self.cumulative_regrets, self.regret_weight_sums, regrets, ts.t_alpha_num,
-                                          ts.t_beta_num, ts.t_alpha_den, ts.t_beta_den,
-                                          self.cfr_type in ("discounted", "discounted_plus"), self.cfr_plus)
-        self.update_policy(t)
+        # `compute_instantaneous_regrets`, the discounted update and the regret matching of `update_policy` in one kernel
+        self._call("p2b_steps_regrets", self.latest_values, self.beliefs, self.to_act, self.child_offsets, self.child_count,
+                   self.uniform_policy, self._t_scalars.t_alpha_num, self.cumulative_regrets, self.regret_weight_sums,
+                   self.policy_probs, self.root_nodes, max(self.top, self.root_nodes), int(self.cfr_type in ("discounted", "discounted_plus")),
+                   int(self.cfr_plus))
+        self._follow_policy(t)
         self.set_leaf_values(t)
         self.compute_expected_values()
 
