@@ -137,145 +137,191 @@ __global__ void indexed_add_rows_kernel(float* __restrict__ out, const long long
 // are `player_stride` floats apart (1326 for packed rows, 1344 for the solver's padded rows).
 constexpr int kHandsPerThread = (P2B_NUM_HANDS + kThreads - 1) / kThreads;  // 6
 
-// A block takes up to kCardsPerBlock consecutive next cards of one root: the root's two belief rows are
-// read once into registers, every card's block-wide sums (mass of the combos that stay allowed, their
-// number) are gathered with one barrier pair for the whole group, then the rows are written.  The
-// per-thread partial sums, the shuffle tree and the order over warps are those of chance_expand_kernel,
-// so the normalised values are the same bits.
-constexpr int kCardsPerBlock = 8;
-constexpr int kCardGroups = (P2B_NUM_CARDS + kCardsPerBlock - 1) / kCardsPerBlock;  // groups per root (the last ones may be empty)
+// A block takes `group` consecutive next cards of one root.  What a card leaves of a player's mass is the total minus the
+// mass of the hands that hold it, from one total and 52 per-card sums a root in fp64 (where less than a millionth is left,
+// the rest is added up by itself); so a card costs its row's quotients and stores alone.  A thread owns three pairs of
+// neighbouring hands and writes two bf16 values at once.  Summing the masses anew for every card took 60 % of the kernel.
+// Measured on 111,360 samples (2320 turn roots): 600 -> 254 us, 2.4 TB/s of network input written.
+constexpr int kPairThreads = 224, kPairs = 3, kPairWarps = kPairThreads / 32;
+static_assert(2 * kPairThreads * kPairs >= P2B_NUM_HANDS && kPairThreads >= 4 * P2B_NUM_CARDS, "every hand and every quarter of a card's hands has a thread");
 
-__global__ void __launch_bounds__(kThreads) chance_expand_features_kernel(
+__global__ void __launch_bounds__(kPairThreads, 4) chance_expand_features_kernel(
     const float* __restrict__ pre_beliefs, long long player_stride, const long long* __restrict__ boards, int board_len,
     const long long* __restrict__ sample_offsets, long long num_roots, const float* __restrict__ context,
     const ComboTable* __restrict__ combos, __nv_bfloat16* __restrict__ features, long long feature_stride,
-    long long* __restrict__ root_lookup) {
-    __shared__ double red[kCardsPerBlock][2][kThreads / 32];
-    __shared__ int cnt[kCardsPerBlock][kThreads / 32];
+    long long* __restrict__ root_lookup, int paired, int group) {
+    __shared__ float xs[2][2 * kPairThreads * kPairs];
+    __shared__ double cs[2][P2B_NUM_CARDS], red[2][kPairWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int groups = (P2B_NUM_CARDS + group - 1) / group;
     // the two cards of this thread's hands do not depend on the root
-    int c1[kHandsPerThread], c2[kHandsPerThread];
+    int c1[2 * kPairs], c2[2 * kPairs];
 #pragma unroll
-    for (int i = 0; i < kHandsPerThread; ++i) {
-        const int h = threadIdx.x + i * kThreads;
-        c1[i] = h < P2B_NUM_HANDS ? combos->c1[h] : 0;
-        c2[i] = h < P2B_NUM_HANDS ? combos->c2[h] : 0;
+    for (int i = 0; i < 2 * kPairs; ++i) {
+        const int h = 2 * (tid + (i >> 1) * kPairThreads) + (i & 1);
+        c1[i] = h < P2B_NUM_HANDS ? combos->c1[h] : -1;
+        c2[i] = h < P2B_NUM_HANDS ? combos->c2[h] : -1;
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (long long task = blockIdx.x; task < num_roots * kCardGroups; task += gridDim.x) {
-        const long long b = task / kCardGroups;
-        const int k0 = (int)(task - b * kCardGroups) * kCardsPerBlock;
+    for (long long task = blockIdx.x; task < num_roots * groups; task += gridDim.x) {
+        const long long b = task / groups;
+        const int k0 = (int)(task - b * groups) * group;
         const long long first = sample_offsets[b];
         const int n_free = (int)(sample_offsets[b + 1] - first);
         if (k0 >= n_free) continue;  // uniform over the block
-        const int n_here = min(kCardsPerBlock, n_free - k0);
+        const int n_here = min(group, n_free - k0);
         unsigned long long board_mask = 0;
         for (int j = 0; j < board_len; ++j) {
             const long long c = boards[b * board_len + j];
             if (c >= 0) board_mask |= 1ull << c;
         }
         // the k0-th free card, in ascending order; the following ones are the next set bits
-        unsigned long long free_cards = ~board_mask & ((1ull << P2B_NUM_CARDS) - 1ull);
-        for (int k = 0; k < k0; ++k) free_cards &= free_cards - 1ull;
-        const float* src0 = pre_beliefs + (b * 2) * player_stride;
-        const float* src1 = src0 + player_stride;
-        float v0[kHandsPerThread], v1[kHandsPerThread];
+        unsigned long long rest = ~board_mask & ((1ull << P2B_NUM_CARDS) - 1ull);
+        for (int k = 0; k < k0; ++k) rest &= rest - 1ull;
+        auto off_board = [&](int i) { return c1[i] >= 0 && (((board_mask >> c1[i]) | (board_mask >> c2[i])) & 1ull) == 0; };
+        float v[2][2 * kPairs];
+        double all[2] = {0.0, 0.0};
+        __syncthreads();  // the previous task's rows and sums have been read
 #pragma unroll
-        for (int i = 0; i < kHandsPerThread; ++i) {
-            const int h = threadIdx.x + i * kThreads;
-            const bool on = h < P2B_NUM_HANDS && (((board_mask >> c1[i]) | (board_mask >> c2[i])) & 1ull) == 0;
-            v0[i] = on ? src0[h] : 0.0f;
-            v1[i] = on ? src1[h] : 0.0f;
-            if (!on) c1[i] |= 64;  // marks a hand that no card of this root allows
+        for (int i = 0; i < 2 * kPairs; ++i) {
+            const int h = 2 * (tid + (i >> 1) * kPairThreads) + (i & 1);
+            const bool on = off_board(i);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                v[p][i] = on ? pre_beliefs[(b * 2 + p) * player_stride + h] : 0.0f;
+                xs[p][h] = v[p][i];
+                all[p] += (double)v[p][i];
+            }
         }
-        __syncthreads();  // the previous task's sums have been read
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) all[p] += __shfl_xor_sync(0xffffffffu, all[p], d);
+            if (lane == 0) red[p][warp] = all[p];
+        }
+        __syncthreads();
+        all[0] = all[1] = 0.0;
+#pragma unroll
+        for (int x = 0; x < kPairWarps; ++x) {
+            all[0] += red[0][x];
+            all[1] += red[1][x];
+        }
         {
-            unsigned long long rest = free_cards;
-            for (int k = 0; k < n_here; ++k) {
-                const int card = __ffsll((long long)rest) - 1;
-                rest &= rest - 1ull;
-                double s0 = 0.0, s1 = 0.0;
-                int n_allowed = 0;
+            // hands that hold a card, a quarter a thread; the threads beyond 207 repeat the last one's, unstored
+            const int t = min(tid, 4 * P2B_NUM_CARDS - 1), c = t >> 2, q = t & 3;
+            double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-                for (int i = 0; i < kHandsPerThread; ++i) {
-                    const bool ok = c1[i] != card && c2[i] != card && c1[i] < 64;
-                    s0 += (double)(ok ? v0[i] : 0.0f);
-                    s1 += (double)(ok ? v1[i] : 0.0f);
-                    n_allowed += ok;
+            for (int i = 0; i < 13; ++i) {
+                const int e = q + 4 * i;
+                if (e < 51) {
+                    const int h = e < c ? combo_index(e, c) : combo_row_offset(c) - c + e;
+                    s0 += (double)xs[0][h];
+                    s1 += (double)xs[1][h];
                 }
+            }
 #pragma unroll
-                for (int d = 16; d > 0; d >>= 1) {
-                    s0 += __shfl_xor_sync(0xffffffffu, s0, d);
-                    s1 += __shfl_xor_sync(0xffffffffu, s1, d);
-                    n_allowed += __shfl_xor_sync(0xffffffffu, n_allowed, d);
-                }
-                if (lane == 0) {
-                    red[k][0][warp] = s0;
-                    red[k][1][warp] = s1;
-                    cnt[k][warp] = n_allowed;
-                }
+            for (int d = 1; d < 4; d <<= 1) {
+                s0 += __shfl_xor_sync(0xffffffffu, s0, d);
+                s1 += __shfl_xor_sync(0xffffffffu, s1, d);
+            }
+            if (q == 0 && tid < 4 * P2B_NUM_CARDS) {
+                cs[0][c] = s0;
+                cs[1][c] = s1;
             }
         }
         __syncthreads();
-        unsigned long long rest = free_cards;
         for (int k = 0; k < n_here; ++k) {
             const int card = __ffsll((long long)rest) - 1;
             rest &= rest - 1ull;
             const long long smp = first + k0 + k;
-            if (threadIdx.x == 0 && root_lookup) root_lookup[smp] = b;
+            if (tid == 0 && root_lookup) root_lookup[smp] = b;
             __nv_bfloat16* row = features + smp * feature_stride;
-            double tot0 = 0.0, tot1 = 0.0;
-            int nall = 0;
+            bool held[2 * kPairs];
 #pragma unroll
-            for (int w = 0; w < kThreads / 32; ++w) {
-                tot0 += red[k][0][w];
-                tot1 += red[k][1][w];
-                nall += cnt[k][w];
-            }
-            const float uni = __fdiv_rn(1.0f, fmaxf((float)nall, 1.0f));
+            for (int i = 0; i < 2 * kPairs; ++i) held[i] = c1[i] == card || c2[i] == card;
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
-                const float sum = (float)(p ? tot1 : tot0);
-                const Divisor d = make_divisor(fmaxf(sum, 1e-12f));  // one divisor per row: exactly rounded quotients
+                double left = all[p] - cs[p][card];
+                if (left < 1e-6 * all[p]) {  // the subtraction has cancelled: add up what is left (uniform over the block)
+                    left = 0.0;
 #pragma unroll
-                for (int i = 0; i < kHandsPerThread; ++i) {
-                    const int h = threadIdx.x + i * kThreads;
+                    for (int i = 0; i < 2 * kPairs; ++i) left += held[i] ? 0.0 : (double)v[p][i];
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) left += __shfl_xor_sync(0xffffffffu, left, d);
+                    __syncthreads();
+                    if (lane == 0) red[p][warp] = left;
+                    __syncthreads();
+                    left = 0.0;
+                    for (int x = 0; x < kPairWarps; ++x) left += red[p][x];
+                }
+                const float sum = (float)left;
+                const Divisor d = make_divisor(fmaxf(sum, 1e-12f));  // one divisor per row: exactly rounded quotients
+                DivGuard g = guard_begin(d.ok);
+                float q[2 * kPairs];
+#pragma unroll
+                for (int i = 0; i < 2 * kPairs; ++i) q[i] = div_g<true>(held[i] ? 0.0f : v[p][i], d.y, d.r, g);
+                if (__builtin_expect(guard_bad(g) || !(sum > 1e-12f), 0)) {
+                    const int cards_left = P2B_NUM_CARDS - 1 - __popcll(board_mask);
+                    const float uni = __fdiv_rn(1.0f, fmaxf((float)(cards_left * (cards_left - 1) / 2), 1.0f));
+#pragma unroll
+                    for (int i = 0; i < 2 * kPairs; ++i)
+                        q[i] = sum > 1e-12f ? __fdiv_rn(held[i] ? 0.0f : v[p][i], d.y) : (off_board(i) && !held[i] ? uni : 0.0f);
+                }
+#pragma unroll
+                for (int j = 0; j < kPairs; ++j) {
+                    const int h = 2 * (tid + j * kPairThreads);
                     if (h < P2B_NUM_HANDS) {
-                        const bool ok = c1[i] != card && c2[i] != card && c1[i] < 64;
-                        const float v = ok ? (p ? v1[i] : v0[i]) : 0.0f;
-                        const float x = sum > 1e-12f ? div_exact(v, d) : (ok ? uni : 0.0f);
-                        row[p * P2B_NUM_HANDS + h] = __float2bfloat16_rn(x);
+                        __nv_bfloat16* at = row + p * P2B_NUM_HANDS + h;
+                        if (paired) {
+                            *reinterpret_cast<__nv_bfloat162*>(at) = __floats2bfloat162_rn(q[2 * j], q[2 * j + 1]);
+                        } else {
+                            at[0] = __float2bfloat16_rn(q[2 * j]);
+                            at[1] = __float2bfloat16_rn(q[2 * j + 1]);
+                        }
                     }
                 }
             }
             // board one-hot, context, padding
-            const unsigned long long mask = board_mask | (1ull << card);
-            for (long long j = 2 * P2B_NUM_HANDS + threadIdx.x; j < feature_stride; j += kThreads) {
+            for (long long j = 2 * P2B_NUM_HANDS + tid; j < feature_stride; j += kPairThreads) {
                 const int r = (int)(j - 2 * P2B_NUM_HANDS);
                 float x = 0.0f;
-                if (r < 52) x = ((mask >> r) & 1ull) ? 1.0f : 0.0f;
+                if (r < 52) x = (((board_mask >> r) & 1ull) || r == card) ? 1.0f : 0.0f;
                 else if (r < 55) x = context[b * 3 + (r - 52)];
                 row[j] = __float2bfloat16_rn(x);
             }
         }
-#pragma unroll
-        for (int i = 0; i < kHandsPerThread; ++i) c1[i] &= 63;
     }
 }
 
 // out[r, p, h] = mean over the samples of root r (rows sample_offsets[r] .. sample_offsets[r+1])
 // of src[sample, p*1326 + h], bf16 -> fp32, added in ascending sample order and divided by
-// max(count, 1) (chance_node_helper.py:462-477).  Each output element is owned by one thread.
+// max(count, 1) (chance_node_helper.py:462-477).  Each output element is owned by one thread, which (PAIRED: rows and base
+// allow it) takes two neighbours with one load a sample.
+template <bool PAIRED>
 __global__ void indexed_mean_bf16_kernel(const __nv_bfloat16* __restrict__ src, long long src_stride,
                                          const long long* __restrict__ sample_offsets, long long num_roots,
                                          float* __restrict__ out, long long out_player_stride) {
-    const long long n = num_roots * 2 * P2B_NUM_HANDS;
+    constexpr int kWide = PAIRED ? 2 : 1, kColumns = 2 * P2B_NUM_HANDS / kWide;
+    const long long n = num_roots * kColumns;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const long long r = e / (2 * P2B_NUM_HANDS);
-        const int c = (int)(e - r * 2 * P2B_NUM_HANDS), p = c >= P2B_NUM_HANDS, h = c - p * P2B_NUM_HANDS;
+        const long long r = e / kColumns;
+        const int c = (int)(e - r * kColumns) * kWide, p = c >= P2B_NUM_HANDS, h = c - p * P2B_NUM_HANDS;
         const long long a = sample_offsets[r], b = sample_offsets[r + 1];
-        float acc = 0.0f;
-        for (long long i = a; i < b; ++i) acc = __fadd_rn(acc, __bfloat162float(src[i * src_stride + c]));
-        out[(r * 2 + p) * out_player_stride + h] = __fdiv_rn(acc, fmaxf((float)(b - a), 1.0f));
+        float acc[kWide];
+#pragma unroll
+        for (int i = 0; i < kWide; ++i) acc[i] = 0.0f;
+#pragma unroll 8
+        for (long long i = a; i < b; ++i) {
+            if constexpr (PAIRED) {
+                const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + i * src_stride + c));
+                acc[0] = __fadd_rn(acc[0], x.x);
+                acc[1] = __fadd_rn(acc[1], x.y);
+            } else {
+                acc[0] = __fadd_rn(acc[0], __bfloat162float(src[i * src_stride + c]));
+            }
+        }
+        const float count = fmaxf((float)(b - a), 1.0f);
+#pragma unroll
+        for (int i = 0; i < kWide; ++i) out[(r * 2 + p) * out_player_stride + h + i] = __fdiv_rn(acc[i], count);
     }
 }
 
@@ -420,12 +466,15 @@ int p2b_chance_expand_features(const float* pre_beliefs, int64_t player_stride, 
         return set_error(P2B_ERR_ARG, "p2b_chance_expand_features: stride too small");
     int rc = ensure_tables();
     if (rc) return rc;
-    long long grid = num_roots * kCardGroups;
+    // all cards of a root in one block where the roots alone fill the chip, else eight at a time
+    const int group = num_roots >= 4ll * sm_count() ? P2B_NUM_CARDS : 8;
+    long long grid = num_roots * ((P2B_NUM_CARDS + group - 1) / group);
     if (grid > (long long)sm_count() * 16) grid = (long long)sm_count() * 16;
-    chance_expand_features_kernel<<<(unsigned)grid, kThreads, 0, (cudaStream_t)stream>>>(
+    chance_expand_features_kernel<<<(unsigned)grid, kPairThreads, 0, (cudaStream_t)stream>>>(
         pre_beliefs, player_stride, (const long long*)boards, board_len, (const long long*)sample_offsets, num_roots,
         context, device_combo_table(), static_cast<__nv_bfloat16*>(features_bf16), feature_stride,
-        (long long*)root_lookup);
+        (long long*)root_lookup,
+        (feature_stride & 1) == 0 && (reinterpret_cast<uintptr_t>(features_bf16) & 3) == 0, group);
     return check_cuda(cudaGetLastError(), "chance_expand_features_kernel");
 }
 
@@ -435,9 +484,11 @@ int p2b_indexed_mean_bf16(const void* src_bf16, int64_t src_stride, const int64_
     if (!src_bf16 || !sample_offsets || !out) return set_error(P2B_ERR_ARG, "p2b_indexed_mean_bf16: null pointer");
     if (src_stride < 2 * P2B_NUM_HANDS || out_player_stride < P2B_NUM_HANDS)
         return set_error(P2B_ERR_ARG, "p2b_indexed_mean_bf16: stride too small");
-    long long blocks = (num_roots * 2 * P2B_NUM_HANDS + kThreads - 1) / kThreads;
+    const bool paired = (src_stride & 1) == 0 && (reinterpret_cast<uintptr_t>(src_bf16) & 3) == 0;
+    long long blocks = (num_roots * 2 * P2B_NUM_HANDS / (paired ? 2 : 1) + kThreads - 1) / kThreads;
     if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-    indexed_mean_bf16_kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(
+    const auto kernel = paired ? indexed_mean_bf16_kernel<true> : indexed_mean_bf16_kernel<false>;
+    kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(
         static_cast<const __nv_bfloat16*>(src_bf16), src_stride, (const long long*)sample_offsets, num_roots, out,
         out_player_stride);
     return check_cuda(cudaGetLastError(), "indexed_mean_bf16_kernel");
