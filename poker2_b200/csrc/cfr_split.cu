@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(32 * kPrepWarps) split_prep_kernel(const CfrPa
 // copied into the warp's part of shared memory while the warp works on the node before, so that neither the child loops have
 // to be unrolled to have loads in flight nor a register is spent on a row that waits: with the loads in registers and a body
 // per child count the kernel ran at 20 warps an SM, half of their stalls on loads and a fifth on instruction fetches.
-constexpr int kUpThreads = 256;  // at most
+constexpr int kUpThreads = 256, kUpSlices = 3;  // of a block, at most
 enum UpSlot { kUpPolicy = 0, kUpSeen = 1, kUpRegret = 2, kUpSum = 3, kUpAverage = 4, kUpValueA = 5, kUpValueO = 6, kUpSlots = 7 };
 constexpr int kUpNodeRows = 3;  // behind the children's rows: regret weights, reach, old average reach
 constexpr int kUpRow = 64;      // floats
@@ -510,8 +510,33 @@ __device__ __forceinline__ void up_stage_values(const SplitWork& w, const SplitI
     }
 }
 
+// The warps of a slice tell one another when the values of a level are stored: an mbarrier a level, at which each warp arrives
+// once.  What follows the values at a node (average, regrets, next policy) does not hold up the levels above.
+__device__ __forceinline__ void level_init(uint64_t* bar, int warps) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(warps) : "memory");
+}
+__device__ __forceinline__ void level_arrive(uint64_t* bar) {  // the whole warp
+    __threadfence_block();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+        asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"((unsigned)__cvta_generic_to_shared(bar)) : "memory");
+}
+__device__ __forceinline__ bool level_wait(uint64_t* bar) {  // false: given up
+    for (int i = 0; i < (1 << 20); ++i) {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred q;\n mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 q, [%1], 0;\n selp.u32 %0, 1, 0, q;\n}"
+            : "=r"(done)
+            : "r"((unsigned)__cvta_generic_to_shared(bar))
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// `stored`: where to arrive once the node's values are stored (null: the warp has another node of this level to come).
 __device__ __forceinline__ void up_node(const CfrParams& p, const SplitWork& w, const UpPass& u, const SplitItem& it, int h,
-                                        float* at) {
+                                        float* at, uint64_t* stored) {
     const int k = it.n_children, a = it.to_act, j = it.node, fc = it.first_child;
     const long long kids = (long long)(it.node_begin + fc) * P2B_HPAD + h;
     const float* node_rows = at + k * kUpSlots * kUpRow;
@@ -541,6 +566,7 @@ __device__ __forceinline__ void up_node(const CfrParams& p, const SplitWork& w, 
         stc<2>(v + a * P2B_HPAD, acc_a);
         stc<2>(v + (1 - a) * P2B_HPAD, acc_o);
     }
+    if (stored) level_arrive(stored);
     if (u.job >= kUpFinal) return;
     if (u.keep_values) {  // the values of this iteration at the node and at the leaves below it
         float* out = p.values_avg + (long long)it.node_begin * 2 * P2B_HPAD + h;
@@ -687,13 +713,13 @@ __device__ __forceinline__ void up_node(const CfrParams& p, const SplitWork& w, 
     }
 }
 
-// A block holds `slices` slices of one subgame with `lanes` warps each, which take the nodes of a level in turn; a level is
-// complete when the warps of a slice meet at its barrier.  `ring`: rows of a warp's staging area; two nodes that follow one
+// A block holds `slices` slices of one subgame with `lanes` warps each, which take the nodes of a level in turn.  `ring`: rows of a warp's staging area; two nodes that follow one
 // another lie at its two ends if they fit together, else the second is copied once the first is done.
 __global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p, const SplitWork w, int job, int pass, bool advance,
                                                               bool mixed, int lanes, int slices, int ring) {
     constexpr int kSlices = P2B_HPAD / kUpRow;
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint64_t ready[kUpSlices][kSplitMaxDepth + 1];
     if (p.work_counter[1] != 0) return;
     const int per_subgame = kSlices / slices;
     const int q = blockIdx.x / per_subgame;
@@ -725,42 +751,54 @@ __global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p,
     u.d_pos = make_divisor(u.sn.den_pos);
     u.d_neg = make_divisor(u.sn.den_neg);
     const int leaf0 = p.leaf_begin ? p.leaf_begin[s] : 0;
+    if (tid < slices * (kSplitMaxDepth + 1)) level_init(&ready[0][0] + tid, lanes);
     __syncthreads();
     launch_next();
     previous_done();
 
-    // one warp a slice: straight up the tree, no barrier
-    const bool alone = lanes == 1;
-    const int n_levels = alone ? 1 : lv->n_levels;
-    auto begin_of = [&](int d) { return alone ? 0 : (int)lv->begin[d]; };
-    auto first_of = [&](int d) { return (alone ? sg.n_internal : (int)lv->begin[d + 1]) - 1 - lane_warp; };
-    int d = n_levels - 1, level = d;
+    uint64_t* level_ready = ready[mine];
+    auto first_of = [&](int d) { return (int)lv->begin[d + 1] - 1 - lane_warp; };
+    const int n_levels = lv->n_levels;
+    int d = n_levels - 1, waited = n_levels;  // levels from `waited` on are known to be stored
     int x = first_of(d);
-    while (d > 0 && x < begin_of(d)) x = first_of(--d);
-    bool any = x >= begin_of(d), top = false;
+    auto skip_empty = [&]() {  // to the warp's next node; it has nothing to store at the levels in between
+        while (x < lv->begin[d]) {
+            level_arrive(level_ready + d);
+            if (d == 0) return false;
+            x = first_of(--d);
+        }
+        return true;
+    };
+    bool any = skip_empty(), top = false;
     if (any) up_stage(p, w, u, items[x], nodes, h, leaf0, stage);
     while (any) {
-        for (; level > d; --level) asm volatile("bar.sync %0, %1;" ::"r"(mine + 1), "r"(32 * lanes) : "memory");
         const SplitItem& it = items[x];
         const int rows = up_rows(it.n_children);
         float* at = stage + (top ? (ring - rows) * kUpRow : 0);
+        if (d + 1 < waited) {  // its children are one level down
+            if (!level_wait(level_ready + d + 1)) atomicMax(p.work_counter + 1, s + 1);
+            waited = d + 1;
+        }
         up_stage_values(w, it, h, at);
         asm volatile("cp.async.wait_all;" ::: "memory");
-        int nx = x - lanes, nd = d;
-        while (nd > 0 && nx < begin_of(nd)) nx = first_of(--nd);
-        const bool more = nx >= begin_of(nd);
-        const int next_rows = more ? up_rows(items[nx].n_children) : 0;
+        uint64_t* stored = nullptr;
+        x -= lanes;
+        if (x < lv->begin[d]) {  // the warp's last node of this level; the empty levels above take its arrival now
+            stored = level_ready + d;
+            any = d > 0;
+            if (any) {
+                x = first_of(--d);
+                any = skip_empty();
+            }
+        }
+        const int next_rows = any ? up_rows(items[x].n_children) : 0;
         float* next_at = stage + (top ? 0 : (ring - next_rows) * kUpRow);
         const bool ahead = rows + next_rows <= ring;
-        if (more && ahead) up_stage(p, w, u, items[nx], nodes, h, leaf0, next_at);
-        up_node(p, w, u, it, h, at);
-        if (more && !ahead) up_stage(p, w, u, items[nx], nodes, h, leaf0, next_at);
-        x = nx;
-        d = nd;
-        any = more;
+        if (any && ahead) up_stage(p, w, u, items[x], nodes, h, leaf0, next_at);
+        up_node(p, w, u, it, h, at, stored);
+        if (any && !ahead) up_stage(p, w, u, items[x], nodes, h, leaf0, next_at);
         top = !top;
     }
-    for (; level > 0; --level) asm volatile("bar.sync %0, %1;" ::"r"(mine + 1), "r"(32 * lanes) : "memory");
     if (advance && lane_warp == 0) advance_root(p, s, h);
 }
 
