@@ -1627,13 +1627,16 @@ int launch_prep(const CfrParams& p, const SplitWork& w, int pass, int max_childr
 
 int launch_up(const CfrParams& p, const SplitWork& w, UpJob job, int pass, bool advance, bool mixed, int max_children, bool follows,
               cudaStream_t stream) {
+    int ring = 40;  // two nodes of two or three actions, the usual ones, fit together
+    if (ring < up_rows(max_children)) ring = up_rows(max_children);
     // Warps a slice: one warp's walk up a tree is the time of a small batch, so nodes of a level are spread over up to eight;
-    // more warps than it takes to keep the memory busy only wait at the levels with few nodes.  Measured (us a pass; 8 / 4 /
+    // but no more warps than twice what the SMs hold at a time, beyond which they only queue.  Measured (us a pass; 8 / 4 /
     // 2 / 1 warps a slice): 1 subgame 17 / 21 / 29 / 49, 37 of 96 nodes 76 / 79 / 114 / 198, 192 of 77 nodes 318 / 257 /
     // 231 / 264, 4096 of 54 nodes - / - / 2550 / 2730.
-    const int lanes = p.num_subgames >= sm_count() ? 2 : 8, slices = lanes == 2 ? 3 : 1;
-    int ring = 40;  // two nodes of two or three actions, the usual ones, fit together; 18 warps an SM
-    if (ring < up_rows(max_children)) ring = up_rows(max_children);
+    const long long held = (long long)sm_count() * (227 * 1024 / (ring * kUpRow * 4));
+    int lanes = 8;
+    while (lanes > 2 && (long long)p.num_subgames * (P2B_HPAD / kUpRow) * lanes > 2 * held) lanes /= 2;
+    const int slices = lanes == 2 ? kUpSlices : 1;
     long long nodes = (long long)p.max_internal * max_children + 1;
     if (nodes > kCfrMaxNodes) nodes = kCfrMaxNodes;
     const int bytes = lanes * slices * ring * kUpRow * 4 + p.max_internal * (int)sizeof(SplitItem) + (int)nodes * (int)sizeof(NodeRecPacked);
