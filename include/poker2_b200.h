@@ -50,6 +50,9 @@ int p2b_compare7_planes(const int8_t* planes, int64_t n, int32_t* out, void* str
  * counterpart of _init_hand_rank_data (src/p2/search/cfr_evaluator.py:406-482). */
 int p2b_rank_hands(const int16_t* boards, int64_t m, int32_t* scores, int64_t* order,
                    unsigned char* tables, void* stream);
+/* the same on int64 boards (of which the low 16 bits count) */
+int p2b_rank_hands_i64(const int64_t* boards, int64_t m, int32_t* scores, int64_t* order,
+                   unsigned char* tables, void* stream);
 
 /* ---- showdown (src/p2/search/cfr_evaluator.py:484-601, _showdown_value_both) ------
  * beliefs/values: `rows` rows of [2,1326] fp32, consecutive rows `*_row_stride` floats

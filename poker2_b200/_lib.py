@@ -31,6 +31,7 @@ _SIGNATURES = {
     "p2b_compare7_cards_i64": [_vp, _i64, _vp, _vp],
     "p2b_compare7_planes": [_vp, _i64, _vp, _vp],
     "p2b_rank_hands": [_vp, _i64, _vp, _vp, _vp, _vp],
+    "p2b_rank_hands_i64": [_vp, _i64, _vp, _vp, _vp, _vp],
     "p2b_showdown_values": [_vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _vp],
     "p2b_showdown_values_at": [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _vp],
     "p2b_showdown_ev_sorted": [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _f32, _vp, _vp],
@@ -151,6 +152,13 @@ def stream_ptr(device: torch.device):
     if _raw_stream is None:
         return torch.cuda.current_stream(device).cuda_stream
     return _raw_stream(torch.cuda.current_device() if device.index is None else device.index)
+
+
+def card_ids(t: torch.Tensor):
+    """(contiguous card ids, suffix of the entry points that read them): int64 and int16 as they are, others as int16."""
+    if t.dtype == torch.int64:
+        return t.contiguous(), "_i64"
+    return t.contiguous().to(torch.int16), ""
 
 
 def require_cuda(t: torch.Tensor, what: str) -> None:

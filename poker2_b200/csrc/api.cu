@@ -12,6 +12,7 @@ int launch_compare7_cards(const int16_t*, int64_t, int32_t*, cudaStream_t);
 int launch_compare7_cards(const int64_t*, int64_t, int32_t*, cudaStream_t);
 int launch_compare7_planes(const int8_t*, int64_t, int32_t*, cudaStream_t);
 int launch_board_setup(const int16_t*, int64_t, unsigned char*, int32_t*, long long*, cudaStream_t);
+int launch_board_setup(const int64_t*, int64_t, unsigned char*, int32_t*, long long*, cudaStream_t);
 int launch_showdown_eval(const unsigned char*, const int32_t*, const int64_t*, const float*, int64_t, const long long*, const float*,
                          float*, int64_t, int64_t, cudaStream_t);
 int launch_showdown_ev_sorted(const float*, const int32_t*, const int32_t*, const int32_t*, const int32_t*, int64_t, int,
@@ -63,6 +64,14 @@ int p2b_compare7_planes(const int8_t* planes, int64_t n, int32_t* out, void* str
 }
 
 int p2b_rank_hands(const int16_t* boards, int64_t m, int32_t* scores, int64_t* order, unsigned char* tables,
+                   void* stream) {
+    P2B_REQUIRE(m >= 0, "negative count");
+    P2B_REQUIRE(m == 0 || boards, "null boards");
+    P2B_REQUIRE(tables == nullptr || (reinterpret_cast<uintptr_t>(tables) & 15) == 0, "tables must be 16-byte aligned");
+    return launch_board_setup(boards, m, tables, scores, reinterpret_cast<long long*>(order), (cudaStream_t)stream);
+}
+
+int p2b_rank_hands_i64(const int64_t* boards, int64_t m, int32_t* scores, int64_t* order, unsigned char* tables,
                    void* stream) {
     P2B_REQUIRE(m >= 0, "negative count");
     P2B_REQUIRE(m == 0 || boards, "null boards");

@@ -22,8 +22,6 @@
 // of the showdown tables) and the barriers between its phases bound it, with half of the issue slots used.  The up kernel
 // is bound by memory at large batches (2.55 ms on 4096 subgames of 54 nodes, 0.9 of the copy bandwidth over the 15 GB it
 // moves) and by the latency of a warp's walk at small ones.
-#include <atomic>
-
 #include "cfr_split.cuh"
 
 #include "cfr_dev.cuh"
@@ -1555,26 +1553,6 @@ __global__ void __launch_bounds__(kRowThreads) split_exploitability_kernel(const
     __syncthreads();
     if (tid == 0) p.exploitability[s] = __fadd_rn(sums[0], sums[1]);
     if (tid < 2 && p.br_values) p.br_values[(long long)s * 2 + tid] = sums[2 + tid];
-}
-
-// Raises a kernel's shared-memory limit on the current device, once for each size it has not had there (the call takes as
-// long as a launch).
-struct SharedLimit {
-    std::atomic<int> bytes[64] = {};
-};
-int allow_shared(SharedLimit& had, const void* kernel, int bytes) {
-    int dev = 0;
-    int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-    if (rc) return rc;
-    const bool known = dev >= 0 && dev < 64;
-    if (known && had.bytes[dev].load() >= bytes) return P2B_OK;
-    rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "shared-memory attribute");
-    if (!rc && known) {
-        int seen = had.bytes[dev].load();
-        while (seen < bytes && !had.bytes[dev].compare_exchange_weak(seen, bytes)) {
-        }
-    }
-    return rc;
 }
 
 // `follows`: the launch before it on the stream was one of these kernels (see launch_next).

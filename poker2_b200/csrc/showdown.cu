@@ -93,11 +93,12 @@ __device__ __forceinline__ void scan_byte_counts(const uint32_t* __restrict__ cn
     __syncthreads();
 }
 
-// boards: [m,5] int16.  Any of tabs / scores / order may be null.
+// boards: [m,5] int16, or int64 (of which the low 16 bits count).  Any of tabs / scores / order may be null.
 //   tabs   : [m, kTabBytes] table blobs used by the showdown evaluation
 //   scores : [m,1326] int32 packed strength of every combo
 //   order  : [m,1326] int64 stable ascending argsort of scores
-__global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const int16_t* __restrict__ boards, int64_t m,
+template <typename T>
+__global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const T* __restrict__ boards, int64_t m,
                                                                        const ComboTable* __restrict__ combos,
                                                                        const RankLut* __restrict__ lut,
                                                                        unsigned char* __restrict__ tabs,
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const int
     // ---- 1. strengths ----
     int bc[5];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) bc[i] = boards[b * 5 + i];
+    for (int i = 0; i < 5; ++i) bc[i] = (int16_t)boards[b * 5 + i];
     uint64_t bsuits = 0;
     RankChain bchain;
 #pragma unroll
@@ -506,17 +507,25 @@ __global__ void __launch_bounds__(kEvalThreads, 2) showdown_eval_kernel(
 
 int sm_count();
 
-int launch_board_setup(const int16_t* boards, int64_t m, unsigned char* tabs, int32_t* scores, long long* order,
+template <typename T>
+static int board_setup(const T* boards, int64_t m, unsigned char* tabs, int32_t* scores, long long* order,
                        cudaStream_t stream) {
     if (m == 0) return P2B_OK;
     int rc = ensure_tables();
     if (rc) return rc;
-    rc = check_cuda(cudaFuncSetAttribute(board_setup_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSetupSmem),
-                    "board_setup_kernel smem attribute");
+    static SharedLimit had;
+    rc = allow_shared(had, reinterpret_cast<const void*>(board_setup_kernel<T>), kSetupSmem);
     if (rc) return rc;
-    board_setup_kernel<<<(unsigned)m, kSetupThreads, kSetupSmem, stream>>>(boards, m, device_combo_table(),
+    board_setup_kernel<T><<<(unsigned)m, kSetupThreads, kSetupSmem, stream>>>(boards, m, device_combo_table(),
                                                                          device_rank_lut(), tabs, scores, order);
     return check_cuda(cudaGetLastError(), "board_setup_kernel");
+}
+
+int launch_board_setup(const int16_t* boards, int64_t m, unsigned char* tabs, int32_t* scores, long long* order, cudaStream_t s) {
+    return board_setup(boards, m, tabs, scores, order, s);
+}
+int launch_board_setup(const int64_t* boards, int64_t m, unsigned char* tabs, int32_t* scores, long long* order, cudaStream_t s) {
+    return board_setup(boards, m, tabs, scores, order, s);
 }
 
 int launch_showdown_eval(const unsigned char* tabs, const int32_t* tab_of_row, const int64_t* row_index, const float* beliefs,
@@ -526,8 +535,8 @@ int launch_showdown_eval(const unsigned char* tabs, const int32_t* tab_of_row, c
     int rc = ensure_tables();
     if (rc) return rc;
     const auto kernel = row_index ? showdown_eval_kernel<true> : showdown_eval_kernel<false>;
-    rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEvalSmem),
-                    "showdown_eval_kernel smem attribute");
+    static SharedLimit had[2];
+    rc = allow_shared(had[row_index != nullptr], reinterpret_cast<const void*>(kernel), kEvalSmem);
     if (rc) return rc;
     int64_t grid = rows;
     const int64_t cap = (int64_t)sm_count() * 2;

@@ -1035,8 +1035,8 @@ int p2b_steps_seen(const float* beliefs, const float* policy, const int64_t* to_
     int rc = ensure_tables();
     if (rc) return rc;
     constexpr int kBytes = (1 + kSeenRows) * (P2B_HPAD * 4 + 53 * 8);
-    rc = check_cuda(cudaFuncSetAttribute(step_seen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes),
-                    "step_seen_kernel shared-memory attribute");
+    static SharedLimit had;
+    rc = allow_shared(had, reinterpret_cast<const void*>(step_seen_kernel), kBytes);
     if (rc) return rc;
     step_seen_kernel<<<(unsigned)num_parents, kRowThreads, kBytes, (cudaStream_t)stream>>>(
         beliefs, policy, (const long long*)to_act, (const long long*)child_offsets, (const long long*)child_count,

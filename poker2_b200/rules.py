@@ -50,26 +50,13 @@ def compare_7_batches(a_batch: torch.Tensor, b_batch: torch.Tensor) -> torch.Ten
     return compare_7_single_batch(torch.stack([a_batch, b_batch], dim=1).bool())
 
 
-def _card_ids(t: torch.Tensor):
-    """(contiguous card ids, suffix of the entry point that reads them): int16 and int64 as they are."""
-    if t.dtype == torch.int64:
-        return t.contiguous(), "_i64"
-    return _as_i16(t), ""
-
-
-def _as_i16(t: torch.Tensor) -> torch.Tensor:
-    if t.dtype == torch.int16 and t.is_contiguous():
-        return t
-    return t.contiguous().to(torch.int16)
-
-
 def compare_7_cards_single_batch(cards_batch: torch.Tensor) -> torch.Tensor:
     """[N,2,7] card ids 0..51 -> int32 [N] in {1,-1,0} (rules_triton.py:78-93)."""
     _require_backend()
     if cards_batch.dim() != 3 or tuple(cards_batch.shape[1:]) != (2, 7):
         raise ValueError(f"Expected [N, 2, 7] input, got {tuple(cards_batch.shape)}")
     _lib.require_cuda(cards_batch, "CUDA hand evaluator")
-    cards, kind = _card_ids(cards_batch)
+    cards, kind = _lib.card_ids(cards_batch)
     out = torch.empty((cards.shape[0],), device=cards.device, dtype=torch.int32)
     with _lib.on(cards.device):
         _lib.call("p2b_compare7_cards" + kind, _lib.ptr(cards), cards.shape[0], _lib.ptr(out),
@@ -84,7 +71,7 @@ def rank_7_cards_single_batch(cards_batch: torch.Tensor) -> torch.Tensor:
     if cards_batch.dim() != 2 or cards_batch.shape[1] != 7:
         raise ValueError(f"Expected [N, 7] input, got {tuple(cards_batch.shape)}")
     _lib.require_cuda(cards_batch, "CUDA hand evaluator")
-    cards, kind = _card_ids(cards_batch)
+    cards, kind = _lib.card_ids(cards_batch)
     out = torch.empty((cards.shape[0],), device=cards.device, dtype=torch.int32)
     with _lib.on(cards.device):
         _lib.call("p2b_rank7_cards" + kind, _lib.ptr(cards), cards.shape[0], _lib.ptr(out),
@@ -99,12 +86,12 @@ def rank_hands(board: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     if board.dim() != 2 or board.shape[1] != 5:
         raise ValueError(f"board must be [M, 5], got {tuple(board.shape)}")
     _lib.require_cuda(board, "CUDA hand evaluator")
-    b16 = _as_i16(board)
-    m = b16.shape[0]
+    ids, kind = _lib.card_ids(board)
+    m = ids.shape[0]
     scores = torch.empty((m, NUM_HANDS), device=board.device, dtype=torch.int32)
     order = torch.empty((m, NUM_HANDS), device=board.device, dtype=torch.int64)
     with _lib.on(board.device):
-        _lib.call("p2b_rank_hands", _lib.ptr(b16), m, _lib.ptr(scores), _lib.ptr(order), None,
+        _lib.call("p2b_rank_hands" + kind, _lib.ptr(ids), m, _lib.ptr(scores), _lib.ptr(order), None,
                   _lib.stream_ptr(board.device))
     return scores, order
 

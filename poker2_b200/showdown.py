@@ -22,11 +22,17 @@ class BoardTables:
         _lib.require_cuda(boards, "BoardTables")
         self.device = boards.device
         self.num_boards = boards.shape[0]
-        b16 = boards.contiguous().to(torch.int16)
+        ids, kind = _lib.card_ids(boards)
         self.blob = torch.empty((self.num_boards, _lib.TABLE_BYTES), device=self.device, dtype=torch.uint8)
         with _lib.on(self.device):
-            _lib.call("p2b_rank_hands", _lib.ptr(b16), self.num_boards, None, None, _lib.ptr(self.blob),
+            _lib.call("p2b_rank_hands" + kind, _lib.ptr(ids), self.num_boards, None, None, _lib.ptr(self.blob),
                       _lib.stream_ptr(self.device))
+
+
+def _there(t: torch.Tensor, device, dtype) -> torch.Tensor:
+    if t.dtype != dtype or t.device != device:
+        t = t.to(device=device, dtype=dtype)
+    return t.contiguous()
 
 
 def showdown_values(
@@ -45,11 +51,11 @@ def showdown_values(
         raise ValueError(f"beliefs must be [R, 2, {NUM_HANDS}], got {tuple(beliefs.shape)}")
     rows = beliefs.shape[0]
     assert beliefs.dtype == torch.float32 and beliefs.is_contiguous()
-    potential = potential.to(device=beliefs.device, dtype=torch.int64).contiguous()
-    scale = scale.to(device=beliefs.device, dtype=torch.float32).contiguous()
+    potential = _there(potential, beliefs.device, torch.int64)
+    scale = _there(scale, beliefs.device, torch.float32)
     assert tuple(potential.shape) == (rows, 2) and tuple(scale.shape) == (rows,)
     if table_of_row is not None:
-        table_of_row = table_of_row.to(device=beliefs.device, dtype=torch.int32).contiguous()
+        table_of_row = _there(table_of_row, beliefs.device, torch.int32)
         assert tuple(table_of_row.shape) == (rows,)
     elif rows != tables.num_boards:
         raise ValueError("table_of_row is required when rows != number of boards")
