@@ -9,13 +9,13 @@ namespace p2b {
 // Board set-up.  One block per board, 352 threads, four keys per thread.
 //   1. strength of every combo (board cards + two hole cards; combos that overlap the board
 //      are scored with repeated card ids, as p2/env/rules_triton.py:139-146 does).  On a fixed
-//      board the rank part of the score (multiplicity category, kickers, straight) depends on
-//      the two hole RANKS only: it is computed once per rank pair (169 threads) and looked up
-//      per combo; only the board's suit with three or more cards, if any, can make a flush,
-//      which costs a combo one table entry of the suit's rank mask;
-//   2. stable LSD radix sort of the 24-bit strengths, four passes of six bits.  A warp ranks
-//      32 consecutive keys with a match instruction; counts per (digit, chunk of 32) are
-//      bytes, scanned in digit-major order to give every key its destination;
+//      board the rank part of the score (multiplicity category, kickers, straight) depends on the
+//      two hole RANKS only, and only the board's suit with three or more cards, if any, can make
+//      a flush, whose score depends on the ranks that the combo adds to it.  So a board has at
+//      most 91 + 91 strengths; each is computed once and numbered by how many of them are lower;
+//   2. stable LSD radix sort of these 8-bit numbers, number and hand in one word, two passes of
+//      four bits.  A warp ranks 32 consecutive keys with four votes; counts per (digit, chunk of
+//      32) are bytes, scanned in digit-major order to give every key its destination;
 //   3. tie groups [L,R) from the sorted strengths (one block-wide max scan);
 //   4. per card, a bit mask over the sorted positions of the hands that hold it, and the
 //      running bit counts per 32-position word;
@@ -23,34 +23,41 @@ namespace p2b {
 //      many entries of those lists lie before L and before R -- each a count of mask bits
 //      below a position.
 // The table blob is assembled in shared memory and written out with 16-byte stores.
+// Bound by shared-memory wavefronts and barriers.  4096 boards and their evaluation: 233 us with 24-bit keys
+// in four passes of six bits, 215 with the 8-bit numbers, 205 with four blocks per SM (40 registers; 47.9 KB).
 // ---------------------------------------------------------------------------------------
 constexpr int kSetupThreads = 352;
 constexpr int kSetupWarps = kSetupThreads / 32;         // 11
 constexpr int kSortChunks = 44;                         // chunks of 32 keys
 constexpr int kSortN = kSortChunks * 32;                // 1408 >= 1326
 constexpr int kSortRounds = kSortChunks / kSetupWarps;  // 4 chunks per warp
-constexpr int kDigitBits = 6, kDigits = 1 << kDigitBits, kSortPasses = 4;
+constexpr int kDigitBits = 4, kDigits = 1 << kDigitBits, kSortPasses = 2;
 static_assert(kSortChunks % 4 == 0, "count bytes are scanned four at a time");
 static_assert(kSortChunks == kSortRounds * kSetupWarps, "every warp sorts the same number of chunks");
-constexpr int kSortCntWords = kDigits * kSortChunks / 4;  // 704 words of four byte counters
+constexpr int kSortCntWords = kDigits * kSortChunks / 4;  // 176 words of four byte counters
+static_assert(kSortCntWords <= kSetupThreads, "a thread scans one word of counters");
+// Strengths one board can give: one per unordered pair of hole ranks (91) and one per set of one or two
+// ranks added to the suit that can make a flush (91); 182 numbers fit the sort's 8 bits with 255 for the pads.
+constexpr int kRankPairs = 91;
+constexpr int kClassPad = 184;  // 2 * kRankPairs, in fours
+static_assert(2 * kRankPairs <= kClassPad && 2 * kRankPairs < (1 << (kDigitBits * kSortPasses)), "classes fit the sorted digits");
 constexpr int kMaskWords = 42;                            // 32-position words of a card's mask (1326 positions, and 1326 itself)
 constexpr int kMaskStride = 43;                           // odd: the cards of one word fall into distinct banks
 static_assert(kMaskWords * 32 > P2B_NUM_HANDS && kMaskStride >= kMaskWords, "a mask covers positions 0..1326");
 
 // shared-memory carve-up (bytes)
-constexpr int kSuKey = 0;                                // uint32 [2][kSortN]
-constexpr int kSuVal = kSuKey + 2 * kSortN * 4;          // uint16 [2][kSortN]
-constexpr int kSuCnt = kSuVal + 2 * kSortN * 2;          // uint32: sort counters [kSortCntWords], then card masks [52][kMaskStride]
+constexpr int kSuItem = 0;                               // uint32 [2][kSortN]  strength class << 16 | hand
+constexpr int kSuCnt = kSuItem + 2 * kSortN * 4;         // uint32: sort counters [kSortCntWords], then card masks [52][kMaskStride]
 constexpr int kSuCntWords = 52 * kMaskStride;            // 2236 >= kSortCntWords
-constexpr int kSuOff = kSuCnt + kSuCntWords * 4;         // rank-pair scores int32 [169], then sort offsets uint16 [64*44],
-constexpr int kSuOffBytes = kDigits * kSortChunks * 2;   // then mask bit counts uint16 [52][kMaskStride]
-static_assert(kSuOffBytes >= 52 * kMaskStride * 2 && kSuOffBytes >= 169 * 4 && kSuCntWords >= kSortCntWords, "shared areas");
+constexpr int kSuOff = kSuCnt + kSuCntWords * 4;         // strengths int32 [kClassPad] and their classes uint8, then sort offsets
+constexpr int kSuOffBytes = (52 * kMaskStride * 2 + 15) / 16 * 16;  // uint16 [16*44], then mask bit counts uint16 [52][kMaskStride]
+static_assert(kSuOffBytes >= kDigits * kSortChunks * 2 && kSuOffBytes >= kClassPad * 5 && kSuCntWords >= kSortCntWords, "shared areas");
 constexpr int kSuLg = kSuOff + kSuOffBytes;              // uint16 [kSortN]   tie-group start per sorted position
 constexpr int kSuRt = kSuLg + kSortN * 2;                // uint16 [kSortN]   tie-group end, indexed by group start
 constexpr int kSuBlob = (kSuRt + kSortN * 2 + 15) / 16 * 16;  // the table blob
 constexpr int kSuWarp = kSuBlob + kTabBytes;             // uint32 [16] warp totals of the block scan
 constexpr int kSetupSmem = kSuWarp + 64;
-static_assert(kSuCnt % 4 == 0 && kSuOff % 4 == 0 && kSuBlob % 16 == 0 && kSuWarp % 4 == 0, "alignment");
+static_assert(kSuCnt % 16 == 0 && kSuOff % 16 == 0 && kSuBlob % 16 == 0 && kSuWarp % 4 == 0, "alignment");
 
 // Exclusive prefix over `words*4` byte counters (in memory order) -> uint16 offsets.  Every
 // thread takes `words_per_thread` consecutive words.  Ends with a barrier.
@@ -98,20 +105,20 @@ __device__ __forceinline__ void scan_byte_counts(const uint32_t* __restrict__ cn
 //   scores : [m,1326] int32 packed strength of every combo
 //   order  : [m,1326] int64 stable ascending argsort of scores
 template <typename T>
-__global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const T* __restrict__ boards, int64_t m,
+__global__ void __launch_bounds__(kSetupThreads, 4) board_setup_kernel(const T* __restrict__ boards, int64_t m,
                                                                        const ComboTable* __restrict__ combos,
                                                                        const RankLut* __restrict__ lut,
                                                                        unsigned char* __restrict__ tabs,
                                                                        int32_t* __restrict__ scores,
                                                                        long long* __restrict__ order) {
     extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t* key = reinterpret_cast<uint32_t*>(smem + kSuKey);
-    uint16_t* val = reinterpret_cast<uint16_t*>(smem + kSuVal);
+    uint32_t* item = reinterpret_cast<uint32_t*>(smem + kSuItem);
     uint32_t* cnt = reinterpret_cast<uint32_t*>(smem + kSuCnt);
     unsigned char* cnt8 = smem + kSuCnt;
     uint32_t* cmask = reinterpret_cast<uint32_t*>(smem + kSuCnt);   // [52][kMaskStride], after the sort
     uint16_t* off = reinterpret_cast<uint16_t*>(smem + kSuOff);
-    int32_t* pair_score = reinterpret_cast<int32_t*>(smem + kSuOff);  // [13][13], before the sort
+    int32_t* strength = reinterpret_cast<int32_t*>(smem + kSuOff);    // [kClassPad], before the sort
+    uint8_t* cls = smem + kSuOff + kClassPad * 4;                     // [kClassPad], before the sort
     uint16_t* cpre = reinterpret_cast<uint16_t*>(smem + kSuOff);      // [52][kMaskStride], after the sort
     uint16_t* lg = reinterpret_cast<uint16_t*>(smem + kSuLg);
     uint16_t* rt = reinterpret_cast<uint16_t*>(smem + kSuRt);
@@ -133,13 +140,6 @@ __global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const T* 
         bsuits |= 1ull << bit;
         bchain.add(1u << (bit & 15));
     }
-    if (tid < 169) {  // rank part per pair of hole ranks (every occurrence of a rank counts, repeated card ids included)
-        const int r1 = tid / 13, r2 = tid - 13 * r1;
-        RankChain ch = bchain;
-        ch.add(1u << r1);
-        ch.add(1u << r2);
-        pair_score[tid] = score_rank_part(ch.classes(), ch.seen);
-    }
     // the one suit of the board that can make a flush (three or more cards), if any
     int fsuit = -1;
     uint32_t fboard = 0;
@@ -151,61 +151,98 @@ __global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const T* 
             fboard = ms;
         }
     }
+    auto rank_pair = [](int a, int c) {
+        const int lo = min(a, c), hi = max(a, c);
+        return hi * (hi + 1) / 2 + lo;
+    };
     for (int i = tid; i < kSortCntWords; i += kSetupThreads) cnt[i] = 0u;
-    __syncthreads();
-    for (int h = tid; h < kSortN; h += kSetupThreads) {
-        uint32_t k = 0xffffffffu;
-        if (h < P2B_NUM_HANDS) {
-            const int b1 = card_bit(combos->c1[h]), b2 = card_bit(combos->c2[h]);
-            int32_t s = pair_score[(b1 & 15) * 13 + (b2 & 15)];
-            if (fsuit >= 0) {
-                const uint32_t fm = fboard | ((b1 >> 4) == fsuit ? 1u << (b1 & 15) : 0u) |
-                                    ((b2 >> 4) == fsuit ? 1u << (b2 & 15) : 0u);
-                if (__popc(fm) >= 5) {  // flush: the five highest ranks of the suit; straight flush: its highest window
+    if (tid < kClassPad) {
+        int32_t s = 0x7fffffff;
+        const bool flush = tid >= kRankPairs;
+        const int t = flush ? tid - kRankPairs : tid;
+        if (t < kRankPairs) {
+            int hi = 0;
+            while ((hi + 1) * (hi + 2) / 2 <= t) ++hi;
+            const int lo = t - hi * (hi + 1) / 2;
+            if (!flush) {  // rank part (every occurrence of a rank counts, repeated card ids included)
+                RankChain ch = bchain;
+                ch.add(1u << lo);
+                ch.add(1u << hi);
+                s = score_rank_part(ch.classes(), ch.seen);
+            } else {  // ranks lo and hi of the suit (lo == hi: one card of it); 0 = no flush, below every rank part
+                const uint32_t fm = fboard | 1u << lo | 1u << hi;
+                s = 0;
+                if (fsuit >= 0 && __popc(fm) >= 5) {  // the five highest ranks of the suit; straight flush: its highest window
                     const uint32_t ef = lut->mask_entry[fm];
-                    s = max(s, (int32_t)((6u << 20) | (ef & 0xFFFFFu)));
+                    s = (int32_t)((6u << 20) | (ef & 0xFFFFFu));
                     const uint32_t sf = ef >> 28;
                     if (sf) s = max(s, (int32_t)((9u << 20) | ((sf - 1u) << 16)));
                 }
             }
-            if (scores) scores[b * P2B_NUM_HANDS + h] = s;
-            k = (uint32_t)s;
         }
-        key[h] = k;
-        val[h] = (uint16_t)h;
+        strength[tid] = s;
+    }
+    __syncthreads();
+    // A strength's class is the number of lower ones among the 182: equal strengths share it and the order stays.
+    const int words = fsuit >= 0 ? kClassPad / 4 : (kRankPairs + 3) / 4;
+    if (tid < 4 * words) {
+        const int32_t s = strength[tid];
+        int below = 0;
+        for (int i = 0; i < words; ++i) {
+            const int4 o = reinterpret_cast<const int4*>(strength)[i];
+            below += (o.x < s) + (o.y < s) + (o.z < s) + (o.w < s);
+        }
+        cls[tid] = (uint8_t)below;
+    }
+    __syncthreads();
+    const int fnone = fsuit >= 0 ? __ffs((int)fboard) - 1 : 0;  // a rank that adds nothing to the board's own cards of the suit
+    for (int h = tid; h < kSortN; h += kSetupThreads) {
+        uint32_t k = 255u;
+        if (h < P2B_NUM_HANDS) {
+            const int b1 = card_bit(combos->c1[h]), b2 = card_bit(combos->c2[h]);
+            const int r1 = b1 & 15, r2 = b2 & 15;
+            const int rp = rank_pair(r1, r2);
+            k = cls[rp];
+            int32_t s = scores ? strength[rp] : 0;
+            if (fsuit >= 0) {
+                const bool f1 = (b1 >> 4) == fsuit, f2 = (b2 >> 4) == fsuit;
+                const int fp = kRankPairs + rank_pair(f1 ? r1 : f2 ? r2 : fnone, f2 ? r2 : f1 ? r1 : fnone);
+                k = max(k, (uint32_t)cls[fp]);
+                if (scores) s = max(s, strength[fp]);
+            }
+            if (scores) scores[b * P2B_NUM_HANDS + h] = s;
+        }
+        item[h] = k << 16 | (uint32_t)h;
     }
     __syncthreads();
 
-    // ---- 2. stable radix sort; buffers alternate, the result ends in buffer 0 ----
-#pragma unroll 1
+    // ---- 2. stable radix sort by class; buffers alternate, the result ends in buffer 0 ----
+#pragma unroll
     for (int pass = 0; pass < kSortPasses; ++pass) {
-        const uint32_t* ksrc = key + (pass & 1) * kSortN;
-        const uint16_t* vsrc = val + (pass & 1) * kSortN;
-        uint32_t* kdst = key + ((pass & 1) ^ 1) * kSortN;
-        uint16_t* vdst = val + ((pass & 1) ^ 1) * kSortN;
-        const int shift = kDigitBits * pass;
+        const uint32_t* src = item + (pass & 1) * kSortN;
+        uint32_t* dst = item + ((pass & 1) ^ 1) * kSortN;
+        const int shift = 16 + kDigitBits * pass;
         uint32_t kk[kSortRounds];
-        uint16_t vv[kSortRounds];
         int slot[kSortRounds], rnk[kSortRounds];
 #pragma unroll
         for (int i = 0; i < kSortRounds; ++i) {
-            const int chunk = warp + kSetupWarps * i, p = 32 * chunk + lane;
-            kk[i] = ksrc[p];
-            vv[i] = vsrc[p];
-            const int d = (int)((kk[i] >> shift) & (kDigits - 1));
-            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const int chunk = warp + kSetupWarps * i;
+            kk[i] = src[32 * chunk + lane];
+            uint32_t peers = 0xffffffffu;  // lanes with this digit
+#pragma unroll
+            for (int bit = 0; bit < kDigitBits; ++bit) {
+                const bool on = (kk[i] >> (shift + bit)) & 1u;
+                const uint32_t vote = __ballot_sync(0xffffffffu, on);
+                peers &= on ? vote : ~vote;
+            }
             rnk[i] = __popc(peers & lt_mask);
-            slot[i] = d * kSortChunks + chunk;
+            slot[i] = (int)((kk[i] >> shift) & (kDigits - 1)) * kSortChunks + chunk;
             if (rnk[i] == 0) cnt8[slot[i]] = (unsigned char)__popc(peers);
         }
         __syncthreads();
-        scan_byte_counts<2>(cnt, kSortCntWords, off, warp_tot);
+        scan_byte_counts<1>(cnt, kSortCntWords, off, warp_tot);
 #pragma unroll
-        for (int i = 0; i < kSortRounds; ++i) {
-            const int dest = off[slot[i]] + rnk[i];
-            kdst[dest] = kk[i];
-            vdst[dest] = vv[i];
-        }
+        for (int i = 0; i < kSortRounds; ++i) dst[off[slot[i]] + rnk[i]] = kk[i];
         // the counters of the next pass, or (after the last one) the card masks that take their place
         for (int i = tid; i < (pass + 1 < kSortPasses ? kSortCntWords : kSuCntWords); i += kSetupThreads) cnt[i] = 0u;
         __syncthreads();
@@ -214,12 +251,12 @@ __global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const T* 
     // ---- 3. tie groups: lg[k] = first position of the run of equal strengths holding k ----
     {
         const int k0 = 4 * tid;
-        uint32_t kprev = k0 > 0 ? key[k0 - 1] : ~key[0];
+        uint32_t kprev = k0 > 0 ? item[k0 - 1] >> 16 : ~0u;
         int run[4];
         int best = 0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t kc = key[k0 + i];
+            const uint32_t kc = item[k0 + i] >> 16;
             if (kc != kprev) best = k0 + i;
             run[i] = best;
             kprev = kc;
@@ -255,7 +292,7 @@ __global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const T* 
 #pragma unroll
     for (int i = 0; i < kSortRounds; ++i) {
         const int k = tid + kSetupThreads * i;
-        hh[i] = k < P2B_NUM_HANDS ? val[k] : 0;
+        hh[i] = k < P2B_NUM_HANDS ? (int)(item[k] & 0xffffu) : 0;
         c1s[i] = combos->c1[hh[i]];
         c2s[i] = combos->c2[hh[i]];
         if (k < P2B_NUM_HANDS) {
@@ -265,7 +302,7 @@ __global__ void __launch_bounds__(kSetupThreads, 3) board_setup_kernel(const T* 
     }
     if (tid < (kTabCardListBytes - 51 * 52 * 2) / 2) cardlist_s[51 * 52 + tid] = 0;
     for (int k = tid; k < kTabSortedPad; k += kSetupThreads) {
-        const uint16_t h = k < P2B_NUM_HANDS ? val[k] : (uint16_t)0;
+        const uint16_t h = k < P2B_NUM_HANDS ? (uint16_t)item[k] : (uint16_t)0;
         sorted_s[k] = h;
         if (order && k < P2B_NUM_HANDS) order[b * P2B_NUM_HANDS + k] = h;
     }
