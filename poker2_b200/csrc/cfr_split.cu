@@ -93,6 +93,15 @@ SplitWork carve(float* scratch, int num_subgames, long long rows) {
     return w;
 }
 
+// Whether the solve has been refused or given up, the same answer for every thread of the block (all of them call it).  Other
+// blocks, and the kernel before this one where it still runs, may set the word meanwhile: if each thread went by what it read
+// itself, some would leave and the rest would wait for them at a barrier.  A kernel that reads the word too early works on
+// rows that no longer mean anything, but on lists that are whole: the record check has finished before any of these starts.
+__device__ __forceinline__ bool block_stops(const CfrParams& p) {
+    const int stop = threadIdx.x == 0 ? *reinterpret_cast<const volatile int32_t*>(p.work_counter + 1) : 0;
+    return __syncthreads_or(stop) != 0;
+}
+
 // ---- work lists -------------------------------------------------------------------------------
 // One block per subgame, one thread per node.  The items of a batch follow the queue order, those of a subgame the
 // node order, which is breadth-first.
@@ -101,8 +110,7 @@ __global__ void __launch_bounds__(kCfrMaxNodes) split_items_kernel(const CfrPara
     const int q = blockIdx.x, i = threadIdx.x;
     if (i == 0) s_before = s_bad = 0;
     if (i <= kSplitMaxDepth) s_depth[i] = 0;
-    __syncthreads();
-    if (p.work_counter[1] != 0) {  // the record check refused the batch
+    if (block_stops(p)) {  // the record check refused the batch
         if (q == 0 && i == 0) w.total[0] = 0;
         return;
     }
@@ -382,7 +390,7 @@ constexpr int kPrepWarps = 4;
 template <int MAXK, int MODE>
 __global__ void __launch_bounds__(32 * kPrepWarps) split_prep_kernel(const CfrParams p, const SplitWork w, int pass) {
     constexpr int kSlices = P2B_HPAD / 64;
-    if (p.work_counter[1] != 0) return;
+    if (block_stops(p)) return;
     const int q = blockIdx.x / kSlices, warp = threadIdx.x >> 5;
     const int h = (blockIdx.x - q * kSlices) * 64 + (threadIdx.x & 31) * 2;
     const int s = p.queue_order ? p.queue_order[q] : q;
@@ -718,7 +726,7 @@ __global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p,
     constexpr int kSlices = P2B_HPAD / kUpRow;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint64_t ready[kUpSlices][kSplitMaxDepth + 1];
-    if (p.work_counter[1] != 0) return;
+    if (block_stops(p)) return;
     const int per_subgame = kSlices / slices;
     const int q = blockIdx.x / per_subgame;
     const int s = p.queue_order ? p.queue_order[q] : q;
@@ -1091,7 +1099,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
     float* sums = reinterpret_cast<float*>(smem + L.sums);
     float* sums_avg = sums + 16;
     const SplitItem& it = *reinterpret_cast<const SplitItem*>(smem + L.item);
-    if (p.work_counter[1] != 0) return;
+    if (block_stops(p)) return;
 
     Hands hi;
 #pragma unroll
@@ -1353,7 +1361,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
 __global__ void __launch_bounds__(kRowThreads) split_values_kernel(const CfrParams p, const SplitWork w) {
     __shared__ __align__(16) float prod[2][P2B_HPAD];
     __shared__ float sums[2];
-    if (p.work_counter[1] != 0) return;
+    if (block_stops(p)) return;
     const int tid = threadIdx.x;
     for (int x = blockIdx.x; x < w.total[0]; x += gridDim.x) {
         const SplitItem& it = w.items[x];
@@ -1441,7 +1449,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_best_response_kernel(con
     float* rows = reinterpret_cast<float*>(smem);  // beliefs of the acting player, then a row a child
     double* cs = reinterpret_cast<double*>(smem + (1 + MAXK) * P2B_HPAD * 4);
     double* S = cs + (1 + MAXK) * 52;
-    if (p.work_counter[1] != 0) return;
+    if (block_stops(p)) return;
     const int tid = threadIdx.x;
     const int q = blockIdx.x / (2 * lanes), rest = blockIdx.x - q * 2 * lanes, deviator = rest / lanes;
     const SplitLevels* lv = w.levels + q;
@@ -1528,7 +1536,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_best_response_kernel(con
 __global__ void __launch_bounds__(kRowThreads) split_exploitability_kernel(const CfrParams p, const SplitWork w) {
     __shared__ __align__(16) float prod[4][P2B_HPAD];
     __shared__ float sums[4];
-    if (p.work_counter[1] != 0) return;
+    if (block_stops(p)) return;
     const int s = blockIdx.x, tid = threadIdx.x;
     const float* cr = p.carry_roots + (long long)s * 4 * P2B_HPAD;
     const float* root = w.rec + (long long)p.subgames[s].node_begin * kRec;

@@ -85,3 +85,23 @@ def test_network_per_leaf_in_place(cuda_device, L, W):
     ev.evaluate_into(beliefs, out)
     assert torch.equal(out[..., :1326], want) and torch.equal(ev(beliefs), want)
     assert (out[..., 1326:] == 7.0).all()
+
+
+@pytest.mark.parametrize("stepped", [False, True])
+def test_refused_batch_stops_every_kernel(cuda_device, stepped):
+    """Malformed records: the status word names the subgame and every split kernel leaves the outputs as they were."""
+    import bench
+    from poker2_b200 import solver, tree as ptree
+
+    boards, ranges, pot, stack = bench.make_inputs(9, 5)
+    trees = ptree.build_trees(ptree.root_states(pot.numpy(), stack.numpy()), [0.5, 1.0], 8, max_raises=2)
+    layout = solver.device_layout(trees, boards.numpy())
+    layout.nodes[int(layout.subgames[6]["node_begin"])]["n_children"] = 9
+    cls = solver.SteppedSolver if stepped else solver.SubgameSolver
+    sv = cls(layout, boards, cuda_device, exploitability=True)
+    outputs = (sv.root_values, sv.values_avg, sv.regrets, sv.policy_avg, sv.exploitability)
+    for x in outputs:
+        x.fill_(-7.0)
+    sv.solve(solver.pad_rows(ranges.to(cuda_device)).contiguous(), solver.iteration_scalars(4))
+    assert sv.status() == 7
+    assert all(bool((x == -7.0).all()) for x in outputs)
