@@ -180,9 +180,10 @@ int p2b_cfr_default_blocks(void);
  * previous setting; a negative argument only queries. */
 int p2b_cfr_path_policy(int32_t policy);
 /* Measurement aid (no counterpart in the upstream project): with timing enabled on the current
- * device, a p2b_cfr_solve of more subgames than SMs (eight times as many where some may exceed the lean
- * kernel's limit, or whenever the lean kernel runs) brackets its iteration passes with CUDA events on the caller's stream; p2b_cfr_iteration_ms waits for it and writes
- * its duration in milliseconds to the HOST float *ms. */
+ * device, a p2b_cfr_solve whose iteration passes run in the lean or in the split kernels brackets them with CUDA events on
+ * the caller's stream; p2b_cfr_iteration_ms waits for the last such solve and writes the duration of its passes in
+ * milliseconds to the HOST float *ms (an error if there has been none: in the general kernel the passes are part of one
+ * launch with the start and the final pass). */
 int p2b_cfr_iteration_timing(int32_t enable);
 int p2b_cfr_iteration_ms(float* ms);
 

@@ -1557,7 +1557,7 @@ int launch_cfr_warm_seed(const NodeRecPacked* nodes, long long rows, const float
     return check_cuda(cudaGetLastError(), "cfr_warm_seed_kernel");
 }
 
-// ---- optional timing of the iteration kernel of a split solve (for benchmarks) ----------------
+// ---- optional timing of the iteration passes of a one-call solve (for benchmarks) --------------
 namespace {
 struct IterTiming {
     bool enabled = false;
@@ -1601,7 +1601,7 @@ int cfr_iteration_timing(int enable) {
 
 int cfr_iteration_ms(float* ms) {
     IterTiming* t = iter_timing_of_current_device();
-    if (!t || !t->recorded) return set_error(P2B_ERR_STATE, "no timed iteration kernel has run on this device");
+    if (!t || !t->recorded) return set_error(P2B_ERR_STATE, "no timed iteration passes have run on this device");
     int rc = check_cuda(cudaEventSynchronize(t->stop), "cudaEventSynchronize");
     if (rc) return rc;
     return check_cuda(cudaEventElapsedTime(ms, t->start, t->stop), "cudaEventElapsedTime");
@@ -1703,7 +1703,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
                       lean_preferred(p.num_subgames, p.max_internal, max_children);
     if (!p.stepped && fast_scratch && !lean && split_applies(p, max_children, p.scratch_floats)) {
         IterTiming* timing = iter_timing_of_current_device();
-        const bool timed = timing && timing->enabled && p.num_subgames > (large ? 8 : 1) * sm_count();
+        const bool timed = timing && timing->enabled;
         CfrParams q = p;
         q.carry_roots = p.scratch + solve_work_floats(p.max_internal, max_children, num_blocks, p.num_subgames, p.rows);
         q.carry_sums = q.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;

@@ -28,7 +28,7 @@ def cuda_device():
     from poker2_b200 import build
 
     build.build()
-    # The fixtures are batches of a few subgames, which the default policy would hand to the general kernel;
+    # The fixtures are batches of a few subgames, which the default policy would hand to the split kernels;
     # the suite wants the lean iteration kernel on them too (tests/test_gpu_path_policy.py covers the default).
     from poker2_b200 import solver
 
