@@ -528,13 +528,13 @@ class SteppedSolver(SubgameSolver):
                 p(sample_pass),
                 p(self.policy_sample), p(self.beliefs_last), p(self.queue_order), p(self.start_policy_rows),
                 _lib.stream_ptr(self.device))
-        self.launches += 1
+        self.launches += 2 if phases == 16 else 1
 
     def solve(self, root_beliefs: torch.Tensor, scalars: np.ndarray, leaf_fn=None, *, cfr_plus: bool = False,
               enforce_zero_sum: bool = False, start_policy: torch.Tensor | None = None, warm_start_iterations: int = 0,
               warm_start_multiplier: float = 1.0, warm_start_scalars: np.ndarray | None = None,
               cfr_avg: bool = False, running_values: bool = False, warm_start_type: str = "model",
-              policy_delta=None, graph: bool = False, joint_sweeps: bool = False) -> SolveResult:
+              policy_delta=None, graph: bool = False, joint_sweeps: bool | None = None) -> SolveResult:
         """scalars: `iteration_scalars(T)` for all T iterations.  start_policy [M,1326] in the
         upstream node order (the policy head's softmax; None = uniform).  With
         warm_start_iterations = w > 0 (needs a start policy) the regrets are seeded from the start
@@ -559,10 +559,10 @@ class SteppedSolver(SubgameSolver):
         launching their kernels and the leaf model's one by one; same kernels, same results.  Ignored
         where the host works between the passes (cfr_avg, running_values, policy_delta).  The leaf model must
         be capturable: device work only, the same shapes every pass, no host synchronisation.
-        joint_sweeps: count the bottom-up sweep of a pass and the top-down sweep of the next one as one in
-        `launches`.  With model leaves the two go into one call (`phases` 16 of `p2b_cfr_step`) in any case, wherever
-        the host has nothing to do between them: that saves deriving the current policy anew (0.09 of 1.4 ms a pass on
-        192 flop subgames of 77 nodes); same results."""
+        joint_sweeps: with model leaves, the bottom-up sweep of a pass and the top-down sweep of the next one go
+        into one call (`phases` 16 of `p2b_cfr_step`) wherever the host has nothing to do between them; False keeps
+        every sweep a call of its own.  Same results; the joint form saves deriving the current policy anew (0.09 of
+        1.4 ms a pass on 192 flop subgames of 77 nodes).  `launches` counts sweeps either way."""
         assert root_beliefs.shape == (self.B, 2, HPAD) and root_beliefs.dtype == torch.float32
         assert root_beliefs.is_contiguous() and root_beliefs.device == self.device
         ws = int(warm_start_iterations)
@@ -614,7 +614,8 @@ class SteppedSolver(SubgameSolver):
             for t, q in pstats.delta_checkpoints(ws, all_scalars.shape[0]).items():
                 delta_at[t - ws + (0 if ws > 0 else -1)] = q
         # the bottom-up sweep of a pass waits for the top-down sweep of the next one where they can share a launch
-        fuse = n_leaves > 0 and graphed is None and not (cfr_avg or running_values or policy_delta is not None)
+        fuse = (joint_sweeps is not False and n_leaves > 0 and graphed is None
+                and not (cfr_avg or running_values or policy_delta is not None))
         pending_up = None
         for pas in range(-1, iterations + 1):
             if pas == 0 and warm_br:
@@ -655,8 +656,6 @@ class SteppedSolver(SubgameSolver):
             if pending_up is not None:
                 self._step(root_beliefs, sc, iterations, flags_pass, pending_up, pas, 16)
                 pending_up = None
-                if not joint_sweeps:
-                    self.launches += 1  # two sweeps
             else:
                 self._step(root_beliefs, sc, iterations, flags_pass, pas, pas, 1)
             if cfr_avg:

@@ -191,8 +191,8 @@ def test_default_bet_sizes_at_depth_three_with_model_leaves(cuda_device):
 
 @pytest.mark.parametrize("warm", [False, True])
 def test_joint_sweeps_equal_separate_launches(cuda_device, warm):
-    """A pass as one launch (bottom-up sweep of the pass before it + its own top-down sweep, `phases` 16) against
-    the two launches per pass: same bits, on trees of 52 ... 282 nodes with model leaves, with and without a
+    """A pass as one call (bottom-up sweep of the pass before it + its own top-down sweep, `phases` 16), which is the default,
+    against the two calls per pass: same bits, on trees of 52 ... 282 nodes with model leaves, with and without a
     warm start (whose seeding keeps the first two sweeps apart)."""
     from oracle import cards
     from poker2_b200 import solver, tree as ptree
@@ -214,18 +214,21 @@ def test_joint_sweeps_equal_separate_launches(cuda_device, warm):
         cc = torch.from_numpy(trees.child_count[trees.parent_index.clip(min=0)]).clamp(min=1)
         kw = dict(start_policy=(1.0 / cc.float())[:, None].expand(-1, 1326).contiguous(), warm_start_iterations=2,
                   warm_start_multiplier=3.0)
-    out, launches = [], []
-    for joint in (False, True):
+    out, calls = [], []
+    for joint in (False, True, None):
         sv = solver.SteppedSolver(layout, torch.from_numpy(boards), cuda_device, exploitability=True, sampling=True)
+        step, made = sv._step, []
+        sv._step = lambda *a, **k: (made.append(a[6]), step(*a, **k))  # the phases of every call
         sv.set_sampling_schedule(torch.tensor([2, 3, 5, 4]), warm_start_iterations=2 if warm else 0)
         res = sv.solve(rb, scal, fn, joint_sweeps=joint, **kw)
         assert sv.status() == 0
-        launches.append(sv.launches)
+        calls.append(made)
         out.append([x.clone() for x in (res.policy_avg, res.regrets, res.weight_sums, res.root_values, res.exploitability,
                                         res.policy_sample, res.beliefs_last)])
-    assert launches[1] < launches[0]
-    for a, b in zip(*out):
-        assert torch.equal(a, b)
+    assert set(calls[0]) == {1, 2} and len(calls[0]) == 2 * (len(scal) - (1 if warm else 0) + 2)
+    assert calls[1].count(16) == len(scal) - (1 if warm else -1) and calls[1] == calls[2]
+    for a, b, c in zip(*out):
+        assert torch.equal(a, b) and torch.equal(a, c)
 
 
 def test_production_tree_shape_against_the_upstream_run(cuda_device, golden_dir):
