@@ -61,19 +61,32 @@ class ValueMLP(torch.nn.Module):
         y = self.net(x)[:, : 2 * NUM_HANDS]
         return y.to(torch.float32).view(S, 2, NUM_HANDS)
 
-
     @torch.no_grad()
     def layers(self, x: torch.Tensor) -> torch.Tensor:
-        """`self.net` on input rows x, activations in place (half the memory traffic and footprint of a GELU, same bits).  A
-        linear layer without hooks is called directly: a pass over few leaves lasts as long as the host takes to launch it."""
+        """`self.net` on input rows x, activations in place (half the memory traffic and footprint of a GELU, same bits) and
+        linear layers without the module's wrapper: a pass over few leaves lasts as long as the host takes to launch it.
+        A network that someone listens to (hooks) or has changed goes through its modules instead."""
+        if type(self.net) is not torch.nn.Sequential or not (_bare(self.net) and all(map(_bare, self.net))):
+            return self.net(x)
         for layer in self.net:
             if type(layer) is torch.nn.GELU and layer.approximate == "none":
                 x = torch.ops.aten.gelu_(x)
-            elif type(layer) is torch.nn.Linear and not (layer._forward_hooks or layer._forward_pre_hooks):
+            elif type(layer) is torch.nn.Linear:
                 x = torch.nn.functional.linear(x, layer.weight, layer.bias)
             else:
                 x = layer(x)
         return x
+
+
+_module_hooks = torch.nn.modules.module
+
+
+def _bare(module: torch.nn.Module) -> bool:
+    """Nothing but the module's own `forward` would run if it were called: no forward hooks, on it or on all modules, no
+    `forward` put in place of the class's, not compiled."""
+    return not (module._forward_hooks or module._forward_pre_hooks or "forward" in module.__dict__
+                or module._compiled_call_impl is not None
+                or _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks)
 
 
 def leaf_context(trees, node_index) -> torch.Tensor:
@@ -161,7 +174,7 @@ class DirectLeafEvaluator:
 
     def evaluate_into(self, leaf_beliefs: torch.Tensor, out: torch.Tensor) -> None:
         """Values of all leaves into out[..., :1326] (fp32 [L,2,W])."""
-        if self._rows is None or not _paired_rows(leaf_beliefs) or not _paired_rows(out):
+        if not (self._direct() and _paired_rows(leaf_beliefs) and _paired_rows(out)):
             out[..., :NUM_HANDS].copy_(self.model(leaf_beliefs[..., :NUM_HANDS].contiguous(), self.boards, self.context))
             return
         p, L = _lib.ptr, leaf_beliefs.shape[0]
@@ -172,8 +185,12 @@ class DirectLeafEvaluator:
             y = self.model.layers(self._rows)
             _lib.call("p2b_leaf_values_bf16", p(y), y.stride(0), L, p(out), out.stride(1), stream)
 
+    def _direct(self) -> bool:
+        """The model's layers may be called on rows kept here instead of the model itself."""
+        return self._rows is not None and type(self.model) is ValueMLP and _bare(self.model)
+
     def __call__(self, leaf_beliefs: torch.Tensor) -> torch.Tensor:
-        if self._rows is None:
+        if not self._direct():
             return self.model(leaf_beliefs[..., :NUM_HANDS].contiguous(), self.boards, self.context)
         out = torch.empty(leaf_beliefs.shape[0], 2, NUM_HANDS, device=leaf_beliefs.device, dtype=torch.float32)
         self.evaluate_into(leaf_beliefs, out)

@@ -1,0 +1,82 @@
+"""Hooks on the leaf network and on its layers fire although its layers are normally called without their modules, and a layer
+whose output a hook has kept is not overwritten by the activation behind it."""
+import pytest
+import torch
+
+from poker2_b200 import leaf_eval
+
+
+def _model():
+    return leaf_eval.ValueMLP(16, 2, dtype=torch.bfloat16, seed=1)
+
+
+def _rows(n=3):
+    return torch.rand(n, leaf_eval.ValueMLP.IN_PADDED, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16)
+
+
+def test_without_hooks_the_layers_give_the_network():
+    model = _model()
+    with torch.no_grad():
+        assert torch.equal(model.layers(_rows()), model.net(_rows()))
+
+
+@pytest.mark.parametrize("where", ["net", "linear", "gelu", "global"])
+@pytest.mark.parametrize("pre", [False, True])
+def test_hooks_on_the_network_fire(where, pre):
+    model, seen = _model(), []
+    target = {"net": model.net, "linear": model.net[0], "gelu": model.net[1]}.get(where)
+    hook = (lambda m, args: seen.append(args[0])) if pre else (lambda m, args, out: seen.append(out))
+    if where == "global":
+        register = (torch.nn.modules.module.register_module_forward_pre_hook if pre
+                    else torch.nn.modules.module.register_module_forward_hook)
+        handle = register(hook)
+    else:
+        handle = (target.register_forward_pre_hook if pre else target.register_forward_hook)(hook)
+    try:
+        got = model.layers(_rows())
+    finally:
+        handle.remove()
+    assert seen
+    with torch.no_grad():
+        assert torch.equal(got, model.net(_rows()))
+        if where == "linear" and not pre:  # what the hook kept is the layer's output, not the activation's
+            assert torch.equal(seen[0], model.net[0](_rows()))
+
+
+@pytest.mark.parametrize("what", ["layer", "net"])
+def test_a_replaced_forward_is_called(what):
+    class Doubled(torch.nn.Module):
+        def __init__(self, net):
+            super().__init__()
+            self.inner = net
+
+        def forward(self, x):
+            return self.inner(x) * 2.0
+
+    model = _model()
+    if what == "layer":
+        model.net[1].forward = lambda x: torch.zeros_like(x)
+    else:
+        model.net = Doubled(model.net)
+    with torch.no_grad():
+        assert torch.equal(model.layers(_rows()), model.net(_rows()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("evaluate", ["call", "into"])
+def test_hooks_on_the_model_of_a_leaf_evaluator_fire(cuda_device, evaluate):
+    model, L, seen = _model().to(cuda_device), 5, []
+    g = torch.Generator(device=cuda_device).manual_seed(3)
+    beliefs = torch.rand(L, 2, 1344, device=cuda_device, generator=g)
+    boards = torch.tensor([[0, 1, 2, -1, -1]], device=cuda_device).expand(L, 5)
+    ev = leaf_eval.DirectLeafEvaluator(model, boards, torch.rand(L, 3, device=cuda_device, generator=g), cuda_device)
+    want = ev(beliefs).clone()
+    handle = model.register_forward_hook(lambda m, args, out: (seen.append(out), out * 2.0)[1])
+    if evaluate == "call":
+        got = ev(beliefs)
+    else:
+        got = torch.zeros(L, 2, 1344, device=cuda_device)
+        ev.evaluate_into(beliefs, got)
+    handle.remove()
+    assert len(seen) == 1 and torch.equal(got[..., :1326], want * 2.0)
+    assert torch.equal(ev(beliefs), want)
