@@ -835,6 +835,18 @@ using namespace p2b;
 #define GRID_ELEMS(n) blocks_for((n), sm_count() * 16)
 #define GRID_ROWS(r) ((int)((r) < (long long)sm_count() * 8 ? ((r) > 0 ? (r) : 1) : (long long)sm_count() * 8))
 
+// The arrays of a whole-step kernel, before anything reaches the device: null or misaligned pointers, sizes that no grid has.
+// (What the index arrays hold is the caller's to keep inside the tree.)
+#define STEPS_REQUIRE(cond, msg) \
+    do {                         \
+        if (!(cond)) return set_error(P2B_ERR_ARG, "%s: %s", __func__, msg); \
+    } while (0)
+template <typename... T>
+static bool arrays_ok(const T*... p) {  // given, and aligned to their elements
+    return ((p != nullptr && reinterpret_cast<uintptr_t>(p) % sizeof(T) == 0) && ...);
+}
+static const char kArrays[] = "null or misaligned array";
+
 extern "C" {
 
 int p2b_step_dcfr_update(const float* regrets, float* cumulative, float* weight_sums, float* positive_out,
@@ -1002,7 +1014,10 @@ int p2b_steps_regrets(const float* values, const float* beliefs, const int64_t* 
                       const int64_t* child_count, const float* uniform, const float* scalars4, float* cumulative,
                       float* weight_sums, float* policy, int64_t num_roots, int64_t num_parents, int apply_dcfr, int cfr_plus,
                       void* stream) {
-    if (num_parents <= 0) return P2B_OK;
+    STEPS_REQUIRE(num_roots >= 0 && num_parents >= 0 && num_parents <= INT32_MAX, "bad count");
+    STEPS_REQUIRE(num_roots <= num_parents, "the roots are among the parents");
+    if (num_parents == 0) return P2B_OK;
+    STEPS_REQUIRE(arrays_ok(values, beliefs, to_act, child_offsets, child_count, uniform, scalars4, cumulative, weight_sums, policy), kArrays);
     const int rc = ensure_tables();
     if (rc) return rc;
     step_regrets_kernel<<<(unsigned)num_parents, kRowThreads, 0, (cudaStream_t)stream>>>(
@@ -1013,7 +1028,14 @@ int p2b_steps_regrets(const float* values, const float* beliefs, const int64_t* 
 
 int p2b_steps_reach(const float* policy, const uint8_t* allowed, const float* allowed_prob, const int32_t* path, int32_t depth,
                     const int64_t* root_index, const float* prior, float* reach, float* beliefs, int64_t nodes, void* stream) {
-    if (nodes <= 0) return P2B_OK;
+    STEPS_REQUIRE(nodes >= 0 && nodes <= INT32_MAX && depth >= 0, "bad count");
+    if (nodes == 0) return P2B_OK;
+    STEPS_REQUIRE(arrays_ok(policy, allowed, reach) && (depth == 0 || arrays_ok(path)), kArrays);
+    if (beliefs) {
+        STEPS_REQUIRE(arrays_ok(beliefs, prior, root_index, allowed_prob), kArrays);
+        // rows of the prior that another block reads must not be the ones that a block writes (a root at least is read)
+        STEPS_REQUIRE(prior + 2 * P2B_NUM_HANDS <= beliefs || beliefs + nodes * 2 * P2B_NUM_HANDS <= prior, "prior and beliefs overlap");
+    }
     step_reach_kernel<<<(unsigned)nodes, kRowThreads, 0, (cudaStream_t)stream>>>(
         policy, allowed, allowed_prob, path, depth, (const long long*)root_index, prior, reach, beliefs);
     STEP_CHECK("step_reach_kernel");
@@ -1022,7 +1044,9 @@ int p2b_steps_reach(const float* policy, const uint8_t* allowed, const float* al
 int p2b_steps_average(const float* reach, const float* reach_avg, const float* policy, const int64_t* to_act,
                       const int64_t* child_offsets, const int64_t* child_count, const float* old_w, const float* new_w,
                       const float* total_w, float* policy_avg, int64_t num_parents, void* stream) {
-    if (num_parents <= 0) return P2B_OK;
+    STEPS_REQUIRE(num_parents >= 0 && num_parents <= INT32_MAX, "bad count");
+    if (num_parents == 0) return P2B_OK;
+    STEPS_REQUIRE(arrays_ok(reach, reach_avg, policy, to_act, child_offsets, child_count, old_w, new_w, total_w, policy_avg), kArrays);
     step_average_kernel<<<(unsigned)num_parents, kRowThreads, 0, (cudaStream_t)stream>>>(
         reach, reach_avg, policy, (const long long*)to_act, (const long long*)child_offsets, (const long long*)child_count,
         old_w, new_w, total_w, policy_avg);
@@ -1031,7 +1055,9 @@ int p2b_steps_average(const float* reach, const float* reach_avg, const float* p
 
 int p2b_steps_seen(const float* beliefs, const float* policy, const int64_t* to_act, const int64_t* child_offsets,
                    const int64_t* child_count, float* seen, int64_t num_parents, void* stream) {
-    if (num_parents <= 0) return P2B_OK;
+    STEPS_REQUIRE(num_parents >= 0 && num_parents <= INT32_MAX, "bad count");
+    if (num_parents == 0) return P2B_OK;
+    STEPS_REQUIRE(arrays_ok(beliefs, policy, to_act, child_offsets, child_count, seen), kArrays);
     int rc = ensure_tables();
     if (rc) return rc;
     constexpr int kBytes = (1 + kSeenRows) * (P2B_HPAD * 4 + 53 * 8);

@@ -51,3 +51,39 @@ def test_tree_builder_rejects_bad_arguments_without_a_gpu():
     assert handle.p2b_tree_count(None, 1, bins, 2, 4, -1, p, p, None) == -1  # null roots
     assert handle.p2b_tree_records(p, None, 5, 1, bins, 2, 4, -1, p, p, p, p, p, p, None, None, None) == -1
     assert handle.p2b_tree_count(p, 0, bins, 2, 4, -1, p, p, None) == 0  # empty batch: nothing to do
+
+
+def test_whole_step_entry_points_reject_bad_arguments_without_a_gpu():
+    """`p2b_steps_*`: null and misaligned arrays, negative sizes and a prior inside the beliefs are refused before any launch."""
+    from poker2_b200 import _lib, build
+
+    build.build()
+    handle = _lib.lib()
+    array = (ctypes.c_int64 * 64)()
+    p = ctypes.addressof(array)
+    good = {
+        "p2b_steps_regrets": [p] * 10 + [1, 1, 1, 0, None],
+        "p2b_steps_reach": [p, p, p, p, 1, p, p, p, p + 2 * 1326 * 4, 1, None],
+        "p2b_steps_average": [p] * 10 + [1, None],
+        "p2b_steps_seen": [p] * 6 + [1, None],
+    }
+    sizes = {"p2b_steps_regrets": (10, 11), "p2b_steps_reach": (4, 9), "p2b_steps_average": (10,), "p2b_steps_seen": (6,)}
+    arrays = {"p2b_steps_regrets": range(10), "p2b_steps_reach": (0, 1, 2, 3, 5, 6, 7), "p2b_steps_average": range(10),
+              "p2b_steps_seen": range(6)}
+
+    def refused(name, args):
+        rc = getattr(handle, name)(*args)
+        return rc == -1 and name.encode() in handle.p2b_last_error()
+
+    for name, args in good.items():
+        for i in arrays[name]:
+            assert refused(name, args[:i] + [None] + args[i + 1:]), (name, i, "null")
+            if (name, i) != ("p2b_steps_reach", 1):  # one byte a hand: any address is aligned
+                assert refused(name, args[:i] + [args[i] + 1] + args[i + 1:]), (name, i, "misaligned")
+        for i in sizes[name]:
+            assert refused(name, args[:i] + [-1] + args[i + 1:]), (name, i, "negative")
+        nothing = [0 if i in sizes[name] else None if i in arrays[name] else a for i, a in enumerate(args)]
+        assert getattr(handle, name)(*nothing) == 0, name  # an empty call: nothing to do
+    reach = good["p2b_steps_reach"]
+    for beliefs in (p, p + 4, p - 4):
+        assert refused("p2b_steps_reach", reach[:8] + [beliefs] + reach[9:]), "overlap"
