@@ -378,6 +378,10 @@ int p2b_step_deep_beliefs(float* out, const float* root_beliefs, const float* re
                           const int64_t* root_index, int64_t num_roots, int64_t total, int32_t H, float eps,
                           void* stream);
 
+/* TScalars.update (:2100): out[0..n) = the n <= 16 floats of the HOST array values, *t_out = t (t_out may be NULL).  The
+ * values travel with the launch: the host waits for nothing, and a captured call replays them */
+int p2b_step_fill_scalars(float* out, const float* values, int32_t n, int64_t* t_out, int64_t t, void* stream);
+
 /* ---- whole steps of one iteration (step_evaluator.StepCFREvaluator) -------------------------
  * Arrays in the upstream layout with rows of 1326: [M,H] or [M,2,H] fp32, level-major topology (children of a node
  * consecutive; child_offsets / child_count / to_act of the first num_parents nodes), index arrays int64.

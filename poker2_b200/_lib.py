@@ -62,6 +62,7 @@ _SIGNATURES = {
     "p2b_step_weighted_parent_sum": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _vp],
     "p2b_step_reach_weights": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _vp],
     "p2b_step_deep_beliefs": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _f32, _vp],
+    "p2b_step_fill_scalars": [_vp, _vp, _i32, _vp, _i64, _vp],
     "p2b_steps_regrets": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i32, _vp],
     "p2b_steps_reach": [_vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _vp, _i64, _vp],
     "p2b_steps_average": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp],

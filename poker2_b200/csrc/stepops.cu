@@ -823,6 +823,19 @@ __global__ void __launch_bounds__(kRowThreads) weighted_parent_rows_kernel(
     for (int p = 0; p < 2; ++p) st_row(values + (par * 2 + p) * H, acc[p]);
 }
 
+// Scalars of an iteration by value: they reach the device with the launch, without a copy that the host would wait for.
+constexpr int kMostScalars = 16;
+struct Scalars {
+    float v[kMostScalars];
+};
+__global__ void fill_scalars_kernel(float* __restrict__ out, const Scalars s, int n, long long* __restrict__ t_out, long long t) {
+    const int i = threadIdx.x;
+#pragma unroll
+    for (int e = 0; e < kMostScalars; ++e)
+        if (i == e && e < n) out[e] = s.v[e];
+    if (i == kMostScalars && t_out) *t_out = t;
+}
+
 }  // namespace
 
 int sm_count();
@@ -1008,6 +1021,16 @@ int p2b_step_deep_beliefs(float* out, const float* root_beliefs, const float* re
     deep_beliefs_kernel<<<GRID_ROWS((total - num_roots) * 2), kThreads, 0, (cudaStream_t)stream>>>(
         out, root_beliefs, reach, allowed_prob, (const long long*)root_index, num_roots, total, H, eps);
     STEP_CHECK("deep_beliefs_kernel");
+}
+
+int p2b_step_fill_scalars(float* out, const float* values, int32_t n, int64_t* t_out, int64_t t, void* stream) {
+    STEPS_REQUIRE(n >= 0 && n <= kMostScalars, "0 to 16 scalars");
+    STEPS_REQUIRE(n == 0 || (arrays_ok(out, values)), kArrays);
+    STEPS_REQUIRE(!t_out || arrays_ok(t_out), kArrays);
+    Scalars s{};
+    for (int i = 0; i < n; ++i) s.v[i] = values[i];
+    fill_scalars_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(out, s, n, reinterpret_cast<long long*>(t_out), t);
+    STEP_CHECK("fill_scalars_kernel");
 }
 
 int p2b_steps_regrets(const float* values, const float* beliefs, const int64_t* to_act, const int64_t* child_offsets,

@@ -8,6 +8,8 @@ index tensors are int64.  The whole-subgame kernel (`poker2_b200.solver`) is the
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -371,7 +373,7 @@ class TScalars:
 
     def __init__(self, device: torch.device, dtype: torch.dtype = torch.float32) -> None:
         self.device, self.dtype = device, dtype
-        # one array, so that an iteration's scalars arrive in one copy
+        # one array, so that an iteration's scalars arrive in one launch
         self._all = torch.zeros(10, dtype=dtype, device=device)
         (self.t_alpha_num, self.t_beta_num, self.t_alpha_den, self.t_beta_den, self.mix_old, self.mix_new, self.mix_total,
          self.mix_inv_total, self.mix_onon, self.mix_oon) = self._all.unbind()
@@ -384,7 +386,12 @@ class TScalars:
         values = [an, bn, an + 1.0, bn + 1.0, old, new, total, 1.0 / total if total != 0.0 else 1.0]
         if new != 0.0:
             values += [total / new, old / new]
-        self._all[: len(values)].copy_(torch.tensor(values, dtype=self.dtype))
+        if self._all.is_cuda and self.dtype == torch.float32:  # by value: the host does not wait for the stream
+            _call("p2b_step_fill_scalars", self._all.device, _p(self._all), (ctypes.c_float * len(values))(*values), len(values),
+                  _p(self.t_tensor), int(t))
+            return
+        for x, v in zip(self._all, values):
+            x.fill_(v)
         self.t_tensor.fill_(int(t))
 
 
