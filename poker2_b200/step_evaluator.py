@@ -113,9 +113,18 @@ class StepCFREvaluator:
         with _lib.on(self.device):
             _lib.call(name, *[a.data_ptr() if torch.is_tensor(a) else a for a in args], _lib.stream_ptr(self.device))
 
+    def _of_nodes(self, *arrays: torch.Tensor, players: bool = True) -> None:
+        """State arrays as the kernels read them, whoever made them: [M,2,1326] or [M,1326] fp32, contiguous, on this device."""
+        shape = (self.total_nodes, 2, NUM_HANDS) if players else (self.total_nodes, NUM_HANDS)
+        for a in arrays:
+            assert a.shape == shape and a.dtype == torch.float32, f"expected fp32 {shape}, got {a.dtype} {tuple(a.shape)}"
+            assert a.is_contiguous() and a.device == self._path.device
+
     def _calculate_reach_weights(self, target: torch.Tensor, policy: torch.Tensor, beliefs: torch.Tensor | None = None) -> None:
         """Reach under `policy`; with `beliefs` also those: every row = its root's row x reach, blocked and normalised (the
         root rows themselves are normalised once more per call, like every other row upstream)."""
+        self._of_nodes(target, *(() if beliefs is None else (beliefs,)))
+        self._of_nodes(policy, players=False)
         prior = None if beliefs is None else beliefs[: self.root_nodes].clone()
         self._call("p2b_steps_reach", policy, self._allowed_bytes, self.allowed_hands_prob, self._path, self._path.shape[1],
                    self.root_of, prior, target, beliefs, self.total_nodes)
@@ -146,6 +155,7 @@ class StepCFREvaluator:
             vals = self.leaf_fn(beliefs[self.model_indices], self.model_indices)
             self.latest_values[self.model_indices] = vals[..., :NUM_HANDS].to(torch.float32)
         if self.showdown_indices.numel():
+            self._of_nodes(beliefs, self.latest_values)
             stride = 2 * NUM_HANDS
             self._call("p2b_showdown_values_at", self._tables.blob, self._sd_table, self.showdown_indices, beliefs, stride,
                        self._sd_potential, self._sd_scale, self.latest_values, stride, self.showdown_indices.numel())
@@ -155,6 +165,8 @@ class StepCFREvaluator:
         beliefs = self.beliefs if beliefs is None else beliefs.contiguous()
         leaf_values = self.latest_values if leaf_values is None else leaf_values
         values = leaf_values if values is None else values
+        self._of_nodes(beliefs, values)
+        self._of_nodes(policy, players=False)
         if leaf_values is not values:  # (in place, the inner rows are overwritten below)
             torch.where(self.leaf_mask[:, None, None], leaf_values, torch.zeros((), device=self.device), out=values)
         self._call("p2b_steps_seen", beliefs, policy, self.to_act, self.child_offsets, self.child_count, self._seen, self.top)
@@ -185,6 +197,8 @@ class StepCFREvaluator:
         if (self.cfr_type in ("discounted", "discounted_plus") and t <= self.dcfr_delay) or t == 0:
             self.policy_probs_avg.copy_(self.policy_probs)
             return
+        self._of_nodes(self.self_reach, self.self_reach_avg)
+        self._of_nodes(self.policy_probs, self.policy_probs_avg, players=False)
         ts = self._t_scalars
         self._call("p2b_steps_average", self.self_reach, self.self_reach_avg, self.policy_probs, self.to_act, self.child_offsets,
                    self.child_count, ts.mix_old, ts.mix_new, ts.mix_total, self.policy_probs_avg, self.top)
@@ -216,6 +230,8 @@ class StepCFREvaluator:
     def cfr_iteration(self, t: int) -> None:
         if not self._skip_t_scalars_update:
             self.prepare_replay(t)
+        self._of_nodes(self.latest_values, self.beliefs)
+        self._of_nodes(self.uniform_policy, self.cumulative_regrets, self.regret_weight_sums, self.policy_probs, players=False)
         # `compute_instantaneous_regrets`, the discounted update and the regret matching of `update_policy` in one kernel
         self._call("p2b_steps_regrets", self.latest_values, self.beliefs, self.to_act, self.child_offsets, self.child_count,
                    self.uniform_policy, self._t_scalars.t_alpha_num, self.cumulative_regrets, self.regret_weight_sums,

@@ -83,3 +83,46 @@ def test_scalars_of_an_iteration(cuda_device, dtype, where, old, new):
     for name, value in want.items():
         assert torch.equal(getattr(s, name).cpu(), torch.tensor(value, dtype=dtype)), name
     assert s.t_tensor.item() == 7
+
+
+@pytest.mark.parametrize("spoil", ["rows", "type", "strides"])
+def test_state_arrays_of_another_form_are_refused(cuda_device, spoil):
+    """Arrays that a caller hands to a step, or puts in place of the evaluator's own, reach the kernels as bare pointers: too few
+    rows, another type or other strides are refused; what can be copied into place (a policy's or beliefs' strides) is."""
+    from poker2_b200 import step_evaluator, tree as ptree
+
+    trees = ptree.build_trees(ptree.root_states(torch.tensor([100]).numpy(), torch.tensor([400]).numpy()), [0.5, 1.0], 8, max_raises=2)
+    ranges = torch.rand(1, 2, 1326, generator=torch.Generator().manual_seed(1))
+    ev = step_evaluator.StepCFREvaluator(trees, torch.tensor([[0, 5, 17, 30, 51]]).numpy(), ranges, cuda_device, iterations=4)
+    ev.evaluate_cfr()
+
+    def spoilt(x):
+        if spoil == "rows":
+            return x[:-1].clone()
+        if spoil == "type":
+            return x.double()
+        wide = torch.zeros(*x.shape[:-1], x.shape[-1] + 2, device=x.device)
+        wide[..., :-2] = x
+        return wide[..., :-2]
+
+    if spoil == "strides":
+        ev.compute_expected_values()
+        want = ev.latest_values.clone()
+        ev.compute_expected_values(policy=spoilt(ev.policy_probs), beliefs=spoilt(ev.beliefs))
+        assert torch.equal(ev.latest_values, want)
+    else:
+        for kw in ({"policy": spoilt(ev.policy_probs)}, {"beliefs": spoilt(ev.beliefs)}):
+            with pytest.raises(AssertionError):
+                ev.compute_expected_values(**kw)
+        with pytest.raises(AssertionError):
+            ev.set_leaf_values(0, beliefs=spoilt(ev.beliefs))
+    with pytest.raises((AssertionError, RuntimeError)):
+        ev.compute_expected_values(values=spoilt(ev.latest_values))
+    for name in ("latest_values", "beliefs", "self_reach", "self_reach_avg", "beliefs_avg", "policy_probs", "policy_probs_avg",
+                 "cumulative_regrets", "regret_weight_sums", "uniform_policy"):
+        own = getattr(ev, name)
+        setattr(ev, name, spoilt(own))
+        with pytest.raises((AssertionError, RuntimeError)):
+            ev.cfr_iteration(3)
+        setattr(ev, name, own)
+    ev.cfr_iteration(3)
