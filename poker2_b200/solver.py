@@ -443,6 +443,16 @@ class SubgameSolver:
             raise RuntimeError(f"subgame {st - 1}: tree records exceed the solver's limits; nothing was solved")
 
 
+def _writes_in_place(leaf_fn) -> bool:
+    """The evaluator has an `evaluate_into`, and no class derived from it has put a `__call__` of its own before that."""
+    for cls in type(leaf_fn).__mro__:
+        if "evaluate_into" in cls.__dict__:
+            return True
+        if "__call__" in cls.__dict__:
+            return False
+    return False
+
+
 class SteppedSolver(SubgameSolver):
     """Solves subgames whose non-terminal leaves are valued by a caller-side model
     (`set_leaf_values`, p2/search/cfr_evaluator.py:1025-1047): every pass is two launches
@@ -502,9 +512,8 @@ class SteppedSolver(SubgameSolver):
         """The caller's values of the first n leaf slots into `out` (default: the rows the bottom-up sweep reads); an
         evaluator that can write in place does."""
         out = self.leaf_values if out is None else out
-        into = getattr(leaf_fn, "evaluate_into", None)
-        if into is not None:
-            into(self.leaf_beliefs[:n], out[:n])
+        if _writes_in_place(leaf_fn):
+            leaf_fn.evaluate_into(self.leaf_beliefs[:n], out[:n])
             return
         vals = leaf_fn(self.leaf_beliefs[:n])
         if vals.shape[-1] == NUM_HANDS:

@@ -62,6 +62,34 @@ def test_a_replaced_forward_is_called(what):
         assert torch.equal(model.layers(_rows()), model.net(_rows()))
 
 
+class _Halved(leaf_eval.DirectLeafEvaluator):
+    def __call__(self, leaf_beliefs):
+        return super().__call__(leaf_beliefs) * 0.5
+
+
+class _HalvedInPlace(leaf_eval.DirectLeafEvaluator):
+    def evaluate_into(self, leaf_beliefs, out):
+        super().evaluate_into(leaf_beliefs, out)
+        out.mul_(0.5)
+
+
+def test_a_subclass_with_a_call_of_its_own_is_called():
+    """The solver writes values in place only where `evaluate_into` is not behind another `__call__`."""
+    from types import SimpleNamespace
+
+    from poker2_b200 import solver
+
+    L = 3
+    beliefs = torch.rand(L, 2, 1344, generator=torch.Generator().manual_seed(5))
+    boards, ctx = torch.tensor([[0, 1, 2, -1, -1]]).expand(L, 5), torch.rand(L, 3)
+    plain, half, in_place = (c(_model(), boards, ctx, torch.device("cpu")) for c in (leaf_eval.DirectLeafEvaluator, _Halved, _HalvedInPlace))
+    want = plain(beliefs)
+    for fn, factor in ((plain, 1.0), (half, 0.5), (in_place, 0.5), (lambda b: plain(b) * 0.25, 0.25)):
+        state = SimpleNamespace(leaf_beliefs=beliefs, leaf_values=torch.zeros(L, 2, 1344))
+        solver.SteppedSolver._value_leaves(state, fn, L)
+        assert torch.equal(state.leaf_values[..., :1326], want * factor)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("evaluate", ["call", "into"])
 def test_hooks_on_the_model_of_a_leaf_evaluator_fire(cuda_device, evaluate):
