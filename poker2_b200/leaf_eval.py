@@ -174,7 +174,7 @@ class DirectLeafEvaluator:
 
     def evaluate_into(self, leaf_beliefs: torch.Tensor, out: torch.Tensor) -> None:
         """Values of all leaves into out[..., :1326] (fp32 [L,2,W])."""
-        if not (self._direct() and _paired_rows(leaf_beliefs) and _paired_rows(out)):
+        if not (self._direct() and _paired_rows(leaf_beliefs, self._rows) and _paired_rows(out, self._rows)):
             out[..., :NUM_HANDS].copy_(self.model(leaf_beliefs[..., :NUM_HANDS].contiguous(), self.boards, self.context))
             return
         p, L = _lib.ptr, leaf_beliefs.shape[0]
@@ -197,7 +197,8 @@ class DirectLeafEvaluator:
         return out
 
 
-def _paired_rows(t: torch.Tensor) -> bool:
-    """[L,2,W] fp32, rows of whole pairs of hands one after the other."""
-    return (t.is_cuda and t.dtype == torch.float32 and t.stride(2) == 1 and t.stride(0) == 2 * t.stride(1)
+def _paired_rows(t: torch.Tensor, network_rows: torch.Tensor) -> bool:
+    """[L,2,W] fp32, rows of whole pairs of hands one after the other, as many leaves as there are network rows."""
+    return (t.is_cuda and t.device == network_rows.device and t.dim() == 3 and t.shape[0] == network_rows.shape[0]
+            and t.shape[1] == 2 and t.shape[2] >= NUM_HANDS and t.dtype == torch.float32 and t.stride(2) == 1 and t.stride(0) == 2 * t.stride(1)
             and t.stride(1) % 2 == 0 and t.data_ptr() % 8 == 0)

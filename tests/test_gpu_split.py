@@ -105,3 +105,25 @@ def test_refused_batch_stops_every_kernel(cuda_device, stepped):
     sv.solve(solver.pad_rows(ranges.to(cuda_device)).contiguous(), solver.iteration_scalars(4))
     assert sv.status() == 7
     assert all(bool((x == -7.0).all()) for x in outputs)
+
+
+@pytest.mark.parametrize("rows,width", [(7, 1344), (3, 1344), (5, 1324)])
+@pytest.mark.parametrize("what", ["beliefs", "out"])
+def test_network_per_leaf_refuses_other_shapes(cuda_device, rows, width, what):
+    """More or fewer leaves than the evaluator was made for, or rows that are too short, do not reach the kernels: the general
+    path refuses them."""
+    from poker2_b200 import leaf_eval
+
+    L = 5
+    g = torch.Generator(device=cuda_device).manual_seed(4)
+    boards = torch.tensor([[0, 1, 2, -1, -1]], device=cuda_device).expand(L, 5)
+    model = leaf_eval.ValueMLP(64, 2, dtype=torch.bfloat16, seed=1).to(cuda_device)
+    ev = leaf_eval.DirectLeafEvaluator(model, boards, torch.rand(L, 3, device=cuda_device, generator=g), cuda_device)
+    shapes = {"beliefs": (L, 2, 1344), "out": (L, 2, 1344)}
+    shapes[what] = (rows, 2, width)
+    beliefs = torch.rand(*shapes["beliefs"], device=cuda_device, generator=g)
+    with pytest.raises((RuntimeError, ValueError)):
+        ev.evaluate_into(beliefs, torch.zeros(*shapes["out"], device=cuda_device))
+    if what == "beliefs":
+        with pytest.raises((RuntimeError, ValueError)):
+            ev(beliefs)
