@@ -66,9 +66,10 @@ class ValueMLP(torch.nn.Module):
         """`self.net` on input rows x, activations in place (half the memory traffic and footprint of a GELU, same bits) and
         linear layers without the module's wrapper: a pass over few leaves lasts as long as the host takes to launch it.
         A network that someone listens to (hooks) or has changed goes through its modules instead."""
-        if type(self.net) is not torch.nn.Sequential or not (_bare(self.net) and all(map(_bare, self.net))):
-            return self.net(x)
-        for layer in self.net:
+        net = self.net
+        if type(net) is not torch.nn.Sequential or not _bare(net, *net._modules.values()):
+            return net(x)
+        for layer in net._modules.values():
             if type(layer) is torch.nn.GELU and layer.approximate == "none":
                 x = torch.ops.aten.gelu_(x)
             elif type(layer) is torch.nn.Linear:
@@ -81,12 +82,16 @@ class ValueMLP(torch.nn.Module):
 _module_hooks = torch.nn.modules.module
 
 
-def _bare(module: torch.nn.Module) -> bool:
-    """Nothing but the module's own `forward` would run if it were called: no forward hooks, on it or on all modules, no
-    `forward` put in place of the class's, not compiled."""
-    return not (module._forward_hooks or module._forward_pre_hooks or "forward" in module.__dict__
-                or module._compiled_call_impl is not None
-                or _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks)
+def _bare(*modules: torch.nn.Module) -> bool:
+    """Nothing but the modules' own `forward` would run if they were called: no forward hooks, on them or on all modules, no
+    `forward` put in place of the class's, not compiled.  (By their dictionaries: asked once a pass, for nine modules.)"""
+    if _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks:
+        return False
+    for m in modules:
+        own = m.__dict__
+        if own["_forward_hooks"] or own["_forward_pre_hooks"] or "forward" in own or own.get("_compiled_call_impl") is not None:
+            return False
+    return True
 
 
 def leaf_context(trees, node_index) -> torch.Tensor:
