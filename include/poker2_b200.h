@@ -104,12 +104,13 @@ int p2b_showdown_ev_sorted(const float* b_sorted, const int32_t* c1_sorted, cons
  *             local exploitability of the average policy and the best-response value of each
  *             player at the root (cfr_evaluator.py:718-764)
  *  rows       number of rows of the state arrays (the record check refuses subgames that reach past it)
- *  scratch    at least p2b_cfr_scratch_floats(max_internal, num_blocks) floats of work space.  With
- *             p2b_cfr_solve_scratch_floats(max_internal, max_children, num_blocks, num_subgames, rows)
- *             floats the solve runs as
- *             three launches (start pass; iteration passes in a leaner kernel; final pass) with the same
- *             results, bit for bit; the extra floats carry the root rows between the launches (very
- *             small batches stay in the one-launch form, see p2b_cfr_path_policy)
+ *  scratch    at least p2b_cfr_scratch_floats(max_internal, num_blocks) floats of work space: the general kernel
+ *             runs the whole solve in one launch, a set of work rows a block.  With
+ *             p2b_cfr_solve_block_scratch_floats(max_internal, max_children, num_blocks, num_subgames, rows) floats,
+ *             which also hold the rows that one launch hands to the next, the lean kernel may run the iteration passes
+ *             and a warm start is possible; with p2b_cfr_solve_scratch_floats(same arguments) the split kernels too,
+ *             for which that is 7 rows of 1344 floats a node (see p2b_cfr_path_policy).  Same results, bit for bit,
+ *             with any of the three
  *  scalars    [iterations] 32-byte records {float t^alpha, t^alpha+1, t^beta, t^beta+1,
  *             mix_old, mix_new, fl(mix_old+mix_new); int32 do_mix (bit 0; bits 1-2 see flags bit 4)}
  *  flags      bit 0: CFR+ (cumulative regrets clamped at zero after every update, cfr_evaluator.py:1366-1368);
@@ -157,7 +158,7 @@ int p2b_showdown_ev_sorted(const float* b_sorted, const int32_t* c1_sorted, cons
  *             that regret matching replays the start policy (warm_start of type `model`, :913-926).  scalars[0]
  *             then belongs to the warm start's own policy update (update_policy(w), :923) and scalars[k], k >= 1,
  *             to iteration w + k - 1; `iterations` counts these passes.  Needs the scratch area of
- *             p2b_cfr_solve_scratch_floats. */
+ *             p2b_cfr_solve_block_scratch_floats. */
 int p2b_cfr_solve(const void* subgames, const void* nodes, int32_t num_subgames, int64_t rows, int32_t max_children,
                   int32_t max_internal, const unsigned char* tables, const float* root_beliefs,
                   float* regrets, float* weight_sums, float* policy_avg, float* policy,
@@ -169,14 +170,17 @@ int p2b_cfr_solve(const void* subgames, const void* nodes, int32_t num_subgames,
 int64_t p2b_cfr_scratch_floats(int32_t max_internal, int32_t num_blocks);
 int64_t p2b_cfr_solve_scratch_floats(int32_t max_internal, int32_t max_children, int32_t num_blocks,
                                      int32_t num_subgames, int64_t rows);
+int64_t p2b_cfr_solve_block_scratch_floats(int32_t max_internal, int32_t max_children, int32_t num_blocks,
+                                           int32_t num_subgames, int64_t rows);
 int64_t p2b_cfr_step_scratch_floats(int32_t max_internal, int32_t num_subgames, int64_t rows);
 int p2b_cfr_default_blocks(void);
 /* Which kernels run the iteration passes of a p2b_cfr_solve whose leaves are all terminal (process-wide
  * setting, no counterpart in the upstream project).  0, the default: the lean kernel, a block per subgame, from
  * two subgames per SM on unless max_internal x max_children + 1 exceeds 160, i.e. some subgame may be too
  * large for it; else, and for solves it does not cover, the split kernels, which spread a subgame over the
- * chip (they need the scratch area of p2b_cfr_solve_scratch_floats as sized under the same setting; else the general
- * kernel runs).  1: the lean kernel whenever it applies.  Results are the same bits either way.  Returns the
+ * chip.  Where the scratch area has no room for those, the general kernel takes batches of at most a subgame per SM
+ * (fewer than eight where some may be large), the lean kernel those above that it covers.  1: the lean kernel
+ * whenever it applies (p2b_cfr_solve_scratch_floats then asks for no more than it needs).  Results are the same bits either way.  Returns the
  * previous setting; a negative argument only queries. */
 int p2b_cfr_path_policy(int32_t policy);
 /* Measurement aid (no counterpart in the upstream project): with timing enabled on the current

@@ -133,6 +133,13 @@ int64_t p2b_cfr_solve_scratch_floats(int32_t max_internal, int32_t max_children,
     return cfr_solve_scratch_floats(max_internal, max_children, num_blocks, num_subgames, rows);
 }
 
+int64_t p2b_cfr_solve_block_scratch_floats(int32_t max_internal, int32_t max_children, int32_t num_blocks,
+                                           int32_t num_subgames, int64_t rows) {
+    if (num_blocks <= 0) num_blocks = cfr_default_blocks();
+    if (num_blocks > num_subgames) num_blocks = num_subgames > 0 ? num_subgames : 1;
+    return cfr_solve_block_scratch_floats(max_internal, max_children, num_blocks, num_subgames, rows);
+}
+
 int p2b_cfr_solve(const void* subgames, const void* nodes, int32_t num_subgames, int64_t rows, int32_t max_children,
                   int32_t max_internal, const unsigned char* tables, const float* root_beliefs, float* regrets,
                   float* weight_sums, float* policy_avg, float* policy, float* root_values, float* values_avg,
@@ -200,11 +207,7 @@ int p2b_cfr_solve(const void* subgames, const void* nodes, int32_t num_subgames,
     p.queue_order = queue_order;
     p.start_policy = start_policy;
     p.warm_weight = warm_start_weight;
-    // with the larger scratch area of p2b_cfr_solve_scratch_floats the iteration passes of a plain
-    // solve run in the lean iteration kernel
-    const bool fast_scratch =
-        scratch_floats >= cfr_solve_scratch_floats(max_internal, max_children, num_blocks, num_subgames, rows);
-    return launch_cfr_solve(p, num_blocks, max_children, (cudaStream_t)stream, fast_scratch);
+    return launch_cfr_solve(p, num_blocks, max_children, (cudaStream_t)stream);
 }
 
 // Part of a solve: the passes pass_begin..pass_end, top-down and/or bottom-up sweeps.

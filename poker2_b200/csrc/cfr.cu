@@ -1615,26 +1615,38 @@ static int clear_counters(int32_t* work_counter, cudaStream_t stream) {
 // Some subgame of the batch may be too large for the lean kernel.
 static bool maybe_large(int max_internal, int max_children) { return (long long)max_internal * max_children + 1 > kIterMaxNodes; }
 
-static bool lean_preferred(int num_subgames, int max_internal, int max_children) {
+// `split`: the split kernels could run the batch; where they cannot (their work space is not there, or a tree is too deep for
+// them) the choice is the one between the lean and the general kernel, whose blocks walk a subgame each: at most one
+// subgame an SM leaves the lean kernel's 448 threads behind the general kernel's 672 (148 subgames x 64 iterations 30.2
+// against 22.3 ms), and with large subgames a small batch would run half empty twice (192 of up to 237 nodes x 24
+// iterations 64 against 36 ms).
+static bool lean_preferred(int num_subgames, int max_internal, int max_children, bool split) {
     if (g_path_policy.load() != 0) return true;
-    return num_subgames >= 2 * sm_count() && !maybe_large(max_internal, max_children);
+    const bool large = maybe_large(max_internal, max_children);
+    if (split) return num_subgames >= 2 * sm_count() && !large;
+    return num_subgames > (large ? 8 * sm_count() - 1 : sm_count());
 }
 
-// Work space of a one-call solve before the hand-over rows: one set of work rows per block, or the space of the split
-// passes, which the start and final pass use in turn.
-static long long solve_work_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows) {
+// Work space of a one-call solve is one set of work rows per block or, for the split kernels, some rows per node; behind it lie
+// the rows that one launch hands to the next.
+static long long block_work_floats(int max_internal, int max_children, int num_blocks) {
     long long per_block = cfr_scratch_floats(max_internal);
-    const long long iter_block = cfr_iter_scratch_floats(max_internal, max_children);
+    const long long iter_block = max_children <= kIterMaxChildren ? cfr_iter_scratch_floats(max_internal, max_children) : 0;
     if (iter_block > per_block) per_block = iter_block;
-    const long long blocks = per_block * num_blocks, split = split_scratch_floats(num_subgames, rows);
-    const bool lean = max_children <= kIterMaxChildren && lean_preferred(num_subgames, max_internal, max_children);
-    return !lean && split > blocks ? split : blocks;
+    return per_block * num_blocks;
+}
+static long long carry_floats(int num_subgames, long long rows) {
+    return (long long)num_subgames * 4 * P2B_HPAD + rows * 4;  // sums: current-policy and, for cfr_avg, average-policy
+}
+
+long long cfr_solve_block_scratch_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows) {
+    return block_work_floats(max_internal, max_children, num_blocks) + carry_floats(num_subgames, rows);
 }
 
 long long cfr_solve_scratch_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows) {
-    const long long carry_sums = rows * 4;  // current-policy sums and, for cfr_avg, average-policy sums
-    return solve_work_floats(max_internal, max_children, num_blocks, num_subgames, rows) + (long long)num_subgames * 4 * P2B_HPAD +
-           carry_sums;
+    const long long blocks = block_work_floats(max_internal, max_children, num_blocks), split = split_scratch_floats(num_subgames, rows);
+    const bool lean = max_children <= kIterMaxChildren && lean_preferred(num_subgames, max_internal, max_children, true);
+    return (!lean && split > blocks ? split : blocks) + carry_floats(num_subgames, rows);
 }
 
 long long cfr_step_scratch_floats(int max_internal, int num_subgames, long long rows) {
@@ -1680,14 +1692,13 @@ static int launch_stepped(const CfrParams& p, int num_blocks, int max_children, 
     return rc;
 }
 
-int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, cudaStream_t stream, bool fast_scratch) {
+int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, cudaStream_t stream) {
     if (params.num_subgames == 0) return P2B_OK;
     if (params.iterations < 1) return set_error(P2B_ERR_ARG, "at least one iteration is required");
     int rc = ensure_tables();
     if (rc) return rc;
     CfrParams p = params;
     p.combos = device_combo_table();
-    // leaves all terminal, uniform start policy, all passes in this call: the iteration kernel applies
     if (p.warm_weight > 0.0f && (!p.start_policy || !p.rows))
         return set_error(P2B_ERR_ARG, "a warm start needs a start policy and the row count of the state arrays");
     // leaves all terminal, all passes in this call: the iteration kernel applies (a start policy only concerns
@@ -1695,17 +1706,18 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
     const bool plain = !p.stepped && !p.leaf_beliefs && !p.leaf_values && !p.cfr_avg && !p.linear;
     if (p.stepped && p.phases != 8 && split_applies(p, max_children, p.scratch_floats))
         return launch_stepped(p, num_blocks, max_children, stream);
-    long long per_block = cfr_scratch_floats(p.max_internal);
-    const long long iter_block = cfr_iter_scratch_floats(p.max_internal, max_children);
-    if (iter_block > per_block) per_block = iter_block;
+    const long long blocks = block_work_floats(p.max_internal, max_children, num_blocks), per_block = blocks / num_blocks;
+    const long long carry = carry_floats(p.num_subgames, p.rows);
+    const bool room = !p.stepped && p.rows > 0 && p.scratch_floats >= blocks + carry;  // for rows that launches hand on
+    const bool split = room && split_applies(p, max_children, p.scratch_floats - carry);
     const bool large = maybe_large(p.max_internal, max_children);
-    const bool lean = plain && fast_scratch && max_children <= kIterMaxChildren &&
-                      lean_preferred(p.num_subgames, p.max_internal, max_children);
-    if (!p.stepped && fast_scratch && !lean && split_applies(p, max_children, p.scratch_floats)) {
+    const bool lean = plain && room && max_children <= kIterMaxChildren &&
+                      lean_preferred(p.num_subgames, p.max_internal, max_children, split);
+    if (split && !lean) {
         IterTiming* timing = iter_timing_of_current_device();
         const bool timed = timing && timing->enabled;
         CfrParams q = p;
-        q.carry_roots = p.scratch + solve_work_floats(p.max_internal, max_children, num_blocks, p.num_subgames, p.rows);
+        q.carry_roots = p.scratch + split_scratch_floats(p.num_subgames, p.rows);
         q.carry_sums = q.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;
         const bool warm = p.warm_weight > 0.0f;  // works on the regrets of the start pass before the iterations read them
         rc = clear_counters(q.work_counter, stream);
@@ -1725,12 +1737,12 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
         if (p.warm_weight > 0.0f) {
             // the general kernel in two launches around the seeding: start pass, then every other pass
             if (p.stepped) return set_error(P2B_ERR_ARG, "a stepped solve seeds its warm start itself");
-            if (!fast_scratch)
-                return set_error(P2B_ERR_ARG, "a warm start needs the scratch area of p2b_cfr_solve_scratch_floats "
+            if (!room)
+                return set_error(P2B_ERR_ARG, "a warm start needs the scratch area of p2b_cfr_solve_block_scratch_floats "
                                               "(hand-over rows between the launches)");
             CfrParams q = p;
             q.scratch_stride = per_block;
-            q.carry_roots = p.scratch + solve_work_floats(p.max_internal, max_children, num_blocks, p.num_subgames, p.rows);
+            q.carry_roots = p.scratch + blocks;
             q.carry_sums = q.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;
             q.stepped = 1;
             q.scratch_per_block = 1;
@@ -1757,7 +1769,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
     // pass with the best responses (cfr_solve_kernel).  Root rows and their sums travel between the
     // launches in the tail of the scratch area; work rows do not, so each launch keeps one set per block.
     p.scratch_stride = per_block;
-    p.carry_roots = p.scratch + solve_work_floats(p.max_internal, max_children, num_blocks, p.num_subgames, p.rows);
+    p.carry_roots = p.scratch + blocks;
     p.carry_sums = p.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;
     p.stepped = 1;
     p.scratch_per_block = 1;

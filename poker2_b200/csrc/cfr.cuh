@@ -158,11 +158,11 @@ __host__ __device__ inline long long cfr_scratch_floats(int max_internal) {
     return (long long)max_internal * 6 * P2B_HPAD;
 }
 
-// `fast_scratch`: the scratch area also holds the hand-over rows of a split solve
-// (cfr_solve_scratch_floats), so a plain solve may run its iteration passes in cfr_iter_kernel.
-int launch_cfr_solve(const CfrParams& p, int num_blocks, int max_children, cudaStream_t stream, bool fast_scratch = false);
+// Which kernels run a one-call solve depends on its size and on the scratch area it brings (p.scratch_floats).
+int launch_cfr_solve(const CfrParams& p, int num_blocks, int max_children, cudaStream_t stream);
 long long cfr_iter_scratch_floats(int max_internal, int max_children);
 long long cfr_solve_scratch_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows);
+long long cfr_solve_block_scratch_floats(int max_internal, int max_children, int num_blocks, int num_subgames, long long rows);
 long long cfr_step_scratch_floats(int max_internal, int num_subgames, long long rows);
 int launch_cfr_iter(const CfrParams& p, int num_blocks, cudaStream_t stream);
 int cfr_path_policy(int policy);  // returns the previous one; < 0 only queries

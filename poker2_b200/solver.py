@@ -299,6 +299,17 @@ class SolveResult:
         return x.index_select(0, layout_tensor(self.layout, "from_level_major", x.device))[..., :NUM_HANDS]
 
 
+def _room_for(num_bytes: int, device: torch.device) -> bool:
+    """Twice that many bytes are free on the device for this process.  Asked for areas above a sixteenth of the card alone:
+    the question takes the driver some 10 us, and the allocation itself says whether a small one fits."""
+    total = torch.cuda.get_device_properties(device).total_memory
+    if num_bytes <= total // 16:
+        return True
+    held = torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)  # the allocator's own, free
+    allowed = int(torch.cuda.get_per_process_memory_fraction(device) * total) - torch.cuda.memory_allocated(device)
+    return 2 * num_bytes <= min(torch.cuda.mem_get_info(device)[0] + held, allowed)
+
+
 class SubgameSolver:
     """Holds the device buffers of one batch shape and runs the fused kernel on them."""
 
@@ -306,8 +317,9 @@ class SubgameSolver:
                  track_weight_sums: bool = True, keep_policy: bool = False, keep_node_values: bool = False,
                  exploitability: bool = False, num_blocks: int = 0, sampling: bool = False,
                  lean_iterations: bool = True):
-        """lean_iterations=False gives the kernel only its minimal scratch area, which keeps every
-        pass of a solve in the general kernel (one launch); results are the same bit for bit."""
+        """lean_iterations=False gives the solve only the minimal scratch area, which keeps every pass
+        in the general kernel (one launch); results are the same bit for bit, and also where the area
+        that a solve runs fastest with does not fit the card (`_allocate_scratch`)."""
         keep_node_values = keep_node_values or exploitability  # best responses read the node values
         if device.type != "cuda":
             raise ValueError("SubgameSolver requires a CUDA device.")
@@ -339,7 +351,6 @@ class SubgameSolver:
         self.beliefs_avg = torch.zeros(rows, 2, HPAD, **f32) if keep_node_values else None
         self.exploitability = torch.zeros(B, **f32) if (exploitability and keep_node_values) else None
         self.br_values = torch.zeros(B, 2, **f32) if (exploitability and keep_node_values) else None
-        self.scratch = torch.empty(self._scratch_floats(lean_iterations), **f32)
         self.work_counter = torch.zeros(4, device=device, dtype=torch.int32)
         # the thread blocks take subgames from a queue: largest trees first, so that the blocks that finish
         # last hold small ones (a stable sort: equal sizes keep their input order)
@@ -352,15 +363,34 @@ class SubgameSolver:
         self.policy_sample = torch.zeros(rows, HPAD, **f32) if sampling else None
         self.beliefs_last = torch.zeros(rows, 2, HPAD, **f32) if sampling else None
         self.sample_pass = torch.full((B,), -2, device=device, dtype=torch.int32) if sampling else None
+        self._more_buffers()
+        self.scratch = self._allocate_scratch(lean_iterations)  # last: what fits is known then
         self.launches = 0
 
-    def _scratch_floats(self, lean_iterations: bool) -> int:
-        """The larger area lets a solve run its iteration passes in the lean or in the split kernels."""
+    def _more_buffers(self) -> None:
+        """Buffers of a derived solver, allocated before the scratch area."""
+
+    def _scratch_floats(self, lean_iterations: bool) -> list[int]:
+        """Sizes a solve runs with, the fastest first."""
         layout, lib = self.layout, _lib.lib()
-        if lean_iterations:
-            return int(lib.p2b_cfr_solve_scratch_floats(layout.max_internal, layout.max_children, self.num_blocks, self.B,
-                                                        layout.rows))
-        return int(lib.p2b_cfr_scratch_floats(layout.max_internal, self.num_blocks))
+        if not lean_iterations:
+            return [int(lib.p2b_cfr_scratch_floats(layout.max_internal, self.num_blocks))]
+        args = (layout.max_internal, layout.max_children, self.num_blocks, self.B, layout.rows)
+        return [int(lib.p2b_cfr_solve_scratch_floats(*args)), int(lib.p2b_cfr_solve_block_scratch_floats(*args))]
+
+    def _allocate_scratch(self, lean_iterations: bool) -> torch.Tensor:
+        """The split kernels' area is 7 work rows a node, as much as the state arrays themselves: where it does not
+        fit beside what the process holds, or would leave a large solve's caller (its leaf model, its results) less than
+        as much again, the solve gets the smaller area and runs in the kernels that walk a subgame a block."""
+        sizes = self._scratch_floats(lean_iterations)
+        for floats in sizes[:-1]:
+            if floats > sizes[-1] and not _room_for(4 * floats, self.device):
+                continue
+            try:
+                return torch.empty(floats, device=self.device, dtype=torch.float32)
+            except torch.OutOfMemoryError:
+                pass
+        return torch.empty(sizes[-1], device=self.device, dtype=torch.float32)
 
     def set_sampling_schedule(self, t_sample: torch.Tensor, warm_start_iterations: int = 0) -> None:
         """t_sample [B]: iteration at whose start each subgame's current policy is kept
@@ -462,18 +492,19 @@ class SteppedSolver(SubgameSolver):
     device (columns 1326.. are padding; slot order = `layout.model_rows`), and returns their
     values for both players in the same shape (or [slots,2,1326]), in chips / scale."""
 
-    def __init__(self, layout: DeviceTreeLayout, boards: torch.Tensor, device: torch.device, **kw):
-        super().__init__(layout, boards, device, **kw)
-        f32 = dict(device=device, dtype=torch.float32)
+    def _more_buffers(self) -> None:
+        layout, f32 = self.layout, dict(device=self.device, dtype=torch.float32)
         self.carry_sums = torch.zeros(2, layout.rows, 2, **f32)  # current-policy sums, average-policy sums
         self.carry_roots = torch.zeros(self.B, 4, HPAD, **f32)
         slots = max(layout.num_model_leaves, 1)
-        self.leaf_begin = layout_tensor(layout, "leaf_begin", device, torch.int32)
+        self.leaf_begin = layout_tensor(layout, "leaf_begin", self.device, torch.int32)
         self.leaf_beliefs = torch.zeros(slots, 2, HPAD, **f32)
         self.leaf_values = torch.zeros(slots, 2, HPAD, **f32)
 
-    def _scratch_floats(self, lean_iterations: bool) -> int:
-        return int(_lib.lib().p2b_cfr_step_scratch_floats(self.layout.max_internal, self.B, self.layout.rows))
+    def _scratch_floats(self, lean_iterations: bool) -> list[int]:
+        layout, lib = self.layout, _lib.lib()
+        return [int(lib.p2b_cfr_step_scratch_floats(layout.max_internal, self.B, layout.rows)),
+                int(lib.p2b_cfr_scratch_floats(layout.max_internal, 1)) * self.B]
 
     start_policy_rows = None  # [rows,1344] policy of the start pass (None: uniform)
     _last_model_values = None  # the model's values of the evaluation before (cfr_avg), padded rows

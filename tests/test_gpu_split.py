@@ -127,3 +127,96 @@ def test_network_per_leaf_refuses_other_shapes(cuda_device, rows, width, what):
     if what == "beliefs":
         with pytest.raises((RuntimeError, ValueError)):
             ev(beliefs)
+
+
+def _kernels_of(fn):
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+        fn()
+        torch.cuda.synchronize()
+    return " ".join(e.name for e in prof.events() if "_kernel" in e.name)
+
+
+@pytest.mark.parametrize("B", [5, 160])  # the general kernel; the lean kernel where it covers the solve
+@pytest.mark.parametrize("kind", ["plain", "eight actions", "cfr_avg", "warm"])
+def test_smaller_scratch_areas(cuda_device, B, kind):
+    """An area without room for the split kernels: the lean or the general kernel runs, with the same bits and without a write
+    behind the area's end."""
+    import bench
+    from poker2_b200 import _lib, solver, tree as ptree
+
+    boards, ranges, pot, stack = bench.make_inputs(B, 3)
+    bins = (0.5, 0.75, 1.0, 1.5, 2.0) if kind == "eight actions" else (0.5, 1.0)
+    trees = ptree.build_trees(ptree.root_states(pot.numpy(), stack.numpy()), list(bins), 8, max_raises=1)
+    layout = solver.device_layout(trees, boards.numpy())
+    rb = solver.pad_rows(ranges.to(cuda_device)).contiguous()
+    kw = {"cfr_avg": True} if kind == "cfr_avg" else {}
+    if kind == "warm":
+        siblings = torch.from_numpy(trees.child_count[trees.parent_index.clip(min=0)]).clamp(min=1)
+        kw = dict(start_policy=(1.0 / siblings.float())[:, None].expand(-1, 1326).contiguous(), warm_start_iterations=2,
+                  warm_start_multiplier=3.0)
+    scal = solver.iteration_scalars(5, warm_start_iterations=2 if kind == "warm" else 0)
+    lib, args = _lib.lib(), (layout.max_internal, layout.max_children, min(B, 148), B, layout.rows)
+    full = int(lib.p2b_cfr_solve_scratch_floats(*args))
+    sizes = [full, int(lib.p2b_cfr_solve_block_scratch_floats(*args))]
+    if kind != "warm":  # which needs rows handed from launch to launch
+        sizes.append(int(lib.p2b_cfr_scratch_floats(layout.max_internal, min(B, 148))))
+    assert sizes == sorted(sizes, reverse=True) and len(set(sizes)) == len(sizes)
+    out = []
+    for n in sizes:
+        sv = solver.SubgameSolver(layout, boards, cuda_device, exploitability=True)
+        assert sv.num_blocks == min(B, 148) and sv.scratch.numel() == full
+        guarded = torch.full((n + (1 << 20),), float("nan"), device=cuda_device)
+        guarded[n:] = 7.0
+        sv.scratch = guarded[:n]
+        names = _kernels_of(lambda: sv.solve(rb, scal, check=True, **kw))
+        assert ("split_rows_kernel" in names) == (n == full)
+        lean = n == sizes[1] and B > 148 and kind in ("plain", "warm")
+        assert ("cfr_iter_kernel" in names) == lean, names
+        assert bool((guarded[n:] == 7.0).all())
+        out.append([x.clone() for x in (sv.policy_avg, sv.regrets, sv.weight_sums, sv.root_values[..., :1326], sv.exploitability)])
+    for other in out[1:]:
+        for a, b in zip(out[0], other):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("stepped", [False, True])
+def test_area_that_does_not_fit(cuda_device, stepped):
+    """A process whose share of the card holds the state arrays but not the split kernels' area: the solver takes the smaller
+    area, with the same results."""
+    import bench
+    from poker2_b200 import solver, tree as ptree
+
+    B = 160
+    boards, ranges, _, _ = bench.make_inputs(B, 4)
+    trees = ptree.build_trees(ptree.root_states(np.full(B, 60), np.full(B, 500)), [0.5, 1.0], 8)
+    layout = solver.device_layout(trees, boards.numpy())
+    rb = solver.pad_rows(ranges.to(cuda_device)).contiguous()
+    scal = solver.iteration_scalars(3)
+    cls = solver.SteppedSolver if stepped else solver.SubgameSolver
+
+    def solved(sv):
+        sv.solve(rb, scal)
+        assert sv.status() == 0
+        return [x.cpu() for x in (sv.policy_avg, sv.regrets, sv.root_values[..., :1326])]
+
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated(cuda_device)
+    sv = cls(layout, boards, cuda_device)
+    full, smallest = sv.scratch.numel(), sv._scratch_floats(True)[-1]
+    assert full == sv._scratch_floats(True)[0] and 4 * (full - smallest) > 512 << 20
+    state = torch.cuda.memory_allocated(cuda_device) - before - 4 * full
+    want = solved(sv)
+    del sv
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(cuda_device).total_memory
+    share = torch.cuda.memory_reserved(cuda_device) + state + 4 * smallest + (256 << 20)
+    torch.cuda.set_per_process_memory_fraction(share / total, cuda_device)
+    try:
+        sv = cls(layout, boards, cuda_device)
+        assert sv.scratch.numel() == smallest
+        got = solved(sv)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, cuda_device)
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
