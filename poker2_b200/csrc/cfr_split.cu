@@ -103,9 +103,40 @@ __device__ __forceinline__ bool block_stops(const CfrParams& p) {
 }
 
 // ---- work lists -------------------------------------------------------------------------------
-// One block per subgame, one thread per node.  The items of a batch follow the queue order, those of a subgame the
-// node order, which is breadth-first.
-__global__ void __launch_bounds__(kCfrMaxNodes) split_items_kernel(const CfrParams p, const SplitWork w) {
+// The items of a batch follow the queue order, those of a subgame the node order, which is breadth-first.
+
+// Where the items of each subgame begin (levels[].item_begin), by one block: a thread adds up a run of subgames, the block the
+// threads' sums.
+constexpr int kBeginThreads = 1024;
+__global__ void __launch_bounds__(kBeginThreads) split_begin_kernel(const CfrParams p, const SplitWork w) {
+    __shared__ int s_warp[kBeginThreads / 32];
+    if (block_stops(p)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int run = (p.num_subgames + kBeginThreads - 1) / kBeginThreads;
+    const int first = min(tid * run, p.num_subgames), last = min(first + run, p.num_subgames);
+    auto items = [&](int q) { return p.subgames[p.queue_order ? p.queue_order[q] : q].n_internal; };
+    int mine = 0;
+#pragma unroll 8
+    for (int q = first; q < last; ++q) mine += items(q);
+    int upto = mine;
+    for (int d = 1; d < 32; d <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= d) upto += x;
+    }
+    if (lane == 31) s_warp[warp] = upto;
+    __syncthreads();
+    int at = upto - mine;
+    for (int x = 0; x < warp; ++x) at += s_warp[x];
+#pragma unroll 8
+    for (int q = first; q < last; ++q) {
+        w.levels[q].item_begin = at;
+        at += items(q);
+    }
+}
+
+// One block per subgame, one thread per node.  `begun`: split_begin_kernel has run; else every block adds up the subgames
+// before its own.
+__global__ void __launch_bounds__(kCfrMaxNodes) split_items_kernel(const CfrParams p, const SplitWork w, bool begun) {
     __shared__ int s_before, s_depth[kSplitMaxDepth + 1], s_bad;
     const int q = blockIdx.x, i = threadIdx.x;
     if (i == 0) s_before = s_bad = 0;
@@ -115,10 +146,14 @@ __global__ void __launch_bounds__(kCfrMaxNodes) split_items_kernel(const CfrPara
         return;
     }
     const int s = p.queue_order ? p.queue_order[q] : q;
-    int before = 0;
-    for (int r = i; r < q; r += kCfrMaxNodes) before += p.subgames[p.queue_order ? p.queue_order[r] : r].n_internal;
-    for (int d = 16; d > 0; d >>= 1) before += __shfl_xor_sync(0xffffffffu, before, d);
-    if ((i & 31) == 0) atomicAdd(&s_before, before);
+    if (begun) {
+        if (i == 0) s_before = w.levels[q].item_begin;
+    } else {
+        int before = 0;
+        for (int r = i; r < q; r += kCfrMaxNodes) before += p.subgames[p.queue_order ? p.queue_order[r] : r].n_internal;
+        for (int d = 16; d > 0; d >>= 1) before += __shfl_xor_sync(0xffffffffu, before, d);
+        if ((i & 31) == 0) atomicAdd(&s_before, before);
+    }
     __syncthreads();
     const SubgameRec sg = p.subgames[s];
     const NodeRecPacked* nodes = p.nodes + sg.node_begin;
@@ -1645,6 +1680,17 @@ bool split_applies(const CfrParams& p, int max_children, long long scratch_float
            scratch_floats >= split_scratch_floats(p.num_subgames, p.rows);
 }
 
+// The work lists.  Adding up in every block what lies before it is quadratic in the batch, a launch of its own costs a few us and
+// more where a thread's run of subgames gets long: measured, us with the launch / without, 2048 subgames 16 / 14, 4096 28 / 26,
+// 8192 50 / 63, 16,384 97 / 182.
+constexpr int kBeginFrom = 6144;  // subgames
+static int launch_lists(const CfrParams& p, const SplitWork& w, cudaStream_t stream) {
+    const bool begun = p.num_subgames >= kBeginFrom;
+    if (begun) split_begin_kernel<<<1, kBeginThreads, 0, stream>>>(p, w);
+    split_items_kernel<<<p.num_subgames, kCfrMaxNodes, 0, stream>>>(p, w, begun);
+    return check_cuda(cudaGetLastError(), "split_items_kernel");
+}
+
 int launch_split_passes(const CfrParams& p, int max_children, int pass_begin, int pass_end, bool down, bool up, bool continued,
                         cudaStream_t stream) {
     const SplitWork w = carve(p.scratch, p.num_subgames, p.rows);
@@ -1652,8 +1698,7 @@ int launch_split_passes(const CfrParams& p, int max_children, int pass_begin, in
     int rc = P2B_OK;
     bool follows = false;
     if (down && !continued) {
-        split_items_kernel<<<p.num_subgames, kCfrMaxNodes, 0, stream>>>(p, w);
-        rc = check_cuda(cudaGetLastError(), "split_items_kernel");
+        rc = launch_lists(p, w, stream);
         if (!rc) rc = launch_prep<kPrepPolicy>(p, w, pass_begin, max_children, stream);
     }
     for (int pass = pass_begin; pass <= pass_end && !rc; ++pass) {
@@ -1679,8 +1724,7 @@ int launch_split_start(const CfrParams& p, int max_children, bool down, bool up,
     const SplitWork w = carve(p.scratch, p.num_subgames, p.rows);
     int rc = P2B_OK;
     if (down) {
-        split_items_kernel<<<p.num_subgames, kCfrMaxNodes, 0, stream>>>(p, w);
-        rc = check_cuda(cudaGetLastError(), "split_items_kernel");
+        rc = launch_lists(p, w, stream);
         if (!rc) rc = launch_rows<kRowStart>(p, w, 0, max_children, false, stream);
     }
     if (!rc && up) rc = launch_up(p, w, kUpStart, -1, advance, true, max_children, down, stream);

@@ -220,3 +220,50 @@ def test_area_that_does_not_fit(cuda_device, stepped):
         torch.cuda.set_per_process_memory_fraction(1.0, cuda_device)
     for a, b in zip(want, got):
         assert torch.equal(a, b)
+
+
+def _small_trees(cuda_device, B):
+    """A batch of small trees off the lean path, on the split kernels."""
+    from poker2_b200 import _lib, device_tree, solver, tree as ptree
+
+    boards = torch.rand(B, 52, generator=torch.Generator().manual_seed(B)).argsort(dim=1)[:, :5]
+    layout = device_tree.build_device_layout(ptree.root_states(np.full(B, 100), 8 + np.arange(B) % 5), boards, [0.5, 1.0], 3,
+                                             max_raises=1, device=cuda_device)
+    layout.max_children = 8  # as if some node had so many actions
+    sv = solver.SubgameSolver(layout, boards, cuda_device)
+    assert sv.scratch.numel() == _lib.lib().p2b_cfr_solve_scratch_floats(layout.max_internal, 8, sv.num_blocks, B, layout.rows)
+    ranges = torch.rand(B, 2, 1344, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(1))
+    ranges[..., 1326:] = 0.0
+    return sv, ranges, solver.iteration_scalars(2)
+
+
+@pytest.mark.parametrize("B", [6143, 6144, 7001])  # below and from where the lists' beginnings are added up by one block
+def test_work_lists_of_large_batches(cuda_device, B):
+    from poker2_b200 import _lib
+
+    sv, ranges, scal = _small_trees(cuda_device, B)
+    outputs = (sv.policy_avg, sv.regrets, sv.root_values[..., :1326])
+    names = _kernels_of(lambda: sv.solve(ranges, scal, check=True))
+    assert "split_rows_kernel" in names and ("split_begin_kernel" in names) == (B >= 6144)
+    got = [x.clone() for x in outputs]
+    sv.scratch = torch.empty(int(_lib.lib().p2b_cfr_scratch_floats(sv.layout.max_internal, sv.num_blocks)), device=cuda_device)
+    assert "split_rows_kernel" not in _kernels_of(lambda: sv.solve(ranges, scal, check=True))
+    for a, b in zip(got, outputs):
+        assert torch.equal(a, b)
+
+
+def test_work_lists_take_time_in_proportion_to_the_batch(cuda_device):
+    def microseconds(B):
+        sv, ranges, scal = _small_trees(cuda_device, B)
+        sv.solve(ranges, scal, check=True)
+        times = []
+        for _ in range(3):
+            torch.cuda.synchronize()
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+                sv.solve(ranges, scal)
+                torch.cuda.synchronize()
+            times.append(sum(e.device_time for e in prof.events() if "split_begin_kernel" in e.name or "split_items_kernel" in e.name))
+        return min(times)
+
+    few, many = microseconds(3072), microseconds(24576)
+    assert 0.0 < many < 12.0 * few, (few, many)  # eight times the subgames; with 64 times the reads it was about 19 times as long
