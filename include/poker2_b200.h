@@ -134,7 +134,9 @@ int p2b_showdown_ev_sorted(const float* b_sorted, const int32_t* c1_sorted, cons
  *  init_depth depth of the deepest tree of the batch (the upstream start pass re-normalises
  *             every belief row once per level of the batch-wide tree)
  *  work_counter four int32, zeroed by the call: [0] the queue the thread blocks take subgames
- *             from; [1] status; [2], [3] internal.  Before every launch a checking kernel compares
+ *             from; [1] status; [2] spare; [3] 1 + a subgame in which a wait between the warps of a block ran out
+ *             (never seen: its limit is there so that a launch always ends), which becomes the status too; it is kept
+ *             over the calls of a stepped solve until the next start pass.  Before every launch a checking kernel compares
  *             every subgame's records with the solver's limits (1..320 nodes per subgame, all
  *             inside the `rows` rows, 1..8 children per internal node, children stored after their
  *             parent and inside the subgame, internal_idx < max_internal, unused record bits zero, root

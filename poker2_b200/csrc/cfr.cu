@@ -1436,6 +1436,10 @@ __global__ void __launch_bounds__(CfrThreads<VPT>::value, 1) cfr_solve_kernel(co
 // solver kernel launched next on the stream finds no work at all.
 __global__ void __launch_bounds__(kCfrMaxNodes) cfr_validate_kernel(const CfrParams p) {
     const int s = blockIdx.x, i = threadIdx.x;
+    if (s == 0 && i == 0 && p.work_counter[kGaveUp] != 0) {  // an earlier call of this solve has left rows that mean nothing
+        atomicMax(p.work_counter + 1, p.work_counter[kGaveUp]);
+        atomicMax(p.work_counter, p.num_subgames);
+    }
     const SubgameRec sg = p.subgames[s];
     int bad = sg.n_nodes < 1 || sg.n_nodes > kCfrMaxNodes || sg.n_internal > p.max_internal || sg.node_begin < 0 ||
               (p.rows > 0 && (long long)sg.node_begin + sg.n_nodes > p.rows) ||
@@ -1607,9 +1611,11 @@ int cfr_iteration_ms(float* ms) {
     return check_cuda(cudaEventElapsedTime(ms, t->start, t->stop), "cudaEventElapsedTime");
 }
 
-static int clear_counters(int32_t* work_counter, cudaStream_t stream) {
-    // [0] subgame queue, [1] status, [2], [3] spare
-    return check_cuda(cudaMemsetAsync(work_counter, 0, 4 * sizeof(int32_t), stream), "cudaMemsetAsync(work counter)");
+// Queue and status; the word of a wait that ran out is cleared with the start pass and kept over the calls of a stepped solve.
+static int clear_counters(const CfrParams& p, cudaStream_t stream) {
+    const bool goes_on = p.stepped && p.pass_begin >= 0;
+    return check_cuda(cudaMemsetAsync(p.work_counter, 0, (goes_on ? kGaveUp : kGaveUp + 1) * sizeof(int32_t), stream),
+                      "cudaMemsetAsync(work counter)");
 }
 
 // Some subgame of the batch may be too large for the lean kernel.
@@ -1659,7 +1665,7 @@ static int general_passes(CfrParams p, int num_blocks, int max_children, int beg
     p.pass_begin = begin;
     p.pass_end = end;
     p.phases = phases;
-    int rc = clear_counters(p.work_counter, stream);
+    int rc = clear_counters(p, stream);
     return rc ? rc : dispatch_cfr(p, num_blocks, max_children, stream);
 }
 
@@ -1672,7 +1678,7 @@ static int launch_stepped(const CfrParams& p, int num_blocks, int max_children, 
         rc = general_passes(p, num_blocks, max_children, -1, -1, p.phases == 16 ? 2 : p.phases, stream);
         if (rc || p.pass_end < 0) return rc;
     }
-    rc = clear_counters(p.work_counter, stream);
+    rc = clear_counters(p, stream);
     if (!rc) rc = check_records(p, stream);
     if (rc) return rc;
     const bool start = p.pass_begin < 0 && !p.iter_values;
@@ -1720,7 +1726,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
         q.carry_roots = p.scratch + split_scratch_floats(p.num_subgames, p.rows);
         q.carry_sums = q.carry_roots + (long long)p.num_subgames * 4 * P2B_HPAD;
         const bool warm = p.warm_weight > 0.0f;  // works on the regrets of the start pass before the iterations read them
-        rc = clear_counters(q.work_counter, stream);
+        rc = clear_counters(q, stream);
         if (!rc) rc = check_records(q, stream);
         if (!rc) rc = launch_split_start(q, max_children, true, true, !warm, stream);
         if (!rc && warm)
@@ -1750,7 +1756,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
             for (int part = 0; part < 2; ++part) {
                 q.pass_begin = part == 0 ? -1 : 0;
                 q.pass_end = part == 0 ? -1 : p.iterations;
-                rc = clear_counters(q.work_counter, stream);
+                rc = clear_counters(q, stream);
                 if (rc) return rc;
                 rc = dispatch_cfr(q, num_blocks, max_children, stream);
                 if (rc) return rc;
@@ -1761,7 +1767,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
             }
             return P2B_OK;
         }
-        rc = clear_counters(p.work_counter, stream);
+        rc = clear_counters(p, stream);
         if (rc) return rc;
         return dispatch_cfr(p, num_blocks, max_children, stream);
     }
@@ -1778,7 +1784,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
         CfrParams q = p;
         q.pass_begin = part == 0 ? -1 : (part == 1 ? 0 : p.iterations);
         q.pass_end = part == 0 ? -1 : (part == 1 ? p.iterations - 1 : p.iterations);
-        rc = clear_counters(q.work_counter, stream);
+        rc = clear_counters(q, stream);
         if (rc) return rc;
         if (part == 1) {
             rc = check_records(q, stream);
@@ -1795,7 +1801,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
             // the general kernel runs their iteration passes.  The batch can only contain such a subgame
             // if the bound below exceeds the limit.
             if (!rc && large) {
-                rc = clear_counters(q.work_counter, stream);
+                rc = clear_counters(q, stream);
                 if (rc) return rc;
                 q.large_only = 1;
                 rc = dispatch_cfr(q, num_blocks, max_children, stream);

@@ -85,6 +85,9 @@ constexpr int kIterMaxNodes = 160;  // what the lean iteration kernel holds; lar
 constexpr int kCfrMaxChildren = 8;   // actions per node (fold, call, five bet sizes, all-in: the upstream dataclass default)
 constexpr int kIterMaxChildren = 6;  // the lean iteration kernel's staging rows; batches with more stay in the general kernel
 
+// Word of work_counter: 1 + a subgame in which a wait on the device ran out since the start pass, 0: none has.
+constexpr int kGaveUp = 3;
+
 struct CfrParams {
     const SubgameRec* subgames;
     const NodeRecPacked* nodes;  // indexed by node_begin + local index
@@ -118,7 +121,7 @@ struct CfrParams {
                                  // passes) the beliefs under the average policy in beliefs_avg: what a caller mixes into
                                  // running average values (`update_average_values`, cfr_evaluator.py:1260-1274)
     int32_t init_depth;          // depth of the deepest tree of the batch the subgames were built in
-    int32_t* work_counter;       // dynamic subgame queue (zeroed by the launcher)
+    int32_t* work_counter;       // four words zeroed by the launcher: [0] subgame queue, [1] status, [2] spare, [kGaveUp]
     const int32_t* queue_order;  // [B] subgame taken at each queue position (may be null: input order); a caller puts
                                  // the largest trees first so that the last blocks to finish hold small ones
     // ---- stepped mode: a launch runs part of the pass sequence and the state that a whole

@@ -93,13 +93,17 @@ SplitWork carve(float* scratch, int num_subgames, long long rows) {
     return w;
 }
 
-// Whether the solve has been refused or given up, the same answer for every thread of the block (all of them call it).  Other
-// blocks, and the kernel before this one where it still runs, may set the word meanwhile: if each thread went by what it read
-// itself, some would leave and the rest would wait for them at a barrier.  A kernel that reads the word too early works on
-// rows that no longer mean anything, but on lists that are whole: the record check has finished before any of these starts.
-__device__ __forceinline__ bool block_stops(const CfrParams& p) {
-    const int stop = threadIdx.x == 0 ? *reinterpret_cast<const volatile int32_t*>(p.work_counter + 1) : 0;
-    return __syncthreads_or(stop) != 0;
+// Whether the solve has been refused (work_counter[1]).  A kernel that nothing runs beside has its block agree on it, as other
+// blocks of the same kernel may set the word.  The two kernels of a pass, which may start before the one ahead of them has
+// ended, read it thread by thread: no kernel that they can meet writes it, a wait that runs out is noted in a word of its own
+// (gave_up), which the record check of the next call and the final pass carry over.
+__device__ __forceinline__ bool refused(const CfrParams& p) { return p.work_counter[1] != 0; }
+__device__ __forceinline__ bool block_refused(const CfrParams& p) {
+    return __syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<const volatile int32_t*>(p.work_counter + 1) != 0) != 0;
+}
+__device__ __forceinline__ int32_t* gave_up(const CfrParams& p) { return p.work_counter + kGaveUp; }
+__device__ __forceinline__ void report_gave_up(const CfrParams& p) {  // one thread of a kernel that has started after the others' end
+    if (blockIdx.x == 0 && threadIdx.x == 0 && *gave_up(p) != 0) atomicMax(p.work_counter + 1, *gave_up(p));
 }
 
 // ---- work lists -------------------------------------------------------------------------------
@@ -110,7 +114,7 @@ __device__ __forceinline__ bool block_stops(const CfrParams& p) {
 constexpr int kBeginThreads = 1024;
 __global__ void __launch_bounds__(kBeginThreads) split_begin_kernel(const CfrParams p, const SplitWork w) {
     __shared__ int s_warp[kBeginThreads / 32];
-    if (block_stops(p)) return;
+    if (block_refused(p)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int run = (p.num_subgames + kBeginThreads - 1) / kBeginThreads;
     const int first = min(tid * run, p.num_subgames), last = min(first + run, p.num_subgames);
@@ -141,7 +145,7 @@ __global__ void __launch_bounds__(kCfrMaxNodes) split_items_kernel(const CfrPara
     const int q = blockIdx.x, i = threadIdx.x;
     if (i == 0) s_before = s_bad = 0;
     if (i <= kSplitMaxDepth) s_depth[i] = 0;
-    if (block_stops(p)) {  // the record check refused the batch
+    if (block_refused(p)) {  // the record check refused the batch
         if (q == 0 && i == 0) w.total[0] = 0;
         return;
     }
@@ -425,7 +429,7 @@ constexpr int kPrepWarps = 4;
 template <int MAXK, int MODE>
 __global__ void __launch_bounds__(32 * kPrepWarps) split_prep_kernel(const CfrParams p, const SplitWork w, int pass) {
     constexpr int kSlices = P2B_HPAD / 64;
-    if (block_stops(p)) return;
+    if (block_refused(p)) return;
     const int q = blockIdx.x / kSlices, warp = threadIdx.x >> 5;
     const int h = (blockIdx.x - q * kSlices) * 64 + (threadIdx.x & 31) * 2;
     const int s = p.queue_order ? p.queue_order[q] : q;
@@ -562,7 +566,7 @@ __device__ __forceinline__ void level_arrive(uint64_t* bar) {  // the whole warp
     if ((threadIdx.x & 31) == 0)
         asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"((unsigned)__cvta_generic_to_shared(bar)) : "memory");
 }
-__device__ __forceinline__ bool level_wait(uint64_t* bar) {  // false: given up
+__device__ __forceinline__ bool level_wait(uint64_t* bar, const int32_t* others) {  // false: given up, the sooner if others have
     for (int i = 0; i < (1 << 20); ++i) {
         unsigned done;
         asm volatile(
@@ -571,6 +575,7 @@ __device__ __forceinline__ bool level_wait(uint64_t* bar) {  // false: given up
             : "r"((unsigned)__cvta_generic_to_shared(bar))
             : "memory");
         if (done) return true;
+        if ((i & 1023) == 1023 && *reinterpret_cast<const volatile int32_t*>(others) != 0) break;
     }
     return false;
 }
@@ -761,7 +766,7 @@ __global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p,
     constexpr int kSlices = P2B_HPAD / kUpRow;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint64_t ready[kUpSlices][kSplitMaxDepth + 1];
-    if (block_stops(p)) return;
+    if (refused(p)) return;
     const int per_subgame = kSlices / slices;
     const int q = blockIdx.x / per_subgame;
     const int s = p.queue_order ? p.queue_order[q] : q;
@@ -817,7 +822,7 @@ __global__ void __launch_bounds__(kUpThreads) split_up_kernel(const CfrParams p,
         const int rows = up_rows(it.n_children);
         float* at = stage + (top ? (ring - rows) * kUpRow : 0);
         if (d + 1 < waited) {  // its children are one level down
-            if (!level_wait(level_ready + d + 1)) atomicMax(p.work_counter + 1, s + 1);
+            if (!level_wait(level_ready + d + 1, gave_up(p))) atomicMax(gave_up(p), s + 1);
             waited = d + 1;
         }
         up_stage_values(w, it, h, at);
@@ -1134,7 +1139,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
     float* sums = reinterpret_cast<float*>(smem + L.sums);
     float* sums_avg = sums + 16;
     const SplitItem& it = *reinterpret_cast<const SplitItem*>(smem + L.item);
-    if (block_stops(p)) return;
+    if (refused(p)) return;
 
     Hands hi;
 #pragma unroll
@@ -1396,8 +1401,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_rows_kernel(const CfrPar
 __global__ void __launch_bounds__(kRowThreads) split_values_kernel(const CfrParams p, const SplitWork w) {
     __shared__ __align__(16) float prod[2][P2B_HPAD];
     __shared__ float sums[2];
-    if (block_stops(p)) return;
+    if (block_refused(p)) return;
     const int tid = threadIdx.x;
+    report_gave_up(p);
     for (int x = blockIdx.x; x < w.total[0]; x += gridDim.x) {
         const SplitItem& it = w.items[x];
         const int leaf0 = p.leaf_begin ? p.leaf_begin[it.subgame] : 0;
@@ -1484,7 +1490,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_best_response_kernel(con
     float* rows = reinterpret_cast<float*>(smem);  // beliefs of the acting player, then a row a child
     double* cs = reinterpret_cast<double*>(smem + (1 + MAXK) * P2B_HPAD * 4);
     double* S = cs + (1 + MAXK) * 52;
-    if (block_stops(p)) return;
+    if (block_refused(p)) return;
     const int tid = threadIdx.x;
     const int q = blockIdx.x / (2 * lanes), rest = blockIdx.x - q * 2 * lanes, deviator = rest / lanes;
     const SplitLevels* lv = w.levels + q;
@@ -1571,7 +1577,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) split_best_response_kernel(con
 __global__ void __launch_bounds__(kRowThreads) split_exploitability_kernel(const CfrParams p, const SplitWork w) {
     __shared__ __align__(16) float prod[4][P2B_HPAD];
     __shared__ float sums[4];
-    if (block_stops(p)) return;
+    if (block_refused(p)) return;
+    report_gave_up(p);
     const int s = blockIdx.x, tid = threadIdx.x;
     const float* cr = p.carry_roots + (long long)s * 4 * P2B_HPAD;
     const float* root = w.rec + (long long)p.subgames[s].node_begin * kRec;

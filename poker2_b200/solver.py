@@ -410,8 +410,9 @@ class SubgameSolver:
 
     def status(self) -> int:
         """0, or 1 + the index of a subgame whose records exceed the kernel's limits, in which
-        case the last solve did nothing.  Reads one word from the device (synchronises)."""
-        return int(self.work_counter[1].item())
+        case the last solve did nothing, or in which a wait on the device ran out.  Reads from the device (synchronises)."""
+        words = self.work_counter.tolist()
+        return words[1] or words[3]
 
     def release(self) -> None:
         """Drops the device buffers (they return to the caching allocator)."""

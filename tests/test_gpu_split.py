@@ -267,3 +267,31 @@ def test_work_lists_take_time_in_proportion_to_the_batch(cuda_device):
 
     few, many = microseconds(3072), microseconds(24576)
     assert 0.0 < many < 12.0 * few, (few, many)  # eight times the subgames; with 64 times the reads it was about 19 times as long
+
+
+def test_a_wait_that_ran_out_is_reported_by_the_whole_solve(cuda_device):
+    """The word a wait leaves when it runs out (put there by hand): every later call of the stepped solve reports it and leaves
+    the outputs alone; the next start pass clears it."""
+    import bench
+    from poker2_b200 import solver, tree as ptree
+
+    boards, ranges, pot, stack = bench.make_inputs(9, 5)
+    trees = ptree.build_trees(ptree.root_states(pot.numpy(), stack.numpy()), [0.5, 1.0], 8, max_raises=2)
+    sv = solver.SteppedSolver(solver.device_layout(trees, boards.numpy()), boards, cuda_device, exploitability=True)
+    rb, scal = solver.pad_rows(ranges.to(cuda_device)).contiguous(), solver.iteration_scalars(4)
+    sv.solve(rb, scal)
+    outputs = (sv.policy_avg, sv.regrets, sv.root_values[..., :1326], sv.exploitability)
+    want = [x.clone() for x in outputs]
+    sv.work_counter[3] = 5
+    for begin, end, phases in ((1, 1, 1), (1, 1, 2), (1, 2, 16), (4, 4, 3), (4, 4, 4)):
+        assert sv.status() == 5
+        sv._step(rb, sv._scalars, 4, 0, begin, end, phases)
+        assert int(sv.work_counter[1]) == 5
+    assert all(torch.equal(a, b) for a, b in zip(want, outputs))
+    sv.solve(rb, scal)
+    assert sv.status() == 0 and all(torch.equal(a, b) for a, b in zip(want, outputs))
+    # a one-call solve begins anew each time
+    one = solver.SubgameSolver(sv.layout, boards, cuda_device)
+    one.work_counter[3] = 5
+    one.solve(rb, scal, check=True)
+    assert torch.equal(one.policy_avg, sv.policy_avg)
