@@ -1444,6 +1444,10 @@ __global__ void __launch_bounds__(kCfrMaxNodes) cfr_validate_kernel(const CfrPar
     int bad = sg.n_nodes < 1 || sg.n_nodes > kCfrMaxNodes || sg.n_internal > p.max_internal || sg.node_begin < 0 ||
               (p.rows > 0 && (long long)sg.node_begin + sg.n_nodes > p.rows) ||
               (p.queue_order && (unsigned)p.queue_order[s] >= (unsigned)p.num_subgames);
+    // What the kernels have room for: the general kernel's two builds go by their own width, the others' shared memory and work
+    // rows by the largest child count that the caller has named, and by no node being without a parent.
+    const int most_children = p.exact_sizes ? p.max_children : p.max_children <= kIterMaxChildren ? kIterMaxChildren : kCfrMaxChildren;
+    if (p.exact_sizes && (long long)sg.n_nodes > (long long)sg.n_internal * most_children + 1) bad = 1;
     if (!bad && i < sg.n_nodes) {
         const NodeRecPacked raw = p.nodes[sg.node_begin + i];
         const NodeRec nd = unpack_node(raw);
@@ -1451,7 +1455,7 @@ __global__ void __launch_bounds__(kCfrMaxNodes) cfr_validate_kernel(const CfrPar
         if (nd.kind > kModelLeaf || (nd.kind == kShowdownLeaf && (sg.table_index < 0 || p.tables == nullptr))) bad = 1;
         if (i == 0 && nd.kind != kInternal) bad = 1;
         if (nd.kind == kInternal &&
-            (nd.n_children < 1 || nd.n_children > kCfrMaxChildren || nd.first_child <= i ||
+            (nd.n_children < 1 || nd.n_children > most_children || nd.first_child <= i ||
              nd.first_child + nd.n_children > sg.n_nodes || nd.internal_idx >= p.max_internal || nd.to_act > 1))
             bad = 1;
         // a leaf valued by the caller's model must own a slot of the leaf arrays
@@ -1710,8 +1714,11 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
     // leaves all terminal, all passes in this call: the iteration kernel applies (a start policy only concerns
     // the start pass, a warm start of type `model` is a kernel of its own between that pass and the iterations)
     const bool plain = !p.stepped && !p.leaf_beliefs && !p.leaf_values && !p.cfr_avg && !p.linear;
-    if (p.stepped && p.phases != 8 && split_applies(p, max_children, p.scratch_floats))
+    p.max_children = max_children;
+    if (p.stepped && p.phases != 8 && split_applies(p, max_children, p.scratch_floats)) {
+        p.exact_sizes = 1;
         return launch_stepped(p, num_blocks, max_children, stream);
+    }
     const long long blocks = block_work_floats(p.max_internal, max_children, num_blocks), per_block = blocks / num_blocks;
     const long long carry = carry_floats(p.num_subgames, p.rows);
     const bool room = !p.stepped && p.rows > 0 && p.scratch_floats >= blocks + carry;  // for rows that launches hand on
@@ -1719,6 +1726,7 @@ int launch_cfr_solve(const CfrParams& params, int num_blocks, int max_children, 
     const bool large = maybe_large(p.max_internal, max_children);
     const bool lean = plain && room && max_children <= kIterMaxChildren &&
                       lean_preferred(p.num_subgames, p.max_internal, max_children, split);
+    p.exact_sizes = split || lean;
     if (split && !lean) {
         IterTiming* timing = iter_timing_of_current_device();
         const bool timed = timing && timing->enabled;
@@ -1882,6 +1890,7 @@ int launch_cfr_solve_static(const CfrParams& params, int max_children, cudaStrea
     if (blocks > sm_count()) blocks = sm_count();
     if (blocks > params.num_subgames) blocks = params.num_subgames;
     CfrParams p = params;
+    p.max_children = max_children;
     p.combos = sp.combos;
     p.scratch = sp.scratch;
     p.scratch_stride = per_block;

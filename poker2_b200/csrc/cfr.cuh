@@ -109,6 +109,8 @@ struct CfrParams {
     long long scratch_stride;    // floats per block
     long long scratch_floats;    // size of the whole scratch area
     int32_t max_internal;        // largest n_internal over the batch
+    int32_t max_children;        // of a node, over the batch
+    int32_t exact_sizes;         // 1: work space is sized by max_children, so the record check holds every subgame to it
     const IterScalars* scalars;  // [iterations]
     int32_t iterations;
     int32_t cfr_plus;

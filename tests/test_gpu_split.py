@@ -295,3 +295,39 @@ def test_a_wait_that_ran_out_is_reported_by_the_whole_solve(cuda_device):
     one.work_counter[3] = 5
     one.solve(rb, scal, check=True)
     assert torch.equal(one.policy_avg, sv.policy_avg)
+
+
+@pytest.mark.parametrize("spoil", ["actions", "orphans"])
+def test_trees_beyond_the_sizes_named_are_refused(cuda_device, spoil):
+    """Work space sized by the largest child count holds no node with more children and no node without a parent: the record
+    check refuses such a subgame wherever the sizes matter, and the general kernel, where they do not, solves it."""
+    import bench
+    from poker2_b200 import solver, tree as ptree
+
+    boards, ranges, pot, stack = bench.make_inputs(6, 8)
+    trees = ptree.build_trees(ptree.root_states(pot.numpy(), stack.numpy()), [0.5, 1.0], 8, max_raises=2)
+    layout = solver.device_layout(trees, boards.numpy())
+    rb, scal = solver.pad_rows(ranges.to(cuda_device)).contiguous(), solver.iteration_scalars(3)
+    sound = solver.SubgameSolver(layout, boards, cuda_device)
+    sound.solve(rb, scal, check=True)
+    assert layout.max_children == 5
+    if spoil == "actions":
+        layout.max_children = 4
+    else:  # leaves behind the last subgame's own that no node has for a child
+        extra = 310 - int(layout.subgames[5]["n_nodes"])
+        leaf = layout.nodes[solver.node_kind(layout.nodes) == ptree.KIND_FOLD][-1]
+        layout.nodes = np.concatenate([layout.nodes, np.repeat(leaf, extra)])
+        layout.subgames[5]["n_nodes"] += extra
+        assert 310 > int(layout.subgames[5]["n_internal"]) * layout.max_children + 1
+    for policy in ("auto", "lean"):
+        solver.set_path_policy(policy)
+        for cls in (solver.SubgameSolver, solver.SteppedSolver):
+            sv = cls(layout, boards, cuda_device)
+            sv.root_values.fill_(-7.0)
+            sv.regrets.fill_(-7.0)
+            sv.solve(rb, scal)
+            assert sv.status() > 0 and bool((sv.root_values == -7.0).all()) and bool((sv.regrets == -7.0).all())
+    general = solver.SubgameSolver(layout, boards, cuda_device, lean_iterations=False)
+    general.solve(rb, scal, check=True)
+    rows = sound.regrets.shape[0]
+    assert torch.equal(general.regrets[:rows], sound.regrets) and torch.equal(general.root_values, sound.root_values)
