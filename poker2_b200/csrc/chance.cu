@@ -241,7 +241,8 @@ __global__ void __launch_bounds__(kPairThreads, 4) chance_expand_features_kernel
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
                 double left = all[p] - cs[p][card];
-                if (left < 1e-6 * all[p]) {  // the subtraction has cancelled: add up what is left (uniform over the block)
+                // the subtraction has cancelled, or what the card takes is no number: add up what is left (uniform over the block)
+                if (!(left >= 1e-6 * all[p])) {
                     left = 0.0;
 #pragma unroll
                     for (int i = 0; i < 2 * kPairs; ++i) left += held[i] ? 0.0 : (double)v[p][i];

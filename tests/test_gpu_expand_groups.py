@@ -29,3 +29,22 @@ def test_features_equal_the_expanded_beliefs(cuda_device, roots, kind):
     assert torch.equal(x[:, :2652], post.reshape(-1, 2652).to(torch.bfloat16))
     assert torch.equal(x[:, 2704:2707], ctx[lookup].to(torch.bfloat16)) and not x[:, 2707:].any()
     assert torch.equal(x[:, 2652:2704].float().sum(dim=1), torch.full((x.shape[0],), 5.0, device=cuda_device))
+
+
+@pytest.mark.parametrize("odd", [float("nan"), float("inf")])
+def test_features_where_a_card_takes_what_is_no_number(cuda_device, odd):
+    """One hand's belief is NaN or infinite: the samples whose card holds that hand are what the unfused expansion, which adds
+    up what a card leaves, gives; so are the others."""
+    from poker2_b200 import chance
+
+    g = torch.Generator(device=cuda_device).manual_seed(3)
+    boards = torch.tensor([[0, 5, 17, 30, -1]], device=cuda_device)
+    pre = torch.rand(1, 2, 1326, device=cuda_device, generator=g)
+    pre[0, 1, 1325] = odd  # cards 50 and 51
+    ctx = torch.rand(1, 3, device=cuda_device, generator=g)
+    off = chance.sample_offsets_of(boards)
+    got = chance.expand_features_bf16(pre, boards, off, 48, ctx, 2720)[:, :2652].view(48, 2, 1326)
+    want, _, samples = chance.expand_next_card(pre, boards)
+    takes = (samples == 50).any(1) | (samples == 51).any(1)
+    assert int(takes.sum()) == 2 and bool(want[takes].isfinite().all())
+    torch.testing.assert_close(got.float(), want.to(torch.bfloat16).float(), rtol=0.0, atol=0.0, equal_nan=True)
