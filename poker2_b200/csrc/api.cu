@@ -157,7 +157,8 @@ int p2b_cfr_solve(const void* subgames, const void* nodes, int32_t num_subgames,
     if (num_subgames == 0) return P2B_OK;
     P2B_REQUIRE(subgames && nodes && root_beliefs && regrets && policy_avg && root_values && scratch && work_counter,
                 "null pointer");
-    P2B_REQUIRE(iterations == 0 || scalars, "null scalars");
+    P2B_REQUIRE(iterations >= 1, "at least one iteration is required");
+    P2B_REQUIRE(scalars, "null scalars");
     P2B_REQUIRE(max_internal >= 1, "max_internal must be positive");
     P2B_REQUIRE(!exploitability || values_avg, "exploitability needs values_avg");
     P2B_REQUIRE(flags >= 0 && flags <= 31 && !(flags & 8),
@@ -331,6 +332,7 @@ int p2b_cfr_solve_noalloc(const void* subgames, const void* nodes, int32_t num_s
                           int32_t iterations, int32_t flags, int32_t init_depth, void* stream) {
     P2B_REQUIRE(num_subgames >= 0 && iterations >= 0 && rows >= 0, "negative count");
     if (num_subgames == 0) return P2B_OK;
+    P2B_REQUIRE(iterations >= 1, "at least one iteration is required");
     P2B_REQUIRE(subgames && nodes && root_beliefs && regrets && policy_avg && root_values && scalars, "null pointer");
     P2B_REQUIRE(max_internal >= 1, "max_internal must be positive");
     P2B_REQUIRE(!exploitability || values_avg, "exploitability needs values_avg");

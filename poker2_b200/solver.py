@@ -447,7 +447,7 @@ class SubgameSolver:
             start_rows = pad_rows(start_policy.to(torch.float32)[order]).to(self.device).contiguous()
         self._start_rows = start_rows  # alive until the kernels have run
         iterations = int(scalars.shape[0])
-        sc = torch.from_numpy(scalars.view(np.uint8).reshape(max(iterations, 0), 32).copy()).to(self.device)
+        sc = torch.from_numpy(scalars.view(np.uint8).reshape(iterations, 32).copy()).to(self.device)
         self._scalars = sc
         p = _lib.ptr
         with _lib.on(self.device):
@@ -457,7 +457,7 @@ class SubgameSolver:
                 p(self.regrets), p(self.weight_sums), p(self.policy_avg), p(self.policy), p(self.root_values),
                 p(self.values_avg), p(self.beliefs_avg), p(self.exploitability), p(self.br_values), p(self.scratch),
                 self.scratch.numel(),
-                p(sc) if iterations else None, iterations,
+                p(sc), iterations,
                 solve_flags(cfr_plus, enforce_zero_sum, cfr_avg, linear=scalars_are_linear(scalars)),
                 self.layout.tree_depth, p(self.work_counter),
                 self.num_blocks, p(self.sample_pass), p(self.policy_sample), p(self.beliefs_last),

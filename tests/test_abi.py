@@ -87,3 +87,28 @@ def test_whole_step_entry_points_reject_bad_arguments_without_a_gpu():
     reach = good["p2b_steps_reach"]
     for beliefs in (p, p + 4, p - 4):
         assert refused("p2b_steps_reach", reach[:8] + [beliefs] + reach[9:]), "overlap"
+
+
+def test_solves_without_iterations_are_refused_without_a_gpu():
+    """No pass of a solve can go without a table of iterations: zero iterations are refused before anything is launched (an empty
+    batch has nothing to do whatever it says)."""
+    from poker2_b200 import _lib, build
+
+    build.build()
+    handle = _lib.lib()
+    area = (ctypes.c_char * 4096)()
+    p = (ctypes.addressof(area) + 63) // 64 * 64
+
+    def solve(subgames, iterations, scalars):
+        return handle.p2b_cfr_solve(p, p, subgames, 8, 5, 2, p, p, p, p, p, p, p, None, None, None, None, p, 1 << 30, scalars,
+                                    iterations, 0, 2, p, 1, None, None, None, None, None, 0.0, None)
+
+    def noalloc(subgames, iterations, scalars):
+        return handle.p2b_cfr_solve_noalloc(p, p, subgames, 8, 5, 2, p, p, p, p, p, p, p, None, None, None, None, scalars,
+                                            iterations, 0, 2, None)
+
+    for call in (solve, noalloc):
+        for scalars in (None, p):
+            assert call(1, 0, scalars) == -1 and b"at least one iteration" in handle.p2b_last_error()
+            assert call(0, 0, scalars) == 0
+        assert call(1, 1, None) == -1 and b"null" in handle.p2b_last_error()
