@@ -1,8 +1,8 @@
 """Subgames with more nodes than the lean iteration kernel holds (160): uncapped river trees of deep stacks
 (up to 261 nodes) next to small ones in one batch, and the largest tree the production search settings can
 produce (depth 5 over {fold, call, half pot, pot, all-in}: 273 nodes) with leaves valued by a stand-in model.
-The one-call solve sends the small subgames through the lean kernel and the large ones through the general
-kernel; results must not depend on that."""
+With the lean policy, which the suite sets, the one-call solve sends the small subgames through the lean kernel and
+the large ones through the general kernel; results must not depend on that."""
 import numpy as np
 import pytest
 import torch
@@ -132,8 +132,9 @@ DEFAULT_BINS = [0.5, 0.75, 1.0, 1.5, 2.0]  # EnvConfig.bet_bins of the upstream 
 
 def test_eight_actions_per_node_on_terminal_trees(cuda_device):
     """River subgames over the dataclass-default bet sizes (fold, call, five bets, all-in) with a raise cap, so
-    that every leaf is terminal: nodes with 6, 7 and 8 children, trees of 59 ... 207 nodes in one batch.  The
-    one-call solve keeps such a batch in the general kernel (its wide build); equal bits with the oracle."""
+    that every leaf is terminal: nodes with 6, 7 and 8 children, trees of 59 ... 207 nodes in one batch.  Such
+    a batch runs in the split kernels, with the minimal scratch area in the general kernel's wide build; equal bits with the
+    oracle."""
     from oracle import cards, cfr as ocfr
     from poker2_b200 import solver, tree as ptree
 
@@ -147,7 +148,7 @@ def test_eight_actions_per_node_on_terminal_trees(cuda_device):
     assert np.bincount(trees.root_of).tolist() == [159, 207, 59, 117] and int(trees.child_count.max()) == 8
     o = ocfr.SubgameOracle(trees.oracle_dict(boards), ranges, iterations=T).solve()
     ex, _ = o.exploitability()
-    for kw in ({}, dict(device_tree=True)):
+    for kw in ({}, dict(device_tree=True), dict(lean_iterations=False)):
         res, _ = solver.solve_subgames(boards, ranges, pot, stack, iterations=T, bet_bins=DEFAULT_BINS, max_depth=12,
                                        max_raises=2, exploitability=True, device=cuda_device, **kw)
         for key, got, want in [("policy_avg", res.level_major(res.policy_avg)[n:], o.policy_avg[n:]),

@@ -253,16 +253,17 @@ def test_model_br_warm_start_matches_upstream(cuda_device, golden_dir):
         _close(f"{tag} seeded regrets", seeded[n:], torch.from_numpy(z[f"{tag}_seeded_regrets"])[n:])
 
 
-def test_linear_cfr_matches_upstream(cuda_device, golden_dir):
-    """cfr_type = linear with the CFR+ clamp: alternating updates, mixing weights (t, 2); every pass in the
-    general kernel.  Through the one-call solve and through the allocation-free entry."""
+@pytest.mark.parametrize("full_area", [True, False])
+def test_linear_cfr_matches_upstream(cuda_device, golden_dir, full_area):
+    """cfr_type = linear with the CFR+ clamp: alternating updates, mixing weights (t, 2).  Through the one-call solve, in the
+    split kernels and, with the minimal scratch area, in the general kernel."""
     from poker2_b200 import solver
 
     z = np.load(os.path.join(golden_dir, "cfr_linear_cap2_t13.npz"))
     res, trees = solver.solve_subgames(z["boards"].astype(np.int64), torch.from_numpy(z["ranges"]), z["pot"], z["stack"],
                                        iterations=int(z["iterations"]), max_depth=int(z["max_depth"]),
                                        max_raises=int(z["cap"]), cfr_type="linear", cfr_plus=True, exploitability=True,
-                                       device=cuda_device)
+                                       device=cuda_device, lean_iterations=full_area)
     assert trees.total_nodes == int(z["total_nodes"])
     n = trees.num_roots
     for name, got in [("regrets", res.regrets), ("weight_sums", res.weight_sums), ("policy_avg", res.policy_avg)]:
@@ -298,7 +299,7 @@ def test_production_search_block_through_the_one_call_solve(cuda_device, golden_
         sv.set_sampling_schedule(torch.from_numpy(z["t_sample"]), warm_start_iterations=ws)
         res = sv.solve(rb, scal, check=True, **args) if lean else None
         if not lean:
-            # the general kernel needs the larger scratch area for the hand-over between its two launches
+            # a warm start is more than one launch in any kernel: the minimal area has no room for the rows handed on
             with pytest.raises(RuntimeError):
                 sv.solve(rb, scal, **args)
             continue

@@ -61,7 +61,7 @@ def test_options(cuda_device, opts):
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("B", [160, 600])  # two warps a slice; beyond the lean kernel's 8 actions limit
+@pytest.mark.parametrize("B", [160, 600])  # two warps a slice; more actions than the lean kernel takes
 def test_wide_batches(cuda_device, B):
     for a, b in zip(*_both(cuda_device, B, bins=(0.5, 0.75, 1.0, 1.5, 2.0), cap=1, iterations=2)[1]):
         assert torch.equal(a, b)
