@@ -81,9 +81,12 @@ int p2b_showdown_ev_sorted(const float* b_sorted, const int32_t* c1_sorted, cons
 
 /* ---- fused subgame CFR (src/p2/search/cfr_evaluator.py:1497-1528 evaluate_cfr with
  * cfr_iteration :1331-1381, on the ragged tree of sparse_cfr_evaluator.py:141-306) ----
- * One persistent kernel runs the start pass, `iterations` DCFR iterations and the final
- * average-policy evaluation for `num_subgames` independent subgames whose leaves are all
- * terminal (fold or showdown).  Rows are 1344 floats (1326 combos + 18 padding floats) so
+ * The start pass, `iterations` >= 1 DCFR iterations and the final average-policy evaluation for
+ * `num_subgames` independent subgames whose leaves are all terminal (fold or showdown).  Three sets
+ * of kernels can run them, with the same results bit for bit: the general kernel, in which a block
+ * walks one subgame after another through a whole solve; the lean kernel, which does so for the
+ * iteration passes alone; and the split kernels, which make a pass one kernel over the nodes of the
+ * whole batch and one over its hands.  Rows are 1344 floats (1326 combos + 18 padding floats) so
  * that every row is 16-byte aligned; all row arrays must be 16-byte aligned.
  *
  *  subgames   [num_subgames] 32-byte records {int32 node_begin, n_nodes, n_internal,
@@ -92,10 +95,10 @@ int p2b_showdown_ev_sorted(const float* b_sorted, const int32_t* c1_sorted, cons
  *             (bits 0-1 kind: 0 internal, 1 fold leaf, 2 showdown leaf, 3 other leaf; bit 7 the
  *             player to act; the other bits zero), depth, internal_idx; float v0, v1},
  *             breadth-first per subgame, local indices.  A subgame has at most 320 nodes (a
- *             depth-5 tree over {fold, call, two bet sizes, all-in} has at most 273); subgames of
- *             up to 160 nodes run their iteration passes in the lean kernel, larger ones in the
- *             general kernel, within the same call; max_children <= 8, and a batch with more than
- *             6 children at some node runs every pass in the general kernel
+ *             depth-5 tree over {fold, call, two bet sizes, all-in} has at most 273) and
+ *             max_children <= 8 actions per node; the lean kernel takes up to 160 nodes (larger ones of
+ *             its batch run their iteration passes in the general kernel, within the same call) and
+ *             batches of up to 6 actions
  *  tables     showdown tables from p2b_rank_hands, indexed by table_index
  *  root_beliefs [num_subgames,2,1344] input ranges
  *  regrets, weight_sums (may be NULL), policy_avg, policy (may be NULL): [rows,1344] out
@@ -122,11 +125,10 @@ int p2b_showdown_ev_sorted(const float* b_sorted, const int32_t* c1_sorted, cons
  *             bit 2: `cfr_avg` upstream (cfr_evaluator.py:1029, :1133): in the iteration passes the showdown
  *             values, the regret weights and the leaf_beliefs handed to the caller's model are taken at the
  *             beliefs under the average policy instead of the current one (the de-averaging of the model's
- *             values, :997-1018, is the caller's part of set_leaf_values); such a solve keeps every pass in
- *             the general kernel;
+ *             values, :997-1018, is the caller's part of set_leaf_values); not in the lean kernel;
  *             bit 4: linear CFR (alternating updates, cfr_evaluator.py:1348-1349): the `do_mix` word of every
  *             scalars record then carries, in bits 1-2, 1 + the player whose actions get no regret at that
- *             iteration; such a solve keeps every pass in the general kernel;
+ *             iteration; not in the lean kernel;
  *             bit 3 (p2b_cfr_step only): the bottom-up sweep of the start pass and of every iteration pass stores
  *             the values of every node in values_avg and (iteration passes) the beliefs under the average
  *             policy, at inner nodes and at the leaves a model values, in beliefs_avg -- the inputs of the
@@ -140,7 +142,8 @@ int p2b_showdown_ev_sorted(const float* b_sorted, const int32_t* c1_sorted, cons
  *             every subgame's records with the solver's limits (1..320 nodes per subgame, all
  *             inside the `rows` rows, 1..8 children per internal node, children stored after their
  *             parent and inside the subgame, internal_idx < max_internal, unused record bits zero, root
- *             internal, a table for every showdown leaf, a slot for every model leaf).
+ *             internal, a table for every showdown leaf, a slot for every model leaf; for the lean and the
+ *             split kernels at most max_children children and no node without a parent).
  *             On a violation status = 1 + the index of an offending subgame and NOTHING is
  *             solved (outputs untouched); otherwise status stays 0
  *  num_blocks 0 = one block per SM
@@ -207,17 +210,16 @@ int p2b_cfr_iteration_ms(float* ms);
  * player who acted - that player's value of the parent under the start policy); the caller multiplies by
  * warm_start_iterations x multiplier, sets the weight sums to that factor and goes on with pass 0.
  * 16 (with pass_end = pass_begin + 1) joins the bottom-up sweep of pass_begin and the top-down sweep of the
- * next pass in one launch: nothing happens on the host between them unless the caller wants it to, and a
- * block then visits a subgame once per pass instead of twice (same results; no faster in our measurements,
- * the time of a pass is the walk over the subgames).
+ * next pass in one call, for callers that have nothing to do between them: the work lists and the current
+ * policy need not be derived anew (0.09 of 1.4 ms a pass on 192 flop subgames of 77 nodes; same results).
  * The caller's loop is: for every pass { step(pass, 1); leaf_values = model(leaf_beliefs);
  * step(pass, 2); }, or step(-1, 1); for every pass { leaf_values = model(leaf_beliefs);
  * pass == iterations ? step(pass, 2) : step(pass..pass+1, 16); }.  Arrays as in p2b_cfr_solve, plus state
  * carried between calls:
  *  scratch      at least p2b_cfr_scratch_floats(max_internal, 1) * num_subgames floats (one set of
  *               work rows per subgame instead of per block).  With p2b_cfr_step_scratch_floats(max_internal,
- *               num_subgames, rows) floats the iteration passes run in the split kernels, which spread a
- *               subgame over the chip; same results, bit for bit.  All calls of a solve pass the same area
+ *               num_subgames, rows) floats the passes run in the split kernels, which spread a subgame
+ *               over the chip, else in the general kernel; same results, bit for bit.  All calls of a solve pass the same area
  *  carry_sums   [rows,2] floats ([2,rows,2] with flags bit 2 or 3), carry_roots [num_subgames,4,1344] floats (opaque)
  *  leaf_begin   [num_subgames] int32: first leaf slot of each subgame; a node of kind 3 uses
  *               slot leaf_begin[subgame] + its internal_idx field; leaf_slots = number of slots
@@ -225,9 +227,9 @@ int p2b_cfr_iteration_ms(float* ms);
  *  leaf_values  [slots,2,1344] in (bottom-up sweep): both players' values there, in the units
  *               of the other leaf values (chips / scale)
  * With leaf_beliefs == NULL / leaf_values == NULL such leaves are skipped / valued 0.
- * queue_order (may be NULL) as in p2b_cfr_solve: the order in which the blocks take the subgames; the
- * largest trees first shortens a launch over a ragged batch (192 subgames of 9..237 nodes: 35.8 against
- * 41.8 ms for 24 iterations). */
+ * queue_order (may be NULL) as in p2b_cfr_solve: the order in which the blocks take the subgames; in the
+ * general kernel the largest trees first shortens a launch over a ragged batch (192 subgames of 9..237
+ * nodes: 35.8 against 41.8 ms for 24 iterations). */
 int p2b_cfr_step(const void* subgames, const void* nodes, int32_t num_subgames, int64_t rows, int32_t max_children,
                  int32_t max_internal, const unsigned char* tables, const float* root_beliefs,
                  float* regrets, float* weight_sums, float* policy_avg, float* policy,

@@ -81,9 +81,9 @@ struct IterScalars {  // 32 bytes
 
 constexpr int kCfrThreads = 672;  // 672 threads x 2 hands cover the 1344-float padded row
 constexpr int kCfrMaxNodes = 320;   // nodes of one subgame (a depth-5 tree over {fold, call, two bets, all-in} has at most 273)
-constexpr int kIterMaxNodes = 160;  // what the lean iteration kernel holds; larger subgames stay in the general kernel
+constexpr int kIterMaxNodes = 160;  // what the lean iteration kernel holds; the general kernel runs the larger ones of its batches
 constexpr int kCfrMaxChildren = 8;   // actions per node (fold, call, five bet sizes, all-in: the upstream dataclass default)
-constexpr int kIterMaxChildren = 6;  // the lean iteration kernel's staging rows; batches with more stay in the general kernel
+constexpr int kIterMaxChildren = 6;  // the lean iteration kernel's staging rows; batches with more do not come to it
 
 // Word of work_counter: 1 + a subgame in which a wait on the device ran out since the start pass, 0: none has.
 constexpr int kGaveUp = 3;
@@ -118,7 +118,7 @@ struct CfrParams {
     int32_t cfr_avg;             // iteration passes: showdown values, regret weights and the beliefs handed to the
                                  // caller's model come from the beliefs under the average policy (:1029, :1133)
     int32_t linear;              // linear CFR (alternating updates, cfr_evaluator.py:1348-1349): the scalars carry the
-                                 // skipped player per iteration; every pass stays in the general kernel
+                                 // skipped player per iteration; not in the lean iteration kernel
     int32_t iter_values;         // start and iteration passes store the values of every node in values_avg and (iteration
                                  // passes) the beliefs under the average policy in beliefs_avg: what a caller mixes into
                                  // running average values (`update_average_values`, cfr_evaluator.py:1260-1274)

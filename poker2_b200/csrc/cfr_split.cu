@@ -16,12 +16,13 @@
 //
 // Arithmetic and results are those of cfr.cu, bit for bit: same operations in the same order, also in the fp64 sums.
 //
-// Measured on a B200, a pass in the general kernel / here: one subgame of 57 nodes 0.32 / 0.033 ms, 37 of 96 nodes
-// 1.15 / 0.16 ms, 192 flop subgames of 77 nodes (largest 271) 1.4 / 0.39 ms.  The row kernel takes 6.3 us an SM and
-// node with two blocks resident; shared-memory wavefronts (0.65 of their peak, mostly the gathers of the per-card sums and
-// of the showdown tables) and the barriers between its phases bound it, with half of the issue slots used.  The up kernel
-// is bound by memory at large batches (2.55 ms on 4096 subgames of 54 nodes, 0.9 of the copy bandwidth over the 15 GB it
-// moves) and by the latency of a warp's walk at small ones.
+// Measured on a B200, a pass in the general kernel / here (the iteration passes by the library's timer, over their number):
+// one subgame of 57 nodes 0.32 / 0.034 ms, 37 of 96 nodes 1.15 / 0.155 ms, 192 flop subgames of 77 nodes (largest 271)
+// 1.4 / 0.39 ms.  The row kernel takes 6.3 us an SM and node with two blocks resident; shared-memory wavefronts (0.59 of
+// their peak on 192 river subgames, mostly the gathers of the per-card sums and of the showdown tables) and the barriers
+// between its phases bound it, with half of the issue slots used.  The up kernel is bound by memory at large batches
+// (2.55 ms on 4096 subgames of 54 nodes, 0.9 of the copy bandwidth over the 15 GB it moves) and by the latency of a warp's walk at
+// small ones (DRAM at 0.44 of its peak on 192 river subgames).
 #include "cfr_split.cuh"
 
 #include "cfr_dev.cuh"

@@ -7,8 +7,9 @@ namespace p2b {
 
 constexpr int kSplitMaxDepth = 16;  // levels of a tree below its root; deeper trees stay in the general kernel
 
-// Floats of work space the passes need: per row the current policy, the opponent-conditioned policy, the regret
-// weights and the values of both players, then one record per internal node and the level bounds per subgame.
+// Floats of work space the passes need: seven rows a node (the current policy, the policy as the other player sees it, the
+// regret weights, the values of both players, the acting player's reach under the current and the old average
+// policy), one record per internal node and the level bounds per subgame.
 long long split_scratch_floats(int num_subgames, long long rows);
 // True if the passes of such a batch can run here: the work space fits and no tree is too deep or too wide.
 bool split_applies(const CfrParams& p, int max_children, long long scratch_floats);

@@ -131,7 +131,7 @@ class SubgameEvaluator:
         kw = dict(exploitability=True, keep_node_values=True, sampling=True)
         # pass by pass only where something happens between the passes: leaves valued by the network, running
         # value averages, the best-response pass of a `model_br` warm start; a warm start of type `model` and a
-        # start policy fit the one-call solve, whose iteration passes run in the lean kernel
+        # start policy fit the one-call solve
         self.stepped = (bool(self.layout.num_model_leaves) or self.running_values or self.policy_delta_stats
                         or (self.warm_start_iterations > 0 and self.warm_start_type == "model_br"))
         if self.layout.num_model_leaves:

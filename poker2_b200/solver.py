@@ -1,5 +1,5 @@
 """Batched subgame solving on the GPU: host-side preparation and the call into the fused
-CFR kernel (`p2b_cfr_solve`).
+CFR kernels (`p2b_cfr_solve`).
 
 `solve_subgames` does, for a batch of independent river subgames, what the upstream
 `initialize_subgame` + `evaluate_cfr` do (p2/search/cfr_evaluator.py:770-828, 1497-1528,
@@ -19,8 +19,8 @@ from .showdown import BoardTables
 
 HPAD = 1344
 NUM_HANDS = 1326
-MAX_NODES = 320  # nodes of one subgame (general kernel); the lean iteration kernel takes those of up to 160
-MAX_CHILDREN = 8  # actions per node (general kernel); batches of up to 6 run their iteration passes in the lean kernel
+MAX_NODES = 320  # nodes of one subgame; the lean iteration kernel takes those of up to 160
+MAX_CHILDREN = 8  # actions per node; the lean iteration kernel takes batches of up to 6
 
 NODE_DTYPE = np.dtype([("parent", "<u2"), ("first_child", "<u2"), ("n_children", "u1"), ("kind_act", "u1"),
                        ("depth", "u1"), ("internal_idx", "u1"), ("v0", "<f4"), ("v1", "<f4")])
@@ -32,8 +32,8 @@ assert NODE_DTYPE.itemsize == 16 and SUBGAME_DTYPE.itemsize == 32 and SCALAR_DTY
 
 
 def set_path_policy(policy: str) -> str:
-    """Which kernel runs the iteration passes of one-call solves in this process: "auto" (default: the lean
-    kernel except for batches so small that the general kernel is quicker, see `p2b_cfr_path_policy`) or "lean"
+    """Which kernels run the iteration passes of one-call solves in this process: "auto" (default: the lean
+    kernel from two subgames an SM on, else the split kernels, see `p2b_cfr_path_policy`) or "lean"
     (the lean kernel whenever it applies).  Returns the previous setting; results do not depend on it."""
     names = ("auto", "lean")
     if policy not in names:
@@ -236,7 +236,7 @@ def solve_flags(cfr_plus: bool, enforce_zero_sum: bool, cfr_avg: bool = False, i
     """The `flags` argument of the solve entry points: bit 0 = CFR+ clamp, bit 1 = zero-sum value outputs,
     bit 2 = leaf values and regret weights at the beliefs under the average policy (`cfr_avg` upstream),
     bit 3 (stepped solves) = keep the node values and average beliefs of every pass, bit 4 = linear CFR (the
-    scalars carry the skipped player; every pass in the general kernel)."""
+    scalars carry the skipped player; not in the lean kernel)."""
     return (int(bool(cfr_plus)) | (int(bool(enforce_zero_sum)) << 1) | (int(bool(cfr_avg)) << 2)
             | (int(bool(iter_values)) << 3) | (int(bool(linear)) << 4))
 
@@ -424,14 +424,12 @@ class SubgameSolver:
               enforce_zero_sum: bool = False, cfr_avg: bool = False, check: bool = False,
               start_policy: torch.Tensor | None = None, warm_start_iterations: int = 0,
               warm_start_multiplier: float = 1.0, warm_start_scalars: np.ndarray | None = None) -> SolveResult:
-        """root_beliefs: [B,2,1344] fp32 on the device (padded).  Enqueues the solve (one to three
-        kernels, one more for a warm start).  start_policy [M,1326] in the upstream node order (the policy head's
+        """root_beliefs: [B,2,1344] fp32 on the device (padded).  Enqueues the solve.  start_policy [M,1326] in the upstream node order (the policy head's
         soft-max; None = uniform); with warm_start_iterations = w > 0 the regrets are seeded from it after the
         start pass (`warm_start` of type `model`, cfr_evaluator.py:887-926) and iterations w..T-1 follow, as in
         `SteppedSolver.solve` (same meaning of `scalars` and `warm_start_scalars`).  enforce_zero_sum: shift the value outputs to zero sum, as upstream does when
         `model.enforce_zero_sum` is set (cfr_evaluator.py:957-980, 1289-1292).  cfr_avg: showdown values
-        and regret weights at the beliefs under the average policy (:1029, :1133; one launch, general
-        kernel).  check: read the status word afterwards (synchronises) and raise if the record check
+        and regret weights at the beliefs under the average policy (:1029, :1133).  check: read the status word afterwards (synchronises) and raise if the record check
         refused the batch."""
         assert root_beliefs.shape == (self.B, 2, HPAD) and root_beliefs.dtype == torch.float32
         assert root_beliefs.is_contiguous() and root_beliefs.device == self.device
@@ -486,8 +484,8 @@ def _writes_in_place(leaf_fn) -> bool:
 
 class SteppedSolver(SubgameSolver):
     """Solves subgames whose non-terminal leaves are valued by a caller-side model
-    (`set_leaf_values`, p2/search/cfr_evaluator.py:1025-1047): every pass is two launches
-    (`p2b_cfr_step`) with the model call in between.
+    (`set_leaf_values`, p2/search/cfr_evaluator.py:1025-1047): the model is called between the two
+    sweeps of every pass (`p2b_cfr_step`).
 
     `leaf_fn(beliefs)` receives the beliefs at the model leaves, [slots,2,1344] fp32 on the
     device (columns 1326.. are padding; slot order = `layout.model_rows`), and returns their

@@ -8,7 +8,7 @@ tests and tools call directly: `initialize_policy_and_beliefs`, `set_leaf_values
 `poker2_b200.fused_cfr` and `poker2_b200.showdown` the way the upstream fused evaluator composes its
 Triton kernels (p2/search/fused_sparse_cfr_evaluator.py:144-527), so the state can be inspected
 between any two steps.  It is the slow, transparent form: a whole solve belongs in
-`solver.SubgameSolver` (three launches), which ends in the same state.  `cfr_iteration` and the steps it is made of run in
+`solver.SubgameSolver`, which ends in the same state.  `cfr_iteration` and the steps it is made of run in
 kernels that do a whole step each (`p2b_steps_*`); the start and `update_policy` by itself go through the one-for-one ones.
 
 Covered: uniform start, `cfr_type` standard / discounted / discounted_plus with optional CFR+ clamp,
