@@ -12,6 +12,8 @@ torch / cuBLAS.
 """
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import torch
 
@@ -169,13 +171,15 @@ class DirectLeafEvaluator:
         # a bf16 `ValueMLP` reads rows that the feature kernel writes: the columns that no pass changes (board
         # one-hot, context, padding) are filled in once
         self._rows = None
-        if type(model) is ValueMLP and model.dtype == torch.bfloat16 and self.boards.shape[0] > 0:
+        self._rows_lock = threading.RLock()
+        if type(model) is ValueMLP and model.dtype == torch.bfloat16 and self.boards.is_cuda and self.boards.shape[0] > 0:
             L, first = self.boards.shape[0], 2 * NUM_HANDS
             x = torch.zeros(L, ValueMLP.IN_PADDED, device=device, dtype=torch.bfloat16)
             card = torch.arange(52, device=device)
             x[:, first: first + 52] = (self.boards[:, :, None] == card).any(dim=1)
             x[:, first + 52: ValueMLP.IN_FEATURES] = self.context
             self._rows = x
+            self._rows_stream = _lib.stream_ptr(x.device)  # where the rows are at home
 
     def evaluate_into(self, leaf_beliefs: torch.Tensor, out: torch.Tensor) -> None:
         """Values of all leaves into out[..., :1326] (fp32 [L,2,W])."""
@@ -183,12 +187,22 @@ class DirectLeafEvaluator:
             out[..., :NUM_HANDS].copy_(self.model(leaf_beliefs[..., :NUM_HANDS].contiguous(), self.boards, self.context))
             return
         p, L = _lib.ptr, leaf_beliefs.shape[0]
-        with _lib.on(out.device), torch.no_grad():
-            stream = _lib.stream_ptr(out.device)
-            _lib.call("p2b_leaf_features_bf16", p(leaf_beliefs), leaf_beliefs.stride(1), L, p(self._rows),
-                      self._rows.stride(0), stream)
-            y = self.model.layers(self._rows)
+        # calls from several threads take the rows in turn, calls on another stream (or recorded for later) a copy of them
+        with _lib.on(out.device), torch.no_grad(), self._rows_lock:
+            stream, rows = _lib.stream_ptr(out.device), self._rows
+            if stream != self._rows_stream:
+                rows = rows.clone()
+                if not torch.cuda.is_current_stream_capturing():
+                    self._rows.record_stream(torch.cuda.current_stream(out.device))
+            _lib.call("p2b_leaf_features_bf16", p(leaf_beliefs), leaf_beliefs.stride(1), L, p(rows), rows.stride(0), stream)
+            y = self.model.layers(rows)
             _lib.call("p2b_leaf_values_bf16", p(y), y.stride(0), L, p(out), out.stride(1), stream)
+
+    def __getstate__(self):  # (a lock is neither copied nor pickled)
+        return {k: v for k, v in self.__dict__.items() if k != "_rows_lock"}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state, _rows_lock=threading.RLock())
 
     def _direct(self) -> bool:
         """The model's layers may be called on rows kept here instead of the model itself."""
@@ -204,6 +218,9 @@ class DirectLeafEvaluator:
 
 def _paired_rows(t: torch.Tensor, network_rows: torch.Tensor) -> bool:
     """[L,2,W] fp32, rows of whole pairs of hands one after the other, as many leaves as there are network rows."""
-    return (t.is_cuda and t.device == network_rows.device and t.dim() == 3 and t.shape[0] == network_rows.shape[0]
-            and t.shape[1] == 2 and t.shape[2] >= NUM_HANDS and t.dtype == torch.float32 and t.stride(2) == 1 and t.stride(0) == 2 * t.stride(1)
-            and t.stride(1) % 2 == 0 and t.data_ptr() % 8 == 0)
+    if t.dim() != 3 or t.dtype != torch.float32 or t.device != network_rows.device:
+        return False
+    leaves, players, width = t.shape
+    per_leaf, per_player, per_hand = t.stride()
+    return (leaves == network_rows.shape[0] and players == 2 and width >= NUM_HANDS and per_hand == 1
+            and per_leaf == 2 * per_player and per_player % 2 == 0 and t.data_ptr() % 8 == 0)

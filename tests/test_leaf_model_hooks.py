@@ -1,5 +1,6 @@
-"""Hooks on the leaf network and on its layers fire although its layers are normally called without their modules, and a layer
-whose output a hook has kept is not overwritten by the activation behind it."""
+"""What the short way through the leaf network must not lose: hooks on the network and on its layers fire, a layer whose output
+a hook has kept is not overwritten by the activation behind it, a derived evaluator's own call is made, and one evaluator
+serves several streams and threads."""
 import pytest
 import torch
 
@@ -108,3 +109,76 @@ def test_hooks_on_the_model_of_a_leaf_evaluator_fire(cuda_device, evaluate):
     handle.remove()
     assert len(seen) == 1 and torch.equal(got[..., :1326], want * 2.0)
     assert torch.equal(ev(beliefs), want)
+
+
+def _two_calls(cuda_device):
+    L = 6
+    g = torch.Generator(device=cuda_device).manual_seed(9)
+    boards = torch.tensor([[0, 1, 2, -1, -1]], device=cuda_device).expand(L, 5)
+    ev = leaf_eval.DirectLeafEvaluator(_model().to(cuda_device), boards, torch.rand(L, 3, device=cuda_device, generator=g), cuda_device)
+    beliefs = [torch.rand(L, 2, 1344, device=cuda_device, generator=g) for _ in range(2)]
+    want = [ev(b) for b in beliefs]
+    torch.cuda.synchronize()
+    assert not torch.equal(*want)
+    return ev, beliefs, want
+
+
+@pytest.mark.gpu
+def test_one_evaluator_on_two_streams(cuda_device, monkeypatch):
+    """A call on another stream while this one's is between its input and its layers."""
+    ev, beliefs, want = _two_calls(cuda_device)
+    other = torch.cuda.Stream(cuda_device)
+    with torch.cuda.stream(other):  # its memory and handles are there: nothing makes the second call wait for the first
+        for _ in range(2):
+            ev(beliefs[1])
+    torch.cuda.synchronize()
+    layers, slow = leaf_eval.ValueMLP.layers, [False, True]  # the first call's layers begin late
+
+    def delayed(self, x):
+        if slow.pop():
+            torch.cuda._sleep(1 << 27)
+        return layers(self, x)
+
+    monkeypatch.setattr(leaf_eval.ValueMLP, "layers", delayed)
+    first = ev(beliefs[0])
+    with torch.cuda.stream(other):
+        second = ev(beliefs[1])
+    torch.cuda.synchronize()
+    assert torch.equal(second, want[1]) and torch.equal(first, want[0])
+
+
+@pytest.mark.gpu
+def test_an_evaluator_can_be_copied(cuda_device):
+    import copy
+    import pickle
+
+    ev, beliefs, want = _two_calls(cuda_device)
+    for other in (copy.deepcopy(ev), pickle.loads(pickle.dumps(ev))):
+        assert torch.equal(other(beliefs[0]), want[0]) and torch.equal(other(beliefs[1]), want[1])
+
+
+@pytest.mark.gpu
+def test_one_evaluator_in_two_threads(cuda_device, monkeypatch):
+    """A second thread's call while the first is between the launches of its input and of its layers."""
+    import threading
+    import time
+
+    ev, beliefs, want = _two_calls(cuda_device)
+    layers, entered = leaf_eval.ValueMLP.layers, threading.Event()
+
+    def delayed(self, x):
+        if not entered.is_set():
+            entered.set()
+            time.sleep(0.2)
+        return layers(self, x)
+
+    monkeypatch.setattr(leaf_eval.ValueMLP, "layers", delayed)
+    got = [None, None]
+    threads = [threading.Thread(target=lambda i=i: got.__setitem__(i, ev(beliefs[i]))) for i in range(2)]
+    threads[0].start()
+    assert entered.wait(5.0)
+    threads[1].start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
